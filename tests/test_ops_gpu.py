@@ -152,6 +152,33 @@ def test_scan_against_oracle_ragged(B, T, Hh):
     assert rel_err(npf(sc), soc) < 2e-5
 
 
+@pytest.mark.parametrize("B,T,Hh", [(1, 9, 148), (1, 16, 149), (2, 7, 148), (3, 17, 99)])
+def test_scan_tile_choice_by_grid(B, T, Hh):
+    """148 / 149 / 296 / 297 CTAs are the edges between the register tiles; T around the block of 8 tokens.  Decays of
+    zero and above one are legal operands.  fp32 sums of 64 terms: 2e-6 of the largest value is about 30 ulp."""
+    r, w, k, v, kk, a = wkv_inputs(B, T, Hh, N, seed=T, dtype=np.float32)
+    w[:, 1, 0], w[:, 2, -1] = 0.0, 1.5
+    rng = np.random.default_rng(T)
+    s0 = (0.1 * rng.standard_normal((B, Hh, N, N))).astype(np.float32)
+    yo, so = O.recurrent_scan(r, w, k, v, kk, a, s0)
+    y, s = hb.fused_recurrent_scan(*(cu(x) for x in (r, w, k, v, kk, a, s0)))
+    assert rel_err(npf(s), so) < 2e-6
+    assert rel_err(npf(y), yo.astype(np.float32)) < 2e-6
+    f = lambda *sh: rng.standard_normal(sh).astype(np.float32)
+    g, rk, gw, gb = f(B, T, Hh, N), 0.1 * f(Hh, N), 1 + 0.1 * f(Hh * N), 0.1 * f(Hh * N)
+    yp, sp = hb.fused_recurrent_scan_output_prepare(*(cu(x) for x in (r, w, k, v, kk, a, s0, g, rk, gw, gb)), eps=EPS)
+    assert torch.equal(sp, s)
+    rows = lambda x: cu(x).reshape(B * T, Hh * N)
+    want = hb.fused_attn_output_prepare(y.reshape(B * T, Hh * N), *(rows(x) for x in (r, k, v, g)), *(cu(x) for x in (rk, gw, gb)),
+                                        num_heads=Hh, head_dim=N, head_v_dim=N, eps=EPS)
+    assert rel_err(npf(yp).reshape(-1), npf(want).reshape(-1)) < 5e-6
+    # a state in fp16: the same recurrence on the rounded state, rounded back once
+    s16 = s0.astype(np.float16)
+    yh, sh = hb.fused_recurrent_scan(*(cu(x.astype(np.float16)) for x in (r, w, k, v, kk, a, s16)))
+    _, soh = O.recurrent_scan(*(x.astype(np.float16) for x in (r, w, k, v, kk, a)), s16.astype(np.float32))
+    assert sh.dtype == torch.float16 and rel_err(npf(sh), soh) < 1e-3
+
+
 def test_scan_empty_sequence_passes_state_through():
     s0 = torch.randn(2, 2, N, N, device="cuda")
     e = torch.empty(2, 0, 2, N, device="cuda", dtype=torch.float16)
