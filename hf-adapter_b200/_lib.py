@@ -15,7 +15,7 @@ LIB_PATH = os.environ.get("RWKV7_B200_LIB") or os.path.join(_HERE, "librwkv7_b20
 
 OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_ALIGN, ERR_CUDA, ERR_WORKSPACE = 0, -1, -2, -3, -4, -5
 F16, BF16, F32 = 0, 1, 2
-EPI_NONE, EPI_RELU2, EPI_ADD = 0, 1, 2
+EPI_NONE, EPI_RELU2, EPI_ADD, EPI_TANH, EPI_SIGMOID = 0, 1, 2, 3, 4
 
 P, I, F, L = c_void_p, c_int, c_float, c_int64
 PP = ctypes.POINTER(c_void_p)
@@ -47,6 +47,7 @@ SIGNATURES = {
     "rwkv7_seq_shift_mix": (I, [P, P, PP, PP, P, I, I, I, I, I, I, P]),
     "rwkv7_dense_small": (I, [P] * 4 + [I, I, I, I, I, I, P]),
     "rwkv7_small_gemm_group": (I, [I, PP, PP, PP, PP, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int), I, I, P]),
+    "rwkv7_rows_gemv": (I, [I, PP, PP, PP, PP, PP] + [ctypes.POINTER(c_int)] * 4 + [I, I, I, P]),
     "rwkv7_prefill_state_prep": (I, [P] * 12 + [I, I, I, I, I, I, I, P]),
     "rwkv7_attn_output_prepare": (I, [P] * 9 + [I, I, I, F, I, P]),
     "rwkv7_w4g_gemv": (I, [P] * 6 + [I, I, I, I, I, I, P]),

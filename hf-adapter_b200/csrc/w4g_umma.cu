@@ -564,7 +564,7 @@ static void mark_tiled_fresh(const void* tiled) {
     std::lock_guard<std::mutex> lk(g_fresh_mu);
     g_fresh_tiled.insert(tiled);
 }
-static bool take_tiled_fresh(const void* tiled) {
+bool take_tiled_fresh(const void* tiled) {
     std::lock_guard<std::mutex> lk(g_fresh_mu);
     return g_fresh_tiled.erase(tiled) != 0;
 }

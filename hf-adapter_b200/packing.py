@@ -20,13 +20,16 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _lib
 from . import gemm as _gemm
 from . import lora as _lora
 from . import norm_mix as _nm
 from . import quant as _q
 from . import recurrent as _rec
+from . import rows as _rowsk
 
 PACK_SLOTS = 41
+_ROWS_MAX_OUT = 32768  # dense out_features up to which the row kernel runs (a vocabulary head keeps its library GEMM)
 _QUANT_TYPES = (_q.MM4Linear, _q.MM8Linear, _q.A8W8Linear)
 
 
@@ -110,10 +113,11 @@ def init_batched_from_packs(packs, batch_size: int, device, dtype, *, state_dtyp
 
 
 # ---------------------------------------------------------------------------------------------- operands
-def apply_linear(op, x, *, relu2=False, residual=None, out=None):
+def apply_linear(op, x, *, relu2=False, residual=None, out=None, static=False):
     """Apply a projection operand of the pack: a quantised module (epilogues fused through its rwkv7_forward_* hooks,
     as the reference's dispatch probes them: rwkv7_hf/native_jit_graph_dispatch.py:487-523), a dense ``[out,in]``
-    weight tensor, or an ``nn.Linear`` (this library's GEMM from 64 rows up in fp16 / bf16, else one library GEMM)."""
+    weight tensor, or an ``nn.Linear`` (fp16 / bf16: this library's GEMM from 64 rows up, its row kernel up to 8; else
+    one library GEMM).  ``static``: the kernel launched just before on this stream does not write a dense weight."""
     if isinstance(op, _QUANT_TYPES):
         if relu2:
             if hasattr(op, "rwkv7_forward_relu2"):
@@ -129,6 +133,14 @@ def apply_linear(op, x, *, relu2=False, residual=None, out=None):
     if rows >= _gemm.MIN_ROWS and _gemm.takes(x, weight) and (bias is None or bias.dtype == x.dtype):
         # many rows over a dense fp16 / bf16 weight: this library's tensor-core GEMM, epilogue fused
         return _gemm.dense_linear(x, weight, bias, relu2=relu2, residual=residual, out=out)
+    N = int(weight.shape[0])
+    whole = lambda t: t is None or (t.dtype == x.dtype and t.is_contiguous() and t.numel() == rows * N)
+    if bias is None and _rowsk.takes_dense(x, weight) and N <= _ROWS_MAX_OUT and whole(residual) and whole(out):
+        epi = _lib.EPI_RELU2 if relu2 else _lib.EPI_ADD if residual is not None else _lib.EPI_NONE
+        y, = _rowsk.rows_gemv((x.reshape(rows, -1),), (weight,), out_features=(N,), fmts=(_rowsk.DENSE,), epilogues=(epi,),
+                              residuals=(None if relu2 else residual,), outs=None if out is None else (out.reshape(rows, N),),
+                              static_weights=static)
+        return y.reshape(*x.shape[:-1], N) if out is None else out
     y = F.linear(x, weight, bias)
     if relu2:
         y = torch.relu(y) ** 2
@@ -160,6 +172,32 @@ def rkv_grouped(ops, xr, xk, xv):
         return _q.w8_tiled_linear_group((xr, xk, xv), tiled, [m.row_scale for m in ops], ops[0].out_features,
                                         ops[0].in_features)
     return _q.w4_tiled_linear_group((xr, xk, xv), tiled, ops[0].out_features, ops[0].in_features)
+
+
+def _rows_operand(op, x):
+    """``(fmt, weight, scale, out_features)`` when the projection ``op`` of the few rows ``x`` runs on the row kernel."""
+    if isinstance(op, _q.MM4Linear) or (isinstance(op, _q.MM8Linear) and op.sm7x_rowwise):
+        tiled = op.tiled_for(x) if op.bias is None and x.is_contiguous() and _q.few_rows_quant(int(x.shape[0]), op.in_features) else None
+        if tiled is None:
+            return None
+        return (_rowsk.INT4, tiled, None, op.out_features) if isinstance(op, _q.MM4Linear) else \
+            (_rowsk.INT8, tiled, op.row_scale, op.out_features)
+    weight = op if isinstance(op, torch.Tensor) else op.weight if isinstance(op, nn.Linear) and op.bias is None else None
+    if weight is None or not _rowsk.takes_dense(x, weight):
+        return None
+    return _rowsk.DENSE, weight, None, int(weight.shape[0])
+
+
+def rows_projections(ops, xs, epilogues=None):
+    """The projections ``ops[i](xs[i])`` of a few rows in one launch, or None when one of them does not take that route.
+    For the inside of a layer step: the kernel before it writes activations only."""
+    if not 1 <= int(xs[0].shape[0]) <= _rowsk.MAX_ROWS or xs[0].dtype not in (torch.float16, torch.bfloat16):
+        return None
+    got = [_rows_operand(o, x) for o, x in zip(ops, xs)]
+    if any(g is None for g in got):
+        return None
+    return _rowsk.rows_gemv(xs, [g[1] for g in got], out_features=[g[3] for g in got], fmts=[g[0] for g in got],
+                            scales=[g[2] for g in got], epilogues=epilogues, static_weights=True)
 
 
 class StepContext:
@@ -203,6 +241,42 @@ class StepContext:
 _DEFAULT_CONTEXT = StepContext()
 
 
+def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
+    """r / k / v and the LoRA pre-activations of a layer step on parallel branches: ``[r, k, v, w, a, g(, v_gate)]``."""
+    xr, xk, xv = xs
+    # The LoRA chain does not depend on r/k/v: it runs on a side stream (a parallel branch of the decode graph once
+    # captured) and joins before the recurrence.
+    main = torch.cuda.current_stream(x.device)
+    side = ctx.side_stream(x.device, 0)
+    side.wait_stream(main)
+    with torch.cuda.stream(side):
+        hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)])
+        lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups])
+    rkv = rkv_grouped(ops, xr, xk, xv) if all(isinstance(o, _QUANT_TYPES) for o in ops) else None
+    if rkv is not None:
+        # int4 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
+        # exchange) instead of three launches competing for the SMs
+        r, k, v = rkv
+        main.wait_stream(side)
+    else:
+        # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
+        sk, sv = ctx.side_stream(x.device, 1), ctx.side_stream(x.device, 2)
+        sk.wait_stream(main)
+        sv.wait_stream(main)
+        with torch.cuda.stream(sk):
+            k = apply_linear(ops[1], xk)
+        with torch.cuda.stream(sv):
+            v = apply_linear(ops[2], xv)
+        r = apply_linear(ops[0], xr)
+        main.wait_stream(side)
+        main.wait_stream(sk)
+        main.wait_stream(sv)
+        xk.record_stream(sk); k.record_stream(sk); xv.record_stream(sv); v.record_stream(sv)
+    for t_ in (*down_x, *lora):
+        t_.record_stream(side)
+    return [r, k, v, *lora]
+
+
 def block_ip_batched(x, state, xpa, xpf, v_first, p, sparse_ffn_out=None, fp16_elapsed=None,
                      fp16_advance_elapsed=False, route_observer=None, *, context: StepContext | None = None):
     """One layer for ``B`` sequences from its pack tuple, recurrent buffers updated in place
@@ -237,65 +311,39 @@ def block_ip_batched(x, state, xpa, xpf, v_first, p, sparse_ffn_out=None, fp16_e
     else:
         xr, xw, xk, xv, xa, xg = _nm.fused_attn_norm_mix6_decode(x, xpa, an_w, an_b, x_r, x_w, x_k, x_v, x_a, x_g,
                                                                  slot_ids=slots)
-    # The LoRA chain does not depend on r/k/v: it runs on a side stream (a parallel branch of the decode graph once
-    # captured) and joins before the recurrence.
-    main = torch.cuda.current_stream(x.device)
-    side = ctx.side_stream(x.device, 0)
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        if int(i) == 0:
-            hs = _lora.small_gemm_group((xw, xa, xg), (_weight_of(w1), _weight_of(a1), _weight_of(g1)), acts=(1, 0, 2))
-            w_raw, a_pre, g = _lora.small_gemm_group(hs, (_weight_of(w2), _weight_of(a2), _weight_of(g2)))
-            extra = dict(v_out=v_first)
-        else:
-            hs = _lora.small_gemm_group((xw, xa, xg, xv), (_weight_of(w1), _weight_of(a1), _weight_of(g1), _weight_of(v1)),
-                                        acts=(1, 0, 2, 0))
-            w_raw, a_pre, g, vg_pre = _lora.small_gemm_group(
-                hs, (_weight_of(w2), _weight_of(a2), _weight_of(g2), _weight_of(v2)))
-            extra = dict(v_first=v_first, v_gate=vg_pre, v_gate_bias=v0, v_gate_is_raw=True)
-    ops = (Rw, Kw, Vw)
-    rkv = rkv_grouped(ops, xr, xk, xv) if all(isinstance(o, _QUANT_TYPES) for o in ops) else None
-    if rkv is not None:
-        # int4 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
-        # exchange) instead of three launches competing for the SMs
-        r, k, v = rkv
-        main.wait_stream(side)
+    first = int(i) == 0
+    downs, ups = ((w1, a1, g1), (w2, a2, g2)) if first else ((w1, a1, g1, v1), (w2, a2, g2, v2))
+    down_x = (xw, xa, xg) if first else (xw, xa, xg, xv)
+    # a few rows: r / k / v and the LoRA "down" products in one launch, the "up" products in the next
+    few = rows_projections((Rw, Kw, Vw) + downs, (xr, xk, xv) + down_x,
+                           ([_lib.EPI_NONE] * 3 + [_lib.EPI_TANH, _lib.EPI_NONE, _lib.EPI_SIGMOID, _lib.EPI_NONE])[:3 + len(downs)])
+    lora = None if few is None else rows_projections(ups, few[3:])
+    if lora is not None:
+        r, k, v = few[:3]
     else:
-        # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
-        sk, sv = ctx.side_stream(x.device, 1), ctx.side_stream(x.device, 2)
-        sk.wait_stream(main)
-        sv.wait_stream(main)
-        with torch.cuda.stream(sk):
-            k = apply_linear(Kw, xk)
-        with torch.cuda.stream(sv):
-            v = apply_linear(Vw, xv)
-        r = apply_linear(Rw, xr)
-        main.wait_stream(side)
-        main.wait_stream(sk)
-        main.wait_stream(sv)
-        xk.record_stream(sk); k.record_stream(sk); xv.record_stream(sv); v.record_stream(sv)
-    for t_ in (xw, xa, xg, xv, w_raw, a_pre, g):
-        t_.record_stream(side)
+        r, k, v, *lora = _wide_projections(ctx, x, (Rw, Kw, Vw), (xr, xk, xv), downs, ups, down_x)
+    w_raw, a_pre, g = lora[:3]
+    extra = dict(v_out=v_first) if first else dict(v_first=v_first, v_gate=lora[3], v_gate_bias=v0, v_gate_is_raw=True)
     elapsed = fp16_elapsed if state.dtype == torch.float16 else None
     # the kernel launched just before the recurrence is a projection: it never writes the state
     out, _ = _rec.fused_recurrent_output_prepare_raw(
         r, w_raw, k, v, a_pre, state, g, k_k, k_a, r_k, gn_w, gn_b, eps=float(eps), new_state=state, w_bias=w0, a_bias=a0,
         a_is_raw=True, state_prefetch=True, elapsed=elapsed,
         advance_elapsed=bool(fp16_advance_elapsed) and elapsed is not None, slot_ids=slots, **extra)
-    attn = apply_linear(Ow, out)
+    attn = apply_linear(Ow, out, static=True)
     if rows_comm is not None:
         x, mixed = rows_comm.ffn_add_norm_mix(x, attn, xpf, fn_w, fn_b, fx_k, slot_ids=slots)
     else:
         x, mixed = _nm.fused_ffn_add_norm_mix_decode(x, ctx.all_reduce(attn), xpf, fn_w, fn_b, fx_k, slot_ids=slots)
-    hidden = apply_linear(fK, mixed, relu2=True)
+    hidden = apply_linear(fK, mixed, relu2=True, static=True)
     if ctx.tp_world > 1:
         # the residual rides in rank 0's partial sum (the projection's add epilogue): no extra add kernel
-        part = apply_linear(fV, hidden, residual=x if ctx.tp_rank == 0 else None)
+        part = apply_linear(fV, hidden, residual=x if ctx.tp_rank == 0 else None, static=True)
         if rows_comm is not None and ctx.defer_sum:
             ctx.pending = True
             return part
         return ctx.all_reduce(part)
-    return apply_linear(fV, hidden, residual=x)
+    return apply_linear(fV, hidden, residual=x, static=True)
 
 
 def step_batched(model, x, state, xpa, xpf, v_first, packs, *, fp16_elapsed=None, context: StepContext | None = None):

@@ -20,6 +20,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from . import rows as _rowsk
 from ._util import dt_code, ptr, require_cuda, stream_ptr
 
 GEMV_MAX_ROWS = 64  # rows up to which the weight-streaming kernels are used; above: dequantise + GEMM
@@ -107,6 +108,14 @@ def w4_repack_tiled(q, scales, in_features, group_size=128, zeros=None):
     return tiled
 
 
+def few_rows_quant(rows: int, in_features: int) -> bool:
+    """Whether a tiled int4 / int8 projection of ``rows`` activation rows runs on the row kernel (csrc/row_gemv.cu) and not on
+    the tcgen05 one.  1 row, tcgen05 against rows: 4096 x 4096 int4 7.6 -> 5.6 us, int8 8.5 -> 6.7; 4096 -> 16384 17.2 -> 15.0 and
+    18.8 -> 17.1; 16384 -> 4096 15.2 -> 14.2 and 17.2 -> 16.0.  At 8 rows the activations weigh as much as the weights of a
+    long row: 16384 -> 4096 int4 14.7 against 16.7."""
+    return 1 <= rows <= _rowsk.MAX_ROWS and (rows <= 4 or in_features <= 10240)
+
+
 def w4_tiled_linear(x, tiled, out_features, in_features, *, out=None, relu2: bool = False, residual=None):
     """y = x @ W^T on the tensor-core kernel from the tiled weight copy (fp16; one weight pass per 64 rows)."""
     K, Nout = int(in_features), int(out_features)
@@ -115,6 +124,10 @@ def w4_tiled_linear(x, tiled, out_features, in_features, *, out=None, relu2: boo
     require_cuda(x2, tiled, what="w4_tiled_linear")
     epi, res = _epi(relu2, residual, M, Nout, x2)
     y = torch.empty((M, Nout), device=x2.device, dtype=x2.dtype) if out is None else out.reshape(M, Nout)
+    if few_rows_quant(M, K) and x2.dtype == torch.float16:
+        _rowsk.rows_gemv((x2,), (tiled,), out_features=(Nout,), fmts=(_rowsk.INT4,), residuals=(res,), outs=(y,), epilogues=(epi,),
+                         static_weights=True)
+        return y.reshape(*x.shape[:-1], Nout)
     _lib.check(_lib.lib.rwkv7_w4g_gemv_tiled(ptr(x2), ptr(tiled), ptr(res), ptr(y), M, K, Nout, epi, dt_code(x2),
                                              stream_ptr(x2)), "w4_tiled_linear")
     return y.reshape(*x.shape[:-1], Nout)
@@ -133,6 +146,10 @@ def w4_tiled_linear_group(xs, tileds, out_features, in_features, *, relu2: bool 
         raise ValueError("grouped projections need the same row count and dtype")
     require_cuda(*x2, *tileds, what="w4_tiled_linear_group")
     ys = [torch.empty((M, Nout), device=x2[0].device, dtype=x2[0].dtype) for _ in range(G)]
+    if few_rows_quant(M, K) and x2[0].dtype == torch.float16:
+        _rowsk.rows_gemv(x2, tileds, out_features=[Nout] * G, fmts=[_rowsk.INT4] * G, outs=ys,
+                         epilogues=[_lib.EPI_RELU2 if relu2 else _lib.EPI_NONE] * G, static_weights=True)
+        return [y.reshape(*x.shape[:-1], Nout) for y, x in zip(ys, xs)]
     arr = lambda ts: (ctypes.c_void_p * G)(*[t.data_ptr() for t in ts])
     _lib.check(_lib.lib.rwkv7_w4g_gemv_tiled_group(arr(x2), arr(tileds), arr(ys), G, M, K, Nout, _lib.EPI_RELU2 if relu2 else
                                                    _lib.EPI_NONE, dt_code(x2[0]), stream_ptr(x2[0])), "w4_tiled_linear_group")
@@ -171,6 +188,10 @@ def w8_tiled_linear_group(xs, tileds, scales, out_features, in_features, *, relu
     if (res is not None or out is not None) and G != 1:
         raise ValueError("residual / out apply to a single projection")
     ys = [torch.empty((M, Nout), device=x2[0].device, dtype=x2[0].dtype) if out is None else out.reshape(M, Nout) for _ in range(G)]
+    if few_rows_quant(M, K) and x2[0].dtype == torch.float16 and all(t.is_contiguous() for t in x2):
+        _rowsk.rows_gemv(x2, tileds, out_features=[Nout] * G, fmts=[_rowsk.INT8] * G, scales=sc, residuals=[res] * G, outs=ys,
+                         epilogues=[epi] * G, static_weights=True)
+        return [y.reshape(*x.shape[:-1], Nout) for y, x in zip(ys, xs)]
     arr = lambda ts: (ctypes.c_void_p * G)(*[t.data_ptr() for t in ts])
     _lib.check(_lib.lib.rwkv7_w8_gemv_tiled_group(arr(x2), arr(tileds), arr(sc), ptr(res), arr(ys), G, M, K, Nout, epi,
                                                    dt_code(x2[0]), stream_ptr(x2[0])), "w8_tiled_linear_group")

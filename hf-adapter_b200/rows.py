@@ -1,0 +1,47 @@
+"""Projections over a few rows (csrc/row_gemv.cu): up to eight independent ones, dense or quantised, in one launch with
+their activation / residual epilogues.  What a decode step of a few sequences runs instead of one library GEMM per
+projection and pointwise kernels behind it (rwkv7_hf/native_jit_graph_dispatch.py:487-523 probes for such fused forms)."""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+
+from . import _lib
+from ._util import dt_code, ptr, require_cuda, stream_ptr
+
+DENSE, INT4, INT8 = 0, 1, 2
+MAX_ROWS = 8
+MAX_PROBLEMS = 8
+
+
+def takes_dense(x, weight) -> bool:
+    """``x @ weight.T`` with a dense weight: fp16 / bf16 CUDA operands of one dtype, contiguous and 16-byte aligned, few
+    rows (anything else keeps its library GEMM)."""
+    return (x.is_cuda and weight.is_cuda and x.dtype == weight.dtype and x.dtype in (torch.float16, torch.bfloat16)
+            and weight.dim() == 2 and weight.is_contiguous() and x.is_contiguous() and int(x.shape[-1]) == int(weight.shape[1])
+            and weight.numel() > 0 and int(weight.shape[1]) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and 1 <= x.numel() // int(weight.shape[1]) <= MAX_ROWS)
+
+
+def rows_gemv(xs, weights, *, out_features, fmts, scales=None, residuals=None, outs=None, epilogues=None, static_weights=False):
+    """``outs[i] = epilogue_i(xs[i] [M,K_i] @ W_i.T)`` in one launch.  ``weights[i]`` is dense ``[N,K]`` or a tiled copy
+    (``quant.w4_repack_tiled`` / ``w8_repack_tiled``).  ``static_weights``: no weight is written by the kernel launched
+    just before this call on the stream."""
+    n = len(xs)
+    M = int(xs[0].shape[0])
+    scales = list(scales) if scales is not None else [None] * n
+    residuals = list(residuals) if residuals is not None else [None] * n
+    epilogues = list(epilogues) if epilogues is not None else [_lib.EPI_NONE] * n
+    require_cuda(*xs, *weights, *scales, *residuals, what="rows_gemv")
+    if any(int(x.shape[0]) != M or x.dtype != xs[0].dtype or not x.is_contiguous() for x in xs):
+        raise ValueError("rows_gemv: all inputs need the same row count and dtype, contiguous")
+    if outs is None:
+        outs = [torch.empty((M, N), device=xs[0].device, dtype=xs[0].dtype) for N in out_features]
+    arr = lambda ts: _lib.ptr_array([ptr(t) for t in ts])
+    (xp, k0), (wp, k1), (sp, k2), (rp, k3), (op, k4) = (arr(t) for t in (xs, weights, scales, residuals, outs))
+    IA = ctypes.c_int * n
+    _lib.check(_lib.lib.rwkv7_rows_gemv(n, xp, wp, sp, rp, op, IA(*[int(x.shape[1]) for x in xs]), IA(*out_features), IA(*fmts),
+                                        IA(*epilogues), M, dt_code(xs[0]), int(bool(static_weights)), stream_ptr(xs[0])),
+               "rows_gemv")
+    return outs

@@ -49,6 +49,8 @@ extern "C" {
 #define RWKV7_EPI_NONE 0
 #define RWKV7_EPI_RELU2 1 /* out = relu(y)^2, y rounded to the activation dtype first */
 #define RWKV7_EPI_ADD 2   /* out = y + residual */
+#define RWKV7_EPI_TANH 3    /* rows_gemv only: out = tanh(y) */
+#define RWKV7_EPI_SIGMOID 4 /* rows_gemv only: out = sigmoid(y) */
 
 int rwkv7_abi_version(void);
 const char* rwkv7_last_error(void);
@@ -216,6 +218,16 @@ int rwkv7_seq_shift_mix(const void* x, const void* initial_prev, const void* con
  * act codes: 0 none, 1 tanh, 2 sigmoid.  Intended for the rank-R projections (K or Nout <= 256). */
 int rwkv7_dense_small(const void* x, const void* W, const void* bias, void* out,
                       int rows, int K, int Nout, int act_in, int act_out, int dtype, void* stream);
+
+/* Up to eight independent projections over 1..8 rows in ONE launch (a decode step of a few sequences):
+ *   out_p[M,N_p] = epilogue_p( x_p[M,K_p] . W_p[N_p,K_p]^T ), the product rounded to the activation dtype first.
+ * fmt: 0 dense [N,K] in the activation dtype (K % 8 == 0), 1 int4 in the tiled copy of rwkv7_w4g_repack, 2 int8 in the tiled
+ * copy of rwkv7_w8_repack with per-channel `scale` (1 and 2: fp16, K % 128 == 0).  epilogue: RWKV7_EPI_*.  scale / residual
+ * may be NULL or hold NULL entries.  static_weights != 0: the caller promises that the kernel launched just before this one
+ * in the stream does not write any W, which is then requested under that kernel's tail. */
+int rwkv7_rows_gemv(int n_problems, const void* const* x, const void* const* W, const void* const* scale,
+                    const void* const* residual, void* const* out, const int* K, const int* N, const int* fmt,
+                    const int* epilogue, int M, int dtype, int static_weights, void* stream);
 
 /* The same for up to four independent problems in ONE launch (the four rank-R "down" projections, or the four "up"
  * projections, of a layer: the reference's _wavg_lora_down_kernel / _wavg_lora_up_kernel pair,

@@ -1,0 +1,70 @@
+"""The few-row projection kernel against fp32 products of the same operands: edges of its channel tiles (16 / 32), of its K
+units (64 dense, 128 quantised), of the warps and cluster ranks that split K, and of the 8 activation rows."""
+import pytest
+import torch
+
+import hf_adapter_b200 as hb
+from hf_adapter_b200 import _lib, rows
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(got, want, dt, p=None):
+    # one rounding of the product p to the storage type and one of the result, each half an ulp; the last term is the fp32
+    # sum's own error and the type's smallest steps
+    ulp = 2.0 ** -10 if dt == torch.float16 else 2.0 ** -7
+    lim = 0.5 * ulp * (want.abs() + (want if p is None else p).abs()) * 1.01 + 1e-5
+    assert bool(((got.float() - want).abs() <= lim).all()), float(((got.float() - want).abs() / lim).max())
+
+
+@pytest.mark.parametrize("M", [1, 3, 8])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shapes", [[(8, 1), (32, 17), (72, 64), (520, 33), (1024, 130), (64, 2560), (128, 300)],
+                                    [(10240, 48)], [(3080, 768), (768, 64)], [(768, 5000)]])
+def test_dense_group_with_epilogues(M, dt, shapes):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    epis = [0, 1, 2, 3, 4, 2, 0][:len(shapes)]
+    xs = [torch.randn(M, K, generator=g, device="cuda").to(dt) for K, _ in shapes]
+    ws = [(torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(dt) for K, N in shapes]
+    res = [torch.randn(M, N, generator=g, device="cuda").to(dt) if e == 2 else None for (_, N), e in zip(shapes, epis)]
+    for static in (False, True):
+        outs = rows.rows_gemv(xs, ws, out_features=[N for _, N in shapes], fmts=[0] * len(xs), residuals=res, epilogues=epis,
+                              static_weights=static)
+        for x, w, r, e, y in zip(xs, ws, res, epis, outs):
+            p = x.double() @ w.double().t()
+            if e == 1:  # the product is rounded before it is squared, which doubles the relative size of that rounding
+                ulp = 2.0 ** -10 if dt == torch.float16 else 2.0 ** -7
+                torch.testing.assert_close(y.double(), torch.relu(p) ** 2, rtol=1.6 * ulp, atol=1e-5)
+                continue
+            want = p if e == 0 else p + r.double() if e == 2 else torch.tanh(p) if e == 3 else torch.sigmoid(p)
+            _close(y, want.float(), dt, p.float())
+
+
+@pytest.mark.parametrize("M", [1, 3, 8])
+@pytest.mark.parametrize("K,N", [(128, 128), (256, 48), (1152, 200), (2560, 2560), (8192, 272)])
+def test_quantised_formats(M, K, N):
+    g = torch.Generator(device="cuda").manual_seed(K + M)
+    x = torch.randn(M, K, generator=g, device="cuda").half()
+    lin = torch.nn.Linear(K, N, bias=False, device="cuda", dtype=torch.float16)
+    with torch.no_grad():
+        lin.weight.normal_(0.0, K ** -0.5, generator=g)
+    m4, m8 = hb.MM4Linear(lin), hb.MM8Linear(lin, rowwise=True)
+    res = torch.randn(M, N, generator=g, device="cuda").half()
+    p4 = (x.double() @ hb.w4_dequant(m4.packed_group, m4.group_scales, K).double().t()).float()
+    p8 = (x.double() @ (m8.q_row.double() * m8.row_scale.double()[:, None]).t()).float()
+    y4, y8 = rows.rows_gemv((x, x), (m4.tiled_for(x), m8.tiled_for(x)), out_features=(N, N), fmts=(1, 2), scales=(None, m8.row_scale),
+                            residuals=(res, None), epilogues=(_lib.EPI_ADD, _lib.EPI_NONE))
+    _close(y4, p4 + res.float(), torch.float16, p4)
+    _close(y8, p8, torch.float16)
+    # the modules give the same whichever kernel their row count and K select
+    _close(m4.rwkv7_forward_add(x, res), p4 + res.float(), torch.float16, p4)
+    _close(m8(x), p8, torch.float16)
+
+
+def test_refusals():
+    x, w = torch.zeros(9, 64, device="cuda").half(), torch.zeros(8, 64, device="cuda").half()
+    with pytest.raises(ValueError):
+        rows.rows_gemv((x,), (w,), out_features=(8,), fmts=(0,))
+    with pytest.raises(ValueError):
+        rows.rows_gemv((x[:1, :60].contiguous(),), (w,), out_features=(8,), fmts=(0,))
+    assert not rows.takes_dense(x[:1].reshape(-1)[1:57].reshape(1, 56), torch.zeros(8, 56, device="cuda").half())  # misaligned
