@@ -354,7 +354,7 @@ class RWKV7ForCausalLM(nn.Module):
         elapsed = elapsed_t if state[0].dtype == torch.float16 else None
         ctx = _pk.StepContext(self._side_stream, self._all_reduce, self.tp_world, self.tp_rank, lane, stream_base,
                               row_sum=self._row_sum)
-        packs, _, _, _ = _pk.extract_graph_packs(self)
+        packs, _, _, _ = _pk.extract_graph_packs(self, unused_as_zeros=False)
         x, *_ = _pk.step_batched(self, x, state, xpa, xpf, v_first, packs, fp16_elapsed=elapsed, context=ctx)
         xn = _nm.layer_norm(x, self.model.norm.weight, self.model.norm.bias)
         return self._head(xn, greedy, lane)

@@ -47,9 +47,11 @@ def graph_linear_is_dense(op) -> bool:
     return isinstance(op, torch.Tensor)
 
 
-def extract_graph_packs(model, *, rkv_policy: str = ""):
+def extract_graph_packs(model, *, rkv_policy: str = "", unused_as_zeros: bool = True):
     """``(packs, H, N, eps)`` for ``model`` (rwkv7_hf/native_jit_packing.py:61-146).  ``rkv_policy="vkwr_auto"`` stacks
-    dense r/k/v weights into slot 40; any other value leaves that slot empty."""
+    dense r/k/v weights into slot 40; any other value leaves that slot empty.  ``unused_as_zeros=False`` leaves None in
+    the slots a layer does not use (its pre-norm, layer 0's v LoRA) instead of the reference's zeros: a decode step builds
+    its packs inside the captured region, where each of those 65 tensors was a fill to replay."""
     layers = model.model.layers
     H = int(layers[0].attn.num_heads)
     N = int(layers[0].attn.head_dim)
@@ -63,12 +65,16 @@ def extract_graph_packs(model, *, rkv_policy: str = ""):
         vl = getattr(a, "v_lora", None)
         if vl is not None:
             v1, v2, v0 = graph_linear_operand(vl.lora[0]), vl.lora[2].weight, vl.lora[2].bias
+        elif not unused_as_zeros:
+            v1 = v2 = v0 = None
         else:
             v1 = torch.zeros(1, hidden, device=emb.device, dtype=emb.dtype)
             v2 = torch.zeros(A, 1, device=emb.device, dtype=emb.dtype)
             v0 = torch.zeros(A, device=emb.device, dtype=emb.dtype)
         if hasattr(layer, "pre_norm"):
             pre_w, pre_b, has_pre = layer.pre_norm.weight, layer.pre_norm.bias, 1
+        elif not unused_as_zeros:
+            pre_w, pre_b, has_pre = None, None, 0
         else:
             pre_w = torch.zeros(hidden, device=emb.device, dtype=emb.dtype)
             pre_b = torch.zeros(hidden, device=emb.device, dtype=emb.dtype)

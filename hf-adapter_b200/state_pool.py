@@ -315,7 +315,7 @@ class RWKV7StatePool:
         m = self.model
         x = torch.nn.functional.embedding(ids, m.model.embeddings.weight)
         ctx = _pk.StepContext(m._side_stream, None, 1, 0, 0, 0, slot_ids=slot_vec)
-        packs, _, _, _ = _pk.extract_graph_packs(m)
+        packs, _, _, _ = _pk.extract_graph_packs(m, unused_as_zeros=False)
         for l, p in enumerate(packs):
             x = _pk.block_ip_batched(x, self.S_pool[l], self.xpa_pool[l], self.xpf_pool[l], self.vfirst_pool, p, context=ctx)
         xn = _nm.layer_norm(x, m.model.norm.weight, m.model.norm.bias)
