@@ -50,6 +50,22 @@ __device__ __forceinline__ float rotator1(int x) {
     return 4.547473508864641e-13f * static_cast<float>(static_cast<int32_t>(bits));
 }
 
+// Four elements in storage type: requested together, converted where they are used, so that the operands of a step cost one
+// trip to memory and not one per branch (zeros when `ok` is false).
+template <typename T> struct alignas(sizeof(T) * 4) Raw4 { T v[4]; };
+template <typename T>
+__device__ __forceinline__ Raw4<T> ld_raw4(const void* base, size_t off, bool ok = true) {
+    Raw4<T> r{};
+    if (ok) r = *reinterpret_cast<const Raw4<T>*>(reinterpret_cast<const T*>(base) + off);
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ void cvt4(const Raw4<T>& r, float (&o)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = to_f<T>(r.v[i]);
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 template <typename TS> struct StateIO;
 template <> struct StateIO<float> {
     static __device__ __forceinline__ float4 load(const void* base, size_t off) {
@@ -104,6 +120,17 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
 #pragma unroll
     for (int it = 0; it < 8; ++it) S[it] = StateIO<TS>::load(p.state_in, sbase + (size_t)(it * 8 + rg) * kN + c0);
 
+    if constexpr (MODE == kRaw) {
+        // the parameters of the head are read after the wait like everything else, but are on their way to L2 by then
+        if (tid < 8) {
+            const void* par[8] = {p.k_k, p.k_a, p.r_k, p.gn_w, p.gn_b, p.w_bias, p.a_bias, p.v_gate_bias};
+            const void* q = par[0];
+#pragma unroll
+            for (int i = 1; i < 8; ++i)
+                if (tid == i) q = par[i];
+            if (q != nullptr) prefetch_l2(reinterpret_cast<const T*>(q) + hbase);
+        }
+    }
     // With the state-prefetch option the loads above are already in flight while the preceding kernel (the r/k/v
     // projection of a decode step) finishes: the caller promises that kernel does not write the state, and every
     // kernel of this library releases its successor only after its own wait, so whatever wrote the state earlier has
@@ -111,25 +138,40 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
     if (p.prefetch_state) grid_dependency_wait();
     if (tid == 0) grid_launch_dependents();  // the output projection sets up and streams weights under this grid's tail
 
-    // ---- column-indexed vectors (4 columns per thread)
+    // ---- all operands of the recurrence, requested before the first is used: four columns per thread, and the value row
+    const bool interp = MODE == kRaw && p.v_first != nullptr && p.v_gate != nullptr;
+    const Raw4<T> q_r = ld_raw4<T>(p.r, vbase + c0), q_a = ld_raw4<T>(p.a, vbase + c0), q_k = ld_raw4<T>(p.k, vbase + c0);
+    const T* vrow = reinterpret_cast<const T*>(p.v) + vbase;
+    T q_v{}, q_gate{}, q_vf{}, q_gb{};
+    if (tid < kN) {
+        q_v = vrow[tid];
+        if (interp) {
+            q_gate = reinterpret_cast<const T*>(p.v_gate)[vbase + tid];
+            q_vf = reinterpret_cast<const T*>(p.v_first)[vsbase + tid];
+            if (p.v_gate_bias) q_gb = reinterpret_cast<const T*>(p.v_gate_bias)[hbase + tid];
+        }
+    }
     float r[4], w[4], k[4], kk[4], a[4];
-    load4(reinterpret_cast<const T*>(p.r) + vbase + c0, r);
-    load4(reinterpret_cast<const T*>(p.a) + vbase + c0, a);
     if constexpr (MODE == kRaw) {
+        const Raw4<T> q_w = ld_raw4<T>(p.w, vbase + c0), q_ks = ld_raw4<T>(p.k_k, hbase + c0), q_ka = ld_raw4<T>(p.k_a, hbase + c0);
+        const bool has_ab = p.a_is_raw && p.a_bias != nullptr;
+        const Raw4<T> q_wb = ld_raw4<T>(p.w_bias, hbase + c0, p.w_bias != nullptr), q_ab = ld_raw4<T>(p.a_bias, hbase + c0, has_ab);
         float wr[4], kr[4], ks[4], ka[4];
-        load4(reinterpret_cast<const T*>(p.w) + vbase + c0, wr);
-        load4(reinterpret_cast<const T*>(p.k) + vbase + c0, kr);
-        load4(reinterpret_cast<const T*>(p.k_k) + hbase + c0, ks);
-        load4(reinterpret_cast<const T*>(p.k_a) + hbase + c0, ka);
+        cvt4(q_r, r);
+        cvt4(q_a, a);
+        cvt4(q_w, wr);
+        cvt4(q_k, kr);
+        cvt4(q_ks, ks);
+        cvt4(q_ka, ka);
         if (p.w_bias) {
             float wb[4];
-            load4(reinterpret_cast<const T*>(p.w_bias) + hbase + c0, wb);
+            cvt4(q_wb, wb);
 #pragma unroll
             for (int c = 0; c < 4; ++c) wr[c] = round_to<T>(wr[c] + wb[c]);
         }
         if (p.a_is_raw) {
-            float ab[4] = {0.f, 0.f, 0.f, 0.f};
-            if (p.a_bias) load4(reinterpret_cast<const T*>(p.a_bias) + hbase + c0, ab);
+            float ab[4];
+            cvt4(q_ab, ab);
 #pragma unroll
             for (int c = 0; c < 4; ++c) a[c] = round_to<T>(sigmoidf_(round_to<T>(a[c] + ab[c])));
         }
@@ -155,9 +197,13 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
             }
         }
     } else {
-        load4(reinterpret_cast<const TW*>(p.w) + vbase + c0, w);
-        load4(reinterpret_cast<const T*>(p.k) + vbase + c0, k);
-        load4(reinterpret_cast<const T*>(p.kk) + vbase + c0, kk);
+        const Raw4<TW> q_w = ld_raw4<TW>(p.w, vbase + c0);
+        const Raw4<T> q_kk = ld_raw4<T>(p.kk, vbase + c0);
+        cvt4(q_r, r);
+        cvt4(q_a, a);
+        cvt4(q_w, w);
+        cvt4(q_k, k);
+        cvt4(q_kk, kk);
     }
     float kka[4];
 #pragma unroll
@@ -165,15 +211,12 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
 
     // ---- row-indexed value vector (with the optional v_first interpolation)
     if (tid < kN) {
-        float vv = to_f<T>(reinterpret_cast<const T*>(p.v)[vbase + tid]);
+        float vv = to_f<T>(q_v);
         if constexpr (MODE == kRaw) {
-            if (p.v_first != nullptr && p.v_gate != nullptr) {
-                float gate = to_f<T>(reinterpret_cast<const T*>(p.v_gate)[vbase + tid]);
-                if (p.v_gate_is_raw) {
-                    const float gb = p.v_gate_bias ? to_f<T>(reinterpret_cast<const T*>(p.v_gate_bias)[hbase + tid]) : 0.f;
-                    gate = round_to<T>(sigmoidf_(round_to<T>(gate + gb)));
-                }
-                const float vf = to_f<T>(reinterpret_cast<const T*>(p.v_first)[vsbase + tid]);
+            if (interp) {
+                float gate = to_f<T>(q_gate);
+                if (p.v_gate_is_raw) gate = round_to<T>(sigmoidf_(round_to<T>(gate + to_f<T>(q_gb))));
+                const float vf = to_f<T>(q_vf);
                 vv = round_to<T>(vv + (vf - vv) * gate);
             }
             if (p.v_out) reinterpret_cast<T*>(p.v_out)[vsbase + tid] = from_f<T>(vv);
@@ -204,7 +247,13 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
     }
 
     float corr = 0.f;
+    T q_gw{}, q_gnb{}, q_g{};
     if constexpr (MODE != kUpdate) {
+        if (tid < kN) {
+            q_gw = reinterpret_cast<const T*>(p.gn_w)[hbase + tid];
+            q_gnb = reinterpret_cast<const T*>(p.gn_b)[hbase + tid];
+            q_g = reinterpret_cast<const T*>(p.g)[vbase + tid];
+        }
         float rk[4];
         load4(reinterpret_cast<const T*>(p.r_k) + hbase + c0, rk);
 #pragma unroll
@@ -226,9 +275,7 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
             const float d0 = y0 - mean, d1 = y1 - mean;
             const float var = group_sum<32>(d0 * d0 + d1 * d1) * (1.0f / kN);
             const float normed = (y - mean) * rsqrtf(var + p.eps);
-            const float gw = to_f<T>(reinterpret_cast<const T*>(p.gn_w)[hbase + tid]);
-            const float gb = to_f<T>(reinterpret_cast<const T*>(p.gn_b)[hbase + tid]);
-            const float gate = to_f<T>(reinterpret_cast<const T*>(p.g)[vbase + tid]);
+            const float gw = to_f<T>(q_gw), gb = to_f<T>(q_gnb), gate = to_f<T>(q_g);
             out[tid] = from_f<T>((normed * gw + gb + corr * s_v[tid]) * gate);
         }
     }
