@@ -11,58 +11,71 @@ namespace rwkv7 {
 // ---------------------------------------------------------------- quantiser
 // one CTA per row; s = max(amax/127, 1e-5); q = clamp(round_half_away(x / s), +-127).  The row is read from memory
 // ONCE: each thread keeps its 8-element chunks in registers between the amax pass and the quantising pass (rows up to
-// 256 * 8 * kQuantChunks elements; longer rows re-read the tail, which then comes from L2).
-constexpr int kQuantChunks = 8;
+// 256 * 8 * CHUNKS elements; longer rows re-read the tail, which then comes from L2).
+//
+// Bound: HBM (3 bytes an fp16 element); the IEEE division per element was what it spent its time on, and registers for
+// eight chunks kept three CTAs on an SM.
 
-__device__ __forceinline__ int8_t quant_one(float v, float s) {
-    const float t = __fdiv_rn(v, s);
-    float r = (t >= 0.f) ? floorf(t + 0.5f) : ceilf(t - 0.5f);
+// The quotient only matters where it rounds: x * (1 / s) is within 1.5 * 2^-23 of x / s relative to it, less than 3e-5 for
+// |x / s| <= 127, so away from a rounding boundary by 1e-4 the product rounds like the IEEE quotient; nearer (and for
+// NaN) the quotient itself is formed.
+__device__ __forceinline__ int8_t quant_one(float v, float s, float inv) {
+    const float u = fabsf(v * inv) + 0.5f, f = floorf(u), d = u - f;
+    float r = copysignf(f, v);
+    if (!(d >= 1e-4f && d <= 0.9999f)) {
+        const float t = __fdiv_rn(v, s);
+        r = (t >= 0.f) ? floorf(t + 0.5f) : ceilf(t - 0.5f);
+    }
     r = fminf(fmaxf(r, -127.f), 127.f);
     return (int8_t)(int)r;
 }
 
-template <typename T>
+template <typename T, int CHUNKS>
 __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, int8_t* __restrict__ q,
                                                        float* __restrict__ scale, int K) {
     __shared__ float red[32];
     const size_t row = blockIdx.x;
     const T* xr = x + row * K;
-    Vec8<T> keep[kQuantChunks];  // the row's chunks in their storage type: 4 registers per chunk for 16-bit inputs
+    Vec8<T> keep[CHUNKS];  // the row's chunks in their storage type: 4 registers per chunk for 16-bit inputs
     float amax = 0.f;
 #pragma unroll
-    for (int c = 0; c < kQuantChunks; ++c) {
+    for (int c = 0; c < CHUNKS; ++c) {
+        const int k = (c * 256 + threadIdx.x) * 8;
+        if (k < K) keep[c] = *reinterpret_cast<const Vec8<T>*>(xr + k);
+    }
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
         const int k = (c * 256 + threadIdx.x) * 8;
         if (k < K) {
-            keep[c] = *reinterpret_cast<const Vec8<T>*>(xr + k);
 #pragma unroll
             for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(to_f<T>(keep[c].v[e])));
         }
     }
-    for (int k = (kQuantChunks * 256 + threadIdx.x) * 8; k < K; k += 256 * 8) {
+    for (int k = (CHUNKS * 256 + threadIdx.x) * 8; k < K; k += 256 * 8) {
         float v[8];
         load8(xr + k, v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
     }
     amax = block_max(amax, red);
-    const float s = fmaxf(__fdiv_rn(amax, 127.0f), 1.0e-5f);
+    const float s = fmaxf(__fdiv_rn(amax, 127.0f), 1.0e-5f), inv = __fdiv_rn(1.0f, s);
     if (threadIdx.x == 0) scale[row] = s;
 #pragma unroll
-    for (int c = 0; c < kQuantChunks; ++c) {
+    for (int c = 0; c < CHUNKS; ++c) {
         const int k = (c * 256 + threadIdx.x) * 8;
         if (k < K) {
             alignas(8) int8_t o[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = quant_one(to_f<T>(keep[c].v[e]), s);
+            for (int e = 0; e < 8; ++e) o[e] = quant_one(to_f<T>(keep[c].v[e]), s, inv);
             *reinterpret_cast<uint2*>(q + row * K + k) = *reinterpret_cast<const uint2*>(o);
         }
     }
-    for (int k = (kQuantChunks * 256 + threadIdx.x) * 8; k < K; k += 256 * 8) {
+    for (int k = (CHUNKS * 256 + threadIdx.x) * 8; k < K; k += 256 * 8) {
         float v[8];
         load8(xr + k, v);
         alignas(8) int8_t o[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = quant_one(v[e], s);
+        for (int e = 0; e < 8; ++e) o[e] = quant_one(v[e], s, inv);
         *reinterpret_cast<uint2*>(q + row * K + k) = *reinterpret_cast<const uint2*>(o);
     }
 }
@@ -259,7 +272,8 @@ extern "C" int rwkv7_a8_quant(const void* x, int8_t* q, float* scale, int rows, 
     RWKV7_REQUIRE(aligned(x, 16) && aligned(q, 8), RWKV7_ERR_ALIGN, "a8_quant: unaligned pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
-        a8_quant_kernel<T><<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K);
+        if (K <= 2 * 256 * 8) a8_quant_kernel<T, 2><<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K);
+        else a8_quant_kernel<T, 8><<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K);
         return check_launch("a8_quant_kernel");
     });
     return RWKV7_OK;

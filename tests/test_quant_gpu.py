@@ -39,6 +39,23 @@ def test_a8_quantiser_bit_exact(rows, K):
     assert np.array_equal(q.cpu().numpy(), qo)
 
 
+@pytest.mark.parametrize("K", [256, 4096, 4104])
+@pytest.mark.parametrize("amax", [127.0, 3.7, 1e-4])
+def test_a8_quantiser_at_rounding_boundaries(K, amax):
+    """Quotients at, just below and just above the half-way points of all 127 steps: the bytes are those of the division."""
+    s = max(np.float32(amax) / np.float32(127.0), np.float32(1e-5))
+    mid = (np.arange(-127, 127) + 0.5).astype(np.float32) * np.float32(s)
+    vals = np.concatenate([mid, np.nextafter(mid, np.float32(np.inf)), np.nextafter(mid, np.float32(-np.inf)),
+                           mid * np.float32(1 + 3e-7), mid * np.float32(1 - 3e-7)])
+    vals = np.clip(vals, -np.float32(amax), np.float32(amax))
+    x = np.resize(vals, (5, K - 1)).astype(np.float32)
+    x = np.concatenate([x, np.full((5, 1), amax, np.float32)], 1)
+    qo, so = O.dynamic_a8_quant(x)
+    q, sc = hb.dynamic_a8_quant(cu(x))
+    np.testing.assert_array_equal(npf(sc).reshape(-1), np.asarray(so, np.float32).reshape(-1))
+    np.testing.assert_array_equal(q.cpu().numpy(), qo)
+
+
 @pytest.mark.parametrize("M,K,Nn", [(1, 16, 8), (17, 64, 24), (64, 256, 96), (130, 4096, 136), (256, 512, 256), (384, 1024, 512)])
 def test_int8_gemm_bit_exact(M, K, Nn):
     rng = np.random.default_rng(M * 7 + Nn)
