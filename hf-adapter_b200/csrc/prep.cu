@@ -95,13 +95,15 @@ __global__ void __launch_bounds__(256) state_prep_kernel(const PrepArgs p) {
     }
     n2 = group_sum<16>(n2);
     const float inv = 1.0f / fmaxf(sqrtf(n2), 1e-12f);
-    float wo[4], ko[4];
+    float wo[4] = {0.f, 0.f, 0.f, 0.f}, ko[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         kk[c] *= inv;
         ko[c] = k[c] * (1.0f + (a[c] - 1.0f) * ka[c]);
-        const float lw = -0.606531f * sigmoidf_(w[c]);
-        wo[c] = p.log_decay ? lw : expf(lw);
+        if (p.w_out) {  // two exponentials and a division an element that the tensor-core scan's caller does not want
+            const float lw = -0.606531f * sigmoidf_(w[c]);
+            wo[c] = p.log_decay ? lw : expf(lw);
+        }
     }
     if (p.v_first && p.v_gate) {
         float vf[4], vg[4];
