@@ -5,8 +5,8 @@
 // One launch covers the four rank-R "down" projections (K = d_model, Nout = rank) or the four "up"
 // projections (K = rank, Nout = attention width) of a layer.  These matrices are tiny (a few MB per
 // layer in total), so the kernel is built for latency: warp-level HMMA (mma.sync m16n8k16, fp32
-// accumulate) on 64 x 64 output tiles, two 64-wide K chunks in flight (cp.async, XOR swizzle for
-// conflict-free ldmatrix; W before the grid-dependency wait where the caller allows it), and split-K across a thread-block cluster whose partial tiles are
+// accumulate) on 64 x 64 output tiles, cp.async double-buffered 64-wide K chunks with an XOR swizzle
+// for conflict-free ldmatrix, and split-K across a thread-block cluster whose partial tiles are
 // reduced through distributed shared memory in fixed rank order (deterministic, no scratch memory).
 #include <cooperative_groups.h>
 
@@ -20,9 +20,6 @@ constexpr int kMaxProblems = 4;
 constexpr int LT = 64;         // tile rows (activations) and tile columns (outputs)
 constexpr int LK = 64;         // K chunk
 constexpr int LTHREADS = 128;  // 4 warps as 2 x 2, warp tile 32 x 32
-constexpr int LSTAGES = 2;     // K chunks in flight: 3 or 4 gain 1 us alone and lose 2..3 % of a step, where the projections want the shared memory
-constexpr int LSTAGE_BYTES = 2 * LT * 128;  // one chunk of x and of W
-static_assert(LT * LT * 4 <= LSTAGE_BYTES, "the partial tile of the split-K reduction fits the first stage");
 
 struct GroupArgs {
     const void* x[kMaxProblems];
@@ -31,7 +28,6 @@ struct GroupArgs {
     void* out[kMaxProblems];
     int K[kMaxProblems], Nout[kMaxProblems], act[kMaxProblems];
     int M, splits, max_tiles;
-    int early;  // W may be read before the grid-dependency wait
 };
 
 __device__ __forceinline__ void lcp16(void* smem, const void* g, bool valid) {
@@ -67,16 +63,18 @@ __device__ __forceinline__ float lora_act(float v, int act) {
 
 template <typename T>
 __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupArgs p) {
-    extern __shared__ __align__(128) unsigned char smem[];  // min(LSTAGES, chunks per CTA) stages of x | W
-    if (!p.early) grid_dependency_wait();
+    __shared__ __align__(128) unsigned char sX[2][LT * 128];
+    __shared__ __align__(128) unsigned char sW[2][LT * 128];
+    __shared__ __align__(16) float sP[LT * LT];  // partial tile for the split-K reduction
+
+    // launched programmatically: resident under the tail of the preceding kernel of the stream, everything below after it
+    grid_dependency_wait();
+    if (threadIdx.x == 0) grid_launch_dependents();
     const int prob = blockIdx.y;
     const int K = p.K[prob], Nout = p.Nout[prob];
     const int n0 = (blockIdx.x % p.max_tiles) * LT;
     const int r0 = (blockIdx.x / p.max_tiles) * LT;  // activation row block
-    if (n0 >= Nout) {  // whole cluster shares blockIdx.x / y, so it leaves together
-        grid_dependency_wait();
-        return;
-    }
+    if (n0 >= Nout) return;  // whole cluster shares blockIdx.x / y, so it leaves together
     const int split = blockIdx.z, S = p.splits;
     const int chunks_total = (K + LK - 1) / LK;
     const int chunks_per = (chunks_total + S - 1) / S;
@@ -95,72 +93,55 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
 
-    auto stage = [&](int c) { return smem + ((c - c_begin) % LSTAGES) * LSTAGE_BYTES; };
-    auto load_w = [&](int c) {
-        if (c >= c_end) return;
+    auto load_chunk = [&](int buf, int c) {
+        const int k0 = c * LK;
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {  // 64 rows x 8 pieces of 16 bytes, 128 threads
-            const int idx = tid + it * LTHREADS, row = idx >> 3, ch = idx & 7, k = c * LK + ch * 8;
-            const bool ok = k < K && (n0 + row) < Nout;
-            lcp16(stage(c) + LT * 128 + lswz(row, ch), ok ? W + (size_t)(n0 + row) * K + k : W, ok);
-        }
-    };
-    auto load_x = [&](int c) {  // ends the chunk's group, which exists also when there is nothing to load
-        if (c < c_end) {
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-                const int idx = tid + it * LTHREADS, row = idx >> 3, ch = idx & 7, k = c * LK + ch * 8;
-                const bool ok = k < K && (r0 + row) < p.M;
-                lcp16(stage(c) + lswz(row, ch), ok ? X + (size_t)(r0 + row) * K + k : X, ok);
-            }
+        for (int it = 0; it < 4; ++it) {  // 64 rows x 8 chunks = 512 chunks per operand, 128 threads
+            const int idx = tid + it * LTHREADS;
+            const int row = idx >> 3, ch = idx & 7;
+            const bool kin = (k0 + ch * 8) < K;
+            const bool vx = kin && (r0 + row) < p.M;
+            const bool vw = kin && (n0 + row) < Nout;
+            lcp16(&sX[buf][lswz(row, ch)], vx ? X + (size_t)(r0 + row) * K + k0 + ch * 8 : X, vx);
+            lcp16(&sW[buf][lswz(row, ch)], vw ? W + (size_t)(n0 + row) * K + k0 + ch * 8 : W, vw);
         }
         asm volatile("cp.async.commit_group;\n" ::);
     };
 
-    for (int i = 0; i < LSTAGES; ++i) load_w(c_begin + i);
-    if (p.early) grid_dependency_wait();
-    if (tid == 0) grid_launch_dependents();
-    for (int i = 0; i < LSTAGES; ++i) load_x(c_begin + i);
+    if (c_begin < c_end) load_chunk(0, c_begin);
     for (int c = c_begin; c < c_end; ++c) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(LSTAGES - 1));
+        const int buf = (c - c_begin) & 1;
+        if (c + 1 < c_end) {
+            load_chunk(buf ^ 1, c + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::);
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::);
+        }
         __syncthreads();
-        const unsigned char *sX = stage(c), *sW = sX + LT * 128;
 #pragma unroll
         for (int ks = 0; ks < LK / 16; ++ks) {
             uint32_t af[2][4], bf[2][4];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int row = wm * 32 + i * 16 + (lane & 15);
-                lldm4(af[i], sX + lswz(row, ks * 2 + (lane >> 4)));
+                lldm4(af[i], &sX[buf][lswz(row, ks * 2 + (lane >> 4))]);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int row = wn * 32 + j * 16 + (lane & 7) + ((lane >> 4) << 3);
-                lldm4(bf[j], sW + lswz(row, ks * 2 + ((lane >> 3) & 1)));
+                lldm4(bf[j], &sW[buf][lswz(row, ks * 2 + ((lane >> 3) & 1))]);
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) hmma<T>(acc[i][j], af[i], bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
         }
-        if (c + LSTAGES < c_end) __syncthreads();  // the stage is filled again
-        load_w(c + LSTAGES);
-        load_x(c + LSTAGES);
+        __syncthreads();
     }
 
     const int gid = lane >> 2, tig = lane & 3;
     cg::cluster_group cluster = cg::this_cluster();
-    const T* bias = reinterpret_cast<const T*>(p.bias[prob]);
-    T* out = reinterpret_cast<T*>(p.out[prob]);
-    const int act = p.act[prob];
-    auto finish = [&](float v, int n) {
-        if (bias) v += to_f<T>(bias[n]);
-        v = round_to<T>(v);
-        return act ? lora_act(v, act) : v;
-    };
     if (S > 1) {
-        float* sP = reinterpret_cast<float*>(smem);  // over the drained ring
-        __syncthreads();
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -171,40 +152,38 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
                     *reinterpret_cast<float2*>(&sP[r * LT + cidx]) = make_float2(acc[i][j][hh * 2], acc[i][j][hh * 2 + 1]);
                 }
         cluster.sync();
-        // rank `split` finishes rows [split*LT/S, (split+1)*LT/S), four columns a thread
+        // rank `split` finishes rows [split*LT/S, (split+1)*LT/S)
         const int rows_per = LT / S;
-        for (int idx = tid; idx < rows_per * LT / 4; idx += LTHREADS) {
-            const int r = split * rows_per + idx / (LT / 4), cidx = idx % (LT / 4) * 4;
-            if (r0 + r >= p.M) continue;
-            float4 part[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (q < S) part[q] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sP, q) + r * LT + cidx);
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (q < S) { v[0] += part[q].x; v[1] += part[q].y; v[2] += part[q].z; v[3] += part[q].w; }
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (n0 + cidx + e < Nout) out[(size_t)(r0 + r) * Nout + n0 + cidx + e] = from_f<T>(finish(v[e], n0 + cidx + e));
+        const T* bias = reinterpret_cast<const T*>(p.bias[prob]);
+        T* out = reinterpret_cast<T*>(p.out[prob]);
+        for (int idx = tid; idx < rows_per * LT; idx += LTHREADS) {
+            const int r = split * rows_per + idx / LT, cidx = idx % LT;
+            float v = 0.f;
+            for (int q = 0; q < S; ++q) v += cluster.map_shared_rank(sP, q)[r * LT + cidx];
+            if (r0 + r < p.M && n0 + cidx < Nout) {
+                if (bias) v += to_f<T>(bias[n0 + cidx]);
+                v = round_to<T>(v);
+                if (p.act[prob]) v = lora_act(v, p.act[prob]);
+                out[(size_t)(r0 + r) * Nout + n0 + cidx] = from_f<T>(v);
+            }
         }
         cluster.sync();
     } else {
+        const T* bias = reinterpret_cast<const T*>(p.bias[prob]);
+        T* out = reinterpret_cast<T*>(p.out[prob]);
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int r = r0 + wm * 32 + i * 16 + gid + hh * 8, n = n0 + wn * 32 + j * 8 + tig * 2;
-                    if (r >= p.M || n >= Nout) continue;
-                    T* dst = out + (size_t)r * Nout + n;
-                    if ((Nout & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0) {
-                        T two[2] = {from_f<T>(finish(acc[i][j][hh * 2], n)), from_f<T>(finish(acc[i][j][hh * 2 + 1], n + 1))};
-                        *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(two);
-                    } else {
-                        dst[0] = from_f<T>(finish(acc[i][j][hh * 2], n));
-                        if (n + 1 < Nout) dst[1] = from_f<T>(finish(acc[i][j][hh * 2 + 1], n + 1));
+                for (int e = 0; e < 4; ++e) {
+                    const int r = wm * 32 + i * 16 + gid + (e >> 1) * 8, cidx = n0 + wn * 32 + j * 8 + tig * 2 + (e & 1);
+                    if (r0 + r < p.M && cidx < Nout) {
+                        float v = acc[i][j][e];
+                        if (bias) v += to_f<T>(bias[cidx]);
+                        v = round_to<T>(v);
+                        if (p.act[prob]) v = lora_act(v, p.act[prob]);
+                        out[(size_t)(r0 + r) * Nout + cidx] = from_f<T>(v);
                     }
                 }
     }
@@ -214,9 +193,9 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
 
 using namespace rwkv7;
 
-static int small_gemm_group_impl(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
-                                 void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
-                                 int static_weights, void* stream) {
+extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
+                                      void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
+                                      void* stream) {
     RWKV7_REQUIRE(n_problems >= 1 && n_problems <= kMaxProblems, RWKV7_ERR_INVALID, "small_gemm_group: 1..%d problems", kMaxProblems);
     RWKV7_REQUIRE(M >= 1 && M <= 16384, RWKV7_ERR_UNSUPPORTED, "small_gemm_group: M must be in 1..16384 (got %d)", M);
     const int row_blocks = (M + LT - 1) / LT;
@@ -242,16 +221,10 @@ static int small_gemm_group_impl(int n_problems, const void* const* x, const voi
     while (splits < 8 && max_tiles * row_blocks * n_problems * splits * 2 <= 160 && chunks / (splits * 2) >= 4) splits *= 2;
     a.splits = splits;
     a.max_tiles = max_tiles;
-    a.early = static_weights != 0;
-    const int per_cta = (chunks + splits - 1) / splits;
-    const int smem = (per_cta < LSTAGES ? per_cta : LSTAGES) * LSTAGE_BYTES;
-    auto kern = dtype == RWKV7_F16 ? small_gemm_group_kernel<__half> : small_gemm_group_kernel<__nv_bfloat16>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LSTAGES * LSTAGE_BYTES);
-    RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "small_gemm_group: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(max_tiles * row_blocks, n_problems, splits);
     cfg.blockDim = dim3(LTHREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = 0;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -262,19 +235,9 @@ static int small_gemm_group_impl(int n_problems, const void* const* x, const voi
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = programmatic_launch_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kern, a);
+    cudaError_t e;
+    if (dtype == RWKV7_F16) e = cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<__half>, a);
+    else e = cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<__nv_bfloat16>, a);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "small_gemm_group launch: %s", cudaGetErrorString(e));
     return RWKV7_OK;
-}
-
-extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
-                                      void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
-                                      void* stream) {
-    return small_gemm_group_impl(n_problems, x, W, bias, out, K, Nout, act_out, M, dtype, 0, stream);
-}
-
-extern "C" int rwkv7_small_gemm_group_static(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
-                                             void* const* out, const int* K, const int* Nout, const int* act_out, int M,
-                                             int dtype, void* stream) {
-    return small_gemm_group_impl(n_problems, x, W, bias, out, K, Nout, act_out, M, dtype, 1, stream);
 }

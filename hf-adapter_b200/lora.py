@@ -29,10 +29,9 @@ def dense_small(x, weight, bias=None, *, act_in: int = 0, act_out: int = 0, out=
     return out.reshape(*x.shape[:-1], Nout)
 
 
-def small_gemm_group(xs, weights, biases=None, acts=None, outs=None, static_weights=False):
+def small_gemm_group(xs, weights, biases=None, acts=None, outs=None):
     """One launch for up to four independent small linears ``out_i = act_i(x_i @ W_i.T + b_i)`` sharing the row
-    count (fp16/bf16: tensor-core kernel, 64-row blocks; fp32: one ``dense_small`` call per problem).
-    ``static_weights``: the kernel launched just before on this stream does not write a weight."""
+    count (fp16/bf16: tensor-core kernel, 64-row blocks; fp32: one ``dense_small`` call per problem)."""
     n = len(xs)
     biases = list(biases) if biases is not None else [None] * n
     acts = list(acts) if acts is not None else [0] * n
@@ -61,8 +60,7 @@ def small_gemm_group(xs, weights, biases=None, acts=None, outs=None, static_weig
     bp, _k3 = _lib.ptr_array([0 if t is None else t.data_ptr() for t in bs])
     op, _k4 = _lib.ptr_array([t.data_ptr() for t in outs])
     IA = _lib.c_int * n
-    launch = _lib.lib.rwkv7_small_gemm_group_static if static_weights else _lib.lib.rwkv7_small_gemm_group
-    _lib.check(launch(n, xp, wp, bp, op, IA(*[int(w.shape[1]) for w in ws]),
+    _lib.check(_lib.lib.rwkv7_small_gemm_group(n, xp, wp, bp, op, IA(*[int(w.shape[1]) for w in ws]),
                                                IA(*[int(w.shape[0]) for w in ws]), IA(*acts), M, dt_code(x2[0]),
                                                stream_ptr(x2[0])), "small_gemm_group")
     return [o.reshape(*x.shape[:-1], int(w.shape[0])) for o, x, w in zip(outs, xs, ws)]

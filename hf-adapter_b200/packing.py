@@ -249,33 +249,38 @@ _DEFAULT_CONTEXT = StepContext()
 
 def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
     """r / k / v and the LoRA pre-activations of a layer step on parallel branches: ``[r, k, v, w, a, g(, v_gate)]``."""
-    # r / k / v do not depend on the LoRA chain and join before the recurrence: they run on side streams (parallel branches
-    # of the decode graph once captured).  The chain, two dependent launches on the critical path, stays on the main stream
-    # and starts under the tail of the kernel before it; the other way round the projections took the SMs first and the
-    # chain ended 18 us after them (256 rows, 4096 wide: 9.62 -> 9.28 ms a step; 64 rows, 2560 wide: 2.74 -> 2.58 ms).
+    xr, xk, xv = xs
+    # The LoRA chain does not depend on r/k/v: it runs on a side stream (a parallel branch of the decode graph once
+    # captured) and joins before the recurrence.
     main = torch.cuda.current_stream(x.device)
-    sides = [ctx.side_stream(x.device, i) for i in range(3)]
-    sides[0].wait_stream(main)
-    with torch.cuda.stream(sides[0]):
-        # int4 / int8 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
-        # exchange) instead of three launches competing for the SMs
-        rkv = rkv_grouped(ops, *xs) if all(isinstance(o, _QUANT_TYPES) for o in ops) else None
+    side = ctx.side_stream(x.device, 0)
+    side.wait_stream(main)
+    with torch.cuda.stream(side):
+        hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)])
+        lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups])
+    rkv = rkv_grouped(ops, xr, xk, xv) if all(isinstance(o, _QUANT_TYPES) for o in ops) else None
     if rkv is not None:
-        sides = sides[:1]
+        # int4 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
+        # exchange) instead of three launches competing for the SMs
+        r, k, v = rkv
+        main.wait_stream(side)
     else:
-        rkv = []
-        for st, op, x_ in zip(sides, ops, xs):  # the tail of one overlaps the ramp-up of the next
-            st.wait_stream(main)
-            with torch.cuda.stream(st):
-                rkv.append(apply_linear(op, x_))
-    hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)], static_weights=True)
-    lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups], static_weights=True)
-    for st in sides:
-        main.wait_stream(st)
-    for i in range(3):
-        xs[i].record_stream(sides[i % len(sides)])
-        rkv[i].record_stream(main)
-    return [*rkv, *lora]
+        # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
+        sk, sv = ctx.side_stream(x.device, 1), ctx.side_stream(x.device, 2)
+        sk.wait_stream(main)
+        sv.wait_stream(main)
+        with torch.cuda.stream(sk):
+            k = apply_linear(ops[1], xk)
+        with torch.cuda.stream(sv):
+            v = apply_linear(ops[2], xv)
+        r = apply_linear(ops[0], xr)
+        main.wait_stream(side)
+        main.wait_stream(sk)
+        main.wait_stream(sv)
+        xk.record_stream(sk); k.record_stream(sk); xv.record_stream(sv); v.record_stream(sv)
+    for t_ in (*down_x, *lora):
+        t_.record_stream(side)
+    return [r, k, v, *lora]
 
 
 def block_ip_batched(x, state, xpa, xpf, v_first, p, sparse_ffn_out=None, fp16_elapsed=None,
