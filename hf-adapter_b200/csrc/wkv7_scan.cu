@@ -30,6 +30,7 @@ struct ScanArgs {
     int ab_mode;         // `kk` holds -kk and `a` holds kk*a (the lane's neg_kk / kka operands)
     const void* w0;      // w_mode 2: per-channel bias [H*64] added to raw w before the decay (may be NULL)
     const int* elapsed;  // w_mode 2: per-sequence step counters [B]; token t uses the dither phase elapsed + channel + t
+    int params_vec;      // r_k, gn_w and gn_b all start on 16 bytes; else (views into a flat buffer) they are read by element
 };
 
 // zero-mean pseudo-random offset of the reference's FP16-state kernels (rwkv7_hf/native_wkv_fp16.py:118-121)
@@ -276,6 +277,15 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
     auto flush = [&](int s, Operands& op) {
         const int t0 = s * kTS, nt = min(kTS, T_ - t0);
         const int l8 = ht & 7, c = l8 * 8;
+        auto load_param = [&](const void* param, float (&o)[8]) {
+            const T* q = reinterpret_cast<const T*>(param) + h * kSN + c;
+            if (p.params_vec) {
+                load8(q, o);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = to_f<T>(q[i]);
+            }
+        };
         for (int tt = ht >> 3; tt < kTS; tt += 8) {
             const bool live = tt < nt;  // the shuffles below run in all lanes
             const size_t o = base + (size_t)(t0 + (live ? tt : 0)) * tok_stride + c;
@@ -287,9 +297,9 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
                 load8<float>(&op.k[live ? tt : 0][c], k);
                 load8<float>(&op.v[live ? tt : 0][c], v);
                 load8(reinterpret_cast<const T*>(p.g) + o, g);
-                load8(reinterpret_cast<const T*>(p.r_k) + h * kSN + c, rk);
-                load8(reinterpret_cast<const T*>(p.gn_w) + h * kSN + c, gw);
-                load8(reinterpret_cast<const T*>(p.gn_b) + h * kSN + c, gb);
+                load_param(p.r_k, rk);
+                load_param(p.gn_w, gw);
+                load_param(p.gn_b, gb);
                 float sum = 0.f, corr = 0.f, var = 0.f;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) { sum += y[i]; corr += r[i] * k[i] * rk[i]; }
@@ -429,7 +439,8 @@ static int scan_impl(const void* r, const void* w, const void* k, const void* v,
     const void* ptrs[] = {r, w, k, v, kk, a, state_in, state_out, y, g};
     for (const void* q : ptrs) RWKV7_REQUIRE(aligned(q, 16), RWKV7_ERR_ALIGN, "wkv7_scan: pointers must be 16-byte aligned");
     RWKV7_REQUIRE((!w0 && !elapsed) || w_mode == 2, RWKV7_ERR_INVALID, "wkv7_scan: w0 / elapsed apply to raw w (w_mode 2)");
-    ScanArgs p{r, w, k, v, kk, a, state_in, state_out, y, g, r_k, gn_w, gn_b, eps, T, H, w_mode, state_f16 != 0, ab_mode != 0, w0, elapsed};
+    ScanArgs p{r, w, k, v, kk, a, state_in, state_out, y, g, r_k, gn_w, gn_b, eps, T, H, w_mode, state_f16 != 0, ab_mode != 0, w0, elapsed,
+               aligned(r_k, 16) && aligned(gn_w, 16) && aligned(gn_b, 16)};
     RWKV7_DISPATCH_DTYPE(dtype, TT, {
         return prep ? dispatch_scan<TT, true>(p, B, st) : dispatch_scan<TT, false>(p, B, st);
     });

@@ -133,6 +133,12 @@ def test_sequence_lane(B, T, Hh):
     assert rel_err(npf(y2), yt.astype(np.float32)) < 4e-3
 
 
+@pytest.mark.parametrize("Hh", [149, 297])
+def test_sequence_lane_on_larger_grids(Hh):
+    """The same operand forms on the other two register tiles of the scan."""
+    test_sequence_lane(1, 9, Hh)
+
+
 def test_model_with_fp16_state_cache():
     """The tiny reference model in fp16 with state_dtype=float16: decode logits track the fp32-state model (cosine
     >= 0.999), the CUDA-graph replay equals the eager step bit for bit (the dither phase lives in the cache), prefill

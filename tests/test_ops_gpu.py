@@ -179,6 +179,28 @@ def test_scan_tile_choice_by_grid(B, T, Hh):
     assert sh.dtype == torch.float16 and rel_err(npf(sh), soh) < 1e-3
 
 
+@pytest.mark.parametrize("dt", ["fp16", "bf16", "fp32"])
+@pytest.mark.parametrize("Hh", [3, 149, 297])
+def test_scan_parameters_of_any_alignment(dt, Hh):
+    """r_k and the GroupNorm parameters as views into one flat buffer at odd element offsets (3 / 149 / 297 CTAs: the
+    three register tiles): the bits of the aligned call."""
+    td = dict(TD, bf16=torch.bfloat16)[dt]
+    gen = torch.Generator(device="cuda").manual_seed(Hh)
+    f = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    T = 9
+    r, k, v, g = (f(1, T, Hh, N).to(td) for _ in range(4))
+    kk = torch.nn.functional.normalize(k.float(), dim=-1).to(td)
+    w, a, s0 = torch.sigmoid(f(1, T, Hh, N)), torch.sigmoid(f(1, T, Hh, N)).to(td), f(1, Hh, N, N)
+    size = Hh * N
+    for off in (1, 3, 8):
+        flat = f(3 * (size + 8) + off).to(td)
+        views = [flat[off + i * (size + (1, 8, 2)[i]):][:size] for i in range(3)]
+        assert off == 8 or any(p.data_ptr() % 16 for p in views)
+        got = hb.fused_recurrent_scan_output_prepare(r, w, k, v, kk, a, s0, g, *views, eps=EPS)
+        want = hb.fused_recurrent_scan_output_prepare(r, w, k, v, kk, a, s0, g, *(p.clone() for p in views), eps=EPS)
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+
+
 def test_scan_empty_sequence_passes_state_through():
     s0 = torch.randn(2, 2, N, N, device="cuda")
     e = torch.empty(2, 0, 2, N, device="cuda", dtype=torch.float16)
