@@ -49,6 +49,23 @@ inline bool programmatic_launch_enabled() {
     return on;
 }
 
+// Whether a launch on `st` may be programmatic.  Under capture the attribute turns EVERY edge into the node into a programmatic
+// one, those of joined branches included, and the kernels' ordering (grid_dependency_wait() stands for the one kernel
+// before this one) is argued for one predecessor: a node that joins branches gets full edges.  Outside capture a join is
+// an event wait in the stream, which orders the launch by itself.
+inline bool programmatic_launch_ok(cudaStream_t st) {
+    if (!programmatic_launch_enabled()) return false;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    size_t predecessors = 0;
+    const cudaGraphNode_t* nodes = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    if (cudaStreamGetCaptureInfo_v3(st, &status, nullptr, nullptr, &nodes, &edges, &predecessors) != cudaSuccess) {
+        cudaGetLastError();  // not this launch's error
+        return false;
+    }
+    return status != cudaStreamCaptureStatusActive || predecessors <= 1;
+}
+
 // Launch with the programmatic-stream-serialization attribute: the kernel may become resident while its predecessor
 // in the stream still runs and must call grid_dependency_wait() before touching anything that kernel writes.
 template <typename... KArgs, typename... Args>
@@ -62,7 +79,7 @@ inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), dim3 grid, dim3
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = programmatic_launch_enabled() ? 1 : 0;
+    cfg.numAttrs = programmatic_launch_ok(st) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

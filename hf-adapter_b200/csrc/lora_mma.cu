@@ -234,7 +234,7 @@ extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, cons
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = programmatic_launch_enabled() ? 2 : 1;
+    cfg.numAttrs = programmatic_launch_ok(cfg.stream) ? 2 : 1;
     cudaError_t e;
     if (dtype == RWKV7_F16) e = cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<__half>, a);
     else e = cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<__nv_bfloat16>, a);

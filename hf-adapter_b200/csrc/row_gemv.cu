@@ -330,7 +330,7 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (programmatic_launch_enabled() && !fresh) ? 2 : 1;
+    cfg.numAttrs = (!fresh && programmatic_launch_ok(cfg.stream)) ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "rows_gemv launch: %s", cudaGetErrorString(e));
     return RWKV7_OK;

@@ -627,7 +627,7 @@ int launch_w4g_umma_tiled(const void* const* xs, const uint8_t* const* tws, cons
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (programmatic_launch_enabled() && !fresh) ? 2 : 1;
+    cfg.numAttrs = (!fresh && programmatic_launch_ok(cfg.stream)) ? 2 : 1;
     const cudaError_t e = NB == 64 ? (fmt == 0 ? launch_variant<64, 0>(cfg, maps, a) : launch_variant<64, 1>(cfg, maps, a))
                                    : (fmt == 0 ? launch_variant<128, 0>(cfg, maps, a) : launch_variant<128, 1>(cfg, maps, a));
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "w4g_gemv_tiled launch: %s", cudaGetErrorString(e));

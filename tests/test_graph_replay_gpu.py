@@ -1,0 +1,97 @@
+"""The decode step's CUDA graph: what orders its nodes, and that replays of one state give one result.
+
+A step forks the LoRA products of a layer from its r / k / v products and joins them before the recurrence.  Kernels
+start under the tail of the one before them (programmatic edges) and wait for it on the device, which orders them behind
+ONE predecessor: a node that joins branches has to have full edges."""
+import collections
+import ctypes
+
+import pytest
+import torch
+
+import hf_adapter_b200 as hb
+
+pytestmark = pytest.mark.gpu
+
+
+class _Edge(ctypes.Structure):  # cudaGraphEdgeData
+    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte), ("reserved", ctypes.c_ubyte * 5)]
+
+
+def _edges(graph):
+    """[(to node, edge type)] of a captured graph (type 0: full, 1: programmatic)."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    raw, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert cu.cuGraphGetEdges_v2(raw, None, None, None, ctypes.byref(n)) == 0
+    a, b, e = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (_Edge * n.value)()
+    assert cu.cuGraphGetEdges_v2(raw, a, b, e, ctypes.byref(n)) == 0
+    return [(b[i], e[i].type) for i in range(n.value)]
+
+
+def _model(weights, D, layers, state=torch.float32, dtype=torch.float16):
+    cfg = hb.NativeRWKV7Config(vocab_size=512, hidden_size=D, num_hidden_layers=layers, num_heads=D // 64, head_dim=64,
+                               intermediate_size=4 * D, decay_low_rank_dim=64, a_low_rank_dim=64, v_low_rank_dim=32,
+                               gate_low_rank_dim=128)
+    old = torch.get_default_dtype()
+    torch.set_default_dtype(dtype)
+    try:
+        with torch.device("cuda"):
+            m = hb.RWKV7ForCausalLM(cfg, state_dtype=state).eval()
+    finally:
+        torch.set_default_dtype(old)
+    gen = torch.Generator(device="cuda").manual_seed(D + layers)
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if p.dim() == 2:
+                p.normal_(0.0, 1.0 if "embeddings" in name else 0.02, generator=gen)
+            elif any(k in name for k in (".x_", "k_k", "k_a")):
+                p.uniform_(0, 1, generator=gen)
+    if weights != "dense":
+        hb.quantize_model(m, weights, min_params=100_000, group_size=128, skip=("lm_head",))
+    return m
+
+
+@pytest.mark.parametrize("weights,batch,state", [("mm4", 64, torch.float32), ("w8", 64, torch.float16), ("dense", 16, torch.float32),
+                                                 ("dense", 80, torch.float32), ("dense", 2, torch.float32)])
+def test_joins_have_full_edges(weights, batch, state):
+    m = _model(weights, 512, 3, state)
+    cache, ids = m.new_cache(batch), torch.zeros(batch, device="cuda", dtype=torch.long)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        m._decode_step(ids, cache)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        m._decode_step(ids, cache)
+    into = collections.defaultdict(list)
+    for node, kind in _edges(graph):
+        into[node].append(kind)
+    assert any(kinds == [1] for kinds in into.values())  # chains are programmatic
+    joins = [kinds for kinds in into.values() if len(kinds) > 1]
+    assert bool(joins) == (batch > 8) and not any(any(kinds) for kinds in joins)
+
+
+@pytest.mark.parametrize("weights,D,batch,state", [("mm4", 4096, b, torch.float32) for b in (1, 8, 9, 64, 128, 256)]
+                         + [("w8", 2560, b, torch.float16) for b in (1, 9, 64, 256)]
+                         + [("dense", 2560, b, torch.float32) for b in (1, 8, 9, 64, 256)])
+def test_replays_of_a_state_agree(weights, D, batch, state):
+    """Two states in turn, 25 replays of each: a value read too early or too late is the other state's."""
+    m = _model(weights, D, 4, state)
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    cache = m.new_cache(batch)
+    starts = []
+    for _ in range(2):
+        cache.reset()
+        m.rwkv7_prefill_native(torch.randint(0, 512, (batch, 4), generator=gen, device="cuda"), cache)
+        starts.append((torch.randint(0, 512, (batch,), generator=gen, device="cuda"), [t.clone() for t in cache._tensors()]))
+    first = [None, None]
+    for i in range(50):
+        ids, tensors = starts[i % 2]
+        for dst, src in zip(cache._tensors(), tensors):
+            dst.copy_(src)
+        got = [m.rwkv7_forward_token(ids, cache), *cache._tensors()]
+        if first[i % 2] is None:
+            first[i % 2] = [t.clone() for t in got]
+        assert all(torch.equal(a, b) for a, b in zip(got, first[i % 2])), f"replay {i // 2} of state {i % 2}"
+    assert not torch.equal(first[0][0], first[1][0])
