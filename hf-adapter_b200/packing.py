@@ -183,7 +183,9 @@ def rkv_grouped(ops, xr, xk, xv):
 def _rows_operand(op, x):
     """``(fmt, weight, scale, out_features)`` when the projection ``op`` of the few rows ``x`` runs on the row kernel."""
     if isinstance(op, _q.MM4Linear) or (isinstance(op, _q.MM8Linear) and op.sm7x_rowwise):
-        tiled = op.tiled_for(x) if op.bias is None and x.is_contiguous() and _q.few_rows_quant(int(x.shape[0]), op.in_features) else None
+        ok = (op.bias is None and x.is_contiguous() and int(x.shape[-1]) == op.in_features
+              and _q.few_rows_quant(int(x.shape[0]), op.in_features))
+        tiled = op.tiled_for(x) if ok else None
         if tiled is None:
             return None
         return (_rowsk.INT4, tiled, None, op.out_features) if isinstance(op, _q.MM4Linear) else \
@@ -197,7 +199,7 @@ def _rows_operand(op, x):
 def rows_projections(ops, xs, epilogues=None):
     """The projections ``ops[i](xs[i])`` of a few rows in one launch, or None when one of them does not take that route.
     For the inside of a layer step: the kernel before it writes activations only."""
-    if not 1 <= int(xs[0].shape[0]) <= _rowsk.MAX_ROWS or xs[0].dtype not in (torch.float16, torch.bfloat16):
+    if xs[0].dim() != 2 or not 1 <= int(xs[0].shape[0]) <= _rowsk.MAX_ROWS or xs[0].dtype not in (torch.float16, torch.bfloat16):
         return None
     got = [_rows_operand(o, x) for o, x in zip(ops, xs)]
     if any(g is None for g in got):

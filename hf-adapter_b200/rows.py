@@ -24,18 +24,45 @@ def takes_dense(x, weight) -> bool:
             and 1 <= x.numel() // int(weight.shape[1]) <= MAX_ROWS)
 
 
+def _check_problem(i, x, w, N, fmt, scale, residual, out):
+    """The kernel takes sizes from ``x`` and ``N`` alone: every other operand has to hold as much."""
+    M, K = (int(v) for v in x.shape)
+    holds = lambda t, n: t.is_contiguous() and t.numel() * t.element_size() >= n
+    if fmt == DENSE:
+        if tuple(w.shape) != (N, K) or w.dtype != x.dtype or not w.is_contiguous():
+            raise ValueError(f"rows_gemv: weight {i} must be a contiguous [{N}, {K}] in the activation dtype, got {tuple(w.shape)}")
+    elif fmt in (INT4, INT8):
+        need = int((_lib.lib.rwkv7_w4g_tiled_bytes if fmt == INT4 else _lib.lib.rwkv7_w8_tiled_bytes)(K, N))
+        if need <= 0 or not holds(w, need):
+            raise ValueError(f"rows_gemv: weight {i} is no tiled copy of [{N}, {K}]")
+    else:
+        raise ValueError(f"rows_gemv: unknown weight format {fmt}")
+    if fmt == INT8 and (scale is None or scale.dtype != x.dtype or not holds(scale, N * scale.element_size())):
+        raise ValueError(f"rows_gemv: scale {i} must be [{N}] in the activation dtype")
+    if residual is not None and (residual.dtype != x.dtype or residual.numel() != M * N or not residual.is_contiguous()):
+        raise ValueError(f"rows_gemv: residual {i} must be a contiguous [{M}, {N}] in the activation dtype")
+    if out is not None and not holds(out, M * N * x.element_size()):
+        raise ValueError(f"rows_gemv: output {i} must be a contiguous [{M}, {N}]")
+
+
 def rows_gemv(xs, weights, *, out_features, fmts, scales=None, residuals=None, outs=None, epilogues=None, static_weights=False):
     """``outs[i] = epilogue_i(xs[i] [M,K_i] @ W_i.T)`` in one launch.  ``weights[i]`` is dense ``[N,K]`` or a tiled copy
     (``quant.w4_repack_tiled`` / ``w8_repack_tiled``).  ``static_weights``: no weight is written by the kernel launched
     just before this call on the stream."""
     n = len(xs)
+    if not 1 <= n <= MAX_PROBLEMS or any(x.dim() != 2 for x in xs):
+        raise ValueError(f"rows_gemv takes 1..{MAX_PROBLEMS} inputs [rows, features]")
     M = int(xs[0].shape[0])
     scales = list(scales) if scales is not None else [None] * n
     residuals = list(residuals) if residuals is not None else [None] * n
     epilogues = list(epilogues) if epilogues is not None else [_lib.EPI_NONE] * n
-    require_cuda(*xs, *weights, *scales, *residuals, what="rows_gemv")
     if any(int(x.shape[0]) != M or x.dtype != xs[0].dtype or not x.is_contiguous() for x in xs):
         raise ValueError("rows_gemv: all inputs need the same row count and dtype, contiguous")
+    if any(len(v) != n for v in (weights, out_features, fmts, scales, residuals, epilogues)) or (outs is not None and len(outs) != n):
+        raise ValueError("rows_gemv: one weight, output width, format, scale, residual, epilogue and output per input")
+    for i, (x, w, N, fmt) in enumerate(zip(xs, weights, out_features, fmts)):
+        _check_problem(i, x, w, int(N), fmt, scales[i], residuals[i], None if outs is None else outs[i])
+    require_cuda(*xs, *weights, *scales, *residuals, *(outs or ()), what="rows_gemv")
     if outs is None:
         outs = [torch.empty((M, N), device=xs[0].device, dtype=xs[0].dtype) for N in out_features]
     arr = lambda ts: _lib.ptr_array([ptr(t) for t in ts])

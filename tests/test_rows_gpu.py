@@ -5,6 +5,7 @@ import torch
 
 import hf_adapter_b200 as hb
 from hf_adapter_b200 import _lib, rows
+from hf_adapter_b200.packing import rows_projections
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +69,28 @@ def test_refusals():
     with pytest.raises(ValueError):
         rows.rows_gemv((x[:1, :60].contiguous(),), (w,), out_features=(8,), fmts=(0,))
     assert not rows.takes_dense(x[:1].reshape(-1)[1:57].reshape(1, 56), torch.zeros(8, 56, device="cuda").half())  # misaligned
+
+
+def test_operands_of_the_wrong_size_are_refused_on_the_host():
+    """Each would be read or written out of range: the kernel has its sizes from x and out_features alone."""
+    h = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.float16)
+    u8 = lambda n: torch.zeros(n, device="cuda", dtype=torch.uint8)
+    x, w = h(2, 128), h(16, 128)
+    w4, w8 = int(_lib.lib.rwkv7_w4g_tiled_bytes(128, 16)), int(_lib.lib.rwkv7_w8_tiled_bytes(128, 16))
+    ok = dict(out_features=(16,), fmts=(rows.DENSE,))
+    for args, kw in [((h(15, 128),), {}), ((h(16, 64),), {}), ((w.float(),), {}), ((w.t().contiguous().t(),), {}),
+                     ((u8(w4 - 1),), dict(fmts=(rows.INT4,))), ((u8(w8 - 1),), dict(fmts=(rows.INT8,), scales=(h(16),))),
+                     ((u8(w8),), dict(fmts=(rows.INT8,), scales=(h(15),))), ((u8(w8),), dict(fmts=(rows.INT8,), scales=(h(16).float(),))),
+                     ((u8(w8),), dict(fmts=(rows.INT8,))), ((u8(w4),), dict(fmts=(3,))),
+                     ((w,), dict(residuals=(h(1, 16),), epilogues=(_lib.EPI_ADD,))),
+                     ((w,), dict(residuals=(h(2, 16).float(),), epilogues=(_lib.EPI_ADD,))),
+                     ((w,), dict(outs=(h(2, 15),))), ((w,), dict(outs=(h(2, 32)[:, ::2],))), ((w, w), {})]:
+        with pytest.raises(ValueError):
+            rows.rows_gemv((x,), args, **{**ok, **kw})
+    assert rows.rows_gemv((x,), (w,), **ok)[0].shape == (2, 16)
+    # a layer step does not hand the kernel activations of another width than the projection's
+    m4 = hb.MM4Linear(torch.nn.Linear(128, 16, bias=False, device="cuda", dtype=torch.float16))
+    assert rows_projections((m4,), (h(2, 256),)) is None and rows_projections((m4,), (h(2, 1, 128),)) is None
+    assert rows_projections((m4,), (x,)) is not None
+    with pytest.raises(ValueError):
+        m4(h(2, 256))
