@@ -162,6 +162,10 @@ def _weight_of(op):
     return op if isinstance(op, torch.Tensor) else op.weight
 
 
+def _out_features(op):
+    return int(op.shape[0]) if isinstance(op, torch.Tensor) else int(op.out_features)
+
+
 def rkv_grouped(ops, xr, xk, xv):
     """r / k / v through one grouped launch when all three are int4 (or row-wise int8) projections of one shape that
     the tensor-core decode kernel takes; None otherwise."""
@@ -322,12 +326,15 @@ def block_ip_batched(x, state, xpa, xpf, v_first, p, sparse_ffn_out=None, fp16_e
     first = int(i) == 0
     downs, ups = ((w1, a1, g1), (w2, a2, g2)) if first else ((w1, a1, g1, v1), (w2, a2, g2, v2))
     down_x = (xw, xa, xg) if first else (xw, xa, xg, xv)
-    # a few rows: r / k / v and the LoRA "down" products in one launch, the "up" products in the next
-    few = rows_projections((Rw, Kw, Vw) + downs, (xr, xk, xv) + down_x,
-                           ([_lib.EPI_NONE] * 3 + [_lib.EPI_TANH, _lib.EPI_NONE, _lib.EPI_SIGMOID, _lib.EPI_NONE])[:3 + len(downs)])
-    lora = None if few is None else rows_projections(ups, few[3:])
-    if lora is not None:
+    # a few rows: r / k / v and the LoRA "down" products in one launch, the "up" products in the next (if they qualify: decided
+    # before the first launch, whose results would be thrown away)
+    few = None
+    if all(_rowsk.takes_weight(_weight_of(u), x.dtype) and int(_weight_of(u).shape[1]) == _out_features(d) for u, d in zip(ups, downs)):
+        few = rows_projections((Rw, Kw, Vw) + downs, (xr, xk, xv) + down_x,
+                               ([_lib.EPI_NONE] * 3 + [_lib.EPI_TANH, _lib.EPI_NONE, _lib.EPI_SIGMOID, _lib.EPI_NONE])[:3 + len(downs)])
+    if few is not None:
         r, k, v = few[:3]
+        lora = rows_projections(ups, few[3:])
     else:
         r, k, v, *lora = _wide_projections(ctx, x, (Rw, Kw, Vw), (xr, xk, xv), downs, ups, down_x)
     w_raw, a_pre, g = lora[:3]

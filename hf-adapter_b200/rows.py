@@ -18,10 +18,14 @@ MAX_PROBLEMS = 8
 def takes_dense(x, weight) -> bool:
     """``x @ weight.T`` with a dense weight: fp16 / bf16 CUDA operands of one dtype, contiguous and 16-byte aligned, few
     rows (anything else keeps its library GEMM)."""
-    return (x.is_cuda and weight.is_cuda and x.dtype == weight.dtype and x.dtype in (torch.float16, torch.bfloat16)
-            and weight.dim() == 2 and weight.is_contiguous() and x.is_contiguous() and int(x.shape[-1]) == int(weight.shape[1])
-            and weight.numel() > 0 and int(weight.shape[1]) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
-            and 1 <= x.numel() // int(weight.shape[1]) <= MAX_ROWS)
+    return (takes_weight(weight, x.dtype) and x.is_cuda and x.is_contiguous() and int(x.shape[-1]) == int(weight.shape[1])
+            and x.data_ptr() % 16 == 0 and 1 <= x.numel() // int(weight.shape[1]) <= MAX_ROWS)
+
+
+def takes_weight(weight, dtype) -> bool:
+    """The part of ``takes_dense`` that the weight decides, for activations of ``dtype``."""
+    return (weight.is_cuda and weight.dtype == dtype and dtype in (torch.float16, torch.bfloat16) and weight.dim() == 2
+            and weight.is_contiguous() and weight.numel() > 0 and int(weight.shape[1]) % 8 == 0 and weight.data_ptr() % 16 == 0)
 
 
 def _check_problem(i, x, w, N, fmt, scale, residual, out):

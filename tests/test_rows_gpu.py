@@ -94,3 +94,32 @@ def test_operands_of_the_wrong_size_are_refused_on_the_host():
     assert rows_projections((m4,), (x,)) is not None
     with pytest.raises(ValueError):
         m4(h(2, 256))
+
+
+@pytest.mark.parametrize("strided", [False, True])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_step_of_a_few_rows_is_the_step_of_many(strided, dt, monkeypatch):
+    """Rows of a batch of 8 against the same rows in a batch of 9, which other kernels compute.  A layer with a strided LoRA "up"
+    weight keeps the route of many rows, and nothing is launched for it and thrown away."""
+    cfg = hb.NativeRWKV7Config(vocab_size=128, hidden_size=256, num_hidden_layers=2, num_heads=4, head_dim=64, intermediate_size=512,
+                               decay_low_rank_dim=16, a_low_rank_dim=24, v_low_rank_dim=16, gate_low_rank_dim=32)
+    torch.manual_seed(9)
+    m = hb.RWKV7ForCausalLM(cfg).to(dt).cuda().eval()
+    if strided:
+        for layer in m.model.layers:
+            up = layer.attn.a_lora.lora[2]
+            up.weight = torch.nn.Parameter(up.weight.t().contiguous().t())
+    launches = []
+    real = rows.rows_gemv
+    monkeypatch.setattr(rows, "rows_gemv", lambda xs, *a, **k: (launches.append(len(xs)), real(xs, *a, **k))[1])
+    ids = torch.randint(0, 128, (9,), device="cuda")
+    caches = [m.new_cache(b) for b in (8, 9)]
+    for _ in range(3):
+        few, many = (m.rwkv7_forward_token(ids[:b], c, use_graph=False) for b, c in zip((8, 9), caches))
+    # r, k, v with the LoRA downs of a layer, then the ups
+    assert [n for n in launches if n > 1] == ([] if strided else [6, 3, 7, 4] * 3)
+    # two layers, three tokens: a few roundings to the activation type on either side
+    ulp = 2.0 ** -11 if dt == torch.float16 else 2.0 ** -8
+    for a, b in zip([few, *caches[0]._tensors()], [many, *caches[1]._tensors()]):
+        a, b = a.float(), b[:8].float() if b.shape[0] == 9 else b.float()
+        assert float((a - b).norm()) <= 4 * ulp * float(b.norm())
