@@ -65,7 +65,7 @@ def extract_graph_packs(model, *, rkv_policy: str = "", unused_as_zeros: bool = 
         vl = getattr(a, "v_lora", None)
         if vl is not None:
             v1, v2, v0 = graph_linear_operand(vl.lora[0]), vl.lora[2].weight, vl.lora[2].bias
-        elif not unused_as_zeros:
+        elif i == 0 and not unused_as_zeros:
             v1 = v2 = v0 = None
         else:
             v1 = torch.zeros(1, hidden, device=emb.device, dtype=emb.dtype)

@@ -1,0 +1,17 @@
+"""Pack tuples of a model on the CPU: which slots a step may leave empty."""
+import torch
+
+import hf_adapter_b200 as hb
+
+
+def test_only_slots_that_a_step_does_not_read_are_left_empty():
+    cfg = hb.NativeRWKV7Config(vocab_size=16, hidden_size=64, num_hidden_layers=3, num_heads=1, head_dim=64, intermediate_size=128,
+                               decay_low_rank_dim=8, a_low_rank_dim=8, v_low_rank_dim=8, gate_low_rank_dim=8)
+    m = hb.RWKV7ForCausalLM(cfg)
+    del m.model.layers[2].attn.v_lora  # its gate is then the one of zero weights, in either form of the packs
+    step, full = (hb.extract_graph_packs(m, unused_as_zeros=z)[0] for z in (False, True))
+    none = [[j for j, v in enumerate(p) if v is None] for p in step]
+    assert none == [[30, 31, 32], [5, 6], [5, 6]]  # layer 0's v LoRA; the pre-norm of the others
+    for a, b in zip(step, full):
+        assert all(x is None or not torch.is_tensor(x) or torch.equal(x, y) for x, y in zip(a, b))
+    assert not any(v is None for p in full for v in p)
