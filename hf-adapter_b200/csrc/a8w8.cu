@@ -4,6 +4,8 @@
 // This file holds the quantiser, the epilogue and a warp-level mma.sync (IMMA
 // m16n8k32) GEMM used for shapes the tcgen05 kernel (gemm_umma.cu) does not take
 // (ragged M/N/K) and as the comparison baseline for it.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace rwkv7 {
@@ -16,13 +18,19 @@ namespace rwkv7 {
 // Bound: HBM (3 bytes an fp16 element); the IEEE division per element was what it spent its time on, and registers for
 // eight chunks kept three CTAs on an SM.
 
+// bf16 rows hold few distinct quotients, which tie in some rows for many elements, and a warp with one tie forms 32
+// quotients after all: below this many rows (few CTAs an SM) bf16 divides without asking.  64 rows of 16384 / 10240 / 4096:
+// 8.72 / 6.32 / 3.60 us with the product, 6.28 / 4.64 / 2.93 without; 4096 rows of 4096: 16.9 us with it (34.7 without).
+constexpr int kA8RecipRows = 512;
+
 // The quotient only matters where it rounds: x * (1 / s) is within 1.5 * 2^-23 of x / s relative to it, less than 3e-5 for
 // |x / s| <= 127, so away from a rounding boundary by 1e-4 the product rounds like the IEEE quotient; nearer (and for
-// NaN) the quotient itself is formed.
+// NaN) the quotient itself is formed.  RECIP false: always.
+template <bool RECIP>
 __device__ __forceinline__ int8_t quant_one(float v, float s, float inv) {
     const float u = fabsf(v * inv) + 0.5f, f = floorf(u), d = u - f;
     float r = copysignf(f, v);
-    if (!(d >= 1e-4f && d <= 0.9999f)) {
+    if (!RECIP || !(d >= 1e-4f && d <= 0.9999f)) {
         const float t = __fdiv_rn(v, s);
         r = (t >= 0.f) ? floorf(t + 0.5f) : ceilf(t - 0.5f);
     }
@@ -30,7 +38,7 @@ __device__ __forceinline__ int8_t quant_one(float v, float s, float inv) {
     return (int8_t)(int)r;
 }
 
-template <typename T, int CHUNKS>
+template <typename T, int CHUNKS, bool RECIP>
 __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, int8_t* __restrict__ q,
                                                        float* __restrict__ scale, int K) {
     __shared__ float red[32];
@@ -38,18 +46,22 @@ __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, 
     const T* xr = x + row * K;
     Vec8<T> keep[CHUNKS];  // the row's chunks in their storage type: 4 registers per chunk for 16-bit inputs
     float amax = 0.f;
+    auto take = [&](int c) {
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-        const int k = (c * 256 + threadIdx.x) * 8;
-        if (k < K) keep[c] = *reinterpret_cast<const Vec8<T>*>(xr + k);
-    }
+        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(to_f<T>(keep[c].v[e])));
+    };
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
         const int k = (c * 256 + threadIdx.x) * 8;
         if (k < K) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(to_f<T>(keep[c].v[e])));
+            keep[c] = *reinterpret_cast<const Vec8<T>*>(xr + k);
+            if (!RECIP) take(c);
         }
+    }
+    if (RECIP) {
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c)
+            if ((c * 256 + threadIdx.x) * 8 < K) take(c);
     }
     for (int k = (CHUNKS * 256 + threadIdx.x) * 8; k < K; k += 256 * 8) {
         float v[8];
@@ -66,7 +78,7 @@ __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, 
         if (k < K) {
             alignas(8) int8_t o[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = quant_one(to_f<T>(keep[c].v[e]), s, inv);
+            for (int e = 0; e < 8; ++e) o[e] = quant_one<RECIP>(to_f<T>(keep[c].v[e]), s, inv);
             *reinterpret_cast<uint2*>(q + row * K + k) = *reinterpret_cast<const uint2*>(o);
         }
     }
@@ -75,7 +87,7 @@ __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, 
         load8(xr + k, v);
         alignas(8) int8_t o[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = quant_one(v[e], s, inv);
+        for (int e = 0; e < 8; ++e) o[e] = quant_one<RECIP>(v[e], s, inv);
         *reinterpret_cast<uint2*>(q + row * K + k) = *reinterpret_cast<const uint2*>(o);
     }
 }
@@ -272,8 +284,15 @@ extern "C" int rwkv7_a8_quant(const void* x, int8_t* q, float* scale, int rows, 
     RWKV7_REQUIRE(aligned(x, 16) && aligned(q, 8), RWKV7_ERR_ALIGN, "a8_quant: unaligned pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
-        if (K <= 2 * 256 * 8) a8_quant_kernel<T, 2><<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K);
-        else a8_quant_kernel<T, 8><<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K);
+        auto launch = [&](auto kern) { kern<<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K); };
+        const bool two = K <= 2 * 256 * 8;
+        if constexpr (sizeof(T) == 2 && !std::is_same<T, __half>::value) {
+            if (rows < kA8RecipRows) {
+                two ? launch(a8_quant_kernel<T, 2, false>) : launch(a8_quant_kernel<T, 8, false>);
+                return check_launch("a8_quant_kernel");
+            }
+        }
+        two ? launch(a8_quant_kernel<T, 2, true>) : launch(a8_quant_kernel<T, 8, true>);
         return check_launch("a8_quant_kernel");
     });
     return RWKV7_OK;
