@@ -28,6 +28,25 @@ def takes_weight(weight, dtype) -> bool:
             and weight.is_contiguous() and weight.numel() > 0 and int(weight.shape[1]) % 8 == 0 and weight.data_ptr() % 16 == 0)
 
 
+def prefers_dense(rows: int, K: int, N: int, fused: bool, early: bool) -> bool:
+    """Whether one dense product of ``rows`` rows on its own is faster here than as a library GEMM with pointwise kernels behind
+    it.  ``fused``: an epilogue rides in it; ``early``: its weights may be requested under the kernel before it.  Library
+    against this kernel in us, fp16, 1 / 8 rows:
+
+    * a short K leaves the reads of x and the epilogue: 64 -> 2560 2.2 against 2.1 / 4.6, + residual 3.6 against 2.3 / 6.0; 256 ->
+      2048 at 0.82 / 0.97 of the library's time, + residual 0.58 / 0.73;
+    * more channels than a wave of CTAs takes: 2560 -> 2560 8.5 against 5.6 / 6.0, but 2560 -> 10240 11.2 against 14.7 / 15.4 and
+      768 -> 32768 11.6 against 15.6 / 16.7; 1024 -> 8192 at 0.84 / 0.93 of the library, 4096 -> 5120 at 1.04 / 1.08, with the
+      residual 0.93 / 0.95;
+    * early, behind a norm kernel: 2560 -> 10240 + relu^2 17.0 against 16.1 / 17.1, 4096 -> 16384 32.8 against 27.8 / 28.5, 8192 ->
+      8192 28.7 against 27.3 / 28.2; but 5120 -> 20480 42.1 against 45.9 / 46.7 and 20480 -> 5120 + residual 48.2 against 51.3 / 53.1."""
+    if K < (32 if fused else 64) * rows or K * N > 1 << 26:
+        return False
+    if early:
+        return N <= 16384
+    return N <= 4096 or (N <= 8192 and (K <= 1024 or (fused and K * N <= 1 << 25)))
+
+
 def _check_problem(i, x, w, N, fmt, scale, residual, out):
     """The kernel takes sizes from ``x`` and ``N`` alone: every other operand has to hold as much."""
     M, K = (int(v) for v in x.shape)

@@ -15,3 +15,13 @@ def test_only_slots_that_a_step_does_not_read_are_left_empty():
     for a, b in zip(step, full):
         assert all(x is None or not torch.is_tensor(x) or torch.equal(x, y) for x, y in zip(a, b))
     assert not any(v is None for p in full for v in p)
+
+
+def test_dense_products_that_stay_on_the_library():
+    from hf_adapter_b200.rows import prefers_dense
+    # (rows, K, N, fused, early): each pair is the two sides of a line
+    for take, leave in [((4, 256, 2048, False, False), (4, 248, 2048, False, False)), ((8, 256, 2048, True, False), (8, 248, 2048, True, False)),
+                        ((1, 2560, 4096, False, False), (1, 2560, 4104, False, False)), ((1, 1024, 8192, False, False), (1, 1024, 8200, False, False)),
+                        ((8, 4096, 8192, True, False), (8, 4104, 8192, True, False)), ((8, 4096, 16384, True, True), (8, 4104, 16384, True, True)),
+                        ((8, 768, 16384, True, True), (8, 768, 16392, True, True)), ((1, 16384, 4096, True, False), (1, 20480, 5120, True, True))]:
+        assert prefers_dense(*take) and not prefers_dense(*leave)
