@@ -108,12 +108,23 @@ def w4_repack_tiled(q, scales, in_features, group_size=128, zeros=None):
     return tiled
 
 
-def few_rows_quant(rows: int, in_features: int) -> bool:
+def few_rows_quant(rows: int, in_features: int, out_features: int) -> bool:
     """Whether a tiled int4 / int8 projection of ``rows`` activation rows runs on the row kernel (csrc/row_gemv.cu) and not on
-    the tcgen05 one.  1 row, tcgen05 against rows: 4096 x 4096 int4 7.6 -> 5.6 us, int8 8.5 -> 6.7; 4096 -> 16384 17.2 -> 15.0 and
-    18.8 -> 17.1; 16384 -> 4096 15.2 -> 14.2 and 17.2 -> 16.0.  At 8 rows the activations weigh as much as the weights of a
-    long row: 16384 -> 4096 int4 14.7 against 16.7."""
-    return 1 <= rows <= _rowsk.MAX_ROWS and (rows <= 4 or in_features <= 10240)
+    the tcgen05 one.  At 8 rows the activations weigh as much as the weights of a long row, and few channels with a long row
+    leave SMs idle.  Time of the row kernel over the other's, int4 / int8, by rows:
+
+        4096 -> 4096    1 0.75 / 0.80   4 0.79 / 0.83   8 0.86 / 0.87
+        2560 -> 10240   1 0.89 / 1.00   5 0.87 / 1.00   8 0.90 / 1.06
+        4096 -> 16384   1 0.86 / 0.87   5 0.82 / 0.84   8 0.89 / 0.96
+        7168 -> 4096    1 0.89 / 0.90   5 0.99 / 0.94   8 0.86 / 0.80
+        8192 -> 8192    1 0.81 / 0.83   7 0.95 / 0.89   8 1.13 / 1.05
+        10240 -> 2560   1 0.84 / 0.83   5 0.98 / 0.88   6 1.05 / 0.96   8 1.09 / 1.00
+        12288 -> 8192   1 0.85 / 0.85   5 0.92 / 0.87   6 1.15 / 1.09   8 1.20 / 1.09
+        16384 -> 4096   1 0.73 / 0.77   3 0.87 / 0.85   4 1.04 / 1.04   8 1.15 / 1.07
+        8192 -> 1024    1 1.00 / 0.94   8 1.06 / 0.98
+        12288 -> 1024   1 1.19 / 1.14   8 1.20 / 1.16"""
+    most = 8 if in_features <= 7168 else 7 if in_features <= 8192 else 5 if in_features <= 12288 else 3
+    return 1 <= rows <= min(most, _rowsk.MAX_ROWS) and in_features < 8 * out_features
 
 
 def w4_tiled_linear(x, tiled, out_features, in_features, *, out=None, relu2: bool = False, residual=None):
@@ -124,7 +135,7 @@ def w4_tiled_linear(x, tiled, out_features, in_features, *, out=None, relu2: boo
     require_cuda(x2, tiled, what="w4_tiled_linear")
     epi, res = _epi(relu2, residual, M, Nout, x2)
     y = torch.empty((M, Nout), device=x2.device, dtype=x2.dtype) if out is None else out.reshape(M, Nout)
-    if few_rows_quant(M, K) and x2.dtype == torch.float16:
+    if few_rows_quant(M, K, Nout) and x2.dtype == torch.float16:
         _rowsk.rows_gemv((x2,), (tiled,), out_features=(Nout,), fmts=(_rowsk.INT4,), residuals=(res,), outs=(y,), epilogues=(epi,),
                          static_weights=True)
         return y.reshape(*x.shape[:-1], Nout)
@@ -146,7 +157,7 @@ def w4_tiled_linear_group(xs, tileds, out_features, in_features, *, relu2: bool 
         raise ValueError("grouped projections need the same row count and dtype")
     require_cuda(*x2, *tileds, what="w4_tiled_linear_group")
     ys = [torch.empty((M, Nout), device=x2[0].device, dtype=x2[0].dtype) for _ in range(G)]
-    if few_rows_quant(M, K) and x2[0].dtype == torch.float16:
+    if few_rows_quant(M, K, Nout) and x2[0].dtype == torch.float16:
         _rowsk.rows_gemv(x2, tileds, out_features=[Nout] * G, fmts=[_rowsk.INT4] * G, outs=ys,
                          epilogues=[_lib.EPI_RELU2 if relu2 else _lib.EPI_NONE] * G, static_weights=True)
         return [y.reshape(*x.shape[:-1], Nout) for y, x in zip(ys, xs)]
@@ -188,7 +199,7 @@ def w8_tiled_linear_group(xs, tileds, scales, out_features, in_features, *, relu
     if (res is not None or out is not None) and G != 1:
         raise ValueError("residual / out apply to a single projection")
     ys = [torch.empty((M, Nout), device=x2[0].device, dtype=x2[0].dtype) if out is None else out.reshape(M, Nout) for _ in range(G)]
-    if few_rows_quant(M, K) and x2[0].dtype == torch.float16 and all(t.is_contiguous() for t in x2):
+    if few_rows_quant(M, K, Nout) and x2[0].dtype == torch.float16 and all(t.is_contiguous() for t in x2):
         _rowsk.rows_gemv(x2, tileds, out_features=[Nout] * G, fmts=[_rowsk.INT8] * G, scales=sc, residuals=[res] * G, outs=ys,
                          epilogues=[epi] * G, static_weights=True)
         return [y.reshape(*x.shape[:-1], Nout) for y, x in zip(ys, xs)]

@@ -25,3 +25,10 @@ def test_dense_products_that_stay_on_the_library():
                         ((8, 4096, 8192, True, False), (8, 4104, 8192, True, False)), ((8, 4096, 16384, True, True), (8, 4104, 16384, True, True)),
                         ((8, 768, 16384, True, True), (8, 768, 16392, True, True)), ((1, 16384, 4096, True, False), (1, 20480, 5120, True, True))]:
         assert prefers_dense(*take) and not prefers_dense(*leave)
+
+
+def test_quantised_products_on_the_row_kernel():
+    from hf_adapter_b200.quant import few_rows_quant
+    for K, N, most in [(128, 24, 8), (128, 16, 0), (7168, 4096, 8), (7296, 4096, 7), (8192, 1032, 7), (8320, 8192, 5), (12288, 8192, 5), (12416, 8192, 3),
+                       (16384, 4096, 3), (12288, 1024, 0)]:
+        assert [m for m in range(10) if few_rows_quant(m, K, N)] == list(range(1, most + 1))
