@@ -92,7 +92,8 @@ struct Mix6Args {
     const int* slots;  // state pool: the shift state of batch row b is row slots[b] of `prev`; NULL = row b
 };
 
-template <typename T, int NV>
+// EARLY: the shift state is requested with the row, not after its statistics (see row_prev_early)
+template <typename T, int NV, bool EARLY>
 __global__ void __launch_bounds__(kNMThreads) attn_norm_mix6_kernel(const Mix6Args p) {
     __shared__ float red[64];
     const size_t row = blockIdx.x;
@@ -114,11 +115,13 @@ __global__ void __launch_bounds__(kNMThreads) attn_norm_mix6_kernel(const Mix6Ar
     grid_dependency_wait();
     if (threadIdx.x == 0) grid_launch_dependents();
     T* prev = reinterpret_cast<T*>(p.prev) + (p.slots ? (size_t)__ldg(p.slots + row) : row) * D;
-    Raw8<T> cp[NV];  // the shift state is requested with the row, not after its statistics
+    Raw8<T> cp[EARLY ? NV : 1];
+    if constexpr (EARLY) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int vi = threadIdx.x + i * kNMThreads;
-        if (vi < nvec) cp[i] = ld_raw8(prev + vi * 8);
+        for (int i = 0; i < NV; ++i) {
+            const int vi = threadIdx.x + i * kNMThreads;
+            if (vi < nvec) cp[i] = ld_raw8(prev + vi * 8);
+        }
     }
     RowStats<T, NV> rs;
     load_row_stats<T, false, NV>(reinterpret_cast<const T*>(p.x) + row * D, nullptr, nullptr, D, p.eps, rs, red);
@@ -129,7 +132,8 @@ __global__ void __launch_bounds__(kNMThreads) attn_norm_mix6_kernel(const Mix6Ar
             float w[8], b[8], pv[8], h[8], d[8];
             cvt8(cw[i], w);
             cvt8(cb[i], b);
-            cvt8(cp[i], pv);
+            if constexpr (EARLY) cvt8(cp[i], pv);
+            else load8(prev + vi * 8, pv);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 h[e] = (rs.x[i][e] - rs.mean) * rs.rstd * w[e] + b[e];
@@ -158,7 +162,7 @@ struct FfnMixArgs {
 
 // ADD: x = res + attn (stored to res_out; normalised from the fp32 sum like the reference's fused kernel)
 // MIX: emit mixed + update prev; otherwise plain LayerNorm into `mixed`.
-template <typename T, bool ADD, bool MIX, int NV>
+template <typename T, bool ADD, bool MIX, int NV, bool EARLY>
 __global__ void __launch_bounds__(kNMThreads) ffn_add_norm_mix_kernel(const FfnMixArgs p) {
     __shared__ float red[64];
     const size_t row = blockIdx.x;
@@ -177,9 +181,9 @@ __global__ void __launch_bounds__(kNMThreads) ffn_add_norm_mix_kernel(const FfnM
     grid_dependency_wait();
     if (threadIdx.x == 0) grid_launch_dependents();
     T* prev = nullptr;
-    Raw8<T> cp[MIX ? NV : 1];
-    if constexpr (MIX) {
-        prev = reinterpret_cast<T*>(p.prev) + (p.slots ? (size_t)__ldg(p.slots + row) : row) * D;
+    Raw8<T> cp[MIX && EARLY ? NV : 1];
+    if constexpr (MIX) prev = reinterpret_cast<T*>(p.prev) + (p.slots ? (size_t)__ldg(p.slots + row) : row) * D;
+    if constexpr (MIX && EARLY) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int vi = threadIdx.x + i * kNMThreads;
@@ -201,7 +205,8 @@ __global__ void __launch_bounds__(kNMThreads) ffn_add_norm_mix_kernel(const FfnM
             for (int e = 0; e < 8; ++e) h[e] = (rs.x[i][e] - rs.mean) * rs.rstd * w[e] + b[e];
             if constexpr (MIX) {
                 float pv[8], mx[8], o[8];
-                cvt8(cp[i], pv);
+                if constexpr (EARLY) cvt8(cp[i], pv);
+                else load8(prev + vi * 8, pv);
                 cvt8(cm[i], mx);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) o[e] = h[e] + (pv[e] - h[e]) * mx[e];
@@ -264,6 +269,18 @@ static void with_row_vectors(int D, F f) {
     else f(std::integral_constant<int, kNMMaxVec>());
 }
 
+// f(EARLY) for a kernel on elements of T: fp32 rows of a few batch rows read the shift state after the statistics, because its
+// registers on top of the row's and the parameters' only spill there (8192 wide, 64 rows: mix of six 11.0 us early, 9.9 late;
+// 8 rows add + norm + mix 5.4 and 5.0); with many rows the earlier request wins all the same (4096 wide, 4096 rows: 77 us
+// against 266).
+template <typename T, typename F>
+static void row_prev_early(int rows, F f) {
+    if constexpr (sizeof(T) == 4) {
+        if (rows < 512) return f(std::false_type());
+    }
+    f(std::true_type());
+}
+
 static int check_row_shape(const char* what, int rows, int D) {
     RWKV7_REQUIRE(rows > 0 && D > 0, RWKV7_ERR_INVALID, "%s: rows and D must be positive", what);
     RWKV7_REQUIRE(D % 8 == 0 && D <= 8 * kNMThreads * kNMMaxVec, RWKV7_ERR_UNSUPPORTED,
@@ -292,7 +309,11 @@ static int attn_norm_mix6_impl(const void* x, void* prev, const int32_t* slots, 
                   "attn_norm_mix6: unaligned pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
-        with_row_vectors(D, [&](auto nv) { launch_programmatic(attn_norm_mix6_kernel<T, decltype(nv)::value>, dim3(rows), dim3(kNMThreads), 0, st, p); });
+        row_prev_early<T>(rows, [&](auto early) {
+            with_row_vectors(D, [&](auto nv) {
+                launch_programmatic(attn_norm_mix6_kernel<T, decltype(nv)::value, decltype(early)::value>, dim3(rows), dim3(kNMThreads), 0, st, p);
+            });
+        });
         return check_launch("attn_norm_mix6_kernel");
     });
     return RWKV7_OK;
@@ -323,8 +344,14 @@ static int ffn_add_norm_mix_impl(const void* residual, const void* attn_out, voi
     FfnMixArgs p{residual, attn_out, norm_w, norm_b, mix, prev, residual_out, mixed, D, eps, slots};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
-        if (attn_out) with_row_vectors(D, [&](auto nv) { launch_programmatic(ffn_add_norm_mix_kernel<T, true, true, decltype(nv)::value>, dim3(rows), dim3(kNMThreads), 0, st, p); });
-        else with_row_vectors(D, [&](auto nv) { launch_programmatic(ffn_add_norm_mix_kernel<T, false, true, decltype(nv)::value>, dim3(rows), dim3(kNMThreads), 0, st, p); });
+        row_prev_early<T>(rows, [&](auto early) {
+            with_row_vectors(D, [&](auto nv) {
+                constexpr int NV = decltype(nv)::value;
+                constexpr bool E = decltype(early)::value;
+                if (attn_out) launch_programmatic(ffn_add_norm_mix_kernel<T, true, true, NV, E>, dim3(rows), dim3(kNMThreads), 0, st, p);
+                else launch_programmatic(ffn_add_norm_mix_kernel<T, false, true, NV, E>, dim3(rows), dim3(kNMThreads), 0, st, p);
+            });
+        });
         return check_launch("ffn_add_norm_mix_kernel");
     });
     return RWKV7_OK;
@@ -355,7 +382,7 @@ extern "C" int rwkv7_layer_norm(const void* x, const void* norm_w, const void* n
     FfnMixArgs p{x, nullptr, norm_w, norm_b, nullptr, nullptr, nullptr, out, D, eps, nullptr};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
-        with_row_vectors(D, [&](auto nv) { launch_programmatic(ffn_add_norm_mix_kernel<T, false, false, decltype(nv)::value>, dim3(rows), dim3(kNMThreads), 0, st, p); });
+        with_row_vectors(D, [&](auto nv) { launch_programmatic(ffn_add_norm_mix_kernel<T, false, false, decltype(nv)::value, true>, dim3(rows), dim3(kNMThreads), 0, st, p); });
         return check_launch("layer_norm_kernel");
     });
     return RWKV7_OK;

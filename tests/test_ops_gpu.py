@@ -245,6 +245,23 @@ def test_norm_mix_lora_prep_against_golden(dt):
     np.testing.assert_allclose(npf(op), g["op_out"].astype(np.float32), **tol(dt, 5))
 
 
+@pytest.mark.parametrize("D", [64, 2048, 2056, 4104, 8192])
+def test_norm_mix_rows_do_not_depend_on_their_number(D):
+    """fp32 reads the shift state after the row statistics below 512 rows and with the row from there on: the same bits."""
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    f = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    x, attn, prev, w, b, mixes = f(512, D), f(512, D), f(512, D), f(D), f(D), [f(D) for _ in range(6)]
+    got = []
+    for n in (512, 511):
+        p1, p2 = prev[:n].clone(), prev[:n].clone()
+        got.append([*hb.fused_attn_norm_mix6_decode(x[:n], p1, w, b, *mixes),
+                    *hb.fused_ffn_add_norm_mix_decode(x[:n], attn[:n], p2, w, b, mixes[0]), p1, p2])
+    assert all(torch.equal(a[:511], c) for a, c in zip(*got))
+    h = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double(), 1e-5)
+    # fp32 sums of up to 8192 terms and a cancelling centre: 1e-5 of the largest value is some 80 ulp
+    assert float((got[0][0].double() - (h + (prev - h) * mixes[0].double())).abs().max()) < 1e-5 * float(got[0][0].abs().max())
+
+
 @pytest.mark.parametrize("rows,D", [(1, 8), (5, 768), (64, 4096), (3, 8192)])
 def test_norm_mix_shapes(rows, D):
     rng = np.random.default_rng(D)
