@@ -1,6 +1,9 @@
 """Host-side helpers shared by the operator wrappers."""
 from __future__ import annotations
 
+import contextlib
+import gc
+
 import torch
 
 from . import _lib
@@ -46,3 +49,17 @@ def ptr(t):
 def no_fallback(force_fallback: bool, what: str) -> None:
     if force_fallback:
         raise RuntimeError(f"{what}: force_fallback=True requests the pure-PyTorch path, which this package does not ship")
+
+
+@contextlib.contextmanager
+def capture(graph):
+    """``torch.cuda.graph(graph)`` with the cyclic collector held off: a model that was dropped leaves its own graphs in a
+    reference cycle, and a graph that the collector destroys in the middle of a capture invalidates that capture."""
+    on = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.graph(graph):
+            yield
+    finally:
+        if on:
+            gc.enable()

@@ -32,6 +32,7 @@ from . import packing as _pk
 from . import prep as _prep
 from . import recurrent as _rec
 from . import sharding as _sh
+from ._util import capture
 from .cache import NativeRWKV7Cache
 
 
@@ -694,7 +695,7 @@ class DecodeGraph:
         torch.cuda.current_stream(dev).wait_stream(side)
         self.cache.reset()
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
+        with capture(self.graph):
             self.logits = model._decode_step(self.ids, self.cache, greedy)
 
     def _static(self):
@@ -754,7 +755,7 @@ class PrefillGraph:
         torch.cuda.current_stream(dev).wait_stream(side)
         self.cache.reset()
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
+        with capture(self.graph):
             self.logits = model._prefill(self.ids, self.cache, keep=self.keep, scan_chunk=scan_chunk)
         self.cache.reset()
 

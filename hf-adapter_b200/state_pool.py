@@ -23,6 +23,7 @@ import torch
 
 from . import norm_mix as _nm
 from . import packing as _pk
+from ._util import capture
 from .cache import NativeRWKV7Cache
 
 
@@ -363,7 +364,7 @@ class PoolDecodeGraph:
         torch.cuda.current_stream(dev).wait_stream(stream)
         torch.cuda.synchronize(dev)
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
+        with capture(self.graph):
             self.out = pool._step(self.ids, self.slots, greedy)
 
     def replay(self, ids, slot_vec):

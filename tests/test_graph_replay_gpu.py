@@ -5,6 +5,7 @@ start under the tail of the one before them (programmatic edges) and wait for it
 ONE predecessor: a node that joins branches has to have full edges."""
 import collections
 import ctypes
+import gc
 
 import pytest
 import torch
@@ -95,3 +96,29 @@ def test_replays_of_a_state_agree(weights, D, batch, state):
             first[i % 2] = [t.clone() for t in got]
         assert all(torch.equal(a, b) for a, b in zip(got, first[i % 2])), f"replay {i // 2} of state {i % 2}"
     assert not torch.equal(first[0][0], first[1][0])
+
+
+def test_a_dropped_model_does_not_break_the_next_capture(monkeypatch):
+    """A dropped model is a reference cycle that holds its graphs; the collector becomes due in the middle of a capture."""
+    from hf_adapter_b200 import packing
+    calls, real, threshold = [], packing.extract_graph_packs, gc.get_threshold()
+
+    def due(*a, **k):
+        calls.append(0)
+        if len(calls) == 3:  # two warm-up steps, then the captured one
+            gc.set_threshold(1)
+            calls.extend([] for _ in range(1000))
+        return real(*a, **k)
+
+    ids = torch.zeros(1, device="cuda", dtype=torch.long)
+    try:
+        gc.set_threshold(10 ** 9)
+        old = _model("dense", 256, 1)
+        old.rwkv7_forward_token(ids, old.new_cache(1))
+        del old
+        m = _model("dense", 256, 1)
+        monkeypatch.setattr(packing, "extract_graph_packs", due)
+        out = m.rwkv7_forward_token(ids, m.new_cache(1))
+        assert len(calls) > 1000 and gc.isenabled() and bool(torch.isfinite(out).all())
+    finally:
+        gc.set_threshold(*threshold)
