@@ -283,10 +283,20 @@ def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
         main.wait_stream(side)
         main.wait_stream(sk)
         main.wait_stream(sv)
-        xk.record_stream(sk); k.record_stream(sk); xv.record_stream(sv); v.record_stream(sv)
-    for t_ in (*down_x, *lora):
+        xk.record_stream(sk); xv.record_stream(sv)
+        _used_on(main, k, v)
+    for t_ in down_x:
         t_.record_stream(side)
+    _used_on(main, *lora)
     return [r, k, v, *lora]
+
+
+def _used_on(stream, *ts):
+    """Results allocated on a branch and used on ``stream``: their memory waits for that use.  (Not under capture: the pool is
+    the graph's own there, and every branch of a later layer starts behind the stream that used them.)"""
+    if not torch.cuda.is_current_stream_capturing():
+        for t in ts:
+            t.record_stream(stream)
 
 
 def block_ip_batched(x, state, xpa, xpf, v_first, p, sparse_ffn_out=None, fp16_elapsed=None,

@@ -122,3 +122,24 @@ def test_a_dropped_model_does_not_break_the_next_capture(monkeypatch):
         assert len(calls) > 1000 and gc.isenabled() and bool(torch.isfinite(out).all())
     finally:
         gc.set_threshold(*threshold)
+
+
+def test_branch_results_outlive_their_use_on_the_main_stream():
+    """Outside capture: memory of results that a branch allocated is not handed out again while the stream they were made for is
+    still busy with them."""
+    from hf_adapter_b200 import packing
+    D, B, R = 256, 16, 32
+    f = lambda *s: torch.randn(*s, device="cuda", dtype=torch.float16)
+    ops, downs, ups = [f(D, D) for _ in range(3)], [f(R, D) for _ in range(4)], [f(D, R) for _ in range(4)]
+    ctx, main = packing.StepContext(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(main):
+        res = packing._wide_projections(ctx, f(B, D), ops, [f(B, D) for _ in range(3)], downs, ups, [f(B, D) for _ in range(4)])
+        torch.cuda._sleep(200_000_000)  # a tenth of a second in which the results are "in use"
+        used = {t.data_ptr() for t in res}
+        del res
+        for i in range(3):
+            with torch.cuda.stream(ctx.side_stream(torch.device("cuda", torch.cuda.current_device()), i)):
+                again = [torch.empty(B, D, device="cuda", dtype=torch.float16) for _ in range(8)]
+            assert not main.query() and not used & {t.data_ptr() for t in again}
+    torch.cuda.synchronize()
