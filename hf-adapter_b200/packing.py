@@ -140,7 +140,8 @@ def apply_linear(op, x, *, relu2=False, residual=None, out=None, static=False):
         return _gemm.dense_linear(x, weight, bias, relu2=relu2, residual=residual, out=out)
     N = int(weight.shape[0])
     whole = lambda t: t is None or (t.dtype == x.dtype and t.is_contiguous() and t.numel() == rows * N)
-    if (bias is None and _rowsk.takes_dense(x, weight) and whole(residual) and whole(out)
+    if (bias is None and rows <= _rowsk.MAX_ROWS and not _rowsk.followed(*(t for t in (x, weight, residual) if t is not None))
+            and _rowsk.takes_dense(x, weight) and whole(residual) and whole(out)
             and _rowsk.prefers_dense(rows, int(weight.shape[1]), N, relu2 or residual is not None, static)):
         epi = _lib.EPI_RELU2 if relu2 else _lib.EPI_ADD if residual is not None else _lib.EPI_NONE
         y, = _rowsk.rows_gemv((x.reshape(rows, -1),), (weight,), out_features=(N,), fmts=(_rowsk.DENSE,), epilogues=(epi,),

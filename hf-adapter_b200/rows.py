@@ -6,6 +6,8 @@ from __future__ import annotations
 import ctypes
 
 import torch
+from torch.autograd import forward_ad
+from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 from . import _lib
 from ._util import dt_code, ptr, require_cuda, stream_ptr
@@ -26,6 +28,14 @@ def takes_weight(weight, dtype) -> bool:
     """The part of ``takes_dense`` that the weight decides, for activations of ``dtype``."""
     return (weight.is_cuda and weight.dtype == dtype and dtype in (torch.float16, torch.bfloat16) and weight.dim() == 2
             and weight.is_contiguous() and weight.numel() > 0 and int(weight.shape[1]) % 8 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def followed(*ts) -> bool:
+    """Whether more than the values of ``ts`` counts: a gradient or tangent to propagate, a functorch transform, a trace, a
+    dispatch mode, a tensor subclass.  A kernel behind ctypes is opaque to all of these; a library GEMM is not."""
+    return ((torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or forward_ad._current_level >= 0
+            or torch._C._are_functorch_transforms_active() or torch.jit.is_tracing() or torch.compiler.is_compiling()
+            or _get_current_dispatch_mode() is not None or any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in ts))
 
 
 def prefers_dense(rows: int, K: int, N: int, fused: bool, early: bool) -> bool:

@@ -123,3 +123,27 @@ def test_step_of_a_few_rows_is_the_step_of_many(strided, dt, monkeypatch):
     for a, b in zip([few, *caches[0]._tensors()], [many, *caches[1]._tensors()]):
         a, b = a.float(), b[:8].float() if b.shape[0] == 9 else b.float()
         assert float((a - b).norm()) <= 4 * ulp * float(b.norm())
+
+
+def test_products_that_something_follows_stay_visible():
+    """Gradients, tangents, vmap and traces of a dense product of a few rows: those of the library GEMM, which it then is."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from hf_adapter_b200.packing import apply_linear
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    f = lambda *s: torch.randn(*s, generator=gen, device="cuda").half()
+    x, w, res, t = f(4, 256), f(64, 256), f(4, 64), f(4, 256)
+    plain = lambda a, b: torch.nn.functional.linear(a, b) + res
+    ours = lambda a, b: apply_linear(b, a, residual=res)
+    grads = []
+    for fn in (plain, ours):
+        a, b = x.clone().requires_grad_(), w.clone().requires_grad_()
+        fn(a, b).float().square().sum().backward()
+        grads.append((a.grad, b.grad))
+    assert all(torch.equal(p, q) for p, q in zip(*grads))
+    assert all(torch.equal(p, q) for p, q in zip(*(torch.func.jvp(lambda a: fn(a, w), (x,), (t,)) for fn in (plain, ours))))
+    x3 = f(3, 4, 256)
+    assert torch.equal(*(torch.func.vmap(lambda a: fn(a, w))(x3) for fn in (plain, ours)))
+    g = make_fx(lambda a: ours(a, w))(x)
+    assert torch.equal(g(t), plain(t, w))
+    with torch.no_grad():  # nothing follows: one rounding of the product, one of the sum
+        _close(ours(x, w), (x.double() @ w.double().t()).float() + res.float(), torch.float16, (x.double() @ w.double().t()).float())
