@@ -122,7 +122,8 @@ def apply_linear(op, x, *, relu2=False, residual=None, out=None, static=False):
     """Apply a projection operand of the pack: a quantised module (epilogues fused through its rwkv7_forward_* hooks,
     as the reference's dispatch probes them: rwkv7_hf/native_jit_graph_dispatch.py:487-523), a dense ``[out,in]``
     weight tensor, or an ``nn.Linear`` (fp16 / bf16: this library's GEMM from 64 rows up, its row kernel up to 8; else
-    one library GEMM).  ``static``: the kernel launched just before on this stream does not write a dense weight."""
+    one library GEMM).  ``static``: a call of a layer step, where the kernel launched just before on this stream does not write
+    a dense weight."""
     if isinstance(op, _QUANT_TYPES):
         if relu2:
             if hasattr(op, "rwkv7_forward_relu2"):
@@ -140,7 +141,9 @@ def apply_linear(op, x, *, relu2=False, residual=None, out=None, static=False):
         return _gemm.dense_linear(x, weight, bias, relu2=relu2, residual=residual, out=out)
     N = int(weight.shape[0])
     whole = lambda t: t is None or (t.dtype == x.dtype and t.is_contiguous() and t.numel() == rows * N)
-    if (bias is None and rows <= _rowsk.MAX_ROWS and not _rowsk.followed(*(t for t in (x, weight, residual) if t is not None))
+    # (inside a layer step, which is opaque to autograd and traces as a whole, nothing is there to follow)
+    seen = not static and rows <= _rowsk.MAX_ROWS and _rowsk.followed(*(t for t in (x, weight, residual) if t is not None))
+    if (bias is None and not seen
             and _rowsk.takes_dense(x, weight) and whole(residual) and whole(out)
             and _rowsk.prefers_dense(rows, int(weight.shape[1]), N, relu2 or residual is not None, static)):
         epi = _lib.EPI_RELU2 if relu2 else _lib.EPI_ADD if residual is not None else _lib.EPI_NONE
