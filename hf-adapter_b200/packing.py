@@ -143,8 +143,7 @@ def apply_linear(op, x, *, relu2=False, residual=None, out=None, static=False):
     whole = lambda t: t is None or (t.dtype == x.dtype and t.is_contiguous() and t.numel() == rows * N)
     # (inside a layer step, which is opaque to autograd and traces as a whole, nothing is there to follow)
     seen = not static and rows <= _rowsk.MAX_ROWS and _rowsk.followed(*(t for t in (x, weight, residual) if t is not None))
-    if (bias is None and not seen
-            and _rowsk.takes_dense(x, weight) and whole(residual) and whole(out)
+    if (bias is None and not seen and _rowsk.takes_dense(x, weight) and whole(residual) and whole(out)
             and _rowsk.prefers_dense(rows, int(weight.shape[1]), N, relu2 or residual is not None, static)):
         epi = _lib.EPI_RELU2 if relu2 else _lib.EPI_ADD if residual is not None else _lib.EPI_NONE
         y, = _rowsk.rows_gemv((x.reshape(rows, -1),), (weight,), out_features=(N,), fmts=(_rowsk.DENSE,), epilogues=(epi,),

@@ -89,7 +89,7 @@ def test_operands_of_the_wrong_size_are_refused_on_the_host():
             rows.rows_gemv((x,), args, **{**ok, **kw})
     assert rows.rows_gemv((x,), (w,), **ok)[0].shape == (2, 16)
     # a layer step does not hand the kernel activations of another width than the projection's
-    m4 = hb.MM4Linear(torch.nn.Linear(128, 16, bias=False, device="cuda", dtype=torch.float16))
+    m4 = hb.MM4Linear(torch.nn.Linear(128, 32, bias=False, device="cuda", dtype=torch.float16))
     assert rows_projections((m4,), (h(2, 256),)) is None and rows_projections((m4,), (h(2, 1, 128),)) is None
     assert rows_projections((m4,), (x,)) is not None
     with pytest.raises(ValueError):
@@ -147,3 +147,29 @@ def test_products_that_something_follows_stay_visible():
     assert torch.equal(g(t), plain(t, w))
     with torch.no_grad():  # nothing follows: one rounding of the product, one of the sum
         _close(ours(x, w), (x.double() @ w.double().t()).float() + res.float(), torch.float16, (x.double() @ w.double().t()).float())
+
+
+@pytest.mark.parametrize("rows_,rank,dt", [(1, 24, torch.float16), (1024, 24, torch.bfloat16), (1025, 24, torch.float16), (8192, 24, torch.float16),
+                                           (8193, 24, torch.bfloat16), (70, 20, torch.float16), (70, 24, torch.float32)])
+@pytest.mark.parametrize("first", [False, True])
+def test_prefill_lora_pairs(rows_, rank, dt, first):
+    """Either side of the row counts up to which the pairs are grouped launches, a rank that those do not take, fp32."""
+    from hf_adapter_b200.model import NativeRWKV7Attention, _prefill_lora
+    cfg = hb.NativeRWKV7Config(vocab_size=16, hidden_size=128, num_hidden_layers=2, num_heads=2, head_dim=64, intermediate_size=256,
+                               decay_low_rank_dim=64, a_low_rank_dim=rank, v_low_rank_dim=16, gate_low_rank_dim=72)
+    torch.manual_seed(rows_ + rank)
+    at = NativeRWKV7Attention(cfg, 1).cuda().to(dt)
+    xs = [torch.randn(1, rows_, 128, device="cuda").to(dt) for _ in range(4)]
+    with torch.no_grad():
+        got = _prefill_lora(at, xs[0], xs[1], xs[2], None if first else xs[3])
+        assert len(got) == 4 and (got[3] is None) == first
+        same = lambda t: t
+        for y, lora, x, act in zip(got, (at.w_lora, at.a_lora, at.g_lora, at.v_lora), xs, (torch.tanh, same, torch.sigmoid, same)):
+            if y is None:
+                continue
+            l = lora.lora.double()
+            want = l[2](act(l[0](x.double())))
+            lora.to(dt)
+            # the hidden value is rounded twice, the result once: each at most half an ulp of its size
+            half_ulp = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -20}[dt]
+            assert y.shape == want.shape and float((y.double() - want).norm()) <= 2 * half_ulp * float(want.norm())
