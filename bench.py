@@ -729,8 +729,9 @@ def main():
                 us4 = time_graph(lambda: [hb.w4_tiled_linear(x, t, Nout, K) for t in tiled], nbuf, reps=5)
                 us8 = time_graph(lambda: [hb.w8_tiled_linear_group((x,), (t,), (s8,), Nout, K) for t in t8], nbuf, reps=5)
                 b4, b8 = w4_launch_bytes(M, K, Nout), w8_launch_bytes(M, K, Nout)
-                entry = {"int4_g128_tcgen05": {"us": us4, "gbs": b4 / us4 / 1e3, "frac": b4 / us4 / 1e3 / hbm_peak},
-                         "int8_per_channel_tcgen05": {"us": us8, "gbs": b8 / us8 / 1e3, "frac": b8 / us8 / 1e3 / hbm_peak}}
+                kernel = "rows" if hb.quant.few_rows_quant(M, K, Nout) else "tcgen05"  # which of the two streams the weights
+                entry = {"kernel": kernel, "int4_g128": {"us": us4, "gbs": b4 / us4 / 1e3, "frac": b4 / us4 / 1e3 / hbm_peak},
+                         "int8_per_channel": {"us": us8, "gbs": b8 / us8 / 1e3, "frac": b8 / us8 / 1e3 / hbm_peak}}
                 if M == 1:  # the CUDA-core GEMV on the reference layout, the small-batch route of w8_linear
                     usg = time_graph(lambda: [hb.w8_linear(x, q, s8) for q in q8], nbuf, reps=5)
                     entry["int8_per_channel_gemv"] = {"us": usg, "gbs": b8 / usg / 1e3, "frac": b8 / usg / 1e3 / hbm_peak}

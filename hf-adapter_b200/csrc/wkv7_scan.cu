@@ -402,8 +402,8 @@ static int launch_scan(const ScanArgs& p, int B, cudaStream_t st) {
 template <typename T, bool PREP>
 static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     // Chosen by how many CTAs an SM gets.  Up to one: the serial chain of a token is all there is, so the rows are spread
-    // over four warps (64 FMAs a thread and token less than the 2 x 32 tile) and loads / conversion / output run on
-    // warps of their own: 242 us for 120 CTAs x 777 tokens against 391 without.  Up to two: the tile with the fewer
+    // over four warps (160 multiply-adds a thread and token, 80 packed, where the 2 x 32 tile has 320) and loads /
+    // conversion / output run on warps of their own: 242 us for 120 CTAs x 777 tokens against 391 without.  Up to two: the tile with the fewer
     // operand reads, still with the extra warps (335 us against 401 for 240 CTAs x 777).  More: six CTAs a SM hide each
     // other's loads and the extra warps only take registers (2211 us against 3159 for 4096 CTAs x 512).
     const int ctas = B * p.H;
