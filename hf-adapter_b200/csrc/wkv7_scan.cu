@@ -403,9 +403,11 @@ template <typename T, bool PREP>
 static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     // Chosen by how many CTAs an SM gets.  Up to one: the serial chain of a token is all there is, so the rows are spread
     // over four warps (160 multiply-adds a thread and token, 80 packed, where the 2 x 32 tile has 320) and loads /
-    // conversion / output run on warps of their own: 242 us for 120 CTAs x 777 tokens against 391 without.  Up to two: the tile with the fewer
-    // operand reads, still with the extra warps (335 us against 401 for 240 CTAs x 777).  More: six CTAs a SM hide each
-    // other's loads and the extra warps only take registers (2211 us against 3159 for 4096 CTAs x 512).
+    // conversion / output run on warps of their own: 242 us for 120 CTAs x 777 tokens against 391 without.  Up to two: the
+    // tile with the fewer operand reads, still with the extra warps (335 us against 401 for 240 CTAs x 777).  More: the CTAs
+    // of an SM hide each other's loads and the extra warps only take registers (2211 us against 3159 for 4096 CTAs x 512).
+    // The three forms in this order, us for 512 tokens, fp16, output prepared: 148 CTAs 158 / 199 / 247, 149 235 / 215 / 250,
+    // 296 235 / 215 / 263, 297 379 / 409 / 370, 448 464 / 426 / 377, 600 602 / 635 / 512, 896 824 / 846 / 697, 2048 1606 / 1486 / 1164.
     const int ctas = B * p.H;
     if (ctas <= kSMs) return launch_scan<T, PREP, 1, 32, true>(p, B, st);
     if (ctas <= 2 * kSMs) return launch_scan<T, PREP, 4, 16, true>(p, B, st);
