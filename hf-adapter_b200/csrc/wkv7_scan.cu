@@ -7,7 +7,9 @@
 // packed pairs; 160 cycles of an SM's FMA pipe per token and head, measured 308 (64 sequences x 512 tokens x 64 heads,
 // fp16, output prepared: 2.21 ms, 6.04 ms with one row half per thread, unpacked, and the conversion in the chain).  Few
 // CTAs are bound by the latency of a token's chain instead: 120 CTAs x 777 tokens 242 us (772 us).  Operands come from
-// shared memory as 16-byte reads that the lanes of a row group share: one 128-byte segment per instruction.
+// shared memory as 16-byte reads that the lanes of a row group share.  Counted in the source, not profiled: the 2 x 32 tile
+// makes 40 of them a thread and token, and at four cycles a warp the two warps of a head hold the shared-memory pipe 320
+// cycles, which is about what a token takes at full grids.
 #include "common.cuh"
 
 namespace rwkv7 {
