@@ -255,27 +255,12 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void umma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// Byte offset of element (row, byte position kbyte along K) inside a K-major SWIZZLE_128B tile of `rows` rows:
-// the tile is a sequence of 128-byte-wide "atoms" along K (rows*128 bytes each); inside an atom the 16-byte chunk
-// index is XORed with (row & 7).  This is the layout make_sw128_kmajor_desc describes.
-__device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t kbyte, uint32_t rows) {
-    const uint32_t atom = kbyte >> 7, inb = kbyte & 127u;
-    return atom * rows * 128u + row * 128u + ((((inb >> 4) ^ (row & 7u)) << 4) | (inb & 15u));
 }
 
 // ---------------------------------------------------------------- host: tensor maps
@@ -335,29 +320,6 @@ inline int make_tmap_x3d(CUtensorMap* map, const void* base, uint64_t rows, uint
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled (3-D activation map) failed with code %d (rows=%llu K=%llu)", (int)r,
                   (unsigned long long)rows, (unsigned long long)K);
-        return RWKV7_ERR_CUDA;
-    }
-    return RWKV7_OK;
-}
-
-// Token vectors [tokens, H, 64] of 2- or 4-byte elements viewed as (64 channels, H, tokens): a box {64, 1, 64} at
-// (0, h, t0) lands the 64-token slice of one head densely ([token][channel], no swizzle).
-inline int make_tmap_tokens(CUtensorMap* map, const void* base, int elem_bytes, uint64_t tokens, uint64_t H) {
-    EncodeTiledFn fn = get_encode_tiled();
-    if (!fn) {
-        set_error("cuTensorMapEncodeTiled is unavailable (no CUDA driver?)");
-        return RWKV7_ERR_CUDA;
-    }
-    cuuint64_t dims[3] = {64, H, tokens};
-    cuuint64_t strides[2] = {(cuuint64_t)64 * elem_bytes, (cuuint64_t)64 * elem_bytes * H};
-    cuuint32_t box[3] = {64, 1, 64};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
-                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled (token map) failed with code %d (tokens=%llu H=%llu)", (int)r,
-                  (unsigned long long)tokens, (unsigned long long)H);
         return RWKV7_ERR_CUDA;
     }
     return RWKV7_OK;

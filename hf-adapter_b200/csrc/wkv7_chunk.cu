@@ -1,38 +1,61 @@
-// Chunked (WY / DPLR) WKV-7 prefill scan with the intra-chunk contractions on tcgen05 tensor cores.
+// Chunked (WY / DPLR) WKV-7 prefill scan, the intra-chunk contractions on tensor cores.
 //
-// One CTA per (sequence, head) walks the sequence in tiles of 64 tokens (the result does not depend on the
-// tile length, so the caller's chunk size is only validated).  With a~ = -kk, b~ = kk*a, per-channel log-decay
-// sums gi (inclusive) / ge (exclusive), gl = gi at the tile end and a centring point gref = gi at token 31:
+// One CTA per (sequence, head), two CTAs an SM.  The sequence is cut into chunks of 16 tokens (the result does not depend on
+// it, so the caller's chunk size is only validated).  With a~ = -kk, b~ = kk*a, P_t the inclusive product of the decays from the
+// chunk's first token on, and S0 the state [value i x key n] before the chunk:
 //
-//   A1 = [ a~ e^{ge-gref} ; r e^{gi-gref} ]   (128 x 64, tf32)      B1 = [ k e^{gref-gi} ; b~ e^{gref-gi} ]  (128 x 64)
-//   D1 = A1 B1^T = [[A_ak A_ab],[A_qk A_qb]]  (128 x 128)           D2 = A1 (S0 e^{gref})^T = [ a~E S0^T ; rP S0^T ]
-//   rhs = D2[0:64] + tril_strict(A_ak) V      (fp16 MMA)            U = (I - tril_strict(A_ab))^-1 rhs   (CUDA cores)
-//   Y   = D2[64:128] + [tril(A_qk) tril(A_qb)] [V ; U]              S' = S0 e^{gl} + [V^T U^T] [k e^{gl-gi} ; b~ e^{gl-gi}]
+//   aE = a~_t P_{t-1}   rP = r_t P_t   kI = k_s / P_s   bI = b~_s / P_s        (16 x 64, tf32 operands)
+//   A_ak = tril_strict(aE kI^T)   A_ab = tril_strict(aE bI^T)   A_qk = tril(rP kI^T)   A_qb = tril(rP bI^T)
+//   U^T = (S0 aE^T + V^T A_ak^T) T^T,   T = (I - A_ab)^-1
+//   Y^T = S0 rP^T + V^T A_qk^T + U^T A_qb^T
+//   S'  = S0 P_15 + V^T (k P_15/P) + U^T (b~ P_15/P)
 //
-// The decay-scaled factors span many orders of magnitude, so the products that contain them run as kind::tf32 on
-// operands rounded to tf32 in shared memory; the products of bounded quantities (A_* against V, U and the
-// end-of-tile-decayed keys) run as kind::f16.  All operands are written by the CTA's threads straight into
-// K-major 128-byte-swizzled tiles; accumulators D1/D2/D3 live in tensor memory (256 columns); the state row of
-// each value index stays in registers between tiles.  Every mbarrier wait is bounded (umma.cuh).
+// What bounds it: the serial chain S0 -> U -> S' of a head and the issue slots around it, not HBM and not the tensor pipe.  So the
+// chain is kept in registers.  Four STATE warps own 16 value rows each; the rows of the state never meet, so these warps never
+// wait for one another, and a warp's state is an mma accumulator that becomes the next product's A operand where it is: the
+// two columns a lane holds of an accumulator tile are read as k positions tq and tq + 4 of the A fragment, and the B operands are
+// read in the same permuted order (physical column 16 p + 4 tq + 2 e + f is column 2 tq + f of tile 2 p + e, so a lane's share of
+// two tiles is one 16-byte piece).  Everything that does not depend on the state is made ahead by four PREP warps, one chunk
+// each in turn, into a ring of six slots: decay products, scaled operands, the four 16 x 16 products, the inverse.  mma.sync
+// and not tcgen05: these products are 16 rows high, and through tensor memory every link of the chain costs a store, a
+// fence, an issue, a commit and a load, about 700 cycles (a tile of 64 tokens with five such links took 16.9 k cycles with one CTA
+// an SM).  8 sequences x 4096 tokens x 32 heads: 1150 -> 435 us (0.38 of the HBM floor of 165 us); the
+// 7.2B model's prefill of 64 x 512 tokens 484 -> 450 ms.
+//
+// Products that contain decay-scaled factors (range e^9.7 over 16 tokens) run on operands rounded to tf32; products of bounded
+// quantities (A_* against V and U, the keys decayed to the chunk's end) run in fp16; T is inverted in fp32, and
+// U = rhs T^T takes both operands as tf32 pairs (hi + lo, three products), which keeps the error of an fp32 solve.  U itself enters
+// its two products as an fp16 pair: the state is rounded to tf32 four times as often as with 64-token tiles, and with U in one
+// fp16 the state's error against 64 bits came out up to 2 % larger than theirs (421 us then); with the pair it is 1 % smaller.
+#include <type_traits>
+
 #include "umma.cuh"
 
 namespace rwkv7 {
 namespace ck {
-constexpr int C = 64, N = 64, THREADS = 512;  // warps 0-7 own the TMEM lanes; warps 8-15 help in the CUDA-core phases
-constexpr int ABS = 68;  // row stride (floats) of the fp32 A_ab / rhs arrays: 16-byte aligned, conflict-free
-// shared-memory regions (bytes)
-constexpr int R_A = 0;                      // A1 (tf32 128x64) | later AE (fp16 128 x 128)
-constexpr int R_B = R_A + 32768;            // B1 (tf32 128x64) | later AB + RH (fp32 64 x 68 each)
-constexpr int R_S0 = R_B + 36864;           // S0 e^{gref} (tf32 64 x 64)
-constexpr int R_AK = R_S0 + 16384;          // tril_strict(A_ak) (fp16 128 x 64, rows 64.. zero)
-constexpr int R_VU = R_AK + 16384;          // [V^T | U^T] (fp16 128 x 128, rows 64.. zero)
-constexpr int R_KB = R_VU + 32768;          // [kD ; bD]^T (fp16 64 x 128)
-constexpr int R_RAW = R_KB + 16384;         // r,k,v,kk,a (T 64x64 each) + w (fp32 64x64)
-constexpr int R_SMALL = R_RAW + 5 * 8192 + 16384;
-constexpr int R_INV = R_SMALL + 4096;     // inverses of the four 16 x 16 diagonal blocks of I - tril_strict(A_ab) (fp32)
-constexpr int INVS = 20;                  // row stride (floats) of one inverse block: conflict-free 16-byte row reads
-constexpr int SMEM_BYTES = R_INV + 4 * 16 * INVS * 4 + 1024;
-constexpr int D1_COL = 0, D2_COL = 128, D3_COL = 192, TMEM_COLS = 256;
+constexpr int C = 16, N = 64;       // tokens per chunk, head size
+constexpr int SLOTS = 6;            // chunks in the ring
+constexpr int STATE_WARPS = 4, PREP_WARPS = 4, THREADS = 32 * (STATE_WARPS + PREP_WARPS);
+// byte offsets in a slot
+constexpr int O_AE = 0;                 // aE [16][64] tf32, 16-byte pieces of odd rows swapped in groups of four
+constexpr int O_RP = O_AE + 4096;       // rP, same layout
+constexpr int O_KD = O_RP + 4096;       // k P_15/P [16][64] fp16 in permuted columns, 16-byte pieces xored by row & 7
+constexpr int O_BD = O_KD + 2048;       // b~ P_15/P, same layout
+constexpr int O_V = O_BD + 2048;        // v [16][64] fp16, pieces xored by row & 7
+constexpr int O_T = O_V + 2048;         // T [16][TS] fp32 (before that A_ab transposed)
+constexpr int TS = 24;                  // row stride of T: the lanes' 8-byte reads of four rows meet no bank twice
+constexpr int O_M = O_T + 16 * TS * 4;  // A_ak, A_qk, A_qb as B fragments: [matrix][lane][4] pairs of fp16
+constexpr int O_GL = O_M + 3 * 512;     // P_15 [64] fp32
+constexpr int SLOT_BYTES = O_GL + 256;
+constexpr int O_KI = O_KD;              // kI [16][64] fp32 while the four products are formed; then k P_15/P and b~ P_15/P
+constexpr int O_BI = O_V;               // bI, likewise; then v, T and the A_* fragments
+static_assert(O_BI + 4096 <= O_GL, "bI fits before P_15");
+constexpr int YS = 48;                  // row stride (bytes) of a state warp's 16 x 16 output tile: conflict-free
+constexpr int O_Y = SLOTS * SLOT_BYTES;
+constexpr int O_BAR = O_Y + STATE_WARPS * 16 * YS;
+constexpr int SMEM_BYTES = O_BAR + 2 * SLOTS * 8 + 16;
+static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs an SM");
+static_assert(SLOT_BYTES % 128 == 0 && O_BAR % 8 == 0, "alignment of the slots and barriers");
 }  // namespace ck
 
 struct ChunkArgs {
@@ -41,513 +64,382 @@ struct ChunkArgs {
     const float* state_in;
     float* state_out;
     __half* y;
-    int T, H, w_mode;
+    int T, H;
     unsigned int* error;
 };
 
 // Round to tf32 (nearest, ties away) with one integer add: the tensor core ignores the 13 low mantissa bits, so adding
-// half an ulp of tf32 to the bit pattern is all the rounding needs (cvt.rna.tf32 runs on the quarter-rate conversion
-// pipe, and this kernel rounds 16k values per tile).
-__device__ __forceinline__ float to_tf32(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
+// half an ulp of tf32 to the bit pattern is all the rounding needs (cvt.rna.tf32 runs on the quarter-rate conversion pipe).
+__device__ __forceinline__ uint32_t tf32_bits(float x) { return __float_as_uint(x) + 0x1000u; }
+// x = hi + lo to 22 bits, both usable as tf32 operands
+__device__ __forceinline__ void tf32_pair(float x, uint32_t& hi, uint32_t& lo) {
+    hi = tf32_bits(x) & 0xffffe000u;
+    lo = tf32_bits(x - __uint_as_float(hi));
+}
 __device__ __forceinline__ float fast_rcp(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&d)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void stmatrix4_trans(uint32_t addr, const uint32_t (&d)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
+                 ::"r"(addr), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]) : "memory");
+}
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
 
-struct ChunkMaps {
-    CUtensorMap m[6];  // r, k, v, kk, a, w viewed as (64 channels, H, B*T tokens)
-};
-
-__global__ void __launch_bounds__(ck::THREADS, 1) wkv7_chunk_kernel(const __grid_constant__ ChunkMaps maps, const ChunkArgs p) {
+// W_MODE 0: decay in fp16, 1: decay in fp32, 2: raw w in fp16 (decay = e^(-0.606531 sigmoid w))
+template <int W_MODE>
+__global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkArgs p) {
     using namespace ck;
-    extern __shared__ unsigned char smem_unaligned[];
-    unsigned char* sm = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
-    float* AB = reinterpret_cast<float*>(sm + R_B);
-    float* RH = AB + C * ABS;
-    float* UU = reinterpret_cast<float*>(sm + R_S0);   // U (fp32 64 x 64) during the solve; the S0 tile is dead by then
-    float* INV = reinterpret_cast<float*>(sm + R_INV);
-    __half* raw_r = reinterpret_cast<__half*>(sm + R_RAW);
-    __half* raw_k = raw_r + 4096;
-    __half* raw_v = raw_k + 4096;
-    __half* raw_kk = raw_v + 4096;
-    __half* raw_a = raw_kk + 4096;
-    float* raw_w = reinterpret_cast<float*>(raw_a + 4096);
-    float* part = reinterpret_cast<float*>(sm + R_SMALL);  // [8][64] partial log-decay sums
-    float* gref = part + 512;                              // [64]
-    float* gl = gref + 64;                                 // [64]
-    float* egref = gl + 64;                                // [64] e^{gref}
-    float* egl = egref + 64;                               // [64] e^{gl}
-    uint64_t* bar = reinterpret_cast<uint64_t*>(egl + 64);
-    uint64_t* raw_bar = bar + 1;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(raw_bar + 1);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    using WPair = typename std::conditional<W_MODE == 1, float2, __half2>::type;
+    extern __shared__ __align__(128) unsigned char sm[];
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + O_BAR);  // [SLOTS] the chunk is in the slot
+    uint64_t* empty = full + SLOTS;                            // [SLOTS] the four state warps have read it
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + SLOTS);
     const AbortCtx actx{abort_flag, p.error};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool main_warp = warp < 8;
-    const int q = warp & 3, hi = (warp >> 2) & 1;  // TMEM lane quarter / column half (main warps)
-    const int tl = q * 32 + lane;            // TMEM lane = accumulator row of this thread
+    const int g = lane >> 2, tq = lane & 3;  // row / column group of a lane in an mma fragment
     const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-    const size_t tok_stride = (size_t)p.H * N;
-    const size_t base = ((size_t)b * p.T * p.H + h) * N;
-    const int wbytes = p.w_mode == 1 ? 4 : 2;
-
+    const size_t stride = (size_t)p.H * N;                      // elements between consecutive tokens
+    const size_t base = ((size_t)b * p.T * p.H + h) * N;        // element offset of token 0
+    const int nchunks = p.T / C;
     if (tid == 0) {
-        mbar_init(bar, 1);
-        mbar_init(raw_bar, 1);
+        for (int s = 0; s < SLOTS; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], STATE_WARPS);
+        }
         *abort_flag = 0;
         mbar_fence_init();
-        for (int i = 0; i < 6; ++i) tma_prefetch_desc(&maps.m[i]);
     }
-    if (warp == 0) tmem_alloc(tmem_slot, TMEM_COLS);
-    // rows 64..127 of the fp16 A-operand tiles stay zero for the whole kernel
-    for (int i = tid; i < (16384 + 32768) / 16; i += THREADS) reinterpret_cast<uint4*>(sm + R_AK)[i] = make_uint4(0, 0, 0, 0);
-
-    // state row of value index i = tl (< 64), columns hi*32..+31, kept in registers across tiles
-    float S[32];
-    if (main_warp && tl < 64) {
-        const float* sp = p.state_in + ((size_t)bh * N + tl) * N + hi * 32;
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) {
-            const float4 t4 = *reinterpret_cast<const float4*>(sp + c);
-            S[c] = t4.x; S[c + 1] = t4.y; S[c + 2] = t4.z; S[c + 3] = t4.w;
-        }
-    }
-
-    // one thread fetches the six [64 tokens x 64 channels] slices of a tile with TMA (rows of the other heads are
-    // skipped by the tensor map); tokens past T in the last tile are masked where they are consumed
-    auto load_raw = [&](int t0) {
-        mbar_expect_tx(raw_bar, 5 * 8192 + 64 * 64 * wbytes);
-        const int row = b * p.T + t0;
-        tma_load_3d(raw_r, &maps.m[0], raw_bar, 0, h, row);
-        tma_load_3d(raw_k, &maps.m[1], raw_bar, 0, h, row);
-        tma_load_3d(raw_v, &maps.m[2], raw_bar, 0, h, row);
-        tma_load_3d(raw_kk, &maps.m[3], raw_bar, 0, h, row);
-        tma_load_3d(raw_a, &maps.m[4], raw_bar, 0, h, row);
-        tma_load_3d(raw_w, &maps.m[5], raw_bar, 0, h, row);
-    };
-
-    tc_fence_before();
     __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16);
-    uint32_t phase = 0;
-    bool ok = true;
-    auto wait_mma = [&]() {  // one polling lane per warp; result broadcast
-        if (lane == 0) ok = mbar_wait(bar, phase, actx, kErrWaitDFull);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        phase ^= 1;
-        tc_fence_after();
-    };
 
-    const int ntiles = (p.T + C - 1) / C;
-    if (tid == 0) load_raw(0);
-    uint32_t raw_phase = 0;
-    for (int tile = 0; tile < ntiles && ok; ++tile) {
-        const int t0 = tile * C;
-        if (lane == 0) ok = mbar_wait(raw_bar, raw_phase, actx, kErrWaitFull);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        raw_phase ^= 1;
-        if (!ok) break;
-        // ---------------- phase A: log-decay prefix sums, decay factors, operand tiles
-        // step 1, thread = (channel n, token quarter tq): prefix sums along tokens, f1 = e^{gi-gref} to shared memory,
-        // and the token-transposed fp16 tiles (rows = channel) with 16-byte stores
-        const int n = tid & 63, tq = tid >> 6;  // tq = 0..7: tokens tq*8 .. tq*8+7
-        float* F1 = reinterpret_cast<float*>(sm + R_S0);  // [64 tokens][64 channels]; the S0 tile is written after phase A
-        float lw[8];
-        {
-            float wv[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int t = tq * 8 + j;
-                wv[j] = p.w_mode == 1 ? raw_w[t * 64 + n] : __half2float(reinterpret_cast<const __half*>(raw_w)[t * 64 + n]);
-            }
-            float run = 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float v = p.w_mode == 2 ? -0.606531f * sigmoidf_(wv[j]) : __logf(wv[j]);
-                v = (t0 + tq * 8 + j < p.T) ? v : 0.f;
-                run += v;
-                lw[j] = v;
-            }
-            part[tq * 64 + n] = run;
-        }
-        __syncthreads();
-        {
-            float gi = 0.f, g_ref = 0.f, g_l = 0.f;
-#pragma unroll
-            for (int qq = 0; qq < 8; ++qq) {
-                const float pv = part[qq * 64 + n];
-                gi += qq < tq ? pv : 0.f;
-                g_ref += qq < 4 ? pv : 0.f;
-                g_l += pv;
-            }
-            if (tq == 0) {
-                gref[n] = g_ref;
-                gl[n] = g_l;
-                egref[n] = __expf(g_ref);
-                egl[n] = __expf(g_l);
-            }
-            // e^{gref-gi} = 1/f1 and e^{gl-gi} = e^{gl-gref}/f1
-            const float e_lr = __expf(g_l - g_ref);
-            float kx[8], bx[8];
-            __half vx[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int t = tq * 8 + j;
-                const bool valid = t0 + t < p.T;
-                const float kv = __half2float(raw_k[t * 64 + n]);
-                const float bv = __half2float(raw_kk[t * 64 + n]) * __half2float(raw_a[t * 64 + n]);
-                const __half vv = raw_v[t * 64 + n];
-                kx[j] = valid ? kv : 0.f;
-                bx[j] = valid ? bv : 0.f;
-                vx[j] = valid ? vv : __float2half(0.f);
-            }
-            uint32_t kdp[4], bdp[4], vvp[4];
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                float f4[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    gi += lw[j + u];
-                    const float f1 = __expf(gi - g_ref);
-                    F1[(tq * 8 + j + u) * 64 + n] = f1;
-                    f4[u] = e_lr * fast_rcp(f1);
-                }
-                const __half2 hk = __floats2half2_rn(kx[j] * f4[0], kx[j + 1] * f4[1]);
-                const __half2 hb = __floats2half2_rn(bx[j] * f4[0], bx[j + 1] * f4[1]);
-                const __half2 hv = __halves2half2(vx[j], vx[j + 1]);
-                kdp[j >> 1] = *reinterpret_cast<const uint32_t*>(&hk);
-                bdp[j >> 1] = *reinterpret_cast<const uint32_t*>(&hb);
-                vvp[j >> 1] = *reinterpret_cast<const uint32_t*>(&hv);
-            }
-            // 8 tokens = one 16-byte chunk of row n
-            const uint32_t kb = tq * 16;
-            *reinterpret_cast<uint4*>(sm + R_KB + sw128_offset(n, kb, 64)) = make_uint4(kdp[0], kdp[1], kdp[2], kdp[3]);
-            *reinterpret_cast<uint4*>(sm + R_KB + sw128_offset(n, 128 + kb, 64)) = make_uint4(bdp[0], bdp[1], bdp[2], bdp[3]);
-            *reinterpret_cast<uint4*>(sm + R_VU + sw128_offset(n, kb, 128)) = make_uint4(vvp[0], vvp[1], vvp[2], vvp[3]);
-        }
-        __syncthreads();  // F1, gref visible
-        // step 2, thread = (token t, 8 channels): the token-major tf32 tiles with 16-byte loads and stores
-        {
-            const int t = tid >> 3, nb = (tid & 7) * 8;
-            const float m = t0 + t < p.T ? 1.f : 0.f;
-            float r8[8], k8[8], kk8[8], a8[8], f1v[8], f2v[8];
-            load8(raw_r + t * 64 + nb, r8);
-            load8(raw_k + t * 64 + nb, k8);
-            load8(raw_kk + t * 64 + nb, kk8);
-            load8(raw_a + t * 64 + nb, a8);
-            load8(F1 + t * 64 + nb, f1v);
-            // e^{ge-gref}: f1 of the previous token; e^{-gref} for the first one
-            if (t > 0) load8(F1 + (t - 1) * 64 + nb, f2v);
-            else {
-                load8(egref + nb, f2v);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f2v[e] = fast_rcp(f2v[e]);
-            }
-            float ae[8], rp[8], ki[8], bi[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float f3 = fast_rcp(f1v[e]) * m;
-                const float kkm = kk8[e] * m;
-                ae[e] = to_tf32(-kkm * f2v[e]);
-                rp[e] = to_tf32(r8[e] * f1v[e] * m);
-                ki[e] = to_tf32(k8[e] * f3);
-                bi[e] = to_tf32(kk8[e] * a8[e] * f3);
-            }
-#pragma unroll
-            for (int c = 0; c < 8; c += 4) {
-                const uint32_t kb = (nb + c) * 4;
-                *reinterpret_cast<float4*>(sm + R_A + sw128_offset(t, kb, 128)) = make_float4(ae[c], ae[c + 1], ae[c + 2], ae[c + 3]);
-                *reinterpret_cast<float4*>(sm + R_A + sw128_offset(64 + t, kb, 128)) = make_float4(rp[c], rp[c + 1], rp[c + 2], rp[c + 3]);
-                *reinterpret_cast<float4*>(sm + R_B + sw128_offset(t, kb, 128)) = make_float4(ki[c], ki[c + 1], ki[c + 2], ki[c + 3]);
-                *reinterpret_cast<float4*>(sm + R_B + sw128_offset(64 + t, kb, 128)) = make_float4(bi[c], bi[c + 1], bi[c + 2], bi[c + 3]);
-            }
-        }
-        __syncthreads();  // raw buffers and F1 consumed
-        if (tid == 0 && tile + 1 < ntiles) {
-            fence_proxy_async_smem();  // generic reads of the raw buffers are ordered before the refill
-            load_raw(t0 + C);
-        }
-        if (main_warp && tl < 64) {  // S0 e^{gref} operand tile and the D3 accumulator initialised with S0 e^{gl}
-            uint32_t d3[32];
-#pragma unroll
-            for (int c = 0; c < 32; c += 4) {
-                float4 o;
-                const float4 er = *reinterpret_cast<const float4*>(egref + hi * 32 + c);
-                o.x = to_tf32(S[c] * er.x);
-                o.y = to_tf32(S[c + 1] * er.y);
-                o.z = to_tf32(S[c + 2] * er.z);
-                o.w = to_tf32(S[c + 3] * er.w);
-                *reinterpret_cast<float4*>(sm + R_S0 + sw128_offset(tl, (hi * 32 + c) * 4, 64)) = o;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) d3[c + e] = __float_as_uint(S[c + e] * egl[hi * 32 + c + e]);
-            }
-            tmem_st16(lane_addr + D3_COL + hi * 32, reinterpret_cast<uint32_t(&)[16]>(d3[0]));
-            tmem_st16(lane_addr + D3_COL + hi * 32 + 16, reinterpret_cast<uint32_t(&)[16]>(d3[16]));
-            tc_wait_st();
-        }
-        fence_proxy_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        // ---------------- phase B: D1 = A1 B1^T, D2 = A1 S0^T (tf32)
-        if (tid == 0) {
-            tc_fence_after();
-            constexpr uint32_t id128 = make_idesc(128, 128, 1, 2, 2), id64 = make_idesc(128, 64, 1, 2, 2);
-            const uint64_t da = make_sw128_kmajor_desc(smem_u32(sm + R_A));
-            const uint64_t db = make_sw128_kmajor_desc(smem_u32(sm + R_B));
-            const uint64_t ds = make_sw128_kmajor_desc(smem_u32(sm + R_S0));
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint64_t oa = (uint64_t)(((j >> 2) * 128 * 128 + (j & 3) * 32) >> 4);
-                const uint64_t os = (uint64_t)(((j >> 2) * 64 * 128 + (j & 3) * 32) >> 4);
-                umma_tf32_ss(tmem + D1_COL, da + oa, db + oa, id128, j > 0);
-                umma_tf32_ss(tmem + D2_COL, da + oa, ds + os, id64, j > 0);
-            }
-            tc_commit(bar);
-        }
-        wait_mma();
-        if (!ok) break;
-        // ---------------- phase C: mask D1 into tril_strict(A_ak) (fp16), tril_strict(A_ab) (fp32), [tril A_qk | tril A_qb] (fp16)
-        for (int i = tid; i < 1024; i += THREADS) {  // rows 0..63 of both AE atoms are zero
-            const int atom = i >> 9, rem = i & 511;
-            reinterpret_cast<uint4*>(sm + R_A + atom * 16384)[rem] = make_uint4(0, 0, 0, 0);
-        }
-        if (main_warp) {
-            const int t = tl & 63;
-            const bool low = tl < 64;  // rows of a~E (low) or rP (high)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + D1_COL + hi * 64 + c * 16, v);
-                tc_wait_ld();
-                if (low && hi == 1) {  // A_ab, strict lower triangle, fp32
-#pragma unroll
-                    for (int e = 0; e < 16; e += 4) {
-                        const int s = c * 16 + e;
-                        float4 o;
-                        o.x = (s + 0 < t) ? __uint_as_float(v[e + 0]) : 0.f;
-                        o.y = (s + 1 < t) ? __uint_as_float(v[e + 1]) : 0.f;
-                        o.z = (s + 2 < t) ? __uint_as_float(v[e + 2]) : 0.f;
-                        o.w = (s + 3 < t) ? __uint_as_float(v[e + 3]) : 0.f;
-                        *reinterpret_cast<float4*>(AB + t * ABS + s) = o;
-                    }
+    if (warp >= STATE_WARPS) {
+        // ------------------------------------------------------------------------------------------------ PREP
+        // lane = channels 2 lane, 2 lane + 1 of all 16 tokens
+        const int pw = warp - STATE_WARPS;
+        const uint32_t f_even = (lane >> 1) * 16 + (lane & 1) * 8;         // fp32 row, even token
+        const uint32_t f_odd = ((lane >> 1) ^ 4) * 16 + (lane & 1) * 8;    // odd token
+        const uint32_t h_piece = (lane >> 3) * 2 + (lane & 1), h_in = ((lane >> 1) & 3) * 4;  // fp16 row: piece and byte of the permuted pair
+        for (int c = pw; c < nchunks; c += PREP_WARPS) {
+            const int slot = c % SLOTS;
+            unsigned char* sl = sm + slot * SLOT_BYTES;
+            const size_t row0 = base + (size_t)c * C * stride;
+            const size_t off = row0 + 2 * lane;
+            if (c + PREP_WARPS < nchunks) {  // the warp's next chunk on its way to L2: lane = token, half of its operands
+                const size_t o = row0 + (size_t)(PREP_WARPS * C + (lane >> 1)) * stride;
+                if (lane & 1) {
+                    prefetch_l2(p.kk + o);
+                    prefetch_l2(p.a + o);
+                    prefetch_l2(reinterpret_cast<const char*>(p.w) + o * (W_MODE == 1 ? 4 : 2));
+                    if (W_MODE == 1) prefetch_l2(reinterpret_cast<const char*>(p.w) + o * 4 + 128);
                 } else {
-                    uint32_t pk[8];
-#pragma unroll
-                    for (int e = 0; e < 16; e += 2) {
-                        const int s = c * 16 + e;
-                        const bool k0 = low ? (s < t) : (s <= t), k1 = low ? (s + 1 < t) : (s + 1 <= t);
-                        const __half2 h2 = __floats2half2_rn(k0 ? __uint_as_float(v[e]) : 0.f, k1 ? __uint_as_float(v[e + 1]) : 0.f);
-                        pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
-                    }
-                    unsigned char* dst = low ? sm + R_AK + sw128_offset(t, c * 32, 128)
-                                             : sm + R_A + sw128_offset(64 + t, (hi * 64 + c * 16) * 2, 128);
-                    // 16 halves = two 16-byte chunks (chunk index differs by one: separate swizzled addresses)
-                    *reinterpret_cast<uint4*>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    unsigned char* dst2 = low ? sm + R_AK + sw128_offset(t, c * 32 + 16, 128)
-                                              : sm + R_A + sw128_offset(64 + t, (hi * 64 + c * 16) * 2 + 16, 128);
-                    *reinterpret_cast<uint4*>(dst2) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                    prefetch_l2(p.r + o);
+                    prefetch_l2(p.k + o);
+                    prefetch_l2(p.v + o);
                 }
             }
-        }
-        // ---------------- phase C2: rhs = D2[0:64] += tril_strict(A_ak) V   (fp16, K = 64)
-        // Warps 0 and 1 wrote tril_strict(A_ak): they hand it to the tensor core at once (named barrier of 64 threads),
-        // so the product runs under the other warps' masks and the block inverses below.
-        if (warp < 2) {
-            fence_proxy_async_smem();
-            tc_fence_before();
-            asm volatile("bar.sync 1, 64;" ::: "memory");
-            if (tid == 0) {
-                tc_fence_after();
-                constexpr uint32_t idh = make_idesc(128, 64, 1, 0, 0);
-                const uint64_t da = make_sw128_kmajor_desc(smem_u32(sm + R_AK));
-                const uint64_t db = make_sw128_kmajor_desc(smem_u32(sm + R_VU));
+            float2 P = make_float2(1.f, 1.f);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_f16_ss(tmem + D2_COL, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), idh, 1);
-                tc_commit(bar);
+            for (int tb = 0; tb < 2; ++tb) {
+                __half2 r2[8], k2[8], kk2[8], a2[8];
+                WPair w2[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const size_t o = off + (size_t)(tb * 8 + j) * stride;
+                    w2[j] = *reinterpret_cast<const WPair*>(reinterpret_cast<const char*>(p.w) + o * (W_MODE == 1 ? 4 : 2));
+                    kk2[j] = *reinterpret_cast<const __half2*>(p.kk + o);
+                    a2[j] = *reinterpret_cast<const __half2*>(p.a + o);
+                    k2[j] = *reinterpret_cast<const __half2*>(p.k + o);
+                    r2[j] = *reinterpret_cast<const __half2*>(p.r + o);
+                }
+                if (tb == 0 && c >= SLOTS && !mbar_wait(&empty[slot], (c / SLOTS - 1) & 1, actx, kErrWaitEmpty)) goto out;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float2 w;
+                    if constexpr (W_MODE == 1) w = w2[j];
+                    else w = __half22float2(w2[j]);
+                    if constexpr (W_MODE == 2) {
+                        w.x = __expf(-0.606531f * fast_rcp(1.f + __expf(-w.x)));
+                        w.y = __expf(-0.606531f * fast_rcp(1.f + __expf(-w.y)));
+                    }
+                    const float2 kk = __half22float2(kk2[j]), a = __half22float2(a2[j]), k = __half22float2(k2[j]), r = __half22float2(r2[j]);
+                    const float2 ae = make_float2(-kk.x * P.x, -kk.y * P.y);
+                    P.x *= w.x;
+                    P.y *= w.y;
+                    const float2 inv = make_float2(fast_rcp(P.x), fast_rcp(P.y));
+                    const uint32_t o = (tb * 8 + j) * 256 + ((j & 1) ? f_odd : f_even);
+                    *reinterpret_cast<uint2*>(sl + O_AE + o) = make_uint2(tf32_bits(ae.x), tf32_bits(ae.y));
+                    *reinterpret_cast<uint2*>(sl + O_RP + o) = make_uint2(tf32_bits(r.x * P.x), tf32_bits(r.y * P.y));
+                    *reinterpret_cast<float2*>(sl + O_KI + o) = make_float2(k.x * inv.x, k.y * inv.y);
+                    *reinterpret_cast<float2*>(sl + O_BI + o) = make_float2(kk.x * a.x * inv.x, kk.y * a.y * inv.y);
+                }
             }
-        }
-        fence_proxy_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        // While that product runs, four helper warps invert the 16 x 16 diagonal blocks of I - tril_strict(A_ab):
-        // lane c of warp 8 + b builds column c of block b by forward substitution in registers.
-        if (warp >= 8 && warp < 12 && lane < 16) {
-            const int blk = warp - 8;
-            const float* L = AB + (blk * 16) * ABS + blk * 16;
-            float x[16];
+            *reinterpret_cast<float2*>(sl + O_GL + lane * 8) = P;
+            uint4 vv[4];  // v of the chunk: 128 pieces of 16 bytes
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                vv[i] = *reinterpret_cast<const uint4*>(p.v + row0 + (size_t)(i * 4 + (lane >> 3)) * stride + (lane & 7) * 8);
+            __syncwarp();
+            // the four products: rows t of aE (0) and rP (1) against kI (n-tiles 0, 1) and bI (2, 3)
+            float acc[2][4][4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[m][q][e] = 0.f;
+#pragma unroll
+            for (int pp = 0; pp < 4; ++pp) {
+                const uint32_t o = g * 256 + tq * 16 + ((pp ^ (g & 1)) * 64);  // row g; row g + 8 has the same parity
+                uint4 A[2][2], B[4];
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    A[0][hf] = *reinterpret_cast<const uint4*>(sl + O_AE + hf * 2048 + o);
+                    A[1][hf] = *reinterpret_cast<const uint4*>(sl + O_RP + hf * 2048 + o);
+                    B[hf] = *reinterpret_cast<const uint4*>(sl + O_KI + hf * 2048 + o);
+                    B[2 + hf] = *reinterpret_cast<const uint4*>(sl + O_BI + hf * 2048 + o);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    B[q].x += 0x1000u; B[q].y += 0x1000u; B[q].z += 0x1000u; B[q].w += 0x1000u;  // round to tf32
+                }
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) mma_tf32(acc[m][q], A[m][0].x, A[m][1].x, A[m][0].y, A[m][1].y, B[q].x, B[q].y);
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) mma_tf32(acc[m][q], A[m][0].z, A[m][1].z, A[m][0].w, A[m][1].w, B[q].z, B[q].w);
+            }
+            // keys decayed to the chunk's end
+            uint32_t kd[16], bd[16];
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
-                float a0 = t == lane ? 1.f : 0.f, a1 = 0.f;
-#pragma unroll
-                for (int ss = 0; ss + 1 < t; ss += 2) {
-                    a0 = fmaf(L[t * ABS + ss], x[ss], a0);
-                    a1 = fmaf(L[t * ABS + ss + 1], x[ss + 1], a1);
-                }
-                if (t & 1) a0 = fmaf(L[t * ABS + t - 1], x[t - 1], a0);
-                x[t] = a0 + a1;
-                INV[(blk * 16 + t) * INVS + lane] = x[t];
+                const uint32_t o = t * 256 + ((t & 1) ? f_odd : f_even);
+                const float2 ki = *reinterpret_cast<const float2*>(sl + O_KI + o), bi = *reinterpret_cast<const float2*>(sl + O_BI + o);
+                kd[t] = pack_half2(ki.x * P.x, ki.y * P.y);
+                bd[t] = pack_half2(bi.x * P.x, bi.y * P.y);
             }
-        }
-        wait_mma();
-        if (!ok) break;
-        // ---------------- phase D: U = (I - tril_strict(A_ab))^-1 rhs
-        if (main_warp && tl < 64) {
+            __syncwarp();  // kI and bI are read: their room is free
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + D2_COL + hi * 32 + c * 16, v);
-                tc_wait_ld();
-#pragma unroll
-                for (int e = 0; e < 16; e += 4)
-                    *reinterpret_cast<float4*>(RH + tl * ABS + hi * 32 + c * 16 + e) =
-                        make_float4(__uint_as_float(v[e]), __uint_as_float(v[e + 1]), __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
+            for (int t = 0; t < 16; ++t) {
+                const uint32_t o = t * 128 + ((h_piece ^ (t & 7)) << 4) + h_in;
+                *reinterpret_cast<uint32_t*>(sl + O_KD + o) = kd[t];
+                *reinterpret_cast<uint32_t*>(sl + O_BD + o) = bd[t];
             }
-        }
-        tc_fence_before();
-        __syncthreads();
-        // Blocked forward substitution on 16-row blocks.  Value columns are independent, so each sweeping warp takes a
-        // group of columns through all four blocks with warp-level syncs only; a lane owns rows rg, rg+4, rg+8, rg+12
-        // of the block and CW columns:
-        //   (a) rhs_b += L[b][0..b) U[0..b)        (b) U_b = inv(I - L_bb) rhs_b
-        constexpr int CW = 2;                   // value columns per lane (measured: 2 columns on 4 warps 1.17 ms, 1 column on 8 warps 1.22 ms)
-        constexpr int SWEEP_WARPS = 8 / CW;     // 8 lanes x CW columns per warp
-        if (warp < SWEEP_WARPS) {
-            const int rg = lane >> 3, col = warp * (8 * CW) + (lane & 7) * CW;
-#pragma unroll 1
-            for (int blk = 0; blk < 4; ++blk) {
-                const int r0 = blk * 16 + rg;
-                if (blk > 0) {
-                    float acc[4][CW];
 #pragma unroll
-                    for (int rr = 0; rr < 4; ++rr)
+            for (int i = 0; i < 4; ++i) {
+                const int t = i * 4 + (lane >> 3);
+                *reinterpret_cast<uint4*>(sl + O_V + t * 128 + (((lane & 7) ^ (t & 7)) << 4)) = vv[i];
+            }
+            // masks; tile q of a product holds (t = g, s = 8 q + 2 tq, + 1) in [0], [1] and t = g + 8 in [2], [3], which is what
+            // the B fragment of its transpose wants in the same lane
+            auto masked = [&](const float (&lo)[4], const float (&hi)[4], int diag, float (&o)[8]) {  // keeps s < t + diag
 #pragma unroll
-                        for (int c = 0; c < CW; ++c) acc[rr][c] = RH[(r0 + 4 * rr) * ABS + col + c];
-#pragma unroll 2
-                    for (int s0 = 0; s0 < blk * 16; s0 += 4) {
-                        float u[4][CW];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-#pragma unroll
-                            for (int c = 0; c < CW; ++c) u[e][c] = UU[(s0 + e) * 64 + col + c];
-#pragma unroll
-                        for (int rr = 0; rr < 4; ++rr) {
-                            const float4 m = *reinterpret_cast<const float4*>(AB + (r0 + 4 * rr) * ABS + s0);
-#pragma unroll
-                            for (int c = 0; c < CW; ++c)
-                                acc[rr][c] = fmaf(m.x, u[0][c], fmaf(m.y, u[1][c], fmaf(m.z, u[2][c], fmaf(m.w, u[3][c], acc[rr][c]))));
-                        }
-                    }
-#pragma unroll
-                    for (int rr = 0; rr < 4; ++rr)
-#pragma unroll
-                        for (int c = 0; c < CW; ++c) RH[(r0 + 4 * rr) * ABS + col + c] = acc[rr][c];
-                    __syncwarp();
+                for (int e = 0; e < 4; ++e) {
+                    const int t = g + (e >> 1) * 8, s = 2 * tq + (e & 1);
+                    o[e] = s < t + diag ? lo[e] : 0.f;
+                    o[4 + e] = s + 8 < t + diag ? hi[e] : 0.f;
                 }
-                float o[4][CW];
+            };
+            auto store_frag = [&](int which, const float (&o)[8]) {
+                *reinterpret_cast<uint4*>(sl + O_M + which * 512 + lane * 16) =
+                    make_uint4(pack_half2(o[0], o[1]), pack_half2(o[4], o[5]), pack_half2(o[2], o[3]), pack_half2(o[6], o[7]));
+            };
+            float mk[8];
+            masked(acc[0][0], acc[0][1], 0, mk);
+            store_frag(0, mk);
+            masked(acc[1][0], acc[1][1], 1, mk);
+            store_frag(1, mk);
+            masked(acc[1][2], acc[1][3], 1, mk);
+            store_frag(2, mk);
+            masked(acc[0][2], acc[0][3], 0, mk);
+            float* Tm = reinterpret_cast<float*>(sl + O_T);
 #pragma unroll
-                for (int rr = 0; rr < 4; ++rr)
+            for (int e = 0; e < 4; ++e) {  // A_ab transposed: row s, column t
+                Tm[(2 * tq + (e & 1)) * TS + g + (e >> 1) * 8] = mk[e];
+                Tm[(8 + 2 * tq + (e & 1)) * TS + g + (e >> 1) * 8] = mk[4 + e];
+            }
+            __syncwarp();
+            // T = (I - A_ab)^-1 by forward substitution, lane = column (both halves of the warp do the same)
+            float x[16];
 #pragma unroll
-                    for (int c = 0; c < CW; ++c) o[rr][c] = 0.f;
+            for (int t = 0; t < 16; ++t) x[t] = t == (lane & 15) ? 1.f : 0.f;
 #pragma unroll
-                for (int s0 = 0; s0 < 16; s0 += 4) {
-                    float x[4][CW];
+            for (int s = 0; s < 15; ++s) {
+#pragma unroll
+                for (int t4 = (s + 1) / 4; t4 < 4; ++t4) {
+                    const float4 l4 = *reinterpret_cast<const float4*>(Tm + s * TS + t4 * 4);
+                    const float l[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e)
-#pragma unroll
-                        for (int c = 0; c < CW; ++c) x[e][c] = RH[(blk * 16 + s0 + e) * ABS + col + c];
-#pragma unroll
-                    for (int rr = 0; rr < 4; ++rr) {
-                        const float4 m = *reinterpret_cast<const float4*>(INV + (r0 + 4 * rr) * INVS + s0);
-#pragma unroll
-                        for (int c = 0; c < CW; ++c)
-                            o[rr][c] = fmaf(m.x, x[0][c], fmaf(m.y, x[1][c], fmaf(m.z, x[2][c], fmaf(m.w, x[3][c], o[rr][c]))));
-                    }
-                }
-#pragma unroll
-                for (int rr = 0; rr < 4; ++rr)
-#pragma unroll
-                    for (int c = 0; c < CW; ++c) UU[(r0 + 4 * rr) * 64 + col + c] = o[rr][c];
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        {
-            const int i = tid & 63, tg = tid >> 6;
-            // U^T into the second K atom of [V^T | U^T]: row = value index i, k = 64 + token; thread (i, tg) packs 8 tokens
-            uint32_t pk[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const __half2 h2 = __floats2half2_rn(UU[(tg * 8 + 2 * e) * 64 + i], UU[(tg * 8 + 2 * e + 1) * 64 + i]);
-                pk[e] = *reinterpret_cast<const uint32_t*>(&h2);
-            }
-            *reinterpret_cast<uint4*>(sm + R_VU + sw128_offset(i, (64 + tg * 8) * 2, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        }
-        fence_proxy_async_smem();
-        __syncthreads();
-        // ---------------- phase E / F: Y = D2[64:128] += [A_qk A_qb][V;U];  S' = D3 += [V^T U^T][kD;bD]   (fp16, K = 128)
-        if (tid == 0) {
-            tc_fence_after();
-            constexpr uint32_t idh = make_idesc(128, 64, 1, 0, 0);
-            const uint64_t dae = make_sw128_kmajor_desc(smem_u32(sm + R_A));
-            const uint64_t dvu = make_sw128_kmajor_desc(smem_u32(sm + R_VU));
-            const uint64_t dkb = make_sw128_kmajor_desc(smem_u32(sm + R_KB));
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint64_t o128 = (uint64_t)(((j >> 2) * 128 * 128 + (j & 3) * 32) >> 4);
-                const uint64_t o64 = (uint64_t)(((j >> 2) * 64 * 128 + (j & 3) * 32) >> 4);
-                umma_f16_ss(tmem + D2_COL, dae + o128, dvu + o128, idh, 1);
-                umma_f16_ss(tmem + D3_COL, dvu + o128, dkb + o64, idh, 1);
-            }
-            tc_commit(bar);
-        }
-        wait_mma();
-        if (!ok) break;
-        // ---------------- phase G: outputs of the tile, new state rows back to registers
-        if (main_warp) {
-            uint32_t v[32];
-            const uint32_t col = (tl < 64 ? D3_COL : D2_COL) + hi * 32;
-            tmem_ld16(lane_addr + col, reinterpret_cast<uint32_t(&)[16]>(v[0]));
-            tmem_ld16(lane_addr + col + 16, reinterpret_cast<uint32_t(&)[16]>(v[16]));
-            tc_wait_ld();
-            if (tl < 64) {
-#pragma unroll
-                for (int c = 0; c < 32; ++c) S[c] = __uint_as_float(v[c]);
-            } else {
-                const int t = tl - 64;
-                if (t0 + t < p.T) {
-                    __half* yp = p.y + base + (size_t)(t0 + t) * tok_stride + hi * 32;
-#pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        uint32_t pk[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const __half2 h2 = __floats2half2_rn(__uint_as_float(v[c + 2 * e]), __uint_as_float(v[c + 2 * e + 1]));
-                            pk[e] = *reinterpret_cast<const uint32_t*>(&h2);
-                        }
-                        *reinterpret_cast<uint4*>(yp + c) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                    }
+                        if (t4 * 4 + e > s) x[t4 * 4 + e] = fmaf(l[e], x[s], x[t4 * 4 + e]);
                 }
             }
+            __syncwarp();
+            if (lane < 16) {
+#pragma unroll
+                for (int t = 0; t < 16; ++t) Tm[t * TS + lane] = x[t];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[slot]);
         }
-        tc_fence_before();
-        __syncthreads();  // accumulators and operand tiles are free for the next tile
+    } else {
+        // ------------------------------------------------------------------------------------------------ STATE
+        // rows 16 warp + g (+ 8); S[j] is accumulator tile j: [0], [1] = row g, [2], [3] = row g + 8
+        float S[8][4];
+        const size_t srow = ((size_t)bh * N + warp * 16 + g) * N + tq * 4;
+#pragma unroll
+        for (int pp = 0; pp < 4; ++pp)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const float4 t4 = *reinterpret_cast<const float4*>(p.state_in + srow + hf * 8 * N + pp * 16);
+                S[2 * pp][2 * hf] = t4.x; S[2 * pp][2 * hf + 1] = t4.y;
+                S[2 * pp + 1][2 * hf] = t4.z; S[2 * pp + 1][2 * hf + 1] = t4.w;
+            }
+        const int l7 = lane & 7, mi = lane >> 3;                              // ldmatrix / stmatrix: row and matrix this lane addresses
+        const uint32_t v_at = (l7 + (mi >> 1) * 8) * 128 + (((2 * warp + (mi & 1)) ^ l7) << 4);
+        const uint32_t d_row = (l7 + (mi & 1) * 8) * 128;
+        unsigned char* ystage = sm + O_Y + warp * 16 * YS;
+        const uint32_t y_st = smem_u32(ystage + (l7 + (mi >> 1) * 8) * YS + (mi & 1) * 16);
+        const uint32_t y_ld = (lane >> 1) * YS + (lane & 1) * 16;
+        __half* yp = p.y + base + (size_t)(lane >> 1) * stride + warp * 16 + (lane & 1) * 8;
+        const uint32_t f_at = g * 256 + tq * 16;
+        for (int c = 0; c < nchunks; ++c) {
+            const int slot = c % SLOTS;
+            const unsigned char* sl = sm + slot * SLOT_BYTES;
+            const uint32_t sl_u32 = smem_u32(sl);
+            if (!mbar_wait(&full[slot], (c / SLOTS) & 1, actx, kErrWaitFull)) goto out;
+            __syncwarp();
+            uint32_t va[4];
+            ldmatrix4_trans(va, sl_u32 + O_V + v_at);
+            const uint4 mak = *reinterpret_cast<const uint4*>(sl + O_M + lane * 16);
+            const uint4 mqk = *reinterpret_cast<const uint4*>(sl + O_M + 512 + lane * 16);
+            float au[2][2][4], ar[2][4];  // [tokens 0..7, 8..15][tiles of even, odd index]: S0 aE^T + V^T A_ak^T, S0 rP^T + V^T A_qk^T
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) au[nt][0][e] = au[nt][1][e] = ar[nt][e] = 0.f;
+            mma_f16(au[0][0], va, mak.x, mak.y);
+            mma_f16(au[1][0], va, mak.z, mak.w);
+            mma_f16(ar[0], va, mqk.x, mqk.y);
+            mma_f16(ar[1], va, mqk.z, mqk.w);
+#pragma unroll
+            for (int pp = 0; pp < 4; ++pp) {
+                const uint32_t o = f_at + ((pp ^ (g & 1)) * 64);
+                const uint4 a0 = *reinterpret_cast<const uint4*>(sl + O_AE + o), a1 = *reinterpret_cast<const uint4*>(sl + O_AE + 2048 + o);
+                const uint4 r0 = *reinterpret_cast<const uint4*>(sl + O_RP + o), r1 = *reinterpret_cast<const uint4*>(sl + O_RP + 2048 + o);
+                const float4 gl = *reinterpret_cast<const float4*>(sl + O_GL + pp * 64 + tq * 16);
+                uint32_t kd[4];
+                ldmatrix4_trans(kd, sl_u32 + O_KD + d_row + (((2 * pp + (mi >> 1)) ^ l7) << 4));
+                float(&s0)[4] = S[2 * pp];
+                float(&s1)[4] = S[2 * pp + 1];
+                const uint32_t e0 = tf32_bits(s0[0]), e1 = tf32_bits(s0[2]), e2 = tf32_bits(s0[1]), e3 = tf32_bits(s0[3]);
+                const uint32_t o0 = tf32_bits(s1[0]), o1 = tf32_bits(s1[2]), o2 = tf32_bits(s1[1]), o3 = tf32_bits(s1[3]);
+                mma_tf32(au[0][0], e0, e1, e2, e3, a0.x, a0.y);
+                mma_tf32(au[1][0], e0, e1, e2, e3, a1.x, a1.y);
+                mma_tf32(au[0][1], o0, o1, o2, o3, a0.z, a0.w);
+                mma_tf32(au[1][1], o0, o1, o2, o3, a1.z, a1.w);
+                mma_tf32(ar[0], e0, e1, e2, e3, r0.x, r0.y);
+                mma_tf32(ar[1], e0, e1, e2, e3, r1.x, r1.y);
+                mma_tf32(ar[0], o0, o1, o2, o3, r0.z, r0.w);
+                mma_tf32(ar[1], o0, o1, o2, o3, r1.z, r1.w);
+                s0[0] *= gl.x; s0[1] *= gl.y; s0[2] *= gl.x; s0[3] *= gl.y;
+                s1[0] *= gl.z; s1[1] *= gl.w; s1[2] *= gl.z; s1[3] *= gl.w;
+                mma_f16(s0, va, kd[0], kd[1]);
+                mma_f16(s1, va, kd[2], kd[3]);
+            }
+            // U^T = rhs T^T: the two halves of T's lower triangle that are not zero, operands as hi + lo
+            uint32_t ua[4], ul[4];  // fp16 and what it leaves
+            {
+                const float* Tm = reinterpret_cast<const float*>(sl + O_T) + g * TS + 2 * tq;
+                const float2 t00 = *reinterpret_cast<const float2*>(Tm), t10 = *reinterpret_cast<const float2*>(Tm + 8 * TS),
+                             t11 = *reinterpret_cast<const float2*>(Tm + 8 * TS + 8);
+                uint32_t th[6], tl[6];
+                tf32_pair(t00.x, th[0], tl[0]); tf32_pair(t00.y, th[1], tl[1]);
+                tf32_pair(t10.x, th[2], tl[2]); tf32_pair(t10.y, th[3], tl[3]);
+                tf32_pair(t11.x, th[4], tl[4]); tf32_pair(t11.y, th[5], tl[5]);
+                uint32_t rh[2][4], rl[2][4];
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) tf32_pair(au[nt][0][e] + au[nt][1][e], rh[nt][e], rl[nt][e]);
+                float u0[4], u1[4], c0[4], c1[4];  // products of the high parts, and the corrections
+#pragma unroll
+                for (int e = 0; e < 4; ++e) u0[e] = u1[e] = c0[e] = c1[e] = 0.f;
+                mma_tf32(u1, rh[0][0], rh[0][2], rh[0][1], rh[0][3], th[2], th[3]);
+                mma_tf32(c1, rl[0][0], rl[0][2], rl[0][1], rl[0][3], th[2], th[3]);
+                mma_tf32(u0, rh[0][0], rh[0][2], rh[0][1], rh[0][3], th[0], th[1]);
+                mma_tf32(c0, rl[0][0], rl[0][2], rl[0][1], rl[0][3], th[0], th[1]);
+                mma_tf32(u1, rh[1][0], rh[1][2], rh[1][1], rh[1][3], th[4], th[5]);
+                mma_tf32(c1, rh[0][0], rh[0][2], rh[0][1], rh[0][3], tl[2], tl[3]);
+                mma_tf32(c0, rh[0][0], rh[0][2], rh[0][1], rh[0][3], tl[0], tl[1]);
+                mma_tf32(c1, rl[1][0], rl[1][2], rl[1][1], rl[1][3], th[4], th[5]);
+                mma_tf32(c1, rh[1][0], rh[1][2], rh[1][1], rh[1][3], tl[4], tl[5]);
+                auto pair = [](float x, float y, uint32_t& hi, uint32_t& lo) {
+                    const __half2 h = __floats2half2_rn(x, y);
+                    const float2 f = __half22float2(h);
+                    hi = *reinterpret_cast<const uint32_t*>(&h);
+                    lo = pack_half2(x - f.x, y - f.y);
+                };
+                pair(u0[0] + c0[0], u0[1] + c0[1], ua[0], ul[0]);
+                pair(u0[2] + c0[2], u0[3] + c0[3], ua[1], ul[1]);
+                pair(u1[0] + c1[0], u1[1] + c1[1], ua[2], ul[2]);
+                pair(u1[2] + c1[2], u1[3] + c1[3], ua[3], ul[3]);
+            }
+#pragma unroll
+            for (int pp = 0; pp < 4; ++pp) {
+                uint32_t bd[4];
+                ldmatrix4_trans(bd, sl_u32 + O_BD + d_row + (((2 * pp + (mi >> 1)) ^ l7) << 4));
+                mma_f16(S[2 * pp], ua, bd[0], bd[1]);
+                mma_f16(S[2 * pp + 1], ua, bd[2], bd[3]);
+                mma_f16(S[2 * pp], ul, bd[0], bd[1]);
+                mma_f16(S[2 * pp + 1], ul, bd[2], bd[3]);
+            }
+            const uint4 mqb = *reinterpret_cast<const uint4*>(sl + O_M + 1024 + lane * 16);
+            mma_f16(ar[0], ua, mqb.x, mqb.y);
+            mma_f16(ar[1], ua, mqb.z, mqb.w);
+            __syncwarp();  // the slot is read; the previous chunk's output tile as well
+            if (lane == 0) mbar_arrive(&empty[slot]);
+            const uint32_t yt[4] = {pack_half2(ar[0][0], ar[0][1]), pack_half2(ar[0][2], ar[0][3]),
+                                    pack_half2(ar[1][0], ar[1][1]), pack_half2(ar[1][2], ar[1][3])};
+            stmatrix4_trans(y_st, yt);  // Y^T fragments as rows of 16 values per token
+            __syncwarp();
+            *reinterpret_cast<uint4*>(yp + (size_t)c * C * stride) = *reinterpret_cast<const uint4*>(ystage + y_ld);
+        }
+#pragma unroll
+        for (int pp = 0; pp < 4; ++pp)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf)
+                *reinterpret_cast<float4*>(p.state_out + srow + hf * 8 * N + pp * 16) =
+                    make_float4(S[2 * pp][2 * hf], S[2 * pp][2 * hf + 1], S[2 * pp + 1][2 * hf], S[2 * pp + 1][2 * hf + 1]);
     }
+out:;
+}
 
-    if (main_warp && tl < 64 && *abort_flag == 0) {
-        float* sp = p.state_out + ((size_t)bh * N + tl) * N + hi * 32;
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(sp + c) = make_float4(S[c], S[c + 1], S[c + 2], S[c + 3]);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        tmem_dealloc(tmem, TMEM_COLS);
-    }
+template <int W_MODE>
+static int launch_chunk(const ChunkArgs& p, int ctas, cudaStream_t st) {
+    const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_kernel<W_MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ck::SMEM_BYTES);
+    RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "wkv7_chunk_scan: %s", cudaGetErrorString(e));
+    wkv7_chunk_kernel<W_MODE><<<ctas, ck::THREADS, ck::SMEM_BYTES, st>>>(p);
+    return check_launch("wkv7_chunk_kernel");
 }
 
 }  // namespace rwkv7
@@ -568,16 +460,8 @@ extern "C" int rwkv7_wkv7_chunk_scan(const void* r, const void* w, const void* k
     for (const void* q : ptrs) RWKV7_REQUIRE(aligned(q, 16), RWKV7_ERR_ALIGN, "wkv7_chunk_scan: pointers must be 16-byte aligned");
     ChunkArgs p{reinterpret_cast<const __half*>(r), reinterpret_cast<const __half*>(k), reinterpret_cast<const __half*>(v),
                 reinterpret_cast<const __half*>(kk), reinterpret_cast<const __half*>(a), w, state_in, state_out,
-                reinterpret_cast<__half*>(y), T, H, w_mode, kernel_error_word()};
+                reinterpret_cast<__half*>(y), T, H, kernel_error_word()};
     RWKV7_REQUIRE(p.error != nullptr, RWKV7_ERR_CUDA, "wkv7_chunk_scan: cannot resolve the device error word");
-    ChunkMaps maps;
-    const void* srcs[6] = {r, k, v, kk, a, w};
-    for (int i = 0; i < 6; ++i) {
-        const bool f32 = (i == 5 && w_mode == 1);
-        if (int e2 = make_tmap_tokens(&maps.m[i], srcs[i], f32 ? 4 : 2, (uint64_t)B * T, H)) return e2;
-    }
-    cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ck::SMEM_BYTES);
-    RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "wkv7_chunk_scan: %s", cudaGetErrorString(e));
-    wkv7_chunk_kernel<<<B * H, ck::THREADS, ck::SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(maps, p);
-    return check_launch("wkv7_chunk_kernel");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return w_mode == 0 ? launch_chunk<0>(p, B * H, st) : w_mode == 1 ? launch_chunk<1>(p, B * H, st) : launch_chunk<2>(p, B * H, st);
 }

@@ -64,7 +64,6 @@ __device__ __forceinline__ void cvt4(const Raw4<T>& r, float (&o)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[i] = to_f<T>(r.v[i]);
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 template <typename TS> struct StateIO;
 template <> struct StateIO<float> {

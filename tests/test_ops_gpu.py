@@ -310,6 +310,23 @@ def test_grouped_lora_gemm_against_oracle(M):
     np.testing.assert_allclose(npf(y1), ref, rtol=4e-3, atol=4e-3)
 
 
+@pytest.mark.parametrize("T", [16, 64, 80, 96, 112, 208])
+def test_chunk_scan_ring_edges_with_raw_decay(T):
+    """The chunked scan around the lengths of its pipeline (four warps prepare 16-token chunks in turn, six chunks in the ring),
+    with the decay formed from raw logits in the kernel: against the sequential recurrence in 64 bits on the decay of those
+    logits.  The bounds are the test below's: fp16 outputs, tf32 / fp16 operands of the products."""
+    B, Hh = 2, 3
+    r, w, k, v, kk, a = wkv_inputs(B, T, Hh, N, seed=T)
+    rng = np.random.default_rng(T)
+    w_raw = (2 * rng.standard_normal((B, T, Hh, N))).astype(np.float16)
+    w = np.exp(-0.606531 / (1 + np.exp(-w_raw.astype(np.float64)))).astype(np.float32)
+    s0 = (0.1 * rng.standard_normal((B, Hh, N, N))).astype(np.float32)
+    yo, so = O.recurrent_scan(r, w, k, v, kk, a, s0, hi=True)
+    y, s = hb.self_chunk_rwkv7(*[cu(x) for x in (r, w_raw, k, v, kk, a, s0)], chunk_size=16, w_is_raw=True)
+    assert rel_err(npf(s), so) < 1e-3
+    assert rel_err(npf(y), yo.astype(np.float32)) < 2e-3
+
+
 @pytest.mark.parametrize("B,T,Hh,chunk", [(1, 64, 1, 64), (2, 128, 3, 16), (2, 192, 2, 32), (1, 1024, 2, 64)])
 def test_chunk_scan_tensor_core_against_oracle(B, T, Hh, chunk):
     """tcgen05 chunked WY scan == the sequential recurrence (fp64 oracle on the same fp16 inputs):
