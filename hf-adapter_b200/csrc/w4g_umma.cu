@@ -1,5 +1,5 @@
 // Decode-time int4 group-wise projection on the 5th-generation tensor cores (any row count; one pass over the
-// weights per 64 activation rows up to 64 rows, per 128 rows above).
+// weights per 64 activation rows up to 64 rows, per 128 or 256 rows above).
 //
 //   out[M, Nout] = epilogue( x[M, K] . W[Nout, K]^T ),  W = round_f16((nibble - zero) * scale)
 //
@@ -17,6 +17,8 @@
 //     the 4x larger fp16 tile never touches shared memory;
 //   * the activation tile [NB rows x 128 k] arrives by TMA (128-byte swizzle) and is the B operand from shared
 //     memory; D [128 x NB] fp32 accumulates in tensor memory;
+//   * without split-K the rounded output tile passes through the (by then free) activation ring and leaves in 16-byte pieces: a lane
+//     is a channel of the accumulator, and its own stores were two bytes each, 3.1 k cycles of epilogue in ffn.key;
 //   * split-K runs as a thread-block cluster along z; every CTA PUSHES the rows of its partial tile that belong to
 //     rank k straight from the accumulator registers into slot [own rank] of rank k's shared memory (remote stores
 //     are fire-and-forget, remote loads would cost a round trip), one cluster barrier, then each rank sums its slots
@@ -71,21 +73,22 @@ constexpr int Z_OFF = SC_OFF + TILE_N * 2;  // then 128 u8 zero-points, then pad
 constexpr int W4_BLOCK_BYTES = 8704;        // one int4 tile block in memory = one bulk copy (68 x 128 B)
 constexpr int W8_BLOCK_BYTES = TILE_N * KB;  // int8 per-channel format: 16 KiB of offset-binary bytes (q + 128), scales apart
 constexpr int TMEM_COLS = 512;
-constexpr int G = 3;                        // dequant groups (four groups with one A buffer each measured the same)
-constexpr int NA = 6;                       // A buffers (two per group) = weight stages = "done" barriers
 constexpr int HANDOFF_THREADS = 128 + 32;   // a dequant group arrives, its issuer warp syncs
 
 // NB = activation rows per weight pass = UMMA N.  64: two issuers, six activation stages sharing the "done" barriers
 // with the A buffers.  128: one issuer (tensor memory holds 6 A buffers + one 128-column accumulator), three
-// activation stages of 32 KiB with their own barriers.
+// activation stages of 32 KiB with their own barriers.  256: one issuer, two activation stages of 64 KiB, and the
+// 256-column accumulator leaves room for four A buffers, so two dequant groups.
 // FMT 0 = int4 group-128 (scales and zero-points inside the block), FMT 1 = int8 with one scale per output channel.
 template <int NB_, int FMT_>
 struct Cfg {
     static constexpr int NB = NB_, FMT = FMT_;
     static constexpr int BLOCK_BYTES = FMT_ == 0 ? W4_BLOCK_BYTES : W8_BLOCK_BYTES;
+    static constexpr int G = NB_ == 256 ? 2 : 3;  // dequant groups (four groups with one A buffer each measured the same)
+    static constexpr int NA = 2 * G;              // A buffers (two per group) = weight stages = "done" barriers
     static constexpr int WRING_BYTES = NA * BLOCK_BYTES;
     static constexpr int NISS = NB_ == 64 ? 2 : 1;
-    static constexpr int XST = NB_ == 64 ? 6 : 3;
+    static constexpr int XST = NB_ == 64 ? 6 : NB_ == 128 ? 3 : 2;
     static constexpr bool SHARED_DONE = XST == NA;  // one commit per block releases the activation stage and the A buffer
     static constexpr int XATOM = NB_ * 128, X_BYTES = 2 * XATOM;
     static constexpr int FIRST_DQ_WARP = 2 + NISS;
@@ -109,6 +112,7 @@ struct W4UmmaArgs {
     const __half* rscale[kW4MaxGroup];  // int8 format: one scale per output channel
     __half* out[kW4MaxGroup];
     const __half* residual;          // add epilogue (single projection only)
+    int vec;  // Nout is a multiple of 8 and every output (and the residual) starts on 16 bytes: rows move in 16-byte pieces
     int M, K, Nout, epilogue, nkb, kbt, splits, row_blocks;  // kbt = K / 128 (k-blocks per channel tile)
     unsigned int* error;
 };
@@ -178,7 +182,7 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
     using namespace w4;
     using C = Cfg<NBT, FMT>;
     constexpr int BLOCK_BYTES = C::BLOCK_BYTES, WRING_BYTES = C::WRING_BYTES;
-    constexpr int NB = C::NB, NISS = C::NISS, XST = C::XST, X_BYTES = C::X_BYTES, XATOM = C::XATOM;
+    constexpr int NB = C::NB, NISS = C::NISS, XST = C::XST, X_BYTES = C::X_BYTES, XATOM = C::XATOM, G = C::G, NA = C::NA;
     constexpr int FIRST_DQ_WARP = C::FIRST_DQ_WARP, NTHREADS = C::NTHREADS, A_COL = C::A_COL, D_COL = C::D_COL;
     extern __shared__ unsigned char smem_unaligned[];
     // the swizzled TMA / UMMA tiles need 1024-byte alignment; the offset is the same in every CTA
@@ -186,6 +190,7 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
     unsigned char* xs = smem;                                   // [XST][atom 0 | atom 1]
     unsigned char* raws = smem + XST * X_BYTES;                 // [NA][nibbles | scales | zeros]
     float* Q = reinterpret_cast<float*>(xs);                    // split-K exchange (after the last MMA)
+    __half* stage = reinterpret_cast<__half*>(xs);              // or the output tile [NB][TILE_N] without split-K
     uint64_t* bars = reinterpret_cast<uint64_t*>(raws + WRING_BYTES);
     uint64_t* full = bars;               // [XST] activation tile landed
     uint64_t* xfree = bars + XST;        // [XST] the MMAs that read the tile completed (unused when SHARED_DONE)
@@ -380,51 +385,34 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
         }
         if (ok && *abort_flag == 0) {
             tc_fence_after();
-            // 16-column chunks of the accumulator (activation rows) are dealt to the groups in turn
-            for (int c = g; c < NB / 16; c += G) {
-                const int col0 = c * 16;
-                uint32_t v[16];
-                tmem_ld16(lane_addr + D_COL + col0, v);
-                tc_wait_ld();
+            // eight columns of the accumulator (activation rows) at a time, dealt to the groups in turn
+            for (int c = g; c < NB / 8; c += G) {
+                const int col0 = c * 8;
+                if (col0 >= m_rows) break;
+                uint32_t v[8];
+                tmem_ld8(lane_addr + D_COL + col0, v);
                 if (NISS == 2 && nkb > 1) {  // the second issuer's accumulator
-                    uint32_t t[16];
-                    tmem_ld16(lane_addr + D_COL + NB + col0, t);
+                    uint32_t t[8];
+                    tmem_ld8(lane_addr + D_COL + NB + col0, t);
                     tc_wait_ld();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(t[e]));
+                    for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(t[e]));
+                } else {
+                    tc_wait_ld();
                 }
                 if (!clustered) {
-                    // No split-K: nothing to exchange, so the accumulator goes straight to global memory (fp16
-                    // rounding, epilogue, 2-byte stores: the 32 lanes of a warp cover 64 contiguous bytes of a row).
-                    const int nn = n0 + row;
-                    grid_dependency_wait();  // returns at once (the accumulator already depends on the activations)
-                    if (nn < p.Nout) {
-                        const float rs = FMT == 1 ? __half2float(p.rscale[grp_idx][nn]) : 1.f;
+                    // No split-K: nothing to exchange.  The rounded values pass through the activation ring, which is free by now, as
+                    // [row][channel], so that rows leave in 16-byte pieces below (a lane is a channel here: its own stores would be
+                    // two bytes each).
+                    const float rs = FMT == 1 && n0 + row < p.Nout ? __half2float(p.rscale[grp_idx][n0 + row]) : 1.f;
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const int m = col0 + e;
-                            if (m >= m_rows) break;
-                            const size_t o = (size_t)(m0 + m) * p.Nout + nn;
-                            float y = __half2float(__float2half_rn(__uint_as_float(v[e]) * rs));
-                            if (p.epilogue == RWKV7_EPI_RELU2) {
-                                y = fmaxf(y, 0.f);
-                                y *= y;
-                            } else if (p.epilogue == RWKV7_EPI_ADD) {
-                                y += __half2float(p.residual[o]);
-                            }
-                            outp[o] = __float2half_rn(y);
-                        }
-                    }
-                } else if (col0 < m_rows) {
+                    for (int e = 0; e < 8; ++e) stage[(col0 + e) * TILE_N + row] = __float2half_rn(__uint_as_float(v[e]) * rs);
+                } else {
                     // 8 consecutive rows never straddle two ranks (rows_per_rank is a multiple of 8)
+                    const int dst = col0 / rows_per_rank;
+                    float* qd = cluster.map_shared_rank(Q, dst) + ((size_t)split * rows_per_rank + (col0 - dst * rows_per_rank)) * TILE_N + row;
 #pragma unroll
-                    for (int h8 = 0; h8 < 2; ++h8) {
-                        const int m = col0 + h8 * 8;
-                        const int dst = m / rows_per_rank;
-                        float* qd = cluster.map_shared_rank(Q, dst) + ((size_t)split * rows_per_rank + (m - dst * rows_per_rank)) * TILE_N + row;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) qd[e * TILE_N] = __uint_as_float(v[h8 * 8 + e]);
-                    }
+                    for (int e = 0; e < 8; ++e) qd[e * TILE_N] = __uint_as_float(v[e]);
                 }
             }
             tc_fence_before();
@@ -444,6 +432,35 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
     }
     const bool aborted = (*abort_flag != 0);
     grid_dependency_wait();  // residual reads and output writes are ordered after the preceding kernel (returns at once here)
+    if (!aborted && !clustered) {
+        // 16-byte pieces of the staged rows: 16 threads cover the 256 bytes of a row
+        for (int idx = tid; idx < m_rows * (TILE_N / 8); idx += NTHREADS) {
+            const int m = idx / (TILE_N / 8), n = n0 + idx % (TILE_N / 8) * 8;
+            if (n >= p.Nout) continue;
+            float y[8];
+            load8(stage + idx * 8, y);
+            const size_t o = (size_t)(m0 + m) * p.Nout + n;
+            if (p.epilogue == RWKV7_EPI_RELU2) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    y[e] = fmaxf(y[e], 0.f);
+                    y[e] *= y[e];
+                }
+            }
+            if (p.vec) {
+                if (p.epilogue == RWKV7_EPI_ADD) {
+                    float r[8];
+                    load8(p.residual + o, r);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) y[e] += r[e];
+                }
+                store8(outp + o, y);
+            } else {
+                for (int e = 0; e < 8 && n + e < p.Nout; ++e)
+                    outp[o + e] = __float2half_rn(p.epilogue == RWKV7_EPI_ADD ? y[e] + __half2float(p.residual[o + e]) : y[e]);
+            }
+        }
+    }
     if (!aborted && clustered) {
         // Each thread owns one channel pair (n, n+1) and walks the rows of this rank's share: float2 loads of the rank
         // slots in fixed order, fp16 rounding, epilogue, one 4-byte store; 64 consecutive threads cover one 256-byte
@@ -580,24 +597,40 @@ static cudaError_t launch_variant(cudaLaunchConfig_t& cfg, const W4Maps& maps, c
     return cudaLaunchKernelEx(&cfg, w4g_umma_kernel<NBT, FMT>, maps, a);
 }
 
+// Activation rows per pass over the weights.  Above 128 a pass of 256 halves the CTAs, which pays where the passes of 128 take
+// more waves than one or the K range of a CTA is long, and costs where it only turns into split-K with its exchange of 256
+// rows.  The estimate counts tens of cycles: 105 / 164 a k-block (at 128 / 256 rows the activations' way through L2 bounds it,
+// 32..40 bytes a clock and SM, not the tensor pipe), 1400 / 2200 for the exchange and what surrounds it, 450 without.  us at 129 / 256 / 257 / 512 rows, int4, 128 -> 256 rows a pass: 4096 -> 16384 39.9 / 41.8 / 59.8 / 81.8 -> 27.7 / 30.2 /
+// 55.7 / 60.7; 3 x 4096 -> 4096 38.7 / 40.6 / 41.0 / 61.0 -> 27.4 / 29.2 / 52.5 / 56.3; 4096 -> 4096 15.3 / 16.2 / 20.3 / 20.7 -> 17.3 / 19.5 /
+// 26.0 / 26.4; 16384 -> 4096 44.4 / 44.9 / 87.0 / 88.4 -> 39.5 / 42.4 / 74.7 / 74.4; 3 x 2560 -> 2560 14.1 / 14.6 / 26.0 / 28.4 -> 20.6 / 22.0 /
+// 19.4 / 20.0; 10240 -> 2560 29.4 / 30.6 / 30.6 / 57.3 -> 28.6 / 31.0 / 48.8 / 52.6.
+static int rows_per_pass(int M, int tiles, int G, int total_kb, int splits128, int splits256) {
+    if (M <= 128) return M > 64 ? 128 : 64;
+    const auto cost = [&](int nb, int splits) {
+        const long long ctas = (long long)tiles * ((M + nb - 1) / nb) * G * splits;
+        const long long exchange = splits == 1 ? 450 : nb == 128 ? 1400 : 2200;
+        return (ctas + 147) / 148 * ((long long)(total_kb / splits) * (nb == 128 ? 105 : 164) + exchange);
+    };
+    return cost(256, splits256) < cost(128, splits128) ? 256 : 128;
+}
+
 // fmt 0: int4 group-wise tiled weights; fmt 1: int8 tiled weights with per-channel scales rscales[g] [Nout].
 int launch_w4g_umma_tiled(const void* const* xs, const uint8_t* const* tws, const void* const* rscales, const void* residual,
                           void* const* outs, int G, int M, int K, int Nout, int epilogue, int fmt, cudaStream_t st) {
     using namespace w4;
     RWKV7_REQUIRE(G >= 1 && G <= kW4MaxGroup, RWKV7_ERR_UNSUPPORTED, "w4g_gemv_tiled: 1..%d projections per launch (got %d)", kW4MaxGroup, G);
-    const int NB = M > 64 ? 128 : 64;          // activation rows per pass over the weights
-    RWKV7_REQUIRE(M >= 1 && (long long)G * ((M + NB - 1) / NB) <= 65535, RWKV7_ERR_UNSUPPORTED, "w4g_gemv_tiled: M out of range (got %d)", M);
-    const int row_blocks = (M + NB - 1) / NB;
+    RWKV7_REQUIRE(M >= 1 && (long long)G * ((M + 127) / 128) <= 65535, RWKV7_ERR_UNSUPPORTED, "w4g_gemv_tiled: M out of range (got %d)", M);
     RWKV7_REQUIRE(K % KB == 0, RWKV7_ERR_UNSUPPORTED, "w4g_gemv_tiled: K must be a multiple of %d (got %d)", KB, K);
     const int tiles = (Nout + TILE_N - 1) / TILE_N;
     const int total_kb = K / KB;
-    int splits = 1;
-    for (int s = 8; s >= 2; s >>= 1) {
-        if (tiles * row_blocks * G * s <= 148 && total_kb % s == 0 && (total_kb / s) >= 4) {
-            splits = s;
-            break;
-        }
-    }
+    const auto splits_for = [&](int nb) {
+        for (int s = 8; s >= 2; s >>= 1)
+            if ((long long)tiles * ((M + nb - 1) / nb) * G * s <= 148 && total_kb % s == 0 && total_kb / s >= 4) return s;
+        return 1;
+    };
+    const int NB = rows_per_pass(M, tiles, G, total_kb, splits_for(128), splits_for(256));
+    const int row_blocks = (M + NB - 1) / NB;
+    const int splits = splits_for(NB);
     const int nkb = total_kb / splits;
     W4Maps maps;
     W4UmmaArgs a{};
@@ -608,6 +641,7 @@ int launch_w4g_umma_tiled(const void* const* xs, const uint8_t* const* tws, cons
         a.rscale[g] = rscales ? reinterpret_cast<const __half*>(rscales[g]) : nullptr;
         a.out[g] = reinterpret_cast<__half*>(outs[g]);
         fresh |= take_tiled_fresh(tws[g]);
+        a.vec = (g == 0 || a.vec) && Nout % 8 == 0 && aligned(outs[g], 16) && aligned(residual, 16);
     }
     for (int g = G; g < kW4MaxGroup; ++g) maps.x[g] = maps.x[0];
     a.residual = reinterpret_cast<const __half*>(residual);
@@ -629,7 +663,8 @@ int launch_w4g_umma_tiled(const void* const* xs, const uint8_t* const* tws, cons
     cfg.attrs = attr;
     cfg.numAttrs = (!fresh && programmatic_launch_ok(cfg.stream)) ? 2 : 1;
     const cudaError_t e = NB == 64 ? (fmt == 0 ? launch_variant<64, 0>(cfg, maps, a) : launch_variant<64, 1>(cfg, maps, a))
-                                   : (fmt == 0 ? launch_variant<128, 0>(cfg, maps, a) : launch_variant<128, 1>(cfg, maps, a));
+                          : NB == 128 ? (fmt == 0 ? launch_variant<128, 0>(cfg, maps, a) : launch_variant<128, 1>(cfg, maps, a))
+                                      : (fmt == 0 ? launch_variant<256, 0>(cfg, maps, a) : launch_variant<256, 1>(cfg, maps, a));
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "w4g_gemv_tiled launch: %s", cudaGetErrorString(e));
     return RWKV7_OK;
 }

@@ -186,6 +186,30 @@ def test_w4g_tensor_core_path(M, K, Nn):
     assert _lib.kernel_status(True) == 0
 
 
+@pytest.mark.parametrize("M", [64, 128, 129, 256, 257])
+@pytest.mark.parametrize("K,Nn", [(128, 128), (640, 130), (1024, 256), (256, 9602), (12288, 2432)])
+def test_tiled_projection_row_blocks_and_output_rows(M, K, Nn):
+    """The tcgen05 projection kernel at the edges of its row blocks (64, 128, 256 activation rows a pass), with and without
+    split-K, with rows that leave in 16-byte pieces and widths that do not allow it, every epilogue, against the
+    oracle.  Bounds as for the other tests of the kernel (fp16 outputs of sums of K products of N(0, 0.02) and N(0, 1)), and for
+    a long K the rounding of the oracle's int8 weights, which the kernel does not do (it scales the sum): 2^-12 / sqrt(3) of a
+    weight on average, eight times the deviation of a sum of K of them."""
+    rng = np.random.default_rng(M + K + Nn)
+    atol = max(2e-3, 8 * 0.02 * np.sqrt(K) * 2.0 ** -12 / np.sqrt(3))
+    W = (0.02 * rng.standard_normal((Nn, K))).astype(np.float16)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    res = rng.standard_normal((M, Nn)).astype(np.float16)
+    packed, scales = O.quantize_w4_groupwise(W, 128)
+    q, s = O.quantize_w8_row(W)
+    t4, t8 = hb.w4_repack_tiled(cu(packed), cu(scales), K, 128), hb.w8_repack_tiled(cu(q))
+    for yo, run in ((O.w4_groupwise_linear(x, packed, scales), lambda **kw: hb.w4_tiled_linear(cu(x), t4, Nn, K, **kw)),
+                    (O.w8_linear(x, q, s), lambda **kw: hb.w8_tiled_linear_group((cu(x),), (t8,), (cu(s),), Nn, K, **kw)[0])):
+        yo = yo.astype(np.float32)
+        np.testing.assert_allclose(npf(run()), yo, rtol=2e-3, atol=atol)
+        np.testing.assert_allclose(npf(run(relu2=True)), np.maximum(yo, 0) ** 2, rtol=4e-3, atol=4e-3)
+        np.testing.assert_allclose(npf(run(residual=cu(res))), yo + res.astype(np.float32), rtol=2e-3, atol=2 * atol)
+
+
 @pytest.mark.parametrize("G,M,K,Nn", [(3, 64, 4096, 4096), (3, 7, 512, 200), (2, 130, 1024, 256), (4, 64, 1024, 128), (1, 33, 2048, 384)])
 def test_w4g_grouped_projections(G, M, K, Nn):
     """G projections of one shape in a single launch: each output equals the oracle (and, where the split-K plan is
