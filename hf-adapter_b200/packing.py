@@ -258,40 +258,37 @@ _DEFAULT_CONTEXT = StepContext()
 
 def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
     """r / k / v and the LoRA pre-activations of a layer step on parallel branches: ``[r, k, v, w, a, g(, v_gate)]``."""
-    xr, xk, xv = xs
-    # The LoRA chain does not depend on r/k/v: it runs on a side stream (a parallel branch of the decode graph once
-    # captured) and joins before the recurrence.
+    # The LoRA chain is two launches long and leads on the main stream, behind the kernel that made its inputs; r / k / v do not
+    # depend on it and branch off (parallel branches of the decode graph once captured), joined before the recurrence.
     main = torch.cuda.current_stream(x.device)
-    side = ctx.side_stream(x.device, 0)
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)])
-        lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups])
-    rkv = rkv_grouped(ops, xr, xk, xv) if all(isinstance(o, _QUANT_TYPES) for o in ops) else None
-    if rkv is not None:
-        # int4 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
+    fork = main.record_event()
+    hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)])
+    lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups])
+    used = []
+
+    def branch(i, t, run):
+        st = ctx.side_stream(x.device, i)
+        if st not in used:
+            st.wait_event(fork)
+            used.append(st)
+        with torch.cuda.stream(st):
+            y = run()
+        for v in t:
+            v.record_stream(st)
+        return y
+
+    rkv = None
+    if all(isinstance(o, _QUANT_TYPES) for o in ops):
+        # int4 / int8 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
         # exchange) instead of three launches competing for the SMs
-        r, k, v = rkv
-        main.wait_stream(side)
-    else:
+        rkv = branch(0, xs, lambda: rkv_grouped(ops, *xs))
+    if rkv is None:
         # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
-        sk, sv = ctx.side_stream(x.device, 1), ctx.side_stream(x.device, 2)
-        sk.wait_stream(main)
-        sv.wait_stream(main)
-        with torch.cuda.stream(sk):
-            k = apply_linear(ops[1], xk)
-        with torch.cuda.stream(sv):
-            v = apply_linear(ops[2], xv)
-        r = apply_linear(ops[0], xr)
-        main.wait_stream(side)
-        main.wait_stream(sk)
-        main.wait_stream(sv)
-        xk.record_stream(sk); xv.record_stream(sv)
-        _used_on(main, k, v)
-    for t_ in down_x:
-        t_.record_stream(side)
-    _used_on(main, *lora)
-    return [r, k, v, *lora]
+        rkv = [branch(i, (t,), lambda: apply_linear(o, t)) for i, (o, t) in enumerate(zip(ops, xs))]
+    for st in used:
+        main.wait_stream(st)
+    _used_on(main, *rkv)
+    return [*rkv, *lora]
 
 
 def _used_on(stream, *ts):
