@@ -5,9 +5,12 @@
 // One launch covers the four rank-R "down" projections (K = d_model, Nout = rank) or the four "up"
 // projections (K = rank, Nout = attention width) of a layer.  These matrices are tiny (a few MB per
 // layer in total), so the kernel is built for latency: warp-level HMMA (mma.sync m16n8k16, fp32
-// accumulate) on 64 x 64 output tiles, cp.async double-buffered 64-wide K chunks with an XOR swizzle
-// for conflict-free ldmatrix, and split-K across a thread-block cluster whose partial tiles are
-// reduced through distributed shared memory in fixed rank order (deterministic, no scratch memory).
+// accumulate) on 64 x 64 output tiles, 64-wide K chunks by cp.async with an XOR swizzle for
+// conflict-free ldmatrix, three of them in flight where a CTA has more than two, and split-K across a
+// thread-block cluster whose partial tiles are reduced through distributed shared memory in fixed
+// rank order (deterministic, no scratch memory).  The pair of launches is the longest branch of a decode
+// step over many rows: with one chunk in flight, weights not announced and outputs stored one by one
+// 64 rows of the 7.2B shape took 3214 us a step, 3152 now, 64 rows of the 2.9B shape 2419 and 2344.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -17,6 +20,7 @@ namespace cg = cooperative_groups;
 namespace rwkv7 {
 
 constexpr int kMaxProblems = 4;
+template <typename T> struct alignas(2 * sizeof(T)) Pair { T x, y; };
 constexpr int LT = 64;         // tile rows (activations) and tile columns (outputs)
 constexpr int LK = 64;         // K chunk
 constexpr int LTHREADS = 128;  // 4 warps as 2 x 2, warp tile 32 x 32
@@ -28,6 +32,7 @@ struct GroupArgs {
     void* out[kMaxProblems];
     int K[kMaxProblems], Nout[kMaxProblems], act[kMaxProblems];
     int M, splits, max_tiles;
+    int pairs;  // every output has an even width and starts on 4 bytes: two columns per store
 };
 
 __device__ __forceinline__ void lcp16(void* smem, const void* g, bool valid) {
@@ -61,20 +66,22 @@ __device__ __forceinline__ float lora_act(float v, int act) {
     return v;
 }
 
-template <typename T>
+// NST: K chunks in shared memory (2, or 4 where a CTA has more than two: then all but one of them are in flight)
+template <typename T, int NST>
 __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupArgs p) {
-    __shared__ __align__(128) unsigned char sX[2][LT * 128];
-    __shared__ __align__(128) unsigned char sW[2][LT * 128];
-    __shared__ __align__(16) float sP[LT * LT];  // partial tile for the split-K reduction
+    extern __shared__ __align__(128) unsigned char lsm[];
+    auto sX = reinterpret_cast<unsigned char(*)[LT * 128]>(lsm);                     // [NST]
+    auto sW = reinterpret_cast<unsigned char(*)[LT * 128]>(lsm + NST * LT * 128);    // [NST]
+    float* sP = reinterpret_cast<float*>(lsm);  // [LT * LT] partial tile for the split-K reduction, over the chunks when they are done
 
-    // launched programmatically: resident under the tail of the preceding kernel of the stream, everything below after it
-    grid_dependency_wait();
-    if (threadIdx.x == 0) grid_launch_dependents();
     const int prob = blockIdx.y;
     const int K = p.K[prob], Nout = p.Nout[prob];
     const int n0 = (blockIdx.x % p.max_tiles) * LT;
     const int r0 = (blockIdx.x / p.max_tiles) * LT;  // activation row block
-    if (n0 >= Nout) return;  // whole cluster shares blockIdx.x / y, so it leaves together
+    if (n0 >= Nout) {  // whole cluster shares blockIdx.x / y, so it leaves together
+        grid_dependency_wait();
+        return;
+    }
     const int split = blockIdx.z, S = p.splits;
     const int chunks_total = (K + LK - 1) / LK;
     const int chunks_per = (chunks_total + S - 1) / S;
@@ -93,10 +100,21 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
 
-    auto load_chunk = [&](int buf, int c) {
+    // launched programmatically: resident under the tail of the preceding kernel of the stream.  The weights are on their way to L2
+    // (a hint: whoever wrote them, the reads below see it), everything is read after that kernel.
+    if (r0 == 0) {
+        for (int i = tid; i < LT * (c_end - c_begin); i += LTHREADS) {
+            const int row = n0 + i % LT, k = (c_begin + i / LT) * LK;
+            if (row < Nout && k < K) prefetch_l2(W + (size_t)row * K + k);
+        }
+    }
+    grid_dependency_wait();
+    if (tid == 0) grid_launch_dependents();
+
+    auto load_chunk = [&](int buf, int c) {  // past the end: an empty group, so that the count of groups stays that of chunks
         const int k0 = c * LK;
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {  // 64 rows x 8 chunks = 512 chunks per operand, 128 threads
+        for (int it = 0; it < 4 && c < c_end; ++it) {  // 64 rows x 8 chunks = 512 chunks per operand, 128 threads
             const int idx = tid + it * LTHREADS;
             const int row = idx >> 3, ch = idx & 7;
             const bool kin = (k0 + ch * 8) < K;
@@ -108,16 +126,13 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
         asm volatile("cp.async.commit_group;\n" ::);
     };
 
-    if (c_begin < c_end) load_chunk(0, c_begin);
+#pragma unroll
+    for (int s = 0; s < NST - 1; ++s) load_chunk(s, c_begin + s);
     for (int c = c_begin; c < c_end; ++c) {
-        const int buf = (c - c_begin) & 1;
-        if (c + 1 < c_end) {
-            load_chunk(buf ^ 1, c + 1);
-            asm volatile("cp.async.wait_group 1;\n" ::);
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::);
-        }
-        __syncthreads();
+        const int buf = (c - c_begin) % NST;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(NST - 2));
+        __syncthreads();  // chunk c is there, and chunk c - 1, whose buffer the next load takes, is read
+        load_chunk((c - c_begin + NST - 1) % NST, c + NST - 1);
 #pragma unroll
         for (int ks = 0; ks < LK / 16; ++ks) {
             uint32_t af[2][4], bf[2][4];
@@ -136,12 +151,12 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
 #pragma unroll
                 for (int j = 0; j < 4; ++j) hmma<T>(acc[i][j], af[i], bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
         }
-        __syncthreads();
     }
 
     const int gid = lane >> 2, tig = lane & 3;
     cg::cluster_group cluster = cg::this_cluster();
     if (S > 1) {
+        __syncthreads();  // the last chunk is read
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -176,17 +191,34 @@ __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupA
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = wm * 32 + i * 16 + gid + (e >> 1) * 8, cidx = n0 + wn * 32 + j * 8 + tig * 2 + (e & 1);
-                    if (r0 + r < p.M && cidx < Nout) {
-                        float v = acc[i][j][e];
-                        if (bias) v += to_f<T>(bias[cidx]);
-                        v = round_to<T>(v);
-                        if (p.act[prob]) v = lora_act(v, p.act[prob]);
-                        out[(size_t)(r0 + r) * Nout + cidx] = from_f<T>(v);
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int r = r0 + wm * 32 + i * 16 + gid + hh * 8, cidx = n0 + wn * 32 + j * 8 + tig * 2;
+                    if (r >= p.M || cidx >= Nout) continue;
+                    T* o = out + (size_t)r * Nout + cidx;
+                    Pair<T> v;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float f = acc[i][j][hh * 2 + e];
+                        if (bias && cidx + e < Nout) f += to_f<T>(bias[cidx + e]);
+                        f = round_to<T>(f);
+                        if (p.act[prob]) f = lora_act(f, p.act[prob]);
+                        (e ? v.y : v.x) = from_f<T>(f);
+                    }
+                    if (p.pairs) {
+                        *reinterpret_cast<Pair<T>*>(o) = v;
+                    } else {
+                        o[0] = v.x;
+                        if (cidx + 1 < Nout) o[1] = v.y;
                     }
                 }
     }
+}
+
+template <typename T, int NST>
+static cudaError_t launch_group(cudaLaunchConfig_t& cfg, const GroupArgs& a) {
+    cfg.dynamicSmemBytes = 2 * NST * LT * 128;
+    const cudaError_t e = cudaFuncSetAttribute(small_gemm_group_kernel<T, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+    return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<T, NST>, a);
 }
 
 }  // namespace rwkv7
@@ -213,6 +245,7 @@ extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, cons
         a.K[i] = K[i]; a.Nout[i] = Nout[i]; a.act[i] = act_out[i];
         max_tiles = max_tiles > (Nout[i] + LT - 1) / LT ? max_tiles : (Nout[i] + LT - 1) / LT;
         max_k = max_k > K[i] ? max_k : K[i];
+        a.pairs = (i == 0 || a.pairs) && Nout[i] % 2 == 0 && aligned(out[i], 4);
     }
     a.M = M;
     // split K across a cluster when there are few output tiles and a long K (the "down" projections)
@@ -224,7 +257,6 @@ extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, cons
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(max_tiles * row_blocks, n_problems, splits);
     cfg.blockDim = dim3(LTHREADS);
-    cfg.dynamicSmemBytes = 0;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -236,8 +268,9 @@ extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, cons
     cfg.attrs = attr;
     cfg.numAttrs = programmatic_launch_ok(cfg.stream) ? 2 : 1;
     cudaError_t e;
-    if (dtype == RWKV7_F16) e = cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<__half>, a);
-    else e = cudaLaunchKernelEx(&cfg, small_gemm_group_kernel<__nv_bfloat16>, a);
+    const bool deep = (chunks + splits - 1) / splits > 2;
+    if (dtype == RWKV7_F16) e = deep ? launch_group<__half, 4>(cfg, a) : launch_group<__half, 2>(cfg, a);
+    else e = deep ? launch_group<__nv_bfloat16, 4>(cfg, a) : launch_group<__nv_bfloat16, 2>(cfg, a);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "small_gemm_group launch: %s", cudaGetErrorString(e));
     return RWKV7_OK;
 }
