@@ -64,63 +64,85 @@ __global__ void __launch_bounds__(256) dense_small_kernel(const DenseArgs p) {
 struct PrepArgs {
     const void *w_raw, *k_raw, *v_raw, *a, *k_k, *k_a, *v_first, *v_gate;
     float* w_out;
-    void *k_out, *v_out, *kk_out;
+    void *k_out, *v_out, *kk_out, *a_out;
     int H, a_is_raw, v_gate_is_raw, log_decay;
     long long total_heads;  // rows * H
 };
 
-// one 16-lane group per (row, head): 4 columns per lane
+// V consecutive columns in storage type, 16 bytes: requested together and converted where they are used
+template <typename T, int V> struct alignas(16) Piece { T v[V]; };
+template <typename T, int V>
+__device__ __forceinline__ Piece<T, V> get_piece(const void* base, size_t off, bool ok = true) {
+    Piece<T, V> r{};
+    if (ok) r = *reinterpret_cast<const Piece<T, V>*>(reinterpret_cast<const T*>(base) + off);
+    return r;
+}
+template <typename T, int V>
+__device__ __forceinline__ void put_piece(void* base, size_t off, const float (&o)[V]) {
+    Piece<T, V> r;
+#pragma unroll
+    for (int c = 0; c < V; ++c) r.v[c] = from_f<T>(o[c]);
+    *reinterpret_cast<Piece<T, V>*>(reinterpret_cast<T*>(base) + off) = r;
+}
+
+// 64 / V lanes per (row, head), V columns per lane.  Bound: HBM.  32768 rows of 4096 fp16 with raw gates, no decay (five tensors read,
+// three written, 2.1 GB): 565 us with four columns a lane and the v gate requested behind the head's norm, 416 now; the gate
+// written as well 438, where a pass of its own took 114.
 template <typename T>
 __global__ void __launch_bounds__(256) state_prep_kernel(const PrepArgs p) {
-    const long long gidx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-    const int l16 = threadIdx.x & 15;
+    constexpr int V = 16 / (int)sizeof(T), LANES = 64 / V;
+    const long long gidx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const int l = threadIdx.x % LANES;
     const bool active = gidx < p.total_heads;
     const long long g = active ? gidx : p.total_heads - 1;  // keep the shuffle groups converged
     const int h = (int)(g % p.H);
-    const size_t off = (size_t)g * 64 + l16 * 4;
-    const int hoff = h * 64 + l16 * 4;
-    float w[4] = {0.f, 0.f, 0.f, 0.f}, k[4], v[4], a[4], ks[4], ka[4];
-    if (p.w_raw) load4(reinterpret_cast<const T*>(p.w_raw) + off, w);  // absent: K / V / KK only (the scan takes raw w)
-    load4(reinterpret_cast<const T*>(p.k_raw) + off, k);
-    load4(reinterpret_cast<const T*>(p.v_raw) + off, v);
-    load4(reinterpret_cast<const T*>(p.a) + off, a);
-    load4(reinterpret_cast<const T*>(p.k_k) + hoff, ks);
-    load4(reinterpret_cast<const T*>(p.k_a) + hoff, ka);
-    float kk[4], n2 = 0.f;
+    const size_t off = (size_t)g * 64 + l * V;
+    const int hoff = h * 64 + l * V;
+    const bool interp = p.v_first && p.v_gate;
+    const Piece<T, V> q_k = get_piece<T, V>(p.k_raw, off), q_a = get_piece<T, V>(p.a, off), q_v = get_piece<T, V>(p.v_raw, off),
+                      q_vf = get_piece<T, V>(p.v_first, off, interp), q_vg = get_piece<T, V>(p.v_gate, off, interp),
+                      q_w = get_piece<T, V>(p.w_raw, off, p.w_raw != nullptr),  // absent: k / v / kk only (the scan takes raw w)
+                      q_ks = get_piece<T, V>(p.k_k, hoff), q_ka = get_piece<T, V>(p.k_a, hoff);
+    float a[V], kk[V], ko[V], n2 = 0.f;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < V; ++c) {
+        a[c] = to_f<T>(q_a.v[c]);
         if (p.a_is_raw) a[c] = sigmoidf_(a[c]);
-        kk[c] = k[c] * ks[c];
+        const float k = to_f<T>(q_k.v[c]);
+        kk[c] = k * to_f<T>(q_ks.v[c]);
+        ko[c] = k * (1.0f + (a[c] - 1.0f) * to_f<T>(q_ka.v[c]));
         n2 += kk[c] * kk[c];
     }
-    n2 = group_sum<16>(n2);
+    n2 = group_sum<LANES>(n2);
     const float inv = 1.0f / fmaxf(sqrtf(n2), 1e-12f);
-    float wo[4] = {0.f, 0.f, 0.f, 0.f}, ko[4];
+    float v[V];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < V; ++c) {
         kk[c] *= inv;
-        ko[c] = k[c] * (1.0f + (a[c] - 1.0f) * ka[c]);
-        if (p.w_out) {  // two exponentials and a division an element that the tensor-core scan's caller does not want
-            const float lw = -0.606531f * sigmoidf_(w[c]);
-            wo[c] = p.log_decay ? lw : expf(lw);
+        v[c] = to_f<T>(q_v.v[c]);
+        if (interp) {
+            float vg = to_f<T>(q_vg.v[c]);
+            if (p.v_gate_is_raw) vg = sigmoidf_(vg);
+            v[c] = v[c] + (to_f<T>(q_vf.v[c]) - v[c]) * vg;
         }
     }
-    if (p.v_first && p.v_gate) {
-        float vf[4], vg[4];
-        load4(reinterpret_cast<const T*>(p.v_first) + off, vf);
-        load4(reinterpret_cast<const T*>(p.v_gate) + off, vg);
+    if (!active) return;
+    if (p.w_out) {  // two exponentials and a division an element that the tensor-core scan's caller does not want
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (p.v_gate_is_raw) vg[c] = sigmoidf_(vg[c]);
-            v[c] = v[c] + (vf[c] - v[c]) * vg[c];
+        for (int c = 0; c < V; c += 4) {
+            float wo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float lw = -0.606531f * sigmoidf_(to_f<T>(q_w.v[c + e]));
+                wo[e] = p.log_decay ? lw : expf(lw);
+            }
+            *reinterpret_cast<float4*>(p.w_out + off + c) = make_float4(wo[0], wo[1], wo[2], wo[3]);
         }
     }
-    if (active) {
-        if (p.w_out) *reinterpret_cast<float4*>(p.w_out + off) = make_float4(wo[0], wo[1], wo[2], wo[3]);
-        store4(reinterpret_cast<T*>(p.k_out) + off, ko);
-        store4(reinterpret_cast<T*>(p.v_out) + off, v);
-        store4(reinterpret_cast<T*>(p.kk_out) + off, kk);
-    }
+    put_piece<T, V>(p.k_out, off, ko);
+    put_piece<T, V>(p.v_out, off, v);
+    put_piece<T, V>(p.kk_out, off, kk);
+    if (p.a_out) put_piece<T, V>(p.a_out, off, a);
 }
 
 // ---------------------------------------------------------------- attn_output_prepare
@@ -188,10 +210,10 @@ extern "C" int rwkv7_dense_small(const void* x, const void* W, const void* bias,
     return RWKV7_OK;
 }
 
-extern "C" int rwkv7_prefill_state_prep(const void* w_raw, const void* k_raw, const void* v_raw, const void* a,
-                                        const void* k_k, const void* k_a, const void* v_first, const void* v_gate,
-                                        float* w_out, void* k_out, void* v_out, void* kk_out, int rows, int H, int N,
-                                        int a_is_raw, int v_gate_is_raw, int log_decay, int dtype, void* stream) {
+extern "C" int rwkv7_prefill_state_prep_gate(const void* w_raw, const void* k_raw, const void* v_raw, const void* a,
+                                             const void* k_k, const void* k_a, const void* v_first, const void* v_gate,
+                                             float* w_out, void* k_out, void* v_out, void* kk_out, void* a_out, int rows, int H, int N,
+                                             int a_is_raw, int v_gate_is_raw, int log_decay, int dtype, void* stream) {
     RWKV7_REQUIRE(N == 64, RWKV7_ERR_UNSUPPORTED, "prefill_state_prep: head size must be 64, got %d", N);
     RWKV7_REQUIRE(rows > 0 && H > 0, RWKV7_ERR_INVALID, "prefill_state_prep: sizes must be positive");
     RWKV7_REQUIRE(k_raw && v_raw && a && k_k && k_a && k_out && v_out && kk_out, RWKV7_ERR_INVALID,
@@ -200,18 +222,26 @@ extern "C" int rwkv7_prefill_state_prep(const void* w_raw, const void* k_raw, co
                   "prefill_state_prep: w_raw and w_out must be given together (both NULL = no decay output)");
     RWKV7_REQUIRE((v_first == nullptr) == (v_gate == nullptr), RWKV7_ERR_INVALID,
                   "prefill_state_prep: v_first and v_gate must be given together");
-    const void* ptrs[] = {w_raw, k_raw, v_raw, a, k_k, k_a, v_first, v_gate, w_out, k_out, v_out, kk_out};
+    const void* ptrs[] = {w_raw, k_raw, v_raw, a, k_k, k_a, v_first, v_gate, w_out, k_out, v_out, kk_out, a_out};
     for (const void* q : ptrs) RWKV7_REQUIRE(aligned(q, 16), RWKV7_ERR_ALIGN, "prefill_state_prep: unaligned pointer");
-    PrepArgs p{w_raw, k_raw, v_raw, a, k_k, k_a, v_first, v_gate, w_out, k_out, v_out, kk_out,
+    PrepArgs p{w_raw, k_raw, v_raw, a, k_k, k_a, v_first, v_gate, w_out, k_out, v_out, kk_out, a_out,
                H, a_is_raw, v_gate_is_raw, log_decay, (long long)rows * H};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long threads = p.total_heads * 16;
+    const long long threads = p.total_heads * (dtype == RWKV7_F32 ? 16 : 8);
     const int grid = (int)((threads + 255) / 256);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
         state_prep_kernel<T><<<grid, 256, 0, st>>>(p);
         return check_launch("state_prep_kernel");
     });
     return RWKV7_OK;
+}
+
+extern "C" int rwkv7_prefill_state_prep(const void* w_raw, const void* k_raw, const void* v_raw, const void* a,
+                                        const void* k_k, const void* k_a, const void* v_first, const void* v_gate,
+                                        float* w_out, void* k_out, void* v_out, void* kk_out, int rows, int H, int N,
+                                        int a_is_raw, int v_gate_is_raw, int log_decay, int dtype, void* stream) {
+    return rwkv7_prefill_state_prep_gate(w_raw, k_raw, v_raw, a, k_k, k_a, v_first, v_gate, w_out, k_out, v_out, kk_out, nullptr,
+                                         rows, H, N, a_is_raw, v_gate_is_raw, log_decay, dtype, stream);
 }
 
 // y = max(x, 0)^2 elementwise (in place allowed), 8 elements per thread

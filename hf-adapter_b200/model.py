@@ -412,20 +412,20 @@ class RWKV7ForCausalLM(nn.Module):
             v_raw = _linear(at.v_proj, xv)
             w_raw, a_pre, g, vg = _prefill_lora(at, xw, xa, xg, xv if i else None)
             vf = v_first if i else None
-            a_sig = torch.sigmoid(a_pre)
             chunked = bool(scan_chunk) and T % scan_chunk == 0 and x.dtype == torch.float16
             if chunked:
                 # the tensor-core scan forms the decay from the raw logits itself: no decay tensor is written or read.
                 # It carries an fp32 state; an fp16 cache is widened for the call and rounded back
-                k, v, kk = _prep.fused_prefill_kv_kk_prep(k_raw, v_raw, a_pre, at.k_k, at.k_a, v_first=vf, v_gate=vg, num_heads=H,
-                                                          head_dim=N, a_is_raw=True, v_gate_is_raw=True)
+                k, v, kk, a_sig = _prep.fused_prefill_kv_kk_prep(
+                    k_raw, v_raw, a_pre, at.k_k, at.k_a, v_first=vf, v_gate=vg, num_heads=H, head_dim=N, a_is_raw=True,
+                    v_gate_is_raw=True, return_gate=True)
                 y, new_state = _rec.self_chunk_rwkv7(r, w_raw, k, v, kk, a_sig, state[i].float(), chunk_size=scan_chunk, w_is_raw=True)
                 out = _prep.fused_attn_output_prepare(y, r, k, v, g, at.r_k, at.g_norm.weight, at.g_norm.bias,
                                                       num_heads=H, head_dim=N, head_v_dim=N, eps=N * 1e-5)
             else:
-                w, k, v, kk = _prep.fused_prefill_state_prep(
+                w, k, v, kk, a_sig = _prep.fused_prefill_state_prep(
                     w_raw, k_raw, v_raw, a_pre, at.k_k, at.k_a, v_first=vf, v_gate=vg, num_heads=H, head_dim=N,
-                    a_is_raw=True, v_gate_is_raw=True)
+                    a_is_raw=True, v_gate_is_raw=True, return_gate=True)
                 out, new_state = _rec.fused_recurrent_scan_output_prepare(
                     r, w, k, v, kk, a_sig, state[i], g, at.r_k, at.g_norm.weight, at.g_norm.bias, eps=N * 1e-5)
             if i == 0:

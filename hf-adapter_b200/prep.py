@@ -16,8 +16,10 @@ def _flat(x, hidden, name):
 
 def fused_prefill_state_prep(w_raw, k_raw, v_raw, a, k_k, k_a, *, v_first=None, v_gate=None, num_heads: int,
                              head_dim: int, w_out_dtype: str = "fp32", w_transform: str = "decay",
-                             a_is_raw: bool = False, v_gate_is_raw: bool = False, force_fallback: bool = False):
-    """Returns ``(w_decay, k_adjusted, v_interpolated, kk_normalized)`` in the input layout."""
+                             a_is_raw: bool = False, v_gate_is_raw: bool = False, force_fallback: bool = False,
+                             return_gate: bool = False):
+    """Returns ``(w_decay, k_adjusted, v_interpolated, kk_normalized)`` in the input layout, and with ``return_gate`` (an
+    extension) the gate ``a`` as the kernel used it (its sigmoid when ``a_is_raw``)."""
     no_fallback(force_fallback, "fused_prefill_state_prep")
     if w_out_dtype not in {"fp32", "input"}:
         raise ValueError(f"w_out_dtype must be 'fp32' or 'input'; got {w_out_dtype!r}")
@@ -45,14 +47,15 @@ def fused_prefill_state_prep(w_raw, k_raw, v_raw, a, k_k, k_a, *, v_first=None, 
     rows = int(w2.shape[0])
     w_out = torch.empty((rows, hidden), device=w2.device, dtype=torch.float32)
     k_out, v_out, kk_out = torch.empty_like(k2), torch.empty_like(k2), torch.empty_like(k2)
-    _lib.check(_lib.lib.rwkv7_prefill_state_prep(
+    a_out = torch.empty_like(a2) if return_gate else None
+    _lib.check(_lib.lib.rwkv7_prefill_state_prep_gate(
         ptr(w2), ptr(k2), ptr(v2), ptr(a2), ptr(kk_c), ptr(ka_c), ptr(vf2), ptr(vg2), ptr(w_out), ptr(k_out),
-        ptr(v_out), ptr(kk_out), rows, int(num_heads), int(head_dim), int(bool(a_is_raw)), int(bool(v_gate_is_raw)),
+        ptr(v_out), ptr(kk_out), ptr(a_out), rows, int(num_heads), int(head_dim), int(bool(a_is_raw)), int(bool(v_gate_is_raw)),
         int(w_transform == "log_decay"), dt_code(w2), stream_ptr(w2)), "fused_prefill_state_prep")
     if w_out_dtype == "input":
         w_out = w_out.to(w2.dtype)
     rs = lambda t: t.reshape(*prefix, hidden)
-    return rs(w_out), rs(k_out), rs(v_out), rs(kk_out)
+    return (rs(w_out), rs(k_out), rs(v_out), rs(kk_out)) + ((rs(a_out),) if return_gate else ())
 
 
 def fused_attn_output_prepare(recurrent_out, r, k, v, g, r_k, group_norm_weight, group_norm_bias, *, num_heads: int,
@@ -78,10 +81,12 @@ def fused_attn_output_prepare(recurrent_out, r, k, v, g, r_k, group_norm_weight,
 
 
 def fused_prefill_kv_kk_prep(k_raw, v_raw, a, k_k, k_a, *, v_first=None, v_gate=None, num_heads: int, head_dim: int,
-                             force_fallback: bool = False, a_is_raw: bool = False, v_gate_is_raw: bool = False):
+                             force_fallback: bool = False, a_is_raw: bool = False, v_gate_is_raw: bool = False,
+                             return_gate: bool = False):
     """State prep without the decay (rwkv7_hf/fused_prefill.py:324), the companion of the raw-w scan.
     Returns ``(k_adjusted, v_interpolated, kk_normalized)`` in the input layout.  ``a_is_raw`` / ``v_gate_is_raw``
-    (extensions, as in ``fused_prefill_state_prep``): the sigmoid of ``a`` / of the v gate is applied in the kernel."""
+    (extensions, as in ``fused_prefill_state_prep``): the sigmoid of ``a`` / of the v gate is applied in the kernel;
+    ``return_gate``: the gate ``a`` so formed is a fourth result."""
     no_fallback(force_fallback, "fused_prefill_kv_kk_prep")
     hidden = int(num_heads) * int(head_dim)
     k2, prefix = _flat(k_raw, hidden, "k_raw")
@@ -103,12 +108,13 @@ def fused_prefill_kv_kk_prep(k_raw, v_raw, a, k_k, k_a, *, v_first=None, v_gate=
     same_dtype(k2, v2, a2, kk_c, ka_c, vf2, vg2, what="fused_prefill_kv_kk_prep")
     rows = int(k2.shape[0])
     k_out, v_out, kk_out = torch.empty_like(k2), torch.empty_like(k2), torch.empty_like(k2)
-    _lib.check(_lib.lib.rwkv7_prefill_state_prep(
+    a_out = torch.empty_like(a2) if return_gate else None
+    _lib.check(_lib.lib.rwkv7_prefill_state_prep_gate(
         None, ptr(k2), ptr(v2), ptr(a2), ptr(kk_c), ptr(ka_c), ptr(vf2), ptr(vg2), None, ptr(k_out), ptr(v_out),
-        ptr(kk_out), rows, int(num_heads), int(head_dim), int(bool(a_is_raw)), int(bool(v_gate_is_raw)), 0, dt_code(k2),
+        ptr(kk_out), ptr(a_out), rows, int(num_heads), int(head_dim), int(bool(a_is_raw)), int(bool(v_gate_is_raw)), 0, dt_code(k2),
         stream_ptr(k2)), "fused_prefill_kv_kk_prep")
     rs = lambda t: t.reshape(*prefix, hidden)
-    return rs(k_out), rs(v_out), rs(kk_out)
+    return (rs(k_out), rs(v_out), rs(kk_out)) + ((rs(a_out),) if return_gate else ())
 
 
 def fused_attn_output_project(recurrent_out, r, k, v, g, r_k, group_norm_weight, group_norm_bias, o_proj_weight,

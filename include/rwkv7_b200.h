@@ -250,6 +250,14 @@ int rwkv7_prefill_state_prep(const void* w_raw, const void* k_raw, const void* v
                              int rows, int H, int N, int a_is_raw, int v_gate_is_raw, int log_decay,
                              int dtype, void* stream);
 
+/* The same with one more output: a_out = the gate the kernel used (sigmoid of `a` when a_is_raw), which the scan takes; NULL =
+ * rwkv7_prefill_state_prep. */
+int rwkv7_prefill_state_prep_gate(const void* w_raw, const void* k_raw, const void* v_raw, const void* a,
+                                  const void* k_k, const void* k_a, const void* v_first, const void* v_gate,
+                                  float* w_out, void* k_out, void* v_out, void* kk_out, void* a_out,
+                                  int rows, int H, int N, int a_is_raw, int v_gate_is_raw, int log_decay,
+                                  int dtype, void* stream);
+
 /* Replaces fused_attn_output_prepare (rwkv7_hf/fused_output.py:190): (GroupNorm(y) + (sum r k r_k) v) * g. */
 int rwkv7_attn_output_prepare(const void* recurrent, const void* r, const void* k, const void* v, const void* g,
                               const void* r_k, const void* gn_w, const void* gn_b, void* out,

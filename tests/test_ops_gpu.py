@@ -310,6 +310,27 @@ def test_grouped_lora_gemm_against_oracle(M):
     np.testing.assert_allclose(npf(y1), ref, rtol=4e-3, atol=4e-3)
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,Hh", [(1, 1), (5, 3), (67, 12)])
+def test_state_prep_returns_its_gate(dt, rows, Hh):
+    """The fourth / fifth result of the prefill state prep is the gate it used: the sigmoid of raw ``a`` rounded once (one
+    unit in the last place between two correct exponentials), ``a`` itself when it is no raw gate; the other results do not
+    depend on whether it is asked for."""
+    n = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dt)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w, k, v, a, vf, vg = (n(rows, Hh * N) for _ in range(6))
+    kk, ka = n(Hh * N), n(Hh * N)
+    ulp = torch.finfo(dt).eps
+    for first in (True, False):
+        kw = dict(num_heads=Hh, head_dim=N, v_gate_is_raw=True, **({} if first else dict(v_first=vf, v_gate=vg)))
+        for raw in (True, False):
+            want = torch.sigmoid(a.float()).to(dt) if raw else a
+            for fn, xs in ((hb.fused_prefill_kv_kk_prep, (k, v, a, kk, ka)), (hb.fused_prefill_state_prep, (w, k, v, a, kk, ka))):
+                *rest, gate = fn(*xs, a_is_raw=raw, return_gate=True, **kw)
+                assert ((gate.float() - want.float()).abs() <= ulp * want.float().abs()).all()
+                assert all(torch.equal(p, q) for p, q in zip(rest, fn(*xs, a_is_raw=raw, **kw)))
+
+
 @pytest.mark.parametrize("T", [16, 64, 80, 96, 112, 208])
 def test_chunk_scan_ring_edges_with_raw_decay(T):
     """The chunked scan around the lengths of its pipeline (four warps prepare 16-token chunks in turn, six chunks in the ring),
