@@ -40,6 +40,7 @@ struct GemmArgs {
     int tiles_m, tiles_n;
     int epi;
     int relu2;  // with EPI_DEQUANT: relu^2 of the dequantised value rounded to the output type (instead of + residual)
+    int bulk_out;  // the CTA-pair kernel with eight epilogue warps stores through a tensor map of C (epilogue_group_bulk)
     int vec;  // 1: N % 8 == 0 and every pointer the epilogue touches is 16-byte aligned
     unsigned int* error;
     // arg-max epilogue: per (row, column tile) the best value rounded to the output type and its column, [M, tiles_n] each
@@ -163,6 +164,44 @@ __device__ __forceinline__ void epilogue_group(const GemmArgs& p, uint32_t* stg,
         }
     }
     __syncwarp();  // the staging tile is overwritten by the next group
+}
+
+// The epilogue of one warp for 64 columns of its 32 rows when the output is the rounded sum (+ bias) and nothing else: the row a thread
+// holds is rounded in registers, goes to shared memory as 128 bytes (16-byte pieces xored by the row, the layout a
+// 128-byte-swizzled tensor map expects) and leaves as one bulk copy of [32 x 64].  The products with a tiny K are all
+// epilogue, and the general form above spends four times the instructions on it: 32768 rows, K 32 / 64 / 128 -> 4096 columns with
+// bias 140 / 140 / 142 us, 79 / 77 / 82 so (41 to write the output).  `buf`: this warp's buffer of 4 KB.
+template <typename TOut>
+__device__ __forceinline__ void epilogue_group_bulk(const GemmArgs& p, const CUtensorMap* tm_c, unsigned char* buf, uint32_t taddr, int row0, int col0, int lane) {
+    uint32_t v[64];
+    tmem_ld64(taddr, v);
+    if (row0 >= p.M || col0 >= p.N) {  // nothing to store: an empty group, so that the groups go on alternating between the buffers
+        tc_wait_ld();
+        if (lane == 0) tma_store_commit();
+        return;
+    }
+    if (lane == 0) tma_store_wait_read<1>();  // the copy before last, from this buffer
+    __syncwarp();
+    tc_wait_ld();
+    const TOut* bias = reinterpret_cast<const TOut*>(p.bias);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        float f[8], bv[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[u * 8 + e]);
+        if (bias && col0 + u * 8 < p.N) {
+            load8(bias + col0 + u * 8, bv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __fadd_rn(f[e], bv[e]);
+        }
+        store8(reinterpret_cast<TOut*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)), f);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+        tma_store_2d(tm_c, buf, col0, row0);
+        tma_store_commit();
+    }
 }
 
 // Arg-max epilogue: nothing of the product is stored.  A thread owns one row of the tile and folds its 256 columns
@@ -343,12 +382,14 @@ constexpr int kbox(int ew) { return ew == 8 ? 1 : 2; }
 constexpr int stages(int ew) { return ew == 8 ? 5 : 3; }
 constexpr int threads(int ew) { return 64 + 32 * ew; }
 constexpr int stage_bytes(int ew) { return kbox(ew) * (A_BYTES + B_BYTES); }
-constexpr int smem_bytes(int ew) { return stages(ew) * stage_bytes(ew) + 256 + ew * gm::STG_WARP_BYTES + 1024; }
+constexpr int BAR_BYTES = 1024;  // barriers; the staging tiles behind them start on 1024 bytes
+constexpr int smem_bytes(int ew) { return stages(ew) * stage_bytes(ew) + BAR_BYTES + ew * gm::STG_WARP_BYTES + 1024; }
 }  // namespace gp
 
 template <int KIND, typename TOut, int EW>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gp::threads(EW), 1)
-gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmArgs p) {
+gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
+                      const GemmArgs p) {
     using namespace gp;
     constexpr int KBOX = kbox(EW), STAGES = stages(EW), STAGE_BYTES = stage_bytes(EW);
     extern __shared__ unsigned char smem_unaligned[];
@@ -360,7 +401,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const AbortCtx actx{abort_flag, p.error};
-    uint32_t* stg = reinterpret_cast<uint32_t*>(sm + STAGES * STAGE_BYTES + 256) + (threadIdx.x >= 64 ? (threadIdx.x >> 5) - 2 : 0) * (32 * 64);
+    uint32_t* stg = reinterpret_cast<uint32_t*>(sm + STAGES * STAGE_BYTES + BAR_BYTES) + (threadIdx.x >= 64 ? (threadIdx.x >> 5) - 2 : 0) * (32 * 64);
 
     constexpr int ES = (KIND == gm::KIND_I8) ? 1 : 2;
     constexpr int BK = BKB / ES;
@@ -488,6 +529,14 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
                     p.part_idx[(size_t)row * p.tiles_n + tn] = best_col;
                 }
                 }
+            } else if (EW == 8 && KIND != gm::KIND_I8 && p.bulk_out) {
+                if constexpr (sizeof(TOut) == 2) {
+                    static_assert(EW != 8 || GPW == 2, "two groups a tile, two buffers");
+#pragma unroll
+                    for (int g2 = 0; g2 < GPW; ++g2)
+                        epilogue_group_bulk<TOut>(p, &tm_c, reinterpret_cast<unsigned char*>(stg) + (g2 & 1) * 4096, lane_addr + (half * GPW + g2) * 64,
+                                                  tm * PAIR_M + (int)rank * BM + q * 32, tn * BN + (half * GPW + g2) * 64, lane);
+                }
             } else {
 #pragma unroll 1
                 for (int gidx = half * GPW; gidx < half * GPW + GPW; ++gidx)
@@ -501,6 +550,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
             }
         }
     }
+    if (EW == 8 && p.bulk_out && warp >= 2 && lane == 0) tma_store_wait_all();
     // neither CTA may free its tensor memory or leave while the other can still touch its memory
     tc_fence_before();
     __syncthreads();
@@ -532,7 +582,7 @@ static int launch_gemm(const void* a, const void* b, GemmArgs g, cudaStream_t st
     constexpr CUtensorMapDataType dt = (KIND == KIND_I8)    ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                        : (KIND == KIND_F16) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                             : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    CUtensorMap tm_a, tm_b;
+    CUtensorMap tm_a, tm_b, tm_c{};
     g.error = kernel_error_word();
     RWKV7_REQUIRE(g.error != nullptr, RWKV7_ERR_CUDA, "gemm: cannot resolve the device error word");
     if (g.M > BM) {
@@ -547,14 +597,20 @@ static int launch_gemm(const void* a, const void* b, GemmArgs g, cudaStream_t st
         // up to four 128-byte K slices the tile's mainloop is shorter than its epilogue: eight epilogue warps
         if ((long long)g.K * ES <= 4 * BKB) {
             auto pk = gemm_umma_pair_kernel<KIND, TOut, 8>;
+            if constexpr (sizeof(TOut) == 2 && KIND != KIND_I8) {
+                if (g.epi == EPI_STORE && g.vec && !g.residual) {
+                    g.bulk_out = 1;
+                    if (int e = make_tmap_2d(&tm_c, dt, ES, g.C, g.M, g.N, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+                }
+            }
             cudaError_t pe = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, gp::smem_bytes(8));
             RWKV7_REQUIRE(pe == cudaSuccess, RWKV7_ERR_CUDA, "gemm: %s", cudaGetErrorString(pe));
-            pk<<<2 * pairs, gp::threads(8), gp::smem_bytes(8), st>>>(tm_a, tm_b, g);
+            pk<<<2 * pairs, gp::threads(8), gp::smem_bytes(8), st>>>(tm_a, tm_b, tm_c, g);
         } else {
             auto pk = gemm_umma_pair_kernel<KIND, TOut, 4>;
             cudaError_t pe = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, gp::smem_bytes(4));
             RWKV7_REQUIRE(pe == cudaSuccess, RWKV7_ERR_CUDA, "gemm: %s", cudaGetErrorString(pe));
-            pk<<<2 * pairs, gp::threads(4), gp::smem_bytes(4), st>>>(tm_a, tm_b, g);
+            pk<<<2 * pairs, gp::threads(4), gp::smem_bytes(4), st>>>(tm_a, tm_b, tm_c, g);
         }
         return check_launch("gemm_umma_pair_kernel");
     }

@@ -45,6 +45,24 @@ def test_gemm_epilogues(M, K, N, dtype):
     assert _lib.kernel_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K,N", [(129, 32, 8), (160, 8, 72), (257, 64, 256), (300, 128, 328), (1000, 256, 2560), (20000, 32, 64)])
+def test_tiny_k_products_store_whole_tiles(M, K, N, dt):
+    """Products whose K fits four 128-byte slices leave as bulk copies of [32 rows x 64 columns]: ragged rows, column groups that
+    are cut or empty, several tiles a CTA, with and without bias, and nothing written beyond the output.  fp32 sums of K terms,
+    rounded once: one unit in the last place."""
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    x, w, b = (torch.randn(*s, generator=g, device="cuda").to(dt) for s in ((M, K), (N, K), (N,)))
+    for bias in (None, b):
+        want = x.double() @ w.double().t() + (0 if bias is None else bias.double())
+        room = torch.full((M * N + 4096,), 7.0, device="cuda", dtype=dt)
+        y = room[:M * N].view(M, N)
+        hb.dense_linear(x, w, bias, out=y)
+        err = (y.double() - want).abs()
+        assert (err <= torch.finfo(dt).eps * want.abs() + 1e-5 * K).all()
+        assert (room[M * N:] == 7).all()
+
+
 def test_gemm_into_views_and_batched_rows():
     x = torch.randn(3, 50, 256, device="cuda", dtype=torch.float16)
     w = torch.randn(384, 256, device="cuda", dtype=torch.float16) / 16
