@@ -6,7 +6,7 @@
 // Bound: 5 * 64 * 64 multiply-adds per token and head in fp32 (1 S.kk, 1 decay, 2 rank-one terms, 1 S.r), issued as
 // packed pairs; 160 cycles of an SM's FMA pipe per token and head, measured 308 (64 sequences x 512 tokens x 64 heads,
 // fp16, output prepared: 2.21 ms, 6.04 ms with one row half per thread, unpacked, and the conversion in the chain).  Few
-// CTAs are bound by the latency of a token's chain instead: 120 CTAs x 777 tokens 242 us (772 us).  Operands come from
+// CTAs are bound by the chain of a token instead and have a kernel of their own.  Operands come from
 // shared memory as 16-byte reads that the lanes of a row group share.  Counted in the source, not profiled: the 2 x 32 tile
 // makes 40 of them a thread and token, and at four cycles a warp the two warps of a head hold the shared-memory pipe 320
 // cycles, which is about what a token takes at full grids.
@@ -188,18 +188,322 @@ __device__ __forceinline__ void scan_block(f2 (&S)[R][C / 2], Operands& op, int 
     }
 }
 
-// A CTA owns one (sequence, head).  (64 / R) * (64 / C) threads run the token loop; 64 threads load and convert a block of
-// tokens, 64 write one out.  SPEC: these are four further warps that prepare block s+1 and write block s-1 while block s
-// runs (for grids that leave an SM with one or two CTAs, where both would otherwise sit in the serial chain); without
-// it the 64 threads of the token loop do all three in turn and the other CTAs of the SM fill the gaps.
-template <typename T, bool PREP, int R, int C, bool SPEC>
-__global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_scan_kernel(const ScanArgs p) {
+// ---- grids that leave an SM with one or two CTAs: the serial chain of a token is all there is -----------------------------
+// Operands of one token in registers: the columns of a lane (4 cg .. + 3 and 32 + 4 cg .. + 3) and the values of its four rows.
+constexpr int kFewRows = 4, kFewLanes = 8;  // rows a thread has eight columns of, lanes that share them
+struct TokenRegs {
+    f2 kk[4], w[4], k[4], nb[4], r[4];
+    float v[kFewRows];
+};
+__device__ __forceinline__ void load_token(TokenRegs& o, const Operands& op, int t, int row0, int cg) {
+    auto load = [&](f2 (&x)[4], const float* src) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(src + j * 32 + cg * 4);
+            x[2 * j] = q.x;
+            x[2 * j + 1] = q.y;
+        }
+    };
+    load(o.kk, op.kk[t]);
+    load(o.w, op.w[t]);
+    load(o.k, op.k[t]);
+    load(o.nb, op.nb[t]);
+    load(o.r, op.r[t]);
+    load4<float>(&op.v[t][row0], o.v);
+}
+
+template <typename T> struct alignas(2 * sizeof(T)) Pair { T x, y; };
+template <typename T> __device__ __forceinline__ float2 to_f2(const Pair<T>& q) { return make_float2(to_f<T>(q.x), to_f<T>(q.y)); }
+
+// A CTA owns one (sequence, head).  Warps 0..3 run the recurrence: 8 lanes share four rows, a lane has 8 columns of each.  Warps
+// 4, 5 read a block of tokens ahead (in registers while the block before it runs) and convert it, warps 6, 7 write out the block that
+// is done.  In the token loop everything that does not wait for S.kk of this token sits in its shadow: the operands of the next
+// token, the decay and the v k^T term, the output sums of the token before.  What bounds it: the shared-memory pipe, which hands
+// a warp its 16-byte operand pieces at four cycles each whoever shares them (with two rows a thread on twice the warps it was
+// busy 80 % and a token took 13 % longer), and the chain of a token: 120 CTAs x 777 tokens 236 -> 203 us (262 ns a token).
+template <typename T, bool PREP, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs p) {
+    constexpr int R = kFewRows, G = kFewLanes, NT = kSN / R * G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Operands* ops = reinterpret_cast<Operands*>(smem_raw);  // [3]
+    const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
+    const int tid = threadIdx.x;
+    const int T_ = p.T;
+    const size_t tok_stride = (size_t)p.H * kSN;
+    const size_t base = ((size_t)b * T_ * p.H + h) * kSN;
+    const int nblocks = (T_ + kTS - 1) / kTS;
+
+    if (tid < NT) {
+        const int cg = tid % G, row0 = tid / G * R;
+        const size_t soff = ((size_t)bh * kSN + row0) * kSN + cg * 4;
+        f2 S[R][4];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const size_t o = soff + (size_t)i * kSN + j * 32;
+                float x[4];
+                if (p.state_f16) load4(reinterpret_cast<const __half*>(p.state_in) + o, x);
+                else load4(reinterpret_cast<const float*>(p.state_in) + o, x);
+                S[i][2 * j] = pack2(x[0], x[1]);
+                S[i][2 * j + 1] = pack2(x[2], x[3]);
+            }
+        float y[R];
+        auto dot = [&](float (&out)[R], const f2 (&x)[4]) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const f2 q0 = fma2(S[i][2], x[2], mul2(S[i][0], x[0])), q1 = fma2(S[i][3], x[3], mul2(S[i][1], x[1]));
+                float a0, a1, a2, a3;
+                unpack2(q0, a0, a1);
+                unpack2(q1, a2, a3);
+                out[i] = (a0 + a1) + (a2 + a3);
+            }
+        };
+        // Sums over the eight lanes of a row group in three steps, with work that does not wait for them in between: S.kk of this
+        // token goes to all lanes; the output of the token before is halved to one row a lane on the way (which rows go up is
+        // decided by the bits of the lane), and one of the lanes that end up with a row stores it.
+        const bool hi4 = (cg & 4) != 0, hi2 = (cg & 2) != 0;
+        const int yrow = row0 + (hi4 ? 2 : 0) + (hi2 ? 1 : 0);
+        const bool ystore = (cg & 1) == 0;
+        auto xchg = [](float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); };
+        auto decay_rows = [&](int i0, const TokenRegs& o) {
+#pragma unroll
+            for (int i = i0; i < i0 + R / 2; ++i) {
+                const f2 v2 = pack2(o.v[i], o.v[i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) S[i][j] = fma2(v2, o.k[j], mul2(S[i][j], o.w[j]));
+            }
+        };
+        float ya[R / 2], yb[R / 2], y1 = 0.f, y1q = 0.f;  // the output sum on its way
+        auto y_step4 = [&] {
+#pragma unroll
+            for (int i = 0; i < R / 2; ++i) {
+                ya[i] = hi4 ? y[R / 2 + i] : y[i];
+                yb[i] = xchg(hi4 ? y[i] : y[R / 2 + i], 4);
+            }
+        };
+        auto y_step2 = [&] {
+#pragma unroll
+            for (int i = 0; i < R / 2; ++i) ya[i] += yb[i];
+            y1 = hi2 ? ya[1] : ya[0];
+            y1q = xchg(hi2 ? ya[0] : ya[1], 2);
+        };
+        auto y_step1 = [&] {
+            y1 += y1q;
+            y1q = xchg(y1, 1);
+        };
+        auto token = [&](Operands& op, int t, bool prev, const TokenRegs& o) {
+            float sa[R], q[R];
+            dot(sa, o.kk);
+#pragma unroll
+            for (int i = 0; i < R; ++i) q[i] = xchg(sa[i], 4);
+            if (prev) y_step4();
+            decay_rows(0, o);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                sa[i] += q[i];
+                q[i] = xchg(sa[i], 2);
+            }
+            if (prev) y_step2();
+            decay_rows(R / 2, o);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                sa[i] += q[i];
+                q[i] = xchg(sa[i], 1);
+            }
+            if (prev) y_step1();
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                sa[i] += q[i];
+                const f2 s2 = pack2(sa[i], sa[i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) S[i][j] = fma2(s2, o.nb[j], S[i][j]);
+            }
+            if (prev && ystore) op.y[t - 1][yrow] = y1 + y1q;
+            dot(y, o.r);
+        };
+        for (int it = -1; it <= nblocks; ++it) {
+            if (it >= 0 && it < nblocks) {
+                Operands& op = ops[it % 3];
+                const int nt = min(kTS, T_ - it * kTS);
+                if (nt == kTS) {
+                    TokenRegs o[CTAS == 1 ? 2 : 1];
+                    load_token(o[0], op, 0, row0, cg);
+#pragma unroll
+                    for (int t = 0; t < kTS; ++t) {
+                        if constexpr (CTAS == 1) {  // the next token's operands a token ahead
+                            if (t + 1 < kTS) load_token(o[(t + 1) & 1], op, t + 1, row0, cg);
+                            token(op, t, t > 0, o[t & 1]);
+                        } else {  // two CTAs an SM: no registers for that, and less need
+                            token(op, t, t > 0, o[0]);
+                            if (t + 1 < kTS) load_token(o[0], op, t + 1, row0, cg);
+                        }
+                    }
+                } else {
+#pragma unroll 1
+                    for (int t = 0; t < nt; ++t) {
+                        TokenRegs o;
+                        load_token(o, op, t, row0, cg);
+                        token(op, t, t > 0, o);
+                    }
+                }
+                y_step4();
+                y_step2();
+                y_step1();
+                if (ystore) op.y[nt - 1][yrow] = y1 + y1q;
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const size_t o = soff + (size_t)i * kSN + j * 32;
+                float x[4];
+                unpack2(S[i][2 * j], x[0], x[1]);
+                unpack2(S[i][2 * j + 1], x[2], x[3]);
+                if (p.state_f16) store4(reinterpret_cast<__half*>(p.state_out) + o, x);
+                else store4(reinterpret_cast<float*>(p.state_out) + o, x);
+            }
+    } else if (tid < NT + 64) {
+        // two channels of four tokens a thread
+        const int ht = tid - NT, c = (ht & 31) * 2, tt0 = (ht >> 5) * 4;
+        const int wsz = p.w_mode == 1 ? 4 : (int)sizeof(T);
+        const int phase0 = p.elapsed ? p.elapsed[b] + h * kSN : 0;
+        float w0[2] = {0.f, 0.f};
+        if (p.w0) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) w0[i] = to_f<T>(reinterpret_cast<const T*>(p.w0)[h * kSN + c + i]);
+        }
+        Pair<T> r[4], k[4], v[4], kk[4], a[4], wt[4];
+        float2 wf[4];
+        auto fetch = [&](int s) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int t = min(s * kTS + tt0 + u, T_ - 1);  // past the end: a token that exists, whose operands nobody uses
+                const size_t o = base + (size_t)t * tok_stride + c;
+                auto get = [&](const void* q) { return *reinterpret_cast<const Pair<T>*>(reinterpret_cast<const T*>(q) + o); };
+                r[u] = get(p.r); k[u] = get(p.k); v[u] = get(p.v); kk[u] = get(p.kk); a[u] = get(p.a);
+                if (p.w_mode == 1) wf[u] = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(p.w) + o);
+                else wt[u] = get(p.w);
+            }
+        };
+        // rows of a later block on their way to L2: eight threads a token, one operand each
+        auto announce = [&](int s) {
+            const int t = s * kTS + (ht >> 3), q = ht & 7;
+            if (t >= T_ || q > 5) return;
+            const void* src = q == 0 ? p.r : q == 1 ? p.k : q == 2 ? p.v : q == 3 ? p.kk : q == 4 ? p.a : p.w;
+            const int size = q == 5 ? wsz : (int)sizeof(T);
+            const char* row = reinterpret_cast<const char*>(src) + (base + (size_t)t * tok_stride) * size;
+            prefetch_l2(row);
+            if (size == 4) prefetch_l2(row + 128);
+        };
+        fetch(0);
+        announce(1);
+        announce(2);
+        for (int it = -1; it <= nblocks; ++it) {
+            const int s = it + 1;
+            if (s < nblocks) {
+                Operands& op = ops[s % 3];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int tt = tt0 + u;
+                    float2 w;
+                    if (p.w_mode == 1) w = wf[u];
+                    else {
+                        w = to_f2(wt[u]);
+                        if (p.w_mode == 2) {
+                            float e[2] = {w.x, w.y};
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                if (p.w0) e[i] += w0[i];
+                                e[i] = decay_from_raw(e[i]);
+                                // (decay - 1 + rotator) rounded to fp16, as the reference's kernel forms its decay operand
+                                if (p.elapsed) e[i] = 1.0f + __half2float(__float2half_rn(e[i] - 1.0f + scan_rotator1(phase0 + c + i + s * kTS + tt)));
+                            }
+                            w = make_float2(e[0], e[1]);
+                        }
+                    }
+                    const float2 kkf = to_f2(kk[u]), af = to_f2(a[u]);
+                    *reinterpret_cast<float2*>(&op.w[tt][c]) = w;
+                    *reinterpret_cast<float2*>(&op.kk[tt][c]) = p.ab_mode ? make_float2(-kkf.x, -kkf.y) : kkf;
+                    *reinterpret_cast<float2*>(&op.nb[tt][c]) = p.ab_mode ? make_float2(-af.x, -af.y) : make_float2(-(kkf.x * af.x), -(kkf.y * af.y));
+                    *reinterpret_cast<float2*>(&op.r[tt][c]) = to_f2(r[u]);
+                    *reinterpret_cast<float2*>(&op.k[tt][c]) = to_f2(k[u]);
+                    *reinterpret_cast<float2*>(&op.v[tt][c]) = to_f2(v[u]);
+                }
+                if (s + 1 < nblocks) fetch(s + 1);
+                announce(s + 3);
+            }
+            __syncthreads();
+        }
+    } else {
+        // eight lanes a token, eight channels a lane
+        const int ht = tid & 63, tt = ht >> 3, c = (ht & 7) * 8;
+        float rk[8], gw[8], gb[8];
+        Vec8<T> g{};
+        if constexpr (PREP) {
+            auto load_param = [&](const void* param, float (&o)[8]) {
+                const T* q = reinterpret_cast<const T*>(param) + h * kSN + c;
+                if (p.params_vec) {
+                    load8(q, o);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[i] = to_f<T>(q[i]);
+                }
+            };
+            load_param(p.r_k, rk);
+            load_param(p.gn_w, gw);
+            load_param(p.gn_b, gb);
+        }
+        for (int it = -1; it <= nblocks; ++it) {
+            const int s = it - 1;
+            if (s >= 0) {
+                const Operands& op = ops[s % 3];
+                const int t = s * kTS + tt;
+                const bool live = t < T_;  // the shuffles below run in all lanes
+                float y[8];
+                load8<float>(&op.y[live ? tt : 0][c], y);
+                if constexpr (PREP) {
+                    float r[8], k[8], v[8];
+                    load8<float>(&op.r[live ? tt : 0][c], r);
+                    load8<float>(&op.k[live ? tt : 0][c], k);
+                    load8<float>(&op.v[live ? tt : 0][c], v);
+                    float sum = 0.f, corr = 0.f, var = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { sum += y[i]; corr += r[i] * k[i] * rk[i]; }
+                    const float mean = group_sum<8>(sum) * (1.0f / kSN);
+                    corr = group_sum<8>(corr);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { y[i] -= mean; var += y[i] * y[i]; }
+                    const float rstd = rsqrtf(group_sum<8>(var) * (1.0f / kSN) + p.eps);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) y[i] = (y[i] * rstd * gw[i] + gb[i] + corr * v[i]) * to_f<T>(g.v[i]);
+                }
+                if (live) store8(reinterpret_cast<T*>(p.y) + base + (size_t)t * tok_stride + c, y);
+            }
+            if constexpr (PREP) {  // the gate of the block that is written next
+                const int t = it * kTS + tt;
+                if (it >= 0 && t < T_) {
+                    const T* q = reinterpret_cast<const T*>(p.g) + base + (size_t)t * tok_stride + c;
+                    reinterpret_cast<uint4*>(&g)[0] = reinterpret_cast<const uint4*>(q)[0];
+                    if constexpr (sizeof(T) == 4) reinterpret_cast<uint4*>(&g)[1] = reinterpret_cast<const uint4*>(q)[1];
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// ---- more CTAs an SM: they hide each other's loads, and 64 threads load, convert, run and write a block in turn ------------
+template <typename T, bool PREP, int R, int C>
+__global__ void __launch_bounds__(kSN / R * (kSN / C)) wkv7_scan_kernel(const ScanArgs p) {
     constexpr int G = kSN / C;
     constexpr int NT = kSN / R * G;  // threads of the token loop
-    static_assert(SPEC || NT == 64, "the helpers are 64 threads");
+    static_assert(NT == 64, "64 threads load and write");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     RawStage<T>* raw = reinterpret_cast<RawStage<T>*>(smem_raw);  // [2]
-    Operands* ops = reinterpret_cast<Operands*>(smem_raw + 2 * sizeof(RawStage<T>));  // [SPEC ? 3 : 1]
+    Operands& op = *reinterpret_cast<Operands*>(smem_raw + 2 * sizeof(RawStage<T>));
 
     const int bh = blockIdx.x;
     const int b = bh / p.H, h = bh % p.H;
@@ -209,10 +513,8 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
     const size_t base = ((size_t)b * T_ * p.H + h) * kSN;     // element offset of token 0
     const int phase0 = p.elapsed ? p.elapsed[b] + h * kSN : 0;
     const int nstages = (T_ + kTS - 1) / kTS;
-    const int ht = SPEC ? (tid - NT) & 63 : tid;  // index among the 64 loading or the 64 writing threads
 
     // ---- in and out--------------------------------------------------------------------------------------------------
-    auto loader_sync = [] { asm volatile("barrier.sync 1, 64;" ::: "memory"); };
     auto issue_stage = [&](int s) {
         constexpr int CH = kSN * (int)sizeof(T) / 16;  // 16-byte chunks per token vector
         RawStage<T>& rs = raw[s & 1];
@@ -222,13 +524,13 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
         T(*dsts[5])[kSN] = {rs.r, rs.k, rs.v, rs.kk, rs.a};
 #pragma unroll
         for (int q = 0; q < 5; ++q)
-            for (int idx = ht; idx < nt * CH; idx += 64) {
+            for (int idx = tid; idx < nt * CH; idx += 64) {
                 const int tt = idx / CH, ch = idx % CH;
                 cp_async16(reinterpret_cast<char*>(dsts[q][tt]) + ch * 16,
                            reinterpret_cast<const char*>(srcs[q] + base + (size_t)(t0 + tt) * tok_stride) + ch * 16);
             }
         const int wsz = (p.w_mode == 1) ? 4 : (int)sizeof(T), chw = kSN * wsz / 16;
-        for (int idx = ht; idx < nt * chw; idx += 64) {
+        for (int idx = tid; idx < nt * chw; idx += 64) {
             const int tt = idx / chw, ch = idx % chw;
             cp_async16(reinterpret_cast<char*>(rs.w[tt]) + ch * 16,
                        reinterpret_cast<const char*>(p.w) + (base + (size_t)(t0 + tt) * tok_stride) * wsz + ch * 16);
@@ -237,17 +539,17 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
     };
 
     // thread = two channels x half of the block's tokens
-    auto convert = [&](int s, Operands& op) {
+    auto convert = [&](int s) {
         RawStage<T>& rs = raw[s & 1];
         const int t0 = s * kTS, nt = min(kTS, T_ - t0);
-        const int c = (ht & 31) * 2;
+        const int c = (tid & 31) * 2;
         auto two = [](const T* q) {
             if constexpr (sizeof(T) == 4) return *reinterpret_cast<const float2*>(q);
             else return make_float2(to_f<T>(q[0]), to_f<T>(q[1]));
         };
 #pragma unroll
         for (int u = 0; u < kTS / 2; ++u) {
-            const int tt = (ht >> 5) * (kTS / 2) + u;
+            const int tt = (tid >> 5) * (kTS / 2) + u;
             if (tt >= nt) continue;
             float2 w;
             if (p.w_mode == 1) w = *reinterpret_cast<const float2*>(&rs.w[tt][c]);
@@ -276,9 +578,9 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
     };
 
     // eight lanes per token, eight channels per lane
-    auto flush = [&](int s, Operands& op) {
+    auto flush = [&](int s) {
         const int t0 = s * kTS, nt = min(kTS, T_ - t0);
-        const int l8 = ht & 7, c = l8 * 8;
+        const int l8 = tid & 7, c = l8 * 8;
         auto load_param = [&](const void* param, float (&o)[8]) {
             const T* q = reinterpret_cast<const T*>(param) + h * kSN + c;
             if (p.params_vec) {
@@ -288,7 +590,7 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
                 for (int i = 0; i < 8; ++i) o[i] = to_f<T>(q[i]);
             }
         };
-        for (int tt = ht >> 3; tt < kTS; tt += 8) {
+        for (int tt = tid >> 3; tt < kTS; tt += 8) {
             const bool live = tt < nt;  // the shuffles below run in all lanes
             const size_t o = base + (size_t)(t0 + (live ? tt : 0)) * tok_stride + c;
             float y[8];
@@ -321,99 +623,61 @@ __global__ void __launch_bounds__(kSN / R * (kSN / C) + (SPEC ? 128 : 0)) wkv7_s
     const int cg = tid % G, row0 = tid / G * R;
     const size_t soff = ((size_t)bh * kSN + row0) * kSN + cg * 4;
     f2 S[R][C / 2];
-    if (!SPEC || tid < NT) {
 #pragma unroll
-        for (int i = 0; i < R; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-            for (int j = 0; j < C / 4; ++j) {
-                const size_t o = soff + (size_t)i * kSN + j * 4 * G;
-                float x[4];
-                if (p.state_f16) load4(reinterpret_cast<const __half*>(p.state_in) + o, x);
-                else load4(reinterpret_cast<const float*>(p.state_in) + o, x);
-                S[i][2 * j] = pack2(x[0], x[1]);
-                S[i][2 * j + 1] = pack2(x[2], x[3]);
-            }
-    }
-    auto run_block = [&](int s, Operands& op) { scan_block<R, C>(S, op, min(kTS, T_ - s * kTS), row0, cg); };
-
-    if constexpr (SPEC) {
-        const bool loader = tid >= NT && tid < NT + 64, writer = tid >= NT + 64;
-        if (loader) {
-            issue_stage(0);
-            if (nstages > 1) issue_stage(1);
+        for (int j = 0; j < C / 4; ++j) {
+            const size_t o = soff + (size_t)i * kSN + j * 4 * G;
+            float x[4];
+            if (p.state_f16) load4(reinterpret_cast<const __half*>(p.state_in) + o, x);
+            else load4(reinterpret_cast<const float*>(p.state_in) + o, x);
+            S[i][2 * j] = pack2(x[0], x[1]);
+            S[i][2 * j + 1] = pack2(x[2], x[3]);
         }
-        for (int s = -1; s <= nstages; ++s) {  // block s+1 in, block s through the recurrence, block s-1 out
-            if (loader) {
-                if (s + 1 < nstages) {
-                    if (s + 2 < nstages) cp_async_wait<1>(); else cp_async_wait<0>();
-                    loader_sync();  // raw block s+1 visible to both loader warps
-                    convert(s + 1, ops[(s + 1) % 3]);
-                    loader_sync();  // ... and read by both
-                    if (s + 3 < nstages) issue_stage(s + 3);
-                }
-            } else if (writer) {
-                if (s >= 1) flush(s - 1, ops[(s - 1) % 3]);
-            } else if (s >= 0 && s < nstages) {
-                run_block(s, ops[s % 3]);
-            }
-            __syncthreads();
+    issue_stage(0);
+    for (int s = 0; s < nstages; ++s) {
+        if (s + 1 < nstages) {
+            issue_stage(s + 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
         }
-    } else {
-        issue_stage(0);
-        for (int s = 0; s < nstages; ++s) {
-            if (s + 1 < nstages) {
-                issue_stage(s + 1);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncthreads();  // raw block visible; the previous block's flush has read the operands
-            convert(s, ops[0]);
-            __syncthreads();
-            run_block(s, ops[0]);
-            __syncthreads();
-            flush(s, ops[0]);
-        }
+        __syncthreads();  // raw block visible; the previous block's flush has read the operands
+        convert(s);
+        __syncthreads();
+        scan_block<R, C>(S, op, min(kTS, T_ - s * kTS), row0, cg);
+        __syncthreads();
+        flush(s);
     }
 
-    if (!SPEC || tid < NT) {
 #pragma unroll
-        for (int i = 0; i < R; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-            for (int j = 0; j < C / 4; ++j) {
-                const size_t o = soff + (size_t)i * kSN + j * 4 * G;
-                float x[4];
-                unpack2(S[i][2 * j], x[0], x[1]);
-                unpack2(S[i][2 * j + 1], x[2], x[3]);
-                if (p.state_f16) store4(reinterpret_cast<__half*>(p.state_out) + o, x);
-                else store4(reinterpret_cast<float*>(p.state_out) + o, x);
-            }
-    }
-}
-
-template <typename T, bool PREP, int R, int C, bool SPEC>
-static int launch_scan(const ScanArgs& p, int B, cudaStream_t st) {
-    constexpr size_t smem = 2 * sizeof(RawStage<T>) + (SPEC ? 3 : 1) * sizeof(Operands);
-    auto kern = wkv7_scan_kernel<T, PREP, R, C, SPEC>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "wkv7_scan: %s", cudaGetErrorString(e));
-    kern<<<B * p.H, kSN / R * (kSN / C) + (SPEC ? 128 : 0), smem, st>>>(p);
-    return check_launch("wkv7_scan_kernel");
+        for (int j = 0; j < C / 4; ++j) {
+            const size_t o = soff + (size_t)i * kSN + j * 4 * G;
+            float x[4];
+            unpack2(S[i][2 * j], x[0], x[1]);
+            unpack2(S[i][2 * j + 1], x[2], x[3]);
+            if (p.state_f16) store4(reinterpret_cast<__half*>(p.state_out) + o, x);
+            else store4(reinterpret_cast<float*>(p.state_out) + o, x);
+        }
 }
 
 template <typename T, bool PREP>
 static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
-    // Chosen by how many CTAs an SM gets.  Up to one: the serial chain of a token is all there is, so the rows are spread
-    // over four warps (160 multiply-adds a thread and token, 80 packed, where the 2 x 32 tile has 320) and loads /
-    // conversion / output run on warps of their own: 242 us for 120 CTAs x 777 tokens against 391 without.  Up to two: the
-    // tile with the fewer operand reads, still with the extra warps (335 us against 401 for 240 CTAs x 777).  More: the CTAs
-    // of an SM hide each other's loads and the extra warps only take registers (2211 us against 3159 for 4096 CTAs x 512).
-    // The three forms in this order, us for 512 tokens, fp16, output prepared: 148 CTAs 158 / 199 / 247, 149 235 / 215 / 250,
-    // 296 235 / 215 / 263, 297 379 / 409 / 370, 448 464 / 426 / 377, 600 602 / 635 / 512, 896 824 / 846 / 697, 2048 1606 / 1486 / 1164.
+    // Chosen by how many CTAs an SM gets.  Up to one, and up to two (with fewer registers a thread): the form with loads, output
+    // and recurrence on warps of their own.  More: the CTAs of an SM hide each other's loads and the extra warps only take
+    // registers.  us for 512 tokens, fp16, output prepared, call included, by CTAs, before -> now: 12 187 -> 152, 148 186 -> 155,
+    // 149 238 -> 221, 296 242 -> 223; 320 405, where the form for fewer took 438.
     const int ctas = B * p.H;
-    if (ctas <= kSMs) return launch_scan<T, PREP, 1, 32, true>(p, B, st);
-    if (ctas <= 2 * kSMs) return launch_scan<T, PREP, 4, 16, true>(p, B, st);
-    return launch_scan<T, PREP, 2, 32, false>(p, B, st);
+    const bool few = ctas <= 2 * kSMs;
+    void (*kern)(const ScanArgs) = ctas <= kSMs ? wkv7_scan_few_kernel<T, PREP, 1> : few ? wkv7_scan_few_kernel<T, PREP, 2> : wkv7_scan_kernel<T, PREP, 2, 32>;
+    const int threads = few ? 256 : 64;
+    const size_t smem = few ? 3 * sizeof(Operands) : 2 * sizeof(RawStage<T>) + sizeof(Operands);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "wkv7_scan: %s", cudaGetErrorString(e));
+    kern<<<ctas, threads, smem, st>>>(p);
+    return check_launch("wkv7_scan_kernel");
 }
 
 }  // namespace rwkv7
