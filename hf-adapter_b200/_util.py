@@ -19,7 +19,8 @@ def dt_code(t: torch.Tensor) -> int:
 
 
 def stream_ptr(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    # (the stream object that torch.cuda.current_stream builds first costs several times this call, once per launch)
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def require_cuda(*tensors, what: str) -> None:
