@@ -44,6 +44,7 @@ SIGNATURES = {
     "rwkv7_wkv7_output_prepare_raw_pool": (I, [P] * 14 + [P, P, I, P, P, P, I, P, I, I, I, I, F, I, P]),
     "rwkv7_ffn_add_norm_mix": (I, [P] * 8 + [I, I, F, I, P]),
     "rwkv7_layer_norm": (I, [P] * 4 + [I, I, F, I, P]),
+    "rwkv7_seq_norm_mix": (I, [P, P, P, P, PP, PP, P, I, I, I, I, F, I, P]),
     "rwkv7_seq_shift_mix": (I, [P, P, PP, PP, P, I, I, I, I, I, I, P]),
     "rwkv7_dense_small": (I, [P] * 4 + [I, I, I, I, I, I, P]),
     "rwkv7_small_gemm_group": (I, [I, PP, PP, PP, PP, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int), I, I, P]),

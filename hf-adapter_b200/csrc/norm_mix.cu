@@ -261,6 +261,110 @@ __global__ void __launch_bounds__(256) seq_shift_mix_kernel(const SeqMixArgs p) 
     }
 }
 
+struct SeqNormMixArgs {
+    const void *x, *nw, *nb, *init_prev;
+    const void* mix[6];
+    void* out[6];
+    void* next_state;
+    int T, D;
+    float eps;
+};
+
+// Raw8 from 16-byte pieces: fp32 rows of a view need not start on 32 bytes
+template <typename T>
+__device__ __forceinline__ Raw8<T> ld_row8(const T* p) {
+    if constexpr (sizeof(T) == 4) {
+        const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+        return Raw8<T>{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+    } else {
+        return ld_raw8(p);
+    }
+}
+
+// LayerNorm and token-shift mixes of a sequence in one pass: a CTA takes one token and normalises its row and the row before it
+// (which L2 has, because the token before is read at about the same time), rounded to the storage type as stored ones would be, so
+// that the normalised sequence is neither written nor read.  The two rows' statistics share their barriers.  A thread has 8 NV
+// elements of each (as many threads as the row needs, up to 512).
+constexpr int kSeqThreads = 512;
+template <typename T, int NMIX, int NV>
+__global__ void __launch_bounds__(kSeqThreads, NV == 1 ? 2 : 1) seq_norm_mix_kernel(const SeqNormMixArgs p) {
+    __shared__ float2 red[2][kSeqThreads / 32];
+    const int D = p.D, nvec = D / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const size_t row = blockIdx.x;
+    const int t = (int)(row % p.T);
+    const size_t b = row / p.T;
+    auto block_sums = [&](float u, float v, float2* r) {
+        u = group_sum<32>(u);
+        v = group_sum<32>(v);
+        if (lane == 0) r[warp] = make_float2(u, v);
+        __syncthreads();
+        const float2 q = lane < warps ? r[lane] : make_float2(0.f, 0.f);
+        return make_float2(group_sum<32>(q.x), group_sum<32>(q.y));
+    };
+    float x[NV][8], pv[NV][8];  // this row and the one before it (t = 0: the initial state, which is normalised already)
+    float sx = 0.f, sp = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int vi = threadIdx.x + i * kSeqThreads;
+        if (vi < nvec) {
+            load8(reinterpret_cast<const T*>(p.x) + row * D + vi * 8, x[i]);
+            load8(t > 0 ? reinterpret_cast<const T*>(p.x) + (row - 1) * D + vi * 8 : reinterpret_cast<const T*>(p.init_prev) + b * D + vi * 8, pv[i]);
+        }
+    }
+    Raw8<T> cw[NV], cb[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int vi = threadIdx.x + i * kSeqThreads;
+        if (vi < nvec) {
+            cw[i] = ld_row8(reinterpret_cast<const T*>(p.nw) + vi * 8);
+            cb[i] = ld_row8(reinterpret_cast<const T*>(p.nb) + vi * 8);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                sx += x[i][e];
+                sp += pv[i][e];
+            }
+        }
+    }
+    float2 mean = block_sums(sx, sp, red[0]);
+    mean.x /= (float)D;
+    mean.y /= (float)D;
+    float qx = 0.f, qp = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        if (threadIdx.x + i * kSeqThreads < nvec) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float dx = x[i][e] - mean.x, dp = pv[i][e] - mean.y;
+                qx += dx * dx;
+                qp += dp * dp;
+            }
+        }
+    }
+    const float2 var = block_sums(qx, qp, red[1]);
+    const float rx = rsqrtf(var.x / (float)D + p.eps), rp = rsqrtf(var.y / (float)D + p.eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int vi = threadIdx.x + i * kSeqThreads;
+        if (vi >= nvec) continue;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float w = to_f<T>(cw[i].v[e]), bb = to_f<T>(cb[i].v[e]);
+            x[i][e] = round_to<T>((x[i][e] - mean.x) * rx * w + bb);
+            const float h = round_to<T>((pv[i][e] - mean.y) * rp * w + bb);
+            pv[i][e] = (t > 0 ? h : pv[i][e]) - x[i][e];
+        }
+        if (t == p.T - 1) store8(reinterpret_cast<T*>(p.next_state) + b * D + vi * 8, x[i]);
+#pragma unroll
+        for (int m = 0; m < NMIX; ++m) {
+            float mx[8], o[8];
+            load8(reinterpret_cast<const T*>(p.mix[m]) + vi * 8, mx);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] = x[i][e] + pv[i][e] * mx[e];
+            store8(reinterpret_cast<T*>(p.out[m]) + row * D + vi * 8, o);
+        }
+    }
+}
+
 // f(std::integral_constant<int, NV>) for the smallest row size the kernels are instantiated for
 template <typename F>
 static void with_row_vectors(int D, F f) {
@@ -384,6 +488,33 @@ extern "C" int rwkv7_layer_norm(const void* x, const void* norm_w, const void* n
     RWKV7_DISPATCH_DTYPE(dtype, T, {
         with_row_vectors(D, [&](auto nv) { launch_programmatic(ffn_add_norm_mix_kernel<T, false, false, decltype(nv)::value, true>, dim3(rows), dim3(kNMThreads), 0, st, p); });
         return check_launch("layer_norm_kernel");
+    });
+    return RWKV7_OK;
+}
+
+extern "C" int rwkv7_seq_norm_mix(const void* x, const void* norm_w, const void* norm_b, const void* initial_prev, const void* const* mixes,
+                                  void* const* outs, void* next_state, int B, int T, int D, int n_mix, float eps, int dtype, void* stream) {
+    RWKV7_REQUIRE(B > 0 && T > 0 && (long long)B * T < (1ll << 31), RWKV7_ERR_INVALID, "seq_norm_mix: bad sizes B=%d T=%d", B, T);
+    if (int e = check_row_shape("seq_norm_mix", B * T, D)) return e;
+    RWKV7_REQUIRE(n_mix == 1 || n_mix == 6, RWKV7_ERR_INVALID, "seq_norm_mix: one mix or six");
+    RWKV7_REQUIRE(x && norm_w && norm_b && initial_prev && mixes && outs && next_state, RWKV7_ERR_INVALID, "seq_norm_mix: null pointer");
+    RWKV7_REQUIRE(initial_prev != next_state, RWKV7_ERR_INVALID, "seq_norm_mix: initial_prev and next_state must not alias");
+    SeqNormMixArgs p{x, norm_w, norm_b, initial_prev, {}, {}, next_state, T, D, eps};
+    for (int m = 0; m < n_mix; ++m) {
+        RWKV7_REQUIRE(mixes[m] && outs[m], RWKV7_ERR_INVALID, "seq_norm_mix: null mix/out pointer %d", m);
+        RWKV7_REQUIRE(aligned(mixes[m], 16) && aligned(outs[m], 16), RWKV7_ERR_ALIGN, "seq_norm_mix: unaligned pointer");
+        p.mix[m] = mixes[m];
+        p.out[m] = outs[m];
+    }
+    const void* ptrs[] = {x, norm_w, norm_b, initial_prev, next_state};
+    for (const void* q : ptrs) RWKV7_REQUIRE(aligned(q, 16), RWKV7_ERR_ALIGN, "seq_norm_mix: unaligned pointer");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    RWKV7_DISPATCH_DTYPE(dtype, TT, {
+        const bool wide = D > 8 * kSeqThreads;
+        auto kern = wide ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 2> : seq_norm_mix_kernel<TT, 1, 2>)
+                         : (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 1> : seq_norm_mix_kernel<TT, 1, 1>);
+        kern<<<B * T, wide ? kSeqThreads : (D / 8 + 31) / 32 * 32, 0, st>>>(p);
+        return check_launch("seq_norm_mix_kernel");
     });
     return RWKV7_OK;
 }

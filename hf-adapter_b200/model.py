@@ -403,9 +403,8 @@ class RWKV7ForCausalLM(nn.Module):
             at, ff = layer.attn, layer.ffn
             if i == 0:
                 x = _nm.layer_norm(x, layer.pre_norm.weight, layer.pre_norm.bias)
-            h = _nm.layer_norm(x, layer.attn_norm.weight, layer.attn_norm.bias)
-            xr, xw, xk, xv, xa, xg, nxt = _nm.fused_attn_sequence_shift_mix(
-                h, xpa[i], at.x_r, at.x_w, at.x_k, at.x_v, at.x_a, at.x_g)
+            (xr, xw, xk, xv, xa, xg), nxt = _nm.sequence_norm_mix(x, xpa[i], layer.attn_norm.weight, layer.attn_norm.bias,
+                                                                  (at.x_r, at.x_w, at.x_k, at.x_v, at.x_a, at.x_g))
             xpa[i].copy_(nxt)
             r = _linear(at.r_proj, xr)
             k_raw = _linear(at.k_proj, xk)
@@ -435,8 +434,7 @@ class RWKV7ForCausalLM(nn.Module):
                 x = _linear(at.o_proj, out, residual=x)  # the residual add rides in the projection's epilogue
             else:
                 x = x + self._all_reduce(_linear(at.o_proj, out))
-            h2 = _nm.layer_norm(x, layer.ffn_norm.weight, layer.ffn_norm.bias)
-            mixed, nxt = _nm.fused_ffn_sequence_shift_mix(h2, xpf[i], ff.x_k)
+            (mixed,), nxt = _nm.sequence_norm_mix(x, xpf[i], layer.ffn_norm.weight, layer.ffn_norm.bias, (ff.x_k,))
             xpf[i].copy_(nxt)
             hidden = _linear(ff.key, mixed, relu2=True)
             if self.tp_world == 1:

@@ -8,6 +8,13 @@ from . import _lib
 from ._util import dt_code, no_fallback, ptr, require_cuda, same_dtype, stream_ptr
 
 
+# Elements of a sequence up to which its norm and its mixes are one kernel.  It normalises every row twice (once as the row before the
+# next), which few CTAs do not notice and many do.  us, two kernels -> one, six mixes / one mix: 512 x 768 fp32 8.0 / 5.1 -> 5.1 / 3.5,
+# 64 x 2560 fp16 5.9 / 4.9 -> 3.9 / 2.8, 1024 x 4096 16.9 / 10.7 -> 15.8 / 11.2, 2331 x 2560 24.3 / 14.7 -> 21.5 / 14.8, 4096 x 4096 60.8 /
+# 34.6 -> 63.4 / 37.8; a launch less either way.
+SEQ_NORM_MIX_ELEMENTS = 6 << 20
+
+
 def _rows(x, name):
     if x.dim() == 1:
         return x.reshape(1, -1), tuple(x.shape)
@@ -148,6 +155,28 @@ def _seq_mix(x, initial_prev, mixes, workspace, name, strict=False):
         storage = torch.empty(expected, device=x.device, dtype=x.dtype)
     nxt = torch.empty((B, D), device=x.device, dtype=x.dtype)
     return src, initial, flat, storage, nxt, (B, T, D), int(bool(strict))
+
+
+def sequence_norm_mix(x, initial_prev, norm_weight, norm_bias, mixes, eps: float = 1e-5):
+    """``layer_norm(x [B,T,C])`` and its token-shift mixes (one, or the six in the order r,w,k,v,a,g): the results of ``layer_norm``
+    followed by the sequence shift-mix.  Returns ``(outs, next_state)``."""
+    src, initial, flat, storage, nxt, (B, T, D), _ = _seq_mix(
+        x, initial_prev, mixes, None, "fused_attn_sequence_shift_mix" if len(mixes) == 6 else "sequence_norm_mix")
+    require_cuda(src, norm_weight, norm_bias, what="sequence_norm_mix")
+    same_dtype(src, norm_weight, norm_bias, what="sequence_norm_mix")
+    slots = storage.unbind(0) if len(mixes) == 6 else (storage,)
+    outs = (slots[0], slots[3], slots[1], slots[2], slots[4], slots[5]) if len(mixes) == 6 else slots
+    nw, nb = norm_weight.contiguous(), norm_bias.contiguous()
+    mp, _k1 = _lib.ptr_array([m.data_ptr() for m in flat])
+    op, _k2 = _lib.ptr_array([o.data_ptr() for o in outs])
+    if B * T * D <= SEQ_NORM_MIX_ELEMENTS:
+        _lib.check(_lib.lib.rwkv7_seq_norm_mix(ptr(src), ptr(nw), ptr(nb), ptr(initial), mp, op, ptr(nxt), B, T, D, len(mixes), float(eps),
+                                               dt_code(src), stream_ptr(src)), "sequence_norm_mix")
+    else:
+        h = layer_norm(src, nw, nb, eps)
+        _lib.check(_lib.lib.rwkv7_seq_shift_mix(ptr(h), ptr(initial), mp, op, ptr(nxt), B, T, D, len(mixes), 0, dt_code(src),
+                                                stream_ptr(src)), "sequence_norm_mix")
+    return outs, nxt
 
 
 def fused_attn_sequence_shift_mix(x, initial_prev, *mixes, block_size: int = 256, num_warps: int = 4, workspace=None,

@@ -201,6 +201,12 @@ int rwkv7_wkv7_output_prepare_raw_pool(const void* r, const void* w_raw, const v
 int rwkv7_layer_norm(const void* x, const void* norm_w, const void* norm_b, void* out,
                      int rows, int D, float eps, int dtype, void* stream);
 
+/* LayerNorm of x [B,T,D] and the token-shift mixes of its rounded rows in one pass (rwkv7_layer_norm, then rwkv7_seq_shift_mix without
+ * strict rounding; the normalised sequence itself is not stored).  n_mix is 1 or 6; next_state [B,D] = the last normalised
+ * row, which must not be initial_prev's memory. */
+int rwkv7_seq_norm_mix(const void* x, const void* norm_w, const void* norm_b, const void* initial_prev, const void* const* mixes,
+                       void* const* outs, void* next_state, int B, int T, int D, int n_mix, float eps, int dtype, void* stream);
+
 /* Replaces fused_attn_sequence_shift_mix / fused_ffn_sequence_shift_mix (rwkv7_hf/fused_time_mix.py:413,470):
  * x [B,T,D] (already normalised), prev_t = x_{t-1} (initial_prev for t = 0), out_m = x + (prev-x)*mix_m for
  * n_mix in {1,6} mixes; next_state [B,D] = x[:, T-1].  strict_rounding != 0 (fp16 only) reproduces the reference's

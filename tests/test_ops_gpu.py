@@ -311,6 +311,30 @@ def test_grouped_lora_gemm_against_oracle(M):
 
 
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,T,D", [(1, 1, 8), (2, 3, 264), (3, 37, 768), (2, 5, 4096), (1, 9, 4104), (2, 2, 8192), (1, 1537, 4096)])
+def test_sequence_norm_mix(dt, B, T, D):
+    """LayerNorm and token-shift mixes in one call, either side of the size at which one kernel becomes two and of the row
+    width at which a thread takes two vectors, against 64 bits on the rounded rows.  The kernel's row may round the other way
+    (one unit of this row and of the one before), and the mix rounds once."""
+    from hf_adapter_b200 import norm_mix as NM
+    g = torch.Generator(device="cuda").manual_seed(B * T + D)
+    n = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dt)
+    x, prev, w, b = n(B, T, D), n(B, D), n(D), n(D)
+    mixes = [torch.rand(D, generator=g, device="cuda").to(dt) for _ in range(6)]
+    xd = x.double()
+    h = (xd - xd.mean(-1, keepdim=True)) * torch.rsqrt(xd.var(-1, unbiased=False, keepdim=True) + 1e-5) * w.double() + b.double()
+    hr = h.to(dt).double()
+    before = torch.cat([prev.double()[:, None], hr[:, :-1]], 1)
+    eps = max(torch.finfo(dt).eps, 2e-6)  # fp32: the statistics of a row
+    room = 2 * eps * (h.abs() + before.abs() + w.double().abs() + b.double().abs())
+    for k in (6, 1):
+        outs, nxt = NM.sequence_norm_mix(x, prev, w, b, mixes[:k])
+        for o, m in zip(outs, mixes):
+            assert ((o.double() - (hr + (before - hr) * m.double())).abs() <= room).all()
+        assert ((nxt.double() - hr[:, -1]).abs() <= room[:, -1]).all()
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,Hh", [(1, 1), (5, 3), (67, 12)])
 def test_state_prep_returns_its_gate(dt, rows, Hh):
     """The fourth / fifth result of the prefill state prep is the gate it used: the sigmoid of raw ``a`` rounded once (one
