@@ -13,7 +13,7 @@
 // Warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2-5 = epilogue (TMEM -> staging -> global); the CTA-pair
 // kernel has a second form with eight epilogue warps for products with a tiny K, which are all epilogue.
 // Ragged M / N / K edges are zero-filled by TMA and masked at the store.  All waits are bounded (umma.cuh).
-// With more than 128 rows the same roles run as CTA pairs on 256 x 256 tiles (second kernel below).
+// With more than 128 rows the same roles run as CTA pairs on tiles of 256 x 256 and narrower (second kernel below).
 #include "umma.cuh"
 
 namespace rwkv7 {
@@ -364,15 +364,15 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 }
 
 // ---------------------------------------------------------------- CTA-pair variant (tcgen05 cta_group::2)
-// Two CTAs of a cluster share one 256 x 256 output tile.  Each stages its own 128 rows of A and 128 of the 256 rows
+// Two CTAs of a cluster share one output tile of 256 x BN.  Each stages its own 128 rows of A and half of the BN rows
 // of B (32 KB per 128 bytes of K instead of 48 KB, so the shared-memory fill per MMA cycle drops by a third); the
 // even CTA issues MMAs of M = 256 that read both CTAs' shared memory and write each CTA's 128 result rows into that
 // CTA's tensor memory.  Barrier protocol: both producers' TMA loads complete on the LEADER's full[s]
 // (armed by the leader with the byte count of both); the leader's commits arrive on empty[s] / acc_full[a] in BOTH
 // CTAs; the epilogue warps of both CTAs arrive on the leader's acc_empty[a].  No TMA multicast.
 namespace gp {
-constexpr int BM = 128, PAIR_M = 256, BN = 256, HALF_N = 128, BKB = 128;
-constexpr int A_BYTES = BM * BKB, B_BYTES = HALF_N * BKB;
+constexpr int BM = 128, PAIR_M = 256, BKB = 128;
+constexpr int A_BYTES = BM * BKB;
 constexpr int TMEM_COLS = 512;
 // Two forms, chosen by the number of epilogue warps EW.  EW = 4 (one per TMEM lane quadrant): a stage holds two
 // 128-byte K slices of both operands, [A slices][B slices], three stages.  EW = 8 (two per quadrant, each on half of the
@@ -381,17 +381,19 @@ constexpr int TMEM_COLS = 512;
 constexpr int kbox(int ew) { return ew == 8 ? 1 : 2; }
 constexpr int stages(int ew) { return ew == 8 ? 5 : 3; }
 constexpr int threads(int ew) { return 64 + 32 * ew; }
-constexpr int stage_bytes(int ew) { return kbox(ew) * (A_BYTES + B_BYTES); }
+constexpr int stage_bytes(int ew, int bn) { return kbox(ew) * (A_BYTES + bn / 2 * BKB); }
 constexpr int BAR_BYTES = 1024;  // barriers; the staging tiles behind them start on 1024 bytes
-constexpr int smem_bytes(int ew) { return stages(ew) * stage_bytes(ew) + BAR_BYTES + ew * gm::STG_WARP_BYTES + 1024; }
+constexpr int smem_bytes(int ew, int bn) { return stages(ew) * stage_bytes(ew, bn) + BAR_BYTES + ew * gm::STG_WARP_BYTES + 1024; }
 }  // namespace gp
 
-template <int KIND, typename TOut, int EW>
+// BN: columns of a tile (256, or 192 / 128 / 64 where that leaves fewer SMs idle)
+template <int KIND, typename TOut, int EW, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gp::threads(EW), 1)
 gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
                       const GemmArgs p) {
     using namespace gp;
-    constexpr int KBOX = kbox(EW), STAGES = stages(EW), STAGE_BYTES = stage_bytes(EW);
+    constexpr int KBOX = kbox(EW), STAGES = stages(EW), STAGE_BYTES = stage_bytes(EW, BN), HALF_N = BN / 2, B_BYTES = HALF_N * BKB;
+    static_assert(B_BYTES % 1024 == 0 && BN % 64 == 0 && 2 * BN <= TMEM_COLS, "swizzled tiles, epilogue groups, tensor memory");
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* sm = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(sm + STAGES * STAGE_BYTES);
@@ -410,7 +412,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
     const bool leader = rank == 0;
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int nk = (p.K + KBOX * BK - 1) / (KBOX * BK);  // stages per tile (a ragged last stage is zero-filled by TMA)
-    const int ntiles = p.tiles_m * p.tiles_n;  // tiles of 256 x 256
+    const int ntiles = p.tiles_m * p.tiles_n;  // tiles of 256 x BN
 
     if (tid == 0) {
         tma_prefetch_desc(&tm_a);
@@ -511,7 +513,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
             tc_fence_after();
             const int row = tm * PAIR_M + (int)rank * BM + q * 32 + lane;
             const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN);
-            constexpr int GPW = 16 / EW;  // 64-column groups per epilogue warp
+            constexpr int GPW = BN / 64 * 4 / EW;  // 64-column groups per epilogue warp
             const int half = (warp - 2) >> 2;
             if (KIND != gm::KIND_I8 && p.epi == gm::EPI_ARGMAX) {
                 if (half == 0) {
@@ -575,6 +577,27 @@ static int sm_count() {
     return n;
 }
 
+template <int KIND, typename TOut, int EW, int BN>
+static int launch_pair(const CUtensorMap& tm_a, const void* b, CUtensorMapDataType dt, int es, GemmArgs g, cudaStream_t st) {
+    CUtensorMap tm_b, tm_c{};
+    if constexpr (EW == 8 && sizeof(TOut) == 2 && KIND != gm::KIND_I8) {
+        if (g.epi == gm::EPI_STORE && g.vec && !g.residual) {
+            g.bulk_out = 1;
+            if (int e = make_tmap_2d(&tm_c, dt, es, g.C, g.M, g.N, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+        }
+    }
+    if (int e = make_tmap_2d(&tm_b, dt, es, b, g.N, g.K, BN / 2, gp::BKB / es, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
+    g.tiles_n = (g.N + BN - 1) / BN;
+    const long long pairs_wanted = (long long)g.tiles_m * g.tiles_n;
+    const int pairs_fit = sm_count() / 2;
+    const int pairs = (int)(pairs_wanted < pairs_fit ? pairs_wanted : pairs_fit);
+    auto pk = gemm_umma_pair_kernel<KIND, TOut, EW, BN>;
+    const cudaError_t pe = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, gp::smem_bytes(EW, BN));
+    RWKV7_REQUIRE(pe == cudaSuccess, RWKV7_ERR_CUDA, "gemm: %s", cudaGetErrorString(pe));
+    pk<<<2 * pairs, gp::threads(EW), gp::smem_bytes(EW, BN), st>>>(tm_a, tm_b, tm_c, g);
+    return check_launch("gemm_umma_pair_kernel");
+}
+
 template <int KIND, typename TOut>
 static int launch_gemm(const void* a, const void* b, GemmArgs g, cudaStream_t st) {
     using namespace gm;
@@ -582,37 +605,36 @@ static int launch_gemm(const void* a, const void* b, GemmArgs g, cudaStream_t st
     constexpr CUtensorMapDataType dt = (KIND == KIND_I8)    ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                        : (KIND == KIND_F16) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                             : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    CUtensorMap tm_a, tm_b, tm_c{};
+    CUtensorMap tm_a, tm_b;
     g.error = kernel_error_word();
     RWKV7_REQUIRE(g.error != nullptr, RWKV7_ERR_CUDA, "gemm: cannot resolve the device error word");
     if (g.M > BM) {
         // more than one 128-row tile: CTA pairs on 256 x 256 tiles
         if (int e = make_tmap_2d(&tm_a, dt, ES, a, g.M, g.K, gp::BM, BKB / ES, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
-        if (int e = make_tmap_2d(&tm_b, dt, ES, b, g.N, g.K, gp::HALF_N, BKB / ES, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
         g.tiles_m = (g.M + gp::PAIR_M - 1) / gp::PAIR_M;
-        g.tiles_n = (g.N + gp::BN - 1) / gp::BN;
-        const long long pairs_wanted = (long long)g.tiles_m * g.tiles_n;
-        const int pairs_fit = sm_count() / 2;
-        const int pairs = (int)(pairs_wanted < pairs_fit ? pairs_wanted : pairs_fit);
         // up to four 128-byte K slices the tile's mainloop is shorter than its epilogue: eight epilogue warps
-        if ((long long)g.K * ES <= 4 * BKB) {
-            auto pk = gemm_umma_pair_kernel<KIND, TOut, 8>;
-            if constexpr (sizeof(TOut) == 2 && KIND != KIND_I8) {
-                if (g.epi == EPI_STORE && g.vec && !g.residual) {
-                    g.bulk_out = 1;
-                    if (int e = make_tmap_2d(&tm_c, dt, ES, g.C, g.M, g.N, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
-                }
-            }
-            cudaError_t pe = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, gp::smem_bytes(8));
-            RWKV7_REQUIRE(pe == cudaSuccess, RWKV7_ERR_CUDA, "gemm: %s", cudaGetErrorString(pe));
-            pk<<<2 * pairs, gp::threads(8), gp::smem_bytes(8), st>>>(tm_a, tm_b, tm_c, g);
-        } else {
-            auto pk = gemm_umma_pair_kernel<KIND, TOut, 4>;
-            cudaError_t pe = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, gp::smem_bytes(4));
-            RWKV7_REQUIRE(pe == cudaSuccess, RWKV7_ERR_CUDA, "gemm: %s", cudaGetErrorString(pe));
-            pk<<<2 * pairs, gp::threads(4), gp::smem_bytes(4), st>>>(tm_a, tm_b, tm_c, g);
+        if ((long long)g.K * ES <= 4 * BKB) return launch_pair<KIND, TOut, 8, 256>(tm_a, b, dt, ES, g, st);
+        const long long fit = sm_count() / 2;
+        // Narrower tiles where 256 columns leave pairs idle.  Cycles a 128-byte slice of K holds a CTA pair on a tile of 256 x bn: the
+        // MMAs (2 bn), or the way of its 128 rows of A and bn / 2 of B from L2 (70 bytes a clock and SM); times the waves of tiles; a
+        // narrower tile has to win by 3 %.  us, fp16, 256 columns -> the chosen width, at 256 / 512 / 1024 / 2331 / 4096 rows: 2560 ->
+        // 2560 21.5 / 22.2 / 22.9 / 34.5 / 47.9 -> 16.1 / 17.6 / 19.8 / 30.0 / 47.7; 10240 -> 2560 58.0 / 58.4 / 59.9 / 111.5 / 174.6 -> 43.0 / 46.0 /
+        // 52.6 / 103.8 / 175.2; 4096 -> 4096 34.7 / 35.5 / 33.7 / 72.1 / 99.4 -> 28.9 / 27.8 / 34.1 / 65.0 / 99.9; 768 -> 3072 19.7 / 20.1 / 20.7 / 30.1 /
+        // 40.8 -> 12.7 / 12.6 / 11.9 / 20.6 / 27.5.
+        const auto cost = [&](int bn) {
+            const long long waves = ((long long)g.tiles_m * ((g.N + bn - 1) / bn) + fit - 1) / fit;
+            return waves * (2 * bn > 234 + bn * 9 / 10 ? 2 * bn : 234 + bn * 9 / 10);
+        };
+        int best = 256;
+        if (g.epi != EPI_ARGMAX)  // (its partial results are counted in tiles of 256 columns)
+            for (int bn : {192, 128, 64})
+                if (cost(bn) * 33 < cost(best) * 32) best = bn;
+        switch (best) {
+            case 64: return launch_pair<KIND, TOut, 4, 64>(tm_a, b, dt, ES, g, st);
+            case 128: return launch_pair<KIND, TOut, 4, 128>(tm_a, b, dt, ES, g, st);
+            case 192: return launch_pair<KIND, TOut, 4, 192>(tm_a, b, dt, ES, g, st);
+            default: return launch_pair<KIND, TOut, 4, 256>(tm_a, b, dt, ES, g, st);
         }
-        return check_launch("gemm_umma_pair_kernel");
     }
     if (int e = make_tmap_2d(&tm_a, dt, ES, a, g.M, g.K, BM, BKB / ES, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
     if (int e = make_tmap_2d(&tm_b, dt, ES, b, g.N, g.K, BN, BKB / ES, CU_TENSOR_MAP_SWIZZLE_128B)) return e;

@@ -63,6 +63,23 @@ def test_tiny_k_products_store_whole_tiles(M, K, N, dt):
         assert (room[M * N:] == 7).all()
 
 
+@pytest.mark.parametrize("M,N", [(200, 520), (1000, 2300), (2300, 2552), (2560, 4608)])
+def test_tile_widths(M, N):
+    """Sizes at which a CTA pair takes tiles of 64, 128, 192 and 256 columns, ragged in rows, columns and K: every fp16 epilogue
+    against a matmul in fp32, and the int8 accumulators exactly."""
+    K = 1096
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, K, device="cuda", generator=g).half(), (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).half()
+    bias, res = torch.randn(N, device="cuda", generator=g).half(), torch.randn(M, N, device="cuda", generator=g).half()
+    for b_, relu2, r_ in ((None, False, None), (bias, False, res), (bias, True, None)):
+        y = hb.dense_linear(x, w, b_, relu2=relu2, residual=r_)
+        tol = 5e-3 if relu2 else 2e-3
+        torch.testing.assert_close(y.float(), _ref(x, w, b_, relu2, r_), rtol=tol, atol=tol)
+    qa, qw = (torch.randint(-127, 128, (n, 1104), device="cuda", dtype=torch.int8, generator=g) for n in (M, N))
+    assert torch.equal(hb.int8_mm(qa, qw).double(), qa.double() @ qw.double().t())
+    assert _lib.kernel_status() == 0
+
+
 def test_gemm_into_views_and_batched_rows():
     x = torch.randn(3, 50, 256, device="cuda", dtype=torch.float16)
     w = torch.randn(384, 256, device="cuda", dtype=torch.float16) / 16
