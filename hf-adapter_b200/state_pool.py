@@ -17,6 +17,7 @@ Prefill gathers the scheduled slots into a dense cache, runs the layer-wise pref
 from __future__ import annotations
 
 import hashlib
+import weakref
 from dataclasses import dataclass, field
 
 import torch
@@ -349,10 +350,16 @@ class RWKV7StatePool:
 class PoolDecodeGraph:
     """A decode step captured once per bucket size over the pools themselves.  The kernels read the slot vector from a
     static device buffer, so replays serve any set of scheduled requests without rebinding or copying state; the graph
-    must be rebuilt only if the pools are reallocated or the model's modules change."""
+    must be rebuilt only if the pools are reallocated or the model's modules change.
+
+    The graph keeps the buffers and the model that it was captured over, not the pool, which keeps the graph: in a cycle
+    both would wait for the cyclic collector, and a graph that is destroyed while another is being captured invalidates that
+    capture."""
 
     def __init__(self, pool: RWKV7StatePool, rows: int, greedy: bool):
-        self.pool, self.rows = pool, int(rows)
+        self.rows = int(rows)
+        self._pool = weakref.ref(pool)
+        self._held = (pool.model, pool.S_pool, pool.xpa_pool, pool.xpf_pool, pool.vfirst_pool)
         dev = pool.S_pool.device
         self.ids = torch.zeros(self.rows, device=dev, dtype=torch.long)
         self.slots = torch.full((self.rows,), pool.scratch_slot, device=dev, dtype=torch.int32)
@@ -366,6 +373,11 @@ class PoolDecodeGraph:
         self.graph = torch.cuda.CUDAGraph()
         with capture(self.graph):
             self.out = pool._step(self.ids, self.slots, greedy)
+
+    @property
+    def pool(self) -> RWKV7StatePool | None:
+        """The pool that the graph was captured for, None once it is gone."""
+        return self._pool()
 
     def replay(self, ids, slot_vec):
         n = int(ids.numel())

@@ -6,6 +6,7 @@ ONE predecessor: a node that joins branches has to have full edges."""
 import collections
 import ctypes
 import gc
+import weakref
 
 import pytest
 import torch
@@ -143,3 +144,26 @@ def test_branch_results_outlive_their_use_on_the_main_stream():
                 again = [torch.empty(B, D, device="cuda", dtype=torch.float16) for _ in range(8)]
             assert not main.query() and not used & {t.data_ptr() for t in again}
     torch.cuda.synchronize()
+
+
+def test_a_dropped_pool_frees_its_graph_without_the_collector():
+    """A graph that waits for the cyclic collector is destroyed at a moment nobody chose, a foreign capture among them.  A graph
+    that is kept longer than its pool keeps the buffers it was captured over."""
+    m = _model("dense", 256, 1)
+    ids = torch.zeros(1, device="cuda", dtype=torch.long)
+    on = gc.isenabled()
+    gc.disable()
+    try:
+        pool = hb.RWKV7StatePool(m, 2)
+        slots, gens = pool.allocate(["a"])
+        pool.decode(ids, slots, gens)
+        (graph,) = pool._graphs.values()
+        assert graph.pool is pool
+        gone, buffers = weakref.ref(pool), weakref.ref(pool.S_pool)
+        del pool
+        assert gone() is None and graph.pool is None and buffers() is not None
+        graph, gone = None, weakref.ref(graph)
+        assert gone() is None and buffers() is None
+    finally:
+        if on:
+            gc.enable()
