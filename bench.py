@@ -303,6 +303,7 @@ def main():
     from hf_adapter_b200 import _lib
     from hf_adapter_b200 import model as hbm
     from hf_adapter_b200 import packing as hpk
+    from hf_adapter_b200._util import capture
 
     local = int(os.environ.get("LOCAL_RANK", "0"))
     torch.cuda.set_device(local)
@@ -520,7 +521,7 @@ def main():
         torch.cuda.current_stream(dev).wait_stream(side)
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):
+        with capture(g):
             fn()
         for _ in range(3):
             g.replay()

@@ -143,3 +143,12 @@ def test_model_state_dict_names_match_reference(golden_dir):
     assert set(model.state_dict()) == ref_names
     for k, v in model.state_dict().items():
         assert tuple(v.shape) == tuple(g["param::" + k].shape), k
+
+
+def test_every_capture_holds_the_collector_off():
+    """Graphs are captured through ``_util.capture``: a graph that the cyclic collector destroys in the middle of a capture
+    invalidates that capture, in the library and in the benchmark alike."""
+    package = os.path.join(ROOT, "hf-adapter_b200")
+    files = [os.path.join(package, f) for f in sorted(os.listdir(package)) if f.endswith(".py")] + [os.path.join(ROOT, "bench.py")]
+    bare = [os.path.basename(f) for f in files if re.search(r"with torch\.cuda\.graph\(", open(f).read())]
+    assert bare == ["_util.py"]
