@@ -107,7 +107,7 @@ def test_quantised_fp16_model_against_oracle(kind):
 
 
 def test_prefill_with_tensor_core_scan_matches_sequential_scan():
-    """fp16 prefill of 128 tokens: the chunked (tcgen05) scan and the sequential scan give the same logits
+    """fp16 prefill of 128 tokens: the chunked (tensor-core) scan and the sequential scan give the same logits
     and final recurrent state within fp16 tolerances."""
     g = golden("model_tiny.npz")
     model = load_tiny(g, torch.float16)

@@ -374,7 +374,7 @@ def test_chunk_scan_ring_edges_with_raw_decay(T):
 
 @pytest.mark.parametrize("B,T,Hh,chunk", [(1, 64, 1, 64), (2, 128, 3, 16), (2, 192, 2, 32), (1, 1024, 2, 64)])
 def test_chunk_scan_tensor_core_against_oracle(B, T, Hh, chunk):
-    """tcgen05 chunked WY scan == the sequential recurrence (fp64 oracle on the same fp16 inputs):
+    """Tensor-core chunked WY scan == the sequential recurrence (fp64 oracle on the same fp16 inputs):
     state relative error <= 1e-3, outputs within fp16 tolerance, no bounded wait gave up."""
     from hf_adapter_b200 import _lib
     r, w, k, v, kk, a = wkv_inputs(B, T, Hh, N, seed=T + chunk)
