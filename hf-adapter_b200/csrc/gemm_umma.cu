@@ -609,7 +609,7 @@ static int launch_gemm(const void* a, const void* b, GemmArgs g, cudaStream_t st
     g.error = kernel_error_word();
     RWKV7_REQUIRE(g.error != nullptr, RWKV7_ERR_CUDA, "gemm: cannot resolve the device error word");
     if (g.M > BM) {
-        // more than one 128-row tile: CTA pairs on 256 x 256 tiles
+        // more than one 128-row tile: CTA pairs on tiles of 256 rows
         if (int e = make_tmap_2d(&tm_a, dt, ES, a, g.M, g.K, gp::BM, BKB / ES, CU_TENSOR_MAP_SWIZZLE_128B)) return e;
         g.tiles_m = (g.M + gp::PAIR_M - 1) / gp::PAIR_M;
         // up to four 128-byte K slices the tile's mainloop is shorter than its epilogue: eight epilogue warps

@@ -42,14 +42,15 @@
 //     the group's 128 threads, bar.sync by the issuer warp: tens of cycles) instead of an mbarrier, whose completion
 //     takes about 175 cycles to become visible to a waiter.
 //
-// Warps: 0 weight-stream producer, 1 activation producer + tensor-memory owner, 2..1+NISS issuers, then three dequant
-// groups of four warps (group g takes k-blocks g, g+3, ...).  Six A buffers (two per group): a group waits for the
-// MMAs of its block before last, never for the previous one.  Weight ring: six stages of one block (two per group,
-// released as soon as the block is in registers).  Stage, A buffer and "done" barrier of block i have index i mod 6
-// and always belong to group i mod 3 and issuer i mod NISS: every waiter sees every phase of the barriers it waits on
-// (a waiter that skips phases passes a parity wait one phase early).  Above 64 rows the split-K exchange buffer aliases the
-// activation ring: a CTA announces that its last MMA completed with a cluster-barrier arrive and peers wait for that
-// phase before they push.
+// Warps: 0 weight-stream producer, 1 activation producer + tensor-memory owner, 2..1+NISS issuers, then G dequant groups of
+// four warps (group g takes k-blocks g, g + G, ...).  NA = 2 G A buffers: a group waits for the MMAs of its block before
+// last, never for the previous one.  Weight ring: NA stages of one block (two per group, released as soon as the block is
+// in registers).  Weight stage, A buffer and "done" barrier of block i have index i mod NA and always belong to group
+// i mod G and issuer i mod NISS (NA is a multiple of both); its activation stage has index i mod XST, released by a barrier of its
+// own, or with XST = NA by the "done" barrier.  So every waiter sees every phase of the barriers it waits on (a waiter
+// that skips phases passes a parity wait one phase early).  G, NA, NISS, XST by rows a pass: Cfg below.  Above 64 rows the split-K
+// exchange buffer aliases the activation ring: a CTA announces that its last MMA completed with a cluster-barrier arrive and
+// peers wait for that phase before they push.
 //
 // Named barriers have no time-out, so nobody may skip one: after a bounded mbarrier wait gave up (abort flag raised)
 // every role keeps walking its blocks, skipping the waits and the work but not the bar.arrive / bar.sync.

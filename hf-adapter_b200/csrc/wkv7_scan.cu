@@ -7,9 +7,7 @@
 // packed pairs; 160 cycles of an SM's FMA pipe per token and head, measured 308 (64 sequences x 512 tokens x 64 heads,
 // fp16, output prepared: 2.21 ms, 6.04 ms with one row half per thread, unpacked, and the conversion in the chain).  Few
 // CTAs are bound by the chain of a token instead and have a kernel of their own.  Operands come from
-// shared memory as 16-byte reads that the lanes of a row group share.  Counted in the source, not profiled: the 2 x 32 tile
-// makes 40 of them a thread and token, and at four cycles a warp the two warps of a head hold the shared-memory pipe 320
-// cycles, which is about what a token takes at full grids.
+// shared memory as 16-byte reads that the lanes of a row group share: 40 a thread and token with the 2 x 32 tile.
 #include "common.cuh"
 
 namespace rwkv7 {
@@ -80,32 +78,24 @@ struct alignas(16) Operands {
     float y[kTS][kSN];
 };
 
-// Sum R row values over the G lanes that share a row group, halving the rows a lane keeps while there is more than one
-// (R - 1 shuffles instead of R log2 G).  On return the lane owns row `row` of the group's R; `first` marks the one lane
-// that owns it when there are more lanes than rows.
-template <int R, int G>
-__device__ __forceinline__ float scatter_sum(float (&v)[R], int cg, int& row, bool& first) {
+// Sum R row values over the R lanes that share a row group, halving the rows a lane keeps (R - 1 shuffles instead of
+// R log2 R).  On return the lane owns row `row` of the group's.
+template <int R>
+__device__ __forceinline__ float scatter_sum(float (&v)[R], int cg, int& row) {
     row = 0;
-    first = true;
-    if constexpr (G == 1) {
+    if constexpr (R == 1) {
         return v[0];
-    } else if constexpr (R == 1) {
-        float t = v[0];
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        first = (cg & (G - 1)) == 0;
-        return t;
     } else {
-        constexpr int HALF = G / 2, RH = R / 2;
-        const bool up = (cg & HALF) != 0;
+        constexpr int RH = R / 2;
+        const bool up = (cg & RH) != 0;
         float keep[RH];
 #pragma unroll
         for (int i = 0; i < RH; ++i) {
             const float mine = up ? v[RH + i] : v[i], send = up ? v[i] : v[RH + i];
-            keep[i] = mine + __shfl_xor_sync(0xffffffffu, send, HALF);
+            keep[i] = mine + __shfl_xor_sync(0xffffffffu, send, RH);
         }
         int sub;
-        const float t = scatter_sum<RH, HALF>(keep, cg, sub, first);
+        const float t = scatter_sum<RH>(keep, cg, sub);
         row = (up ? RH : 0) + sub;
         return t;
     }
@@ -116,6 +106,7 @@ __device__ __forceinline__ float scatter_sum(float (&v)[R], int cg, int& row, bo
 template <int R, int C>
 __device__ __forceinline__ void scan_block(f2 (&S)[R][C / 2], Operands& op, int nt, int row0, int cg) {
     constexpr int G = kSN / C;
+    static_assert(R == G, "as many rows as lanes: each ends up with one row's sum");
     auto load = [&](f2 (&x)[C / 2], const float* src) {
 #pragma unroll
         for (int j = 0; j < C / 4; ++j) {
@@ -158,9 +149,8 @@ __device__ __forceinline__ void scan_block(f2 (&S)[R][C / 2], Operands& op, int 
             for (int i = 0; i < R; ++i) sa[i] += __shfl_xor_sync(0xffffffffu, sa[i], o);
         if (tt > 0) {
             int row;
-            bool first;
-            const float ysum = scatter_sum<R, G>(y, cg, row, first);
-            if (first) op.y[tt - 1][row0 + row] = ysum;
+            const float ysum = scatter_sum<R>(y, cg, row);
+            op.y[tt - 1][row0 + row] = ysum;
         }
 #pragma unroll
         for (int i = 0; i < R; ++i) {
@@ -182,9 +172,8 @@ __device__ __forceinline__ void scan_block(f2 (&S)[R][C / 2], Operands& op, int 
     }
     {
         int row;
-        bool first;
-        const float ysum = scatter_sum<R, G>(y, cg, row, first);
-        if (first) op.y[nt - 1][row0 + row] = ysum;
+        const float ysum = scatter_sum<R>(y, cg, row);
+        op.y[nt - 1][row0 + row] = ysum;
     }
 }
 
@@ -677,7 +666,7 @@ static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "wkv7_scan: %s", cudaGetErrorString(e));
     kern<<<ctas, threads, smem, st>>>(p);
-    return check_launch("wkv7_scan_kernel");
+    return check_launch(few ? "wkv7_scan_few_kernel" : "wkv7_scan_kernel");
 }
 
 }  // namespace rwkv7
