@@ -310,6 +310,29 @@ def test_grouped_lora_gemm_against_oracle(M):
     np.testing.assert_allclose(npf(y1), ref, rtol=4e-3, atol=4e-3)
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M", [1, 65])
+@pytest.mark.parametrize("K,Nout", [((72,), (41,)), ((328, 328), (40, 1)), ((520,), (64,)), ((520, 520, 520), (66, 65, 2)),
+                                    ((4104,), (41,)), ((4104, 72, 8), (40, 41, 1)), ((4104, 4096), (64, 32))])
+def test_grouped_lora_gemm_odd_widths_and_ragged_k(dt, M, K, Nout):
+    """Widths that are not pairs (one of a group makes all of it store by element), rows that end in the middle of a pair, K that
+    ends in the middle of a chunk on the deep ring, with and without split K, and shares of K that are empty.  fp32 sums of exact
+    products: K units of 2^-24 of the sum of magnitudes, then one rounding.  Nothing behind an output is written, nothing behind a
+    bias counts."""
+    from hf_adapter_b200.lora import small_gemm_group
+    g = torch.Generator(device="cuda").manual_seed(M + sum(K) + sum(Nout))
+    n = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dt)
+    xs, ws = [n(M, k) for k in K], [n(o, k) for k, o in zip(K, Nout)]
+    biases = [torch.cat([n(o), torch.full((8,), float("nan"), device="cuda", dtype=dt)])[:o] for o in Nout]
+    flat = [torch.full((M * o + 8,), 7.0, device="cuda", dtype=dt) for o in Nout]
+    small_gemm_group(xs, ws, biases, outs=[f[:M * o].view(M, o) for f, o in zip(flat, Nout)])
+    for x, w, b, f, k, o in zip(xs, ws, biases, flat, K, Nout):
+        assert bool((f[M * o:] == 7.0).all())
+        ref = x.double() @ w.double().T + b.double()
+        room = torch.finfo(dt).eps * ref.abs() + k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+        assert bool(((f[:M * o].view(M, o).double() - ref).abs() <= room).all())
+
+
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,T,D", [(1, 1, 8), (2, 3, 264), (3, 37, 768), (2, 5, 4096), (1, 9, 4104), (2, 2, 8192), (1, 1537, 4096)])
 def test_sequence_norm_mix(dt, B, T, D):
