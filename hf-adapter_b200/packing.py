@@ -169,22 +169,29 @@ def _out_features(op):
     return int(op.shape[0]) if isinstance(op, torch.Tensor) else int(op.out_features)
 
 
-def rkv_grouped(ops, xr, xk, xv):
-    """r / k / v through one grouped launch when all three are int4 (or row-wise int8) projections of one shape that
-    the tensor-core decode kernel takes; None otherwise."""
+def _rkv_tiled(ops, xs):
+    """The tiled weights of r / k / v when all three are int4 (or row-wise int8) projections of one shape that the
+    tensor-core decode kernel takes in one launch; None otherwise."""
     int4 = all(isinstance(m, _q.MM4Linear) for m in ops)
     int8 = all(isinstance(m, _q.MM8Linear) and m.sm7x_rowwise for m in ops)
     if not (int4 or int8) or any(m.bias is not None for m in ops):
         return None
     if len({(m.in_features, m.out_features) for m in ops}) != 1:
         return None
-    tiled = [m.tiled_for(x_) for m, x_ in zip(ops, (xr, xk, xv))]
-    if any(t is None for t in tiled):
-        return None
-    if int8:
-        return _q.w8_tiled_linear_group((xr, xk, xv), tiled, [m.row_scale for m in ops], ops[0].out_features,
-                                        ops[0].in_features)
-    return _q.w4_tiled_linear_group((xr, xk, xv), tiled, ops[0].out_features, ops[0].in_features)
+    tiled = [m.tiled_for(x_) for m, x_ in zip(ops, xs)]
+    return None if any(t is None for t in tiled) else tiled
+
+
+def _rkv_launch(ops, xs, tiled):
+    if isinstance(ops[0], _q.MM8Linear):
+        return _q.w8_tiled_linear_group(xs, tiled, [m.row_scale for m in ops], ops[0].out_features, ops[0].in_features)
+    return _q.w4_tiled_linear_group(xs, tiled, ops[0].out_features, ops[0].in_features)
+
+
+def rkv_grouped(ops, xr, xk, xv):
+    """r / k / v through one grouped launch where ``_rkv_tiled`` has their weights; None otherwise."""
+    tiled = _rkv_tiled(ops, (xr, xk, xv))
+    return None if tiled is None else _rkv_launch(ops, (xr, xk, xv), tiled)
 
 
 def _rows_operand(op, x):
@@ -261,6 +268,8 @@ def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
     # The LoRA chain is two launches long and leads on the main stream, behind the kernel that made its inputs; r / k / v do not
     # depend on it and branch off (parallel branches of the decode graph once captured), joined before the recurrence.
     main = torch.cuda.current_stream(x.device)
+    # (tiled weights that are built on first use belong to the stream that outlives the branches: ahead of the fork)
+    tiled = _rkv_tiled(ops, xs)
     fork = main.record_event()
     hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)])
     lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups])
@@ -268,21 +277,19 @@ def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
 
     def branch(i, t, run):
         st = ctx.side_stream(x.device, i)
-        if st not in used:
-            st.wait_event(fork)
-            used.append(st)
+        st.wait_event(fork)
+        used.append(st)
         with torch.cuda.stream(st):
             y = run()
         for v in t:
             v.record_stream(st)
         return y
 
-    rkv = None
-    if all(isinstance(o, _QUANT_TYPES) for o in ops):
+    if tiled is not None:
         # int4 / int8 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
         # exchange) instead of three launches competing for the SMs
-        rkv = branch(0, xs, lambda: rkv_grouped(ops, *xs))
-    if rkv is None:
+        rkv = branch(0, xs, lambda: _rkv_launch(ops, xs, tiled))
+    else:
         # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
         rkv = [branch(i, (t,), lambda: apply_linear(o, t)) for i, (o, t) in enumerate(zip(ops, xs))]
     for st in used:

@@ -167,3 +167,26 @@ def test_a_dropped_pool_frees_its_graph_without_the_collector():
     finally:
         if on:
             gc.enable()
+
+
+@pytest.mark.parametrize("weights,cls", [("mm4", "MM4Linear"), ("w8", "MM8Linear")])
+def test_tiled_weights_are_built_on_the_stream_of_the_step(weights, cls, monkeypatch):
+    """The tiled copy that a projection makes on first use outlives the step: its memory belongs to the stream that the program
+    runs on, not to a branch of one step, whose later allocations would not wait for the readers of a copy that was dropped."""
+    from hf_adapter_b200 import quant
+    m = _model(weights, 512, 1)
+    linear, seen = getattr(quant, cls), []
+    real = linear.tiled_for
+
+    def tiled_for(self, x):
+        if self._tiled is None:
+            seen.append(torch.cuda.current_stream())
+        return real(self, x)
+
+    monkeypatch.setattr(linear, "tiled_for", tiled_for)
+    main = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(main), torch.no_grad():
+        m._decode_step(torch.zeros(16, device="cuda", dtype=torch.long), m.new_cache(16))
+    torch.cuda.synchronize()
+    assert len(seen) >= 6 and all(s == main for s in seen)  # r, k, v, o and the two of the FFN
