@@ -1,14 +1,19 @@
 // Chunked (WY / DPLR) WKV-7 prefill scan, the intra-chunk contractions on tensor cores.
 //
 // One CTA per (sequence, head), two CTAs an SM.  The sequence is cut into chunks of 16 tokens (the result does not depend on
-// it, so the caller's chunk size is only validated).  With a~ = -kk, b~ = kk*a, P_t the inclusive product of the decays from the
-// chunk's first token on, and S0 the state [value i x key n] before the chunk:
+// it, so the caller's chunk size is only validated).  With a~ = -kk, b~ = kk*a, the state S0 [value i x key n] before the chunk, R_t
+// the product of the decays of the chunk's tokens behind t, R_-1 that of all sixteen:
 //
-//   aE = a~_t P_{t-1}   rP = r_t P_t   kI = k_s / P_s   bI = b~_s / P_s        (16 x 64, tf32 operands)
-//   A_ak = tril_strict(aE kI^T)   A_ab = tril_strict(aE bI^T)   A_qk = tril(rP kI^T)   A_qb = tril(rP bI^T)
-//   U^T = (S0 aE^T + V^T A_ak^T) T^T,   T = (I - A_ab)^-1
-//   Y^T = S0 rP^T + V^T A_qk^T + U^T A_qb^T
-//   S'  = S0 P_15 + V^T (k P_15/P) + U^T (b~ P_15/P)
+//   S0d = S0 R_-1   aE = a~_t / R_{t-1}   rP = r_t / R_t   kD = k_s R_s   bD = b~_s R_s        (16 x 64, tf32 operands)
+//   A_ak = tril_strict(aE kD^T)   A_ab = tril_strict(aE bD^T)   A_qk = tril(rP kD^T)   A_qb = tril(rP bD^T)
+//   U^T = (S0d aE^T + V^T A_ak^T) T^T,   T = (I - A_ab)^-1
+//   Y^T = S0d rP^T + V^T A_qk^T + U^T A_qb^T
+//   S'  = S0d + V^T kD + U^T bD
+//
+// (Scaled to the chunk's end, so that the keys which enter the state and those which the tokens behind them read are rounded alike:
+// a rounded key is then a slightly other key in the same recurrence, and the delta rule takes part of the difference back.  Scaled to
+// its start the states came out 2..4 % further from 64 bits; 16 tokens, 4 sequences x 40 heads, relative error of y / state 4.18e-4 /
+// 1.617e-4 so, 4.147e-4 / 1.581e-4 now, and 4.146e-4 / 1.595e-4 with the former tiles of 64 tokens.)
 //
 // What bounds it: the serial chain S0 -> U -> S' of a head and the issue slots around it, not HBM and not the tensor pipe.  So the
 // chain is kept in registers.  Four STATE warps own 16 value rows each; the rows of the state never meet, so these warps never
@@ -19,14 +24,15 @@
 // each in turn, into a ring of six slots: decay products, scaled operands, the four 16 x 16 products, the inverse.  mma.sync
 // and not tcgen05: these products are 16 rows high, and through tensor memory every link of the chain costs a store, a
 // fence, an issue, a commit and a load, about 700 cycles (a tile of 64 tokens with five such links took 16.9 k cycles with one CTA
-// an SM).  8 sequences x 4096 tokens x 32 heads: 1150 -> 435 us (0.38 of the HBM floor of 165 us); the
-// 7.2B model's prefill of 64 x 512 tokens 484 -> 450 ms.
+// an SM).  8 sequences x 4096 tokens x 32 heads, in a row: 1154 -> 412 us (0.40 of the HBM floor of 165 us).
 //
-// Products that contain decay-scaled factors (range e^9.7 over 16 tokens) run on operands rounded to tf32; products of bounded
-// quantities (A_* against V and U, the keys decayed to the chunk's end) run in fp16; T is inverted in fp32, and
-// U = rhs T^T takes both operands as tf32 pairs (hi + lo, three products), which keeps the error of an fp32 solve.  U itself enters
-// its two products as an fp16 pair: the state is rounded to tf32 four times as often as with 64-token tiles, and with U in one
-// fp16 the state's error against 64 bits came out up to 2 % larger than theirs (421 us then); with the pair it is 1 % smaller.
+// Products that contain decay-scaled factors (range e^9.7 over 16 tokens with the model's decays) run on operands rounded to tf32;
+// products of bounded quantities (A_* against V and U, the keys decayed to the chunk's end) run in fp16; T is inverted in fp32.
+// U = rhs T^T takes both operands as tf32 pairs (hi + lo, three products: 21 bits, where a substitution in fp32 has 24; rhs itself
+// has the 11 of its operands).  U enters the state as an fp16 pair: the state is rounded to tf32 as an operand four times as
+// often as with 64-token tiles, and with U in one fp16 its error against 64 bits came out up to 2 % larger than theirs.  Relative
+// errors now, over 16..4096 tokens, three forms of decay, slow and fast: y 4.05e-4..4.71e-4, states 1.19e-4..3.07e-4; with the former tiles
+// 4.06e-4..5.29e-4 and 1.23e-4..4.07e-4.
 #include <type_traits>
 
 #include "umma.cuh"
@@ -39,17 +45,17 @@ constexpr int STATE_WARPS = 4, PREP_WARPS = 4, THREADS = 32 * (STATE_WARPS + PRE
 // byte offsets in a slot
 constexpr int O_AE = 0;                 // aE [16][64] tf32, 16-byte pieces of odd rows swapped in groups of four
 constexpr int O_RP = O_AE + 4096;       // rP, same layout
-constexpr int O_KD = O_RP + 4096;       // k P_15/P [16][64] fp16 in permuted columns, 16-byte pieces xored by row & 7
-constexpr int O_BD = O_KD + 2048;       // b~ P_15/P, same layout
+constexpr int O_KD = O_RP + 4096;       // kD [16][64] fp16 in permuted columns, 16-byte pieces xored by row & 7
+constexpr int O_BD = O_KD + 2048;       // bD, same layout
 constexpr int O_V = O_BD + 2048;        // v [16][64] fp16, pieces xored by row & 7
 constexpr int O_T = O_V + 2048;         // T [16][TS] fp32 (before that A_ab transposed)
 constexpr int TS = 24;                  // row stride of T: the lanes' 8-byte reads of four rows meet no bank twice
 constexpr int O_M = O_T + 16 * TS * 4;  // A_ak, A_qk, A_qb as B fragments: [matrix][lane][4] pairs of fp16
-constexpr int O_GL = O_M + 3 * 512;     // P_15 [64] fp32
+constexpr int O_GL = O_M + 3 * 512;     // product of all decays of the chunk [64] fp32
 constexpr int SLOT_BYTES = O_GL + 256;
-constexpr int O_KI = O_KD;              // kI [16][64] fp32 while the four products are formed; then k P_15/P and b~ P_15/P
-constexpr int O_BI = O_V;               // bI, likewise; then v, T and the A_* fragments
-static_assert(O_BI + 4096 <= O_GL, "bI fits before P_15");
+constexpr int O_KD32 = O_KD;            // kD [16][64] fp32 while the four products are formed; then kD and bD in fp16
+constexpr int O_BD32 = O_V;             // bD, likewise; then v, T and the A_* fragments
+static_assert(O_BD32 + 4096 <= O_GL, "bD fits before the decays");
 constexpr int YS = 48;                  // row stride (bytes) of a state warp's 16 x 16 output tile: conflict-free
 constexpr int O_Y = SLOTS * SLOT_BYTES;
 constexpr int O_BAR = O_Y + STATE_WARPS * 16 * YS;
@@ -154,9 +160,10 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                     prefetch_l2(p.v + o);
                 }
             }
-            float2 P = make_float2(1.f, 1.f);
+            // from the last token to the first: R = product of the decays behind a token, inv = 1 / R
+            float2 R = make_float2(1.f, 1.f);
 #pragma unroll
-            for (int tb = 0; tb < 2; ++tb) {
+            for (int tb = 1; tb >= 0; --tb) {
                 __half2 r2[8], k2[8], kk2[8], a2[8];
                 WPair w2[8];
 #pragma unroll
@@ -168,35 +175,35 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                     k2[j] = *reinterpret_cast<const __half2*>(p.k + o);
                     r2[j] = *reinterpret_cast<const __half2*>(p.r + o);
                 }
-                if (tb == 0 && c >= SLOTS && !mbar_wait(&empty[slot], (c / SLOTS - 1) & 1, actx, kErrWaitEmpty)) goto out;
+                float2 inv = make_float2(fast_rcp(R.x), fast_rcp(R.y));
+                if (tb == 1 && c >= SLOTS && !mbar_wait(&empty[slot], (c / SLOTS - 1) & 1, actx, kErrWaitEmpty)) goto out;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 7; j >= 0; --j) {
                     float2 w;
                     if constexpr (W_MODE == 1) w = w2[j];
                     else w = __half22float2(w2[j]);
+                    const float2 kk = __half22float2(kk2[j]), a = __half22float2(a2[j]), k = __half22float2(k2[j]), r = __half22float2(r2[j]);
+                    const uint32_t o = (tb * 8 + j) * 256 + ((j & 1) ? f_odd : f_even);
+                    *reinterpret_cast<float2*>(sl + O_KD32 + o) = make_float2(k.x * R.x, k.y * R.y);
+                    *reinterpret_cast<float2*>(sl + O_BD32 + o) = make_float2(kk.x * a.x * R.x, kk.y * a.y * R.y);
+                    *reinterpret_cast<uint2*>(sl + O_RP + o) = make_uint2(tf32_bits(r.x * inv.x), tf32_bits(r.y * inv.y));
                     if constexpr (W_MODE == 2) {
                         w.x = __expf(-0.606531f * fast_rcp(1.f + __expf(-w.x)));
                         w.y = __expf(-0.606531f * fast_rcp(1.f + __expf(-w.y)));
                     }
-                    const float2 kk = __half22float2(kk2[j]), a = __half22float2(a2[j]), k = __half22float2(k2[j]), r = __half22float2(r2[j]);
-                    const float2 ae = make_float2(-kk.x * P.x, -kk.y * P.y);
-                    P.x *= w.x;
-                    P.y *= w.y;
-                    const float2 inv = make_float2(fast_rcp(P.x), fast_rcp(P.y));
-                    const uint32_t o = (tb * 8 + j) * 256 + ((j & 1) ? f_odd : f_even);
-                    *reinterpret_cast<uint2*>(sl + O_AE + o) = make_uint2(tf32_bits(ae.x), tf32_bits(ae.y));
-                    *reinterpret_cast<uint2*>(sl + O_RP + o) = make_uint2(tf32_bits(r.x * P.x), tf32_bits(r.y * P.y));
-                    *reinterpret_cast<float2*>(sl + O_KI + o) = make_float2(k.x * inv.x, k.y * inv.y);
-                    *reinterpret_cast<float2*>(sl + O_BI + o) = make_float2(kk.x * a.x * inv.x, kk.y * a.y * inv.y);
+                    R.x *= w.x;
+                    R.y *= w.y;
+                    inv = make_float2(fast_rcp(R.x), fast_rcp(R.y));
+                    *reinterpret_cast<uint2*>(sl + O_AE + o) = make_uint2(tf32_bits(-kk.x * inv.x), tf32_bits(-kk.y * inv.y));
                 }
             }
-            *reinterpret_cast<float2*>(sl + O_GL + lane * 8) = P;
+            *reinterpret_cast<float2*>(sl + O_GL + lane * 8) = R;
             uint4 vv[4];  // v of the chunk: 128 pieces of 16 bytes
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 vv[i] = *reinterpret_cast<const uint4*>(p.v + row0 + (size_t)(i * 4 + (lane >> 3)) * stride + (lane & 7) * 8);
             __syncwarp();
-            // the four products: rows t of aE (0) and rP (1) against kI (n-tiles 0, 1) and bI (2, 3)
+            // the four products: rows t of aE (0) and rP (1) against kD (n-tiles 0, 1) and bD (2, 3)
             float acc[2][4][4];
 #pragma unroll
             for (int m = 0; m < 2; ++m)
@@ -212,8 +219,8 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                 for (int hf = 0; hf < 2; ++hf) {
                     A[0][hf] = *reinterpret_cast<const uint4*>(sl + O_AE + hf * 2048 + o);
                     A[1][hf] = *reinterpret_cast<const uint4*>(sl + O_RP + hf * 2048 + o);
-                    B[hf] = *reinterpret_cast<const uint4*>(sl + O_KI + hf * 2048 + o);
-                    B[2 + hf] = *reinterpret_cast<const uint4*>(sl + O_BI + hf * 2048 + o);
+                    B[hf] = *reinterpret_cast<const uint4*>(sl + O_KD32 + hf * 2048 + o);
+                    B[2 + hf] = *reinterpret_cast<const uint4*>(sl + O_BD32 + hf * 2048 + o);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -228,16 +235,16 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
 #pragma unroll
                     for (int q = 0; q < 4; ++q) mma_tf32(acc[m][q], A[m][0].z, A[m][1].z, A[m][0].w, A[m][1].w, B[q].z, B[q].w);
             }
-            // keys decayed to the chunk's end
+            // kD and bD in fp16
             uint32_t kd[16], bd[16];
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
                 const uint32_t o = t * 256 + ((t & 1) ? f_odd : f_even);
-                const float2 ki = *reinterpret_cast<const float2*>(sl + O_KI + o), bi = *reinterpret_cast<const float2*>(sl + O_BI + o);
-                kd[t] = pack_half2(ki.x * P.x, ki.y * P.y);
-                bd[t] = pack_half2(bi.x * P.x, bi.y * P.y);
+                const float2 k2 = *reinterpret_cast<const float2*>(sl + O_KD32 + o), b2 = *reinterpret_cast<const float2*>(sl + O_BD32 + o);
+                kd[t] = pack_half2(k2.x, k2.y);
+                bd[t] = pack_half2(b2.x, b2.y);
             }
-            __syncwarp();  // kI and bI are read: their room is free
+            __syncwarp();  // kD and bD are read: their room is free
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
                 const uint32_t o = t * 128 + ((h_piece ^ (t & 7)) << 4) + h_in;
@@ -332,7 +339,7 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
             ldmatrix4_trans(va, sl_u32 + O_V + v_at);
             const uint4 mak = *reinterpret_cast<const uint4*>(sl + O_M + lane * 16);
             const uint4 mqk = *reinterpret_cast<const uint4*>(sl + O_M + 512 + lane * 16);
-            float au[2][2][4], ar[2][4];  // [tokens 0..7, 8..15][tiles of even, odd index]: S0 aE^T + V^T A_ak^T, S0 rP^T + V^T A_qk^T
+            float au[2][2][4], ar[2][4];  // [tokens 0..7, 8..15][tiles of even, odd index]: S0d aE^T + V^T A_ak^T, S0d rP^T + V^T A_qk^T
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -351,6 +358,8 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                 ldmatrix4_trans(kd, sl_u32 + O_KD + d_row + (((2 * pp + (mi >> 1)) ^ l7) << 4));
                 float(&s0)[4] = S[2 * pp];
                 float(&s1)[4] = S[2 * pp + 1];
+                s0[0] *= gl.x; s0[1] *= gl.y; s0[2] *= gl.x; s0[3] *= gl.y;
+                s1[0] *= gl.z; s1[1] *= gl.w; s1[2] *= gl.z; s1[3] *= gl.w;
                 const uint32_t e0 = tf32_bits(s0[0]), e1 = tf32_bits(s0[2]), e2 = tf32_bits(s0[1]), e3 = tf32_bits(s0[3]);
                 const uint32_t o0 = tf32_bits(s1[0]), o1 = tf32_bits(s1[2]), o2 = tf32_bits(s1[1]), o3 = tf32_bits(s1[3]);
                 mma_tf32(au[0][0], e0, e1, e2, e3, a0.x, a0.y);
@@ -361,8 +370,6 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                 mma_tf32(ar[1], e0, e1, e2, e3, r1.x, r1.y);
                 mma_tf32(ar[0], o0, o1, o2, o3, r0.z, r0.w);
                 mma_tf32(ar[1], o0, o1, o2, o3, r1.z, r1.w);
-                s0[0] *= gl.x; s0[1] *= gl.y; s0[2] *= gl.x; s0[3] *= gl.y;
-                s1[0] *= gl.z; s1[1] *= gl.w; s1[2] *= gl.z; s1[3] *= gl.w;
                 mma_f16(s0, va, kd[0], kd[1]);
                 mma_f16(s1, va, kd[2], kd[3]);
             }

@@ -425,6 +425,26 @@ def test_chunk_scan_tensor_core_against_oracle(B, T, Hh, chunk):
         hb.self_chunk_rwkv7(*args, chunk_size=48)
 
 
+def test_chunk_scan_single_chunk_error_against_64_bits():
+    """One chunk of 16 tokens: the state no further from a float64 recurrence than with the 64-token tiles of the former kernel
+    (1.5954e-4 over these inputs; 1.617e-4 with a chunk's operands scaled to its start, 1.581e-4 scaled to its end)."""
+    errors = []
+    for seed in range(8):
+        g = torch.Generator(device="cuda").manual_seed(100 * seed + 16)
+        n = lambda: torch.randn(4, 16, 40, N, generator=g, device="cuda")
+        r, k, v = n().half(), n().half(), n().half()
+        kk, a = torch.nn.functional.normalize(k.float(), dim=-1).half(), torch.sigmoid(n()).half()
+        w = torch.exp(-0.606531 * torch.sigmoid(n().half().float()))
+        s = torch.zeros(4, 40, N, N, device="cuda")
+        _, got = hb.self_chunk_rwkv7(r, w, k, v, kk, a, s, chunk_size=16)
+        s = s.double()
+        for t in range(16):
+            kd, vd, kkd, ad, wd = (x[:, t].double() for x in (k, v, kk, a, w))
+            s = s * wd.unsqueeze(-2) - (s @ kkd.unsqueeze(-1)) * (kkd * ad).unsqueeze(-2) + vd.unsqueeze(-1) * kd.unsqueeze(-2)
+        errors.append(float((got.double() - s).norm() / s.norm()))
+    assert sum(errors) / len(errors) < 1.5955e-4
+
+
 def test_scan_full_size_config2():
     """Isolated WKV-7 op at the benchmark's size (B8 T4096 H32 N64, zero state): chunked tensor-core scan vs the
     sequential kernel over all heads (state rel-err <= 1e-3, outputs <= 2e-3 relative), and both against the fp64
