@@ -24,7 +24,7 @@
 // each in turn, into a ring of six slots: decay products, scaled operands, the four 16 x 16 products, the inverse.  mma.sync
 // and not tcgen05: these products are 16 rows high, and through tensor memory every link of the chain costs a store, a
 // fence, an issue, a commit and a load, about 700 cycles (a tile of 64 tokens with five such links took 16.9 k cycles with one CTA
-// an SM).  8 sequences x 4096 tokens x 32 heads, in a row: 1154 -> 412 us (0.40 of the HBM floor of 165 us).
+// an SM).  8 sequences x 4096 tokens x 32 heads, in a row: 1154 -> 412 us (0.40 of the HBM floor of 165 us), raw decays 1209 -> 454.
 //
 // Products that contain decay-scaled factors (range e^9.7 over 16 tokens with the model's decays) run on operands rounded to tf32;
 // products of bounded quantities (A_* against V and U, the keys decayed to the chunk's end) run in fp16; T is inverted in fp32.
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                 }
             }
             // from the last token to the first: R = product of the decays behind a token, inv = 1 / R
-            float2 R = make_float2(1.f, 1.f);
+            float2 R = make_float2(1.f, 1.f), lr = make_float2(0.f, 0.f);
 #pragma unroll
             for (int tb = 1; tb >= 0; --tb) {
                 __half2 r2[8], k2[8], kk2[8], a2[8];
@@ -188,11 +188,16 @@ __global__ void __launch_bounds__(ck::THREADS, 2) wkv7_chunk_kernel(const ChunkA
                     *reinterpret_cast<float2*>(sl + O_BD32 + o) = make_float2(kk.x * a.x * R.x, kk.y * a.y * R.y);
                     *reinterpret_cast<uint2*>(sl + O_RP + o) = make_uint2(tf32_bits(r.x * inv.x), tf32_bits(r.y * inv.y));
                     if constexpr (W_MODE == 2) {
-                        w.x = __expf(-0.606531f * fast_rcp(1.f + __expf(-w.x)));
-                        w.y = __expf(-0.606531f * fast_rcp(1.f + __expf(-w.y)));
+                        // logarithms are summed, and what the state itself is multiplied by, chunk after chunk, is rounded to nearest: an
+                        // approximate exponential a token, multiplied up, took 6.1e-5 off a state that 8192 tokens hardly decay
+                        // (raw w of -6), this 1.2e-6, and the former tiles 1.9e-6
+                        lr.x -= 0.606531f * fast_rcp(1.f + __expf(-w.x));
+                        lr.y -= 0.606531f * fast_rcp(1.f + __expf(-w.y));
+                        R = tb == 0 && j == 0 ? make_float2(1.f + expm1f(lr.x), 1.f + expm1f(lr.y)) : make_float2(__expf(lr.x), __expf(lr.y));
+                    } else {
+                        R.x *= w.x;
+                        R.y *= w.y;
                     }
-                    R.x *= w.x;
-                    R.y *= w.y;
                     inv = make_float2(fast_rcp(R.x), fast_rcp(R.y));
                     *reinterpret_cast<uint2*>(sl + O_AE + o) = make_uint2(tf32_bits(-kk.x * inv.x), tf32_bits(-kk.y * inv.y));
                 }

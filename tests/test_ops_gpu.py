@@ -445,6 +445,18 @@ def test_chunk_scan_single_chunk_error_against_64_bits():
     assert sum(errors) / len(errors) < 1.5955e-4
 
 
+def test_chunk_scan_raw_decay_does_not_drift():
+    """A state that is only decayed, by raw logits of about -6 over 8192 tokens.  A chunk's factor and its product with the state
+    are rounded to nearest, half a unit each with either sign; allowed is a bias of a quarter unit for each of the 512 chunks."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    raw = (0.5 * torch.randn(1, 8192, 8, N, generator=g, device="cuda") - 6).half()
+    s0 = torch.randn(1, 8, N, N, generator=g, device="cuda") + 2
+    z = torch.zeros_like(raw)
+    _, got = hb.self_chunk_rwkv7(z, raw, z, z, z, z, s0.clone(), chunk_size=16, w_is_raw=True)
+    exact = s0.double() * torch.exp(-0.606531 * torch.sigmoid(raw.double()).sum(1)).unsqueeze(-2)
+    assert abs(float(((got.double() - exact) / exact).mean())) < 512 * 2.0 ** -24 / 4
+
+
 def test_scan_full_size_config2():
     """Isolated WKV-7 op at the benchmark's size (B8 T4096 H32 N64, zero state): chunked tensor-core scan vs the
     sequential kernel over all heads (state rel-err <= 1e-3, outputs <= 2e-3 relative), and both against the fp64
