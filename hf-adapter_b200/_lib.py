@@ -48,6 +48,7 @@ SIGNATURES = {
     "rwkv7_seq_shift_mix": (I, [P, P, PP, PP, P, I, I, I, I, I, I, P]),
     "rwkv7_dense_small": (I, [P] * 4 + [I, I, I, I, I, I, P]),
     "rwkv7_small_gemm_group": (I, [I, PP, PP, PP, PP, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int), I, I, P]),
+    "rwkv7_small_gemm_group_lean": (I, [I, PP, PP, PP, PP, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int), I, I, P]),
     "rwkv7_rows_gemv": (I, [I, PP, PP, PP, PP, PP] + [ctypes.POINTER(c_int)] * 4 + [I, I, I, P]),
     "rwkv7_prefill_state_prep_gate": (I, [P] * 13 + [I, I, I, I, I, I, I, P]),
     "rwkv7_prefill_state_prep": (I, [P] * 12 + [I, I, I, I, I, I, I, P]),

@@ -225,9 +225,8 @@ static cudaError_t launch_group(cudaLaunchConfig_t& cfg, const GroupArgs& a) {
 
 using namespace rwkv7;
 
-extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
-                                      void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
-                                      void* stream) {
+static int small_gemm_group(int n_problems, const void* const* x, const void* const* W, const void* const* bias, void* const* out,
+                            const int* K, const int* Nout, const int* act_out, int M, int dtype, bool lean, void* stream) {
     RWKV7_REQUIRE(n_problems >= 1 && n_problems <= kMaxProblems, RWKV7_ERR_INVALID, "small_gemm_group: 1..%d problems", kMaxProblems);
     RWKV7_REQUIRE(M >= 1 && M <= 16384, RWKV7_ERR_UNSUPPORTED, "small_gemm_group: M must be in 1..16384 (got %d)", M);
     const int row_blocks = (M + LT - 1) / LT;
@@ -268,9 +267,23 @@ extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, cons
     cfg.attrs = attr;
     cfg.numAttrs = programmatic_launch_ok(cfg.stream) ? 2 : 1;
     cudaError_t e;
-    const bool deep = (chunks + splits - 1) / splits > 2;
+    const bool deep = !lean && (chunks + splits - 1) / splits > 2;
     if (dtype == RWKV7_F16) e = deep ? launch_group<__half, 4>(cfg, a) : launch_group<__half, 2>(cfg, a);
     else e = deep ? launch_group<__nv_bfloat16, 4>(cfg, a) : launch_group<__nv_bfloat16, 2>(cfg, a);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "small_gemm_group launch: %s", cudaGetErrorString(e));
     return RWKV7_OK;
+}
+
+extern "C" int rwkv7_small_gemm_group(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
+                                      void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
+                                      void* stream) {
+    return small_gemm_group(n_problems, x, W, bias, out, K, Nout, act_out, M, dtype, false, stream);
+}
+
+// Two K chunks and 32 KB a CTA whatever K is: beside kernels that want most of an SM's shared memory (r / k / v of a dense step as
+// three GEMMs) the CTAs of the deep ring, 64 KB each, hold theirs off.
+extern "C" int rwkv7_small_gemm_group_lean(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
+                                           void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
+                                           void* stream) {
+    return small_gemm_group(n_problems, x, W, bias, out, K, Nout, act_out, M, dtype, true, stream);
 }

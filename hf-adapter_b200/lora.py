@@ -29,9 +29,10 @@ def dense_small(x, weight, bias=None, *, act_in: int = 0, act_out: int = 0, out=
     return out.reshape(*x.shape[:-1], Nout)
 
 
-def small_gemm_group(xs, weights, biases=None, acts=None, outs=None):
+def small_gemm_group(xs, weights, biases=None, acts=None, outs=None, *, lean: bool = False):
     """One launch for up to four independent small linears ``out_i = act_i(x_i @ W_i.T + b_i)`` sharing the row
-    count (fp16/bf16: tensor-core kernel, 64-row blocks; fp32: one ``dense_small`` call per problem)."""
+    count (fp16/bf16: tensor-core kernel, 64-row blocks; fp32: one ``dense_small`` call per problem).  ``lean``: the same
+    from CTAs with less shared memory, for a launch beside kernels that need it."""
     n = len(xs)
     biases = list(biases) if biases is not None else [None] * n
     acts = list(acts) if acts is not None else [0] * n
@@ -60,9 +61,9 @@ def small_gemm_group(xs, weights, biases=None, acts=None, outs=None):
     bp, _k3 = _lib.ptr_array([0 if t is None else t.data_ptr() for t in bs])
     op, _k4 = _lib.ptr_array([t.data_ptr() for t in outs])
     IA = _lib.c_int * n
-    _lib.check(_lib.lib.rwkv7_small_gemm_group(n, xp, wp, bp, op, IA(*[int(w.shape[1]) for w in ws]),
-                                               IA(*[int(w.shape[0]) for w in ws]), IA(*acts), M, dt_code(x2[0]),
-                                               stream_ptr(x2[0])), "small_gemm_group")
+    entry = _lib.lib.rwkv7_small_gemm_group_lean if lean else _lib.lib.rwkv7_small_gemm_group
+    _lib.check(entry(n, xp, wp, bp, op, IA(*[int(w.shape[1]) for w in ws]), IA(*[int(w.shape[0]) for w in ws]), IA(*acts), M,
+                     dt_code(x2[0]), stream_ptr(x2[0])), "small_gemm_group")
     return [o.reshape(*x.shape[:-1], int(w.shape[0])) for o, x, w in zip(outs, xs, ws)]
 
 

@@ -263,38 +263,61 @@ class StepContext:
 _DEFAULT_CONTEXT = StepContext()
 
 
+def _lora_leads(op, rows: int, features: int) -> bool:
+    """Whether the LoRA chain stays on the main stream when r / k / v are three products like ``op`` (of ``features`` inputs)."""
+    # The longer branch leads: it starts on the programmatic edge of the kernel before it.  The chain is two launches whatever the width,
+    # the products grow with it.  us a step, dense fp16 / bf16, chain first -> r first, at 9 / 16 / 32 / 48 / 63 rows (library GEMMs):
+    # 768 wide 617 / 633 / 656 / 679 / 705 -> 652 / 669 / 690 / 708 / 729; 1536 1270 / 1313 / 1437 / 1499 / 1790 -> 1358 / 1315 / 1509 /
+    # 1612 / 1715; 2048 1492 / 1539 / 1733 / 2014 / 1990 -> 1540 / 1590 / 1731 / 1885 / 2022; 2560 2486 / 2576 / 2799 / 3208 / 3312 -> 2417 /
+    # 2504 / 2793 / 3045 / 3086.  At 64 / 128 / 256 rows (this library's GEMM): 768 1124 / 1213 / 1139 -> 1135 / 1219 / 1132; 1024 2297 / 2653 /
+    # 2585 -> 2262 / 2484 / 2381; 2560 5835 / 6595 / 6936 -> 5634 / 6176 / 6442.  Affine int8, 2560 wide, 12 / 32 / 64 rows 10350 / 19217 / 9218 ->
+    # 10190 / 19055 / 9235.  int8 x int8 (a quantiser and a product each), 12 / 64 rows: 7332 / 4913 -> 7312 / 4861 on one card, 7519 /
+    # 5120 -> 8317 / 5497 on another.
+    if isinstance(op, _q.A8W8Linear):
+        return True
+    return _out_features(op) * features < (2048 * 2048 if rows < _gemm.MIN_ROWS else 1024 * 1024)
+
+
 def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
-    """r / k / v and the LoRA pre-activations of a layer step on parallel branches: ``[r, k, v, w, a, g(, v_gate)]``."""
-    # The LoRA chain is two launches long and leads on the main stream, behind the kernel that made its inputs; r / k / v do not
-    # depend on it and branch off (parallel branches of the decode graph once captured), joined before the recurrence.
+    """r / k / v and the LoRA pre-activations of a layer step on parallel branches (of the decode graph once captured):
+    ``[r, k, v, w, a, g(, v_gate)]``."""
     main = torch.cuda.current_stream(x.device)
     # (tiled weights that are built on first use belong to the stream that outlives the branches: ahead of the fork)
     tiled = _rkv_tiled(ops, xs)
     fork = main.record_event()
-    hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)])
-    lora = _lora.small_gemm_group(hs, [_weight_of(w) for w in ups])
     used = []
 
-    def branch(i, t, run):
+    def branch(i, ts, run):
         st = ctx.side_stream(x.device, i)
         st.wait_event(fork)
         used.append(st)
         with torch.cuda.stream(st):
             y = run()
-        for v in t:
-            v.record_stream(st)
+        for t in ts:
+            t.record_stream(st)
         return y
+
+    def lora_chain(lean=False):
+        hs = _lora.small_gemm_group(down_x, [_weight_of(w) for w in downs], acts=(1, 0, 2, 0)[:len(downs)], lean=lean)
+        return _lora.small_gemm_group(hs, [_weight_of(w) for w in ups], lean=lean)
 
     if tiled is not None:
         # int4 / int8 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
-        # exchange) instead of three launches competing for the SMs
-        rkv = branch(0, xs, lambda: _rkv_launch(ops, xs, tiled))
-    else:
+        # exchange).  The LoRA chain is two launches long and leads, behind the kernel that made its inputs; they branch off
+        lora = lora_chain()
+        branched = rkv = branch(0, xs, lambda: _rkv_launch(ops, xs, tiled))
+    elif _lora_leads(ops[0], int(x.shape[0]), int(xs[0].shape[-1])):
         # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
-        rkv = [branch(i, (t,), lambda: apply_linear(o, t)) for i, (o, t) in enumerate(zip(ops, xs))]
+        lora = lora_chain()
+        branched = rkv = [branch(i, (t,), lambda: apply_linear(o, t)) for i, (o, t) in enumerate(zip(ops, xs))]
+    else:
+        # they are the longer branch: r leads, and the LoRA kernels leave them the SMs' shared memory
+        lora = branch(0, down_x, lambda: lora_chain(lean=True))
+        k, v = (branch(i, (xs[i],), lambda: apply_linear(ops[i], xs[i])) for i in (1, 2))
+        rkv, branched = [apply_linear(ops[0], xs[0]), k, v], (k, v, *lora)
     for st in used:
         main.wait_stream(st)
-    _used_on(main, *rkv)
+    _used_on(main, *branched)
     return [*rkv, *lora]
 
 

@@ -243,6 +243,10 @@ int rwkv7_rows_gemv(int n_problems, const void* const* x, const void* const* W, 
 int rwkv7_small_gemm_group(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
                            void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
                            void* stream);
+/* The same results from CTAs of at most 32 KB of shared memory (64 otherwise), for a call beside kernels that need it. */
+int rwkv7_small_gemm_group_lean(int n_problems, const void* const* x, const void* const* W, const void* const* bias,
+                                void* const* out, const int* K, const int* Nout, const int* act_out, int M, int dtype,
+                                void* stream);
 
 /* ------------------------------------------------------------------ prefill state / output prep
  * Replaces fused_prefill_state_prep (rwkv7_hf/fused_prefill.py:184): per row of [rows,H*64]

@@ -190,3 +190,24 @@ def test_tiled_weights_are_built_on_the_stream_of_the_step(weights, cls, monkeyp
         m._decode_step(torch.zeros(16, device="cuda", dtype=torch.long), m.new_cache(16))
     torch.cuda.synchronize()
     assert len(seen) >= 6 and all(s == main for s in seen)  # r, k, v, o and the two of the FFN
+
+
+@pytest.mark.parametrize("weights,D,rows,leads", [("dense", 512, 16, True), ("dense", 2048, 16, False), ("dense", 512, 64, True),
+                                                  ("dense", 1024, 64, False), ("mm8", 2048, 16, False), ("a8w8", 2048, 16, True),
+                                                  ("mm4", 2048, 16, True)])
+def test_longer_branch_of_a_layer_stays_on_the_stream_of_the_step(weights, D, rows, leads, monkeypatch):
+    """Where r / k / v are three products of wide weights, r stays on the step's stream and the LoRA chain branches off, in its form
+    with little shared memory; else the chain stays."""
+    from hf_adapter_b200 import lora, packing
+    m = _model(weights, D, 1)
+    chain, products = [], []
+    real_chain, real_linear = lora.small_gemm_group, packing.apply_linear
+    monkeypatch.setattr(lora, "small_gemm_group", lambda *a, **k: (chain.append((torch.cuda.current_stream(), bool(k.get("lean")))), real_chain(*a, **k))[1])
+    monkeypatch.setattr(packing, "apply_linear", lambda *a, **k: (products.append(torch.cuda.current_stream()), real_linear(*a, **k))[1])
+    with torch.no_grad():
+        m._decode_step(torch.zeros(rows, device="cuda", dtype=torch.long), m.new_cache(rows))
+    torch.cuda.synchronize()
+    main = torch.cuda.current_stream()
+    assert [(s == main, lean) for s, lean in chain] == [(leads, not leads)] * 2
+    if weights != "mm4":  # (one grouped launch)
+        assert sum(s == main for s in products[:3]) == (0 if leads else 1)
