@@ -8,11 +8,16 @@ from . import _lib
 from ._util import dt_code, no_fallback, ptr, require_cuda, same_dtype, stream_ptr
 
 
-# Elements of a sequence up to which its norm and its mixes are one kernel.  It normalises every row twice (once as the row before the
-# next), which few CTAs do not notice and many do.  us, two kernels -> one, six mixes / one mix: 512 x 768 fp32 8.0 / 5.1 -> 5.1 / 3.5,
-# 64 x 2560 fp16 5.9 / 4.9 -> 3.9 / 2.8, 1024 x 4096 16.9 / 10.7 -> 15.8 / 11.2, 2331 x 2560 24.3 / 14.7 -> 21.5 / 14.8, 4096 x 4096 60.8 /
-# 34.6 -> 63.4 / 37.8; a launch less either way.
-SEQ_NORM_MIX_ELEMENTS = 6 << 20
+def _one_norm_mix(rows: int, width: int, dtype) -> bool:
+    """Whether the norm and the mixes of a sequence are one kernel, which normalises every row twice (once as the row before the next):
+    few CTAs do not notice, many do, and the fewer fit an SM the sooner (a CTA is width / 8 threads up to 4096, above that 512 with
+    two vectors each)."""
+    # us, two kernels -> one, six mixes / one mix.  fp16: 2331 x 2560 25.7 / 17.6 -> 24.9 / 16.5, 2048 x 3072 25.7 / 17.5 -> 24.7 / 16.1; 768 x 4096
+    # 16.5 / 9.4 -> 15.4 / 9.4, 1024 x 4096 18.1 / 11.4 -> 18.6 / 11.4, 1400 x 4096 22.2 / 15.3 -> 24.9 / 16.0; 128 x 5120 7.1 / 5.8 -> 6.8 / 4.2, 256 x 5120
+    # 9.4 / 6.4 -> 10.5 / 6.3, 1024 x 5120 24.2 / 16.7 -> 32.3 / 20.3; 128 x 8192 8.4 / 6.3 -> 6.8 / 4.8, 384 x 8192 16.2 / 9.4 -> 19.0 / 9.8.  fp32, which
+    # waits for memory: 2048 x 768 21.3 / 9.1 -> 13.9 / 6.3, 1600 x 3584 56.2 / 22.7 -> 44.2 / 21.7, 768 x 8192 65.2 / 29.3 -> 59.6 / 27.3.
+    most = 6 if dtype == torch.float32 or width <= 3072 else 3 if width <= 4096 else 1
+    return rows * width <= most << 20
 
 
 def _rows(x, name):
@@ -169,7 +174,7 @@ def sequence_norm_mix(x, initial_prev, norm_weight, norm_bias, mixes, eps: float
     nw, nb = norm_weight.contiguous(), norm_bias.contiguous()
     mp, _k1 = _lib.ptr_array([m.data_ptr() for m in flat])
     op, _k2 = _lib.ptr_array([o.data_ptr() for o in outs])
-    if B * T * D <= SEQ_NORM_MIX_ELEMENTS:
+    if _one_norm_mix(B * T, D, x.dtype):
         _lib.check(_lib.lib.rwkv7_seq_norm_mix(ptr(src), ptr(nw), ptr(nb), ptr(initial), mp, op, ptr(nxt), B, T, D, len(mixes), float(eps),
                                                dt_code(src), stream_ptr(src)), "sequence_norm_mix")
     else:

@@ -152,3 +152,11 @@ def test_every_capture_holds_the_collector_off():
     files = [os.path.join(package, f) for f in sorted(os.listdir(package)) if f.endswith(".py")] + [os.path.join(ROOT, "bench.py")]
     bare = [os.path.basename(f) for f in files if re.search(r"with torch\.cuda\.graph\(", open(f).read())]
     assert bare == ["_util.py"]
+
+
+@pytest.mark.parametrize("dtype,width,one,two", [(torch.float16, 2560, 2331, 2458), (torch.bfloat16, 3072, 2048, 2049), (torch.float16, 4096, 768, 1024),
+                                                 (torch.float16, 5120, 128, 256), (torch.float16, 8192, 128, 384), (torch.float32, 3584, 1600, 1756),
+                                                 (torch.float32, 8192, 768, 769)])
+def test_norm_and_mixes_are_one_kernel_up_to_the_size_at_which_that_was_faster(dtype, width, one, two):
+    from hf_adapter_b200 import norm_mix
+    assert norm_mix._one_norm_mix(one, width, dtype) and not norm_mix._one_norm_mix(two, width, dtype)

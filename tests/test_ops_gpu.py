@@ -336,7 +336,8 @@ def test_grouped_lora_gemm_odd_widths_and_ragged_k(dt, M, K, Nout):
 
 
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("B,T,D", [(1, 1, 8), (2, 3, 264), (3, 37, 768), (2, 5, 4096), (1, 9, 4104), (2, 2, 8192), (1, 1537, 4096)])
+@pytest.mark.parametrize("B,T,D", [(1, 1, 8), (2, 3, 264), (3, 37, 768), (2, 5, 4096), (1, 9, 4104), (2, 2, 8192), (1, 1537, 4096),
+                                   (1, 768, 4096), (1, 769, 4096), (1, 128, 8192), (1, 129, 8192)])
 def test_sequence_norm_mix(dt, B, T, D):
     """LayerNorm and token-shift mixes in one call, either side of the size at which one kernel becomes two and of the row
     width at which a thread takes two vectors, against 64 bits on the rounded rows.  The kernel's row may round the other way
