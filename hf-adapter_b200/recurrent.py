@@ -316,7 +316,9 @@ def self_chunk_rwkv7(r, w_decay, k, v, kk, a_gate, state_native, *, chunk_size: 
     """Chunked WY/DPLR scan on tensor cores (rwkv7_hf/self_chunk_rwkv7.py:33).  ``T`` must be a
     multiple of ``chunk_size`` and the head size 64, as in the reference (:56-62).  ``w_is_raw`` (an extension):
     ``w_decay`` holds the raw decay logits and the kernel forms ``exp(-0.606531 * sigmoid(w))`` itself, as the
-    reference's clamp-w scans do (rwkv7_hf/fused_recurrent_update.py:1420), so no decay tensor is materialised."""
+    reference's clamp-w scans do (rwkv7_hf/fused_recurrent_update.py:1420), so no decay tensor is materialised.  Other
+    decays than the model's, in fp16 activations: at least 0.0086 each (the kernel divides by products of 16 of them; a
+    zero gives NaN, where the sequential scan takes any)."""
     if w_is_raw:
         if w_is_log:
             raise ValueError("w_is_raw and w_is_log exclude each other")
@@ -338,7 +340,7 @@ def self_chunk_rwkv7(r, w_decay, k, v, kk, a_gate, state_native, *, chunk_size: 
 def dplr_chunk_scan(r, w, k, v, kk, a, state, *, chunk_size: int = 64, force_fallback: bool = False, algorithm=None):
     """rwkv7_hf/dplr_prefill.py:505: any positive chunk size; the result does not depend on it.
     Chunk sizes the tensor-core kernel takes (16/32/64 dividing T) use it, others run the
-    sequential kernel, which computes the same recurrence."""
+    sequential kernel, which computes the same recurrence.  Decays of the former: as in ``self_chunk_rwkv7``."""
     no_fallback(force_fallback, "dplr_chunk_scan")
     if int(chunk_size) <= 0:
         raise ValueError("chunk_size must be positive")

@@ -152,7 +152,9 @@ int rwkv7_wkv7_scan_f16state(const void* r, const void* w, const void* k, const 
 
 /* Chunked (WY / DPLR) form of the same scan with the intra-chunk products on tensor cores.
  * chunk in {16, 32, 64}; T % chunk == 0; fp16 activations only (RWKV7_ERR_UNSUPPORTED otherwise: callers route
- * other dtypes to rwkv7_wkv7_scan, which computes the same recurrence).  Same arguments as above. */
+ * other dtypes to rwkv7_wkv7_scan, which computes the same recurrence).  Same arguments as above, but it divides by products of
+ * decays: in w_mode 0 and 1 the product over the 16 tokens of a chunk has to be at least 2^-110 in every channel (decays of
+ * 0.0086 and more), or that head's results are NaN.  The decays of w_mode 2 are never below 0.54. */
 int rwkv7_wkv7_chunk_scan(const void* r, const void* w, const void* k, const void* v, const void* kk, const void* a,
                           const float* state_in, float* state_out, void* y,
                           int B, int T, int H, int N, int chunk, int dtype, int w_mode, void* stream);

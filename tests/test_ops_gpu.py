@@ -460,6 +460,29 @@ def test_chunk_scan_raw_decay_does_not_drift():
     assert abs(float(((got.double() - exact) / exact).mean())) < 512 * 2.0 ** -24 / 4
 
 
+@pytest.mark.parametrize("f32", [False, True])
+def test_chunk_scan_strong_decays(f32):
+    """Decays down to the smallest that the chunked form admits (2^-6.85 for all 16 tokens of a chunk in some channels, anything
+    above it in the others), against a float64 recurrence; the bounds of the other chunked tests."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    B, T, Hh = 2, 64, 3
+    n = lambda: torch.randn(B, T, Hh, N, generator=g, device="cuda")
+    r, k, v = n().half(), n().half(), n().half()
+    kk, a = torch.nn.functional.normalize(k.float(), dim=-1).half(), torch.sigmoid(n()).half()
+    log2 = -6.85 * torch.rand(B, T, Hh, N, generator=g, device="cuda")
+    log2[..., ::8] = -6.85
+    w = torch.exp2(log2) if f32 else torch.exp2(log2).half()
+    s0 = torch.randn(B, Hh, N, N, generator=g, device="cuda")
+    y, got = hb.self_chunk_rwkv7(r, w, k, v, kk, a, s0, chunk_size=16)
+    s, ys = s0.double(), []
+    for t in range(T):
+        rd, kd, vd, kkd, ad, wd = (x[:, t].double() for x in (r, k, v, kk, a, w))
+        s = s * wd.unsqueeze(-2) - (s @ kkd.unsqueeze(-1)) * (kkd * ad).unsqueeze(-2) + vd.unsqueeze(-1) * kd.unsqueeze(-2)
+        ys.append((s @ rd.unsqueeze(-1)).squeeze(-1))
+    assert rel_err(npf(got), npf(s)) < 1e-3
+    assert rel_err(npf(y), npf(torch.stack(ys, 1))) < 2e-3
+
+
 def test_scan_full_size_config2():
     """Isolated WKV-7 op at the benchmark's size (B8 T4096 H32 N64, zero state): chunked tensor-core scan vs the
     sequential kernel over all heads (state rel-err <= 1e-3, outputs <= 2e-3 relative), and both against the fp64
