@@ -69,8 +69,8 @@ struct PrepArgs {
     long long total_heads;  // rows * H
 };
 
-// V consecutive columns in storage type, 16 bytes: requested together and converted where they are used
-template <typename T, int V> struct alignas(16) Piece { T v[V]; };
+// V consecutive columns in storage type, 8 or 16 bytes: requested together and converted where they are used
+template <typename T, int V> struct alignas(V * sizeof(T)) Piece { T v[V]; };
 template <typename T, int V>
 __device__ __forceinline__ Piece<T, V> get_piece(const void* base, size_t off, bool ok = true) {
     Piece<T, V> r{};
@@ -87,10 +87,10 @@ __device__ __forceinline__ void put_piece(void* base, size_t off, const float (&
 
 // 64 / V lanes per (row, head), V columns per lane.  Bound: HBM.  32768 rows of 4096 fp16 with raw gates, no decay (five tensors read,
 // three written, 2.1 GB): 565 us with four columns a lane and the v gate requested behind the head's norm, 416 now; the gate
-// written as well 438, where a pass of its own took 114.
-template <typename T>
+// written as well 438, where a pass of its own took 114.  V: 16 bytes of columns a lane, or 8 where the heads are too few to fill the SMs.
+template <typename T, int V>
 __global__ void __launch_bounds__(256) state_prep_kernel(const PrepArgs p) {
-    constexpr int V = 16 / (int)sizeof(T), LANES = 64 / V;
+    constexpr int LANES = 64 / V;
     const long long gidx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
     const int l = threadIdx.x % LANES;
     const bool active = gidx < p.total_heads;
@@ -227,10 +227,14 @@ extern "C" int rwkv7_prefill_state_prep_gate(const void* w_raw, const void* k_ra
     PrepArgs p{w_raw, k_raw, v_raw, a, k_k, k_a, v_first, v_gate, w_out, k_out, v_out, kk_out, a_out,
                H, a_is_raw, v_gate_is_raw, log_decay, (long long)rows * H};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long threads = p.total_heads * (dtype == RWKV7_F32 ? 16 : 8);
+    // us with 8 / 4 columns a lane, fp16, decay written: 16 x 40 heads 4.8 / 3.8, 150 x 64 5.9 / 5.4, 800 x 12 5.9 / 5.3, 1024 x 12 6.4 / 6.4, 450 x 40 6.9 / 7.3,
+    // 1024 x 64 19.5 / 20.3
+    const bool wide = dtype != RWKV7_F32 && p.total_heads >= 12288;
+    const long long threads = p.total_heads * (wide ? 8 : 16);
     const int grid = (int)((threads + 255) / 256);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
-        state_prep_kernel<T><<<grid, 256, 0, st>>>(p);
+        if (wide) state_prep_kernel<T, sizeof(T) == 2 ? 8 : 4><<<grid, 256, 0, st>>>(p);
+        else state_prep_kernel<T, 4><<<grid, 256, 0, st>>>(p);
         return check_launch("state_prep_kernel");
     });
     return RWKV7_OK;
