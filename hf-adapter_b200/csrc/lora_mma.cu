@@ -6,7 +6,7 @@
 // projections (K = rank, Nout = attention width) of a layer.  These matrices are tiny (a few MB per
 // layer in total), so the kernel is built for latency: warp-level HMMA (mma.sync m16n8k16, fp32
 // accumulate) on 64 x 64 output tiles, 64-wide K chunks by cp.async with an XOR swizzle for
-// conflict-free ldmatrix, three of them in flight where a CTA has more than two, and split-K across a
+// conflict-free ldmatrix, two or three of them in flight where a CTA has more than two, and split-K across a
 // thread-block cluster whose partial tiles are reduced through distributed shared memory in fixed
 // rank order (deterministic, no scratch memory).  The pair of launches is the longest branch of a decode
 // step over many rows: with one chunk in flight, weights not announced and outputs stored one by one
@@ -66,7 +66,7 @@ __device__ __forceinline__ float lora_act(float v, int act) {
     return v;
 }
 
-// NST: K chunks in shared memory (2, or 4 where a CTA has more than two: then all but one of them are in flight)
+// NST: K chunks in shared memory, 16 KB each: 2, or 3 or 4 where a CTA has more than two, of which all but one are in flight
 template <typename T, int NST>
 __global__ void __launch_bounds__(LTHREADS) small_gemm_group_kernel(const GroupArgs p) {
     extern __shared__ __align__(128) unsigned char lsm[];
@@ -233,7 +233,7 @@ static int small_gemm_group(int n_problems, const void* const* x, const void* co
     RWKV7_REQUIRE(dtype == RWKV7_F16 || dtype == RWKV7_BF16, RWKV7_ERR_UNSUPPORTED, "small_gemm_group: fp16 / bf16 only");
     RWKV7_REQUIRE(x && W && out && K && Nout && act_out, RWKV7_ERR_INVALID, "small_gemm_group: null argument array");
     GroupArgs a{};
-    int max_tiles = 0, max_k = 0;
+    int max_tiles = 0, max_k = 0, tiles = 0;
     for (int i = 0; i < n_problems; ++i) {
         RWKV7_REQUIRE(x[i] && W[i] && out[i], RWKV7_ERR_INVALID, "small_gemm_group: null pointer in problem %d", i);
         RWKV7_REQUIRE(K[i] > 0 && Nout[i] > 0 && K[i] % 8 == 0, RWKV7_ERR_UNSUPPORTED,
@@ -244,6 +244,7 @@ static int small_gemm_group(int n_problems, const void* const* x, const void* co
         a.K[i] = K[i]; a.Nout[i] = Nout[i]; a.act[i] = act_out[i];
         max_tiles = max_tiles > (Nout[i] + LT - 1) / LT ? max_tiles : (Nout[i] + LT - 1) / LT;
         max_k = max_k > K[i] ? max_k : K[i];
+        tiles += (Nout[i] + LT - 1) / LT;
         a.pairs = (i == 0 || a.pairs) && Nout[i] % 2 == 0 && aligned(out[i], 4);
     }
     a.M = M;
@@ -268,8 +269,13 @@ static int small_gemm_group(int n_problems, const void* const* x, const void* co
     cfg.numAttrs = programmatic_launch_ok(cfg.stream) ? 2 : 1;
     cudaError_t e;
     const bool deep = !lean && (chunks + splits - 1) / splits > 2;
-    if (dtype == RWKV7_F16) e = deep ? launch_group<__half, 4>(cfg, a) : launch_group<__half, 2>(cfg, a);
-    else e = deep ? launch_group<__nv_bfloat16, 4>(cfg, a) : launch_group<__nv_bfloat16, 2>(cfg, a);
+    // An SM holds three CTAs of four chunks and four of three: the fourth pays while it costs no second wave.  us with 4 / 3 / 2 chunks, the
+    // four downs of a layer (ranks 64, 64, 128, 32; fp16): 2560 wide 2331 rows 33.9 / 35.1 / 35.6, 4096 rows 36.1 / 44.1 / 51.0, 6000 54.8 / 45.8 / 54.6,
+    // 12000 85.4 / 74.8 / 92.0; 4096 wide 4096 rows 50.6 / 63.6 / 75.0, 6000 79.3 / 65.8 / 81.8, 12000 125.4 / 102.2 / 134.6; 768 wide 6000 24.3 / 20.7 / 21.7,
+    // 12000 38.1 / 33.4 / 33.0
+    const bool one_wave = tiles * row_blocks * splits <= 3 * 148;
+    if (dtype == RWKV7_F16) e = !deep ? launch_group<__half, 2>(cfg, a) : one_wave ? launch_group<__half, 4>(cfg, a) : launch_group<__half, 3>(cfg, a);
+    else e = !deep ? launch_group<__nv_bfloat16, 2>(cfg, a) : one_wave ? launch_group<__nv_bfloat16, 4>(cfg, a) : launch_group<__nv_bfloat16, 3>(cfg, a);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "small_gemm_group launch: %s", cudaGetErrorString(e));
     return RWKV7_OK;
 }

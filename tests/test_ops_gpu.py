@@ -311,7 +311,7 @@ def test_grouped_lora_gemm_against_oracle(M):
 
 
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("M", [1, 65])
+@pytest.mark.parametrize("M", [1, 65, 14300])  # (14300: more CTAs of a K above 128 than one wave, which take a ring of three)
 @pytest.mark.parametrize("K,Nout", [((72,), (41,)), ((328, 328), (40, 1)), ((520,), (64,)), ((520, 520, 520), (66, 65, 2)),
                                     ((4104,), (41,)), ((4104, 72, 8), (40, 41, 1)), ((4104, 4096), (64, 32))])
 def test_grouped_lora_gemm_odd_widths_and_ragged_k(dt, M, K, Nout):
