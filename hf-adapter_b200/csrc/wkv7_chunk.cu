@@ -16,11 +16,12 @@
 // 1.617e-4 so, 4.147e-4 / 1.581e-4 now, and 4.146e-4 / 1.595e-4 with the former tiles of 64 tokens.)
 //
 // What bounds it: the shared-memory pipe on an SM with two heads (99 % of its active cycles in the fullest SM, 85 % on average; tensor
-// pipe 52 / 45 %, issue slots 57 / 49 %, HBM 27 %) and the serial chain S0 -> U -> S' of a head, which is kept in registers.  Four STATE warps own 16 value rows each; the rows of the state never meet, so these warps never
-// wait for one another, and a warp's state is an mma accumulator that becomes the next product's A operand where it is: the
-// two columns a lane holds of an accumulator tile are read as k positions tq and tq + 4 of the A fragment, and the B operands are
-// read in the same permuted order (physical column 16 p + 4 tq + 2 e + f is column 2 tq + f of tile 2 p + e, so a lane's share of
-// two tiles is one 16-byte piece).  Everything that does not depend on the state is made ahead by four PREP warps, one chunk
+// pipe 52 / 45 %, issue slots 57 / 49 %, HBM 27 %) and the serial chain S0 -> U -> S' of a head, which is kept in
+// registers.  Four STATE warps own 16 value rows each; the rows of the state never meet, so these warps never wait for one another,
+// and a warp's state is an mma accumulator that becomes the next product's A operand where it is: the two columns a lane holds of an
+// accumulator tile are read as k positions tq and tq + 4 of the A fragment, and the B operands are read in the same permuted order
+// (physical column 16 p + 4 tq + 2 e + f is column 2 tq + f of tile 2 p + e, so a lane's share of two tiles is one 16-byte
+// piece).  Everything that does not depend on the state is made ahead by four PREP warps, one chunk
 // each in turn, into a ring of six slots: decay products, scaled operands, the four 16 x 16 products, the inverse.  mma.sync
 // and not tcgen05: these products are 16 rows high, and through tensor memory every link of the chain costs a store, a
 // fence, an issue, a commit and a load, about 700 cycles (a tile of 64 tokens with five such links took 16.9 k cycles with one CTA
