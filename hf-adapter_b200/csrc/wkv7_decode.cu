@@ -15,6 +15,11 @@
 // Thread map (128 threads): lane16 = tid & 15 owns columns 4*lane16..+3 (key
 // index j), rowgroup = tid >> 4 owns rows rowgroup + 8*it (value index i), so a
 // warp instruction touches two full 256-byte state rows = 512 contiguous bytes.
+//
+// What it costs beside the state is instructions, of which a head has few warps to hide them: the vectors of the head are
+// made once, by one warp each (when all eight row groups made them for themselves that was two thirds of the kernel), and the
+// sums over the columns of a thread's eight rows run together (sum_rows).  us a launch, before -> now: 64 rows of 64 heads, fp32
+// state 27.7 -> 22.9 (5.9 TB/s), 256 rows 100 -> 82 (6.5); 64 rows of 40 heads, fp16 state 18.3 -> 13; one row of 12 heads 5.9 -> 4.0.
 #include "common.cuh"
 
 namespace rwkv7 {
@@ -50,26 +55,32 @@ __device__ __forceinline__ float rotator1(int x) {
     return 4.547473508864641e-13f * static_cast<float>(static_cast<int32_t>(bits));
 }
 
-// Four elements in storage type: requested together, converted where they are used, so that the operands of a step cost one
+// Two elements in storage type: requested together, converted where they are used, so that the operands of a step cost one
 // trip to memory and not one per branch (zeros when `ok` is false).
-template <typename T> struct alignas(sizeof(T) * 4) Raw4 { T v[4]; };
+template <typename T> struct alignas(sizeof(T) * 2) Raw2 { T v[2]; };
 template <typename T>
-__device__ __forceinline__ Raw4<T> ld_raw4(const void* base, size_t off, bool ok = true) {
-    Raw4<T> r{};
-    if (ok) r = *reinterpret_cast<const Raw4<T>*>(reinterpret_cast<const T*>(base) + off);
+__device__ __forceinline__ Raw2<T> ld_raw2(const void* base, size_t off, bool ok = true) {
+    Raw2<T> r{};
+    if (ok) r = *reinterpret_cast<const Raw2<T>*>(reinterpret_cast<const T*>(base) + off);
     return r;
 }
 template <typename T>
-__device__ __forceinline__ void cvt4(const Raw4<T>& r, float (&o)[4]) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = to_f<T>(r.v[i]);
+__device__ __forceinline__ float2 cvt2(const Raw2<T>& r) { return make_float2(to_f<T>(r.v[0]), to_f<T>(r.v[1])); }
+template <typename T>
+__device__ __forceinline__ void st2(void* base, size_t off, float x, float y) {
+    Raw2<T> r;
+    r.v[0] = from_f<T>(x);
+    r.v[1] = from_f<T>(y);
+    *reinterpret_cast<Raw2<T>*>(reinterpret_cast<T*>(base) + off) = r;
 }
 
 template <typename TS> struct StateIO;
 template <> struct StateIO<float> {
-    static __device__ __forceinline__ float4 load(const void* base, size_t off) {
+    typedef float4 Raw;  // four columns as they are stored
+    static __device__ __forceinline__ Raw load(const void* base, size_t off) {
         return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + off);  // plain load: may alias state_out
     }
+    static __device__ __forceinline__ float4 value(const Raw& r) { return r; }
     // streaming store: the new state is not read again before the next token, so it should not linger in L2 and
     // be written back under the kernels that follow (measured: -8 % time)
     static __device__ __forceinline__ void store(void* base, size_t off, const float4& s) {
@@ -77,8 +88,11 @@ template <> struct StateIO<float> {
     }
 };
 template <> struct StateIO<__half> {
-    static __device__ __forceinline__ float4 load(const void* base, size_t off) {
-        const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(base) + off);
+    typedef uint2 Raw;
+    static __device__ __forceinline__ Raw load(const void* base, size_t off) {
+        return *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(base) + off);
+    }
+    static __device__ __forceinline__ float4 value(const Raw& u) {
         const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
         const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
         return make_float4(a.x, a.y, b.x, b.y);
@@ -92,11 +106,30 @@ template <> struct StateIO<__half> {
     }
 };
 
+// Sums over the 16 lanes of a row group, of eight rows at once: each exchange halves the rows that a lane goes on with, so eight sums
+// cost eight shuffles and not 32.  Lane l16 ends with the sum of row (l16 & 7) (lanes l16 and l16 ^ 8 alike).
+__device__ __forceinline__ float sum_rows(const float (&v)[8], int l16) {
+    float a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // rows 2 i and 2 i + 1: the lane keeps the one of its bit 0
+        const float keep = l16 & 1 ? v[2 * i + 1] : v[2 * i], give = l16 & 1 ? v[2 * i] : v[2 * i + 1];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float keep = l16 & 2 ? a[2 * i + 1] : a[2 * i], give = l16 & 2 ? a[2 * i] : a[2 * i + 1];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+    const float keep = l16 & 4 ? b[1] : b[0], give = l16 & 4 ? b[0] : b[1];
+    const float c = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    return c + __shfl_xor_sync(0xffffffffu, c, 8);
+}
+
 template <typename T, typename TW, int MODE, typename TS, bool POOL = false>
 __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepArgs p) {  // 64 registers: 8 CTAs per SM (measured: 7 -> 8 CTAs is -9 % time)
     const int bh = blockIdx.x;
     const int h = bh % p.H;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int l16 = tid & 15;
     const int rg = tid >> 4;
     const size_t vbase = (size_t)bh * kN;
@@ -106,16 +139,16 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
     const size_t sbh = POOL ? (size_t)srow * p.H + h : (size_t)bh;
     const size_t vsbase = sbh * kN;
     const int hbase = h * kN;
-    const int c0 = l16 * 4;
+    const int c0 = l16 * 4, c2 = lane * 2;
 
-    __shared__ float s_v[kN];
-    __shared__ float s_y[kN];
+    __shared__ __align__(16) float s_w[kN], s_k[kN], s_kk[kN], s_kka[kN], s_r[kN], s_v[kN], s_y[kN];
+    __shared__ float s_corr;
 
     // Launched programmatically: resident under the tail of the preceding kernel.  By default everything waits for it.
     if (!p.prefetch_state) grid_dependency_wait();
     // ---- state tile: issue all 8 row loads first (memory-level parallelism)
     const size_t sbase = sbh * kN * kN;
-    float4 S[8];
+    typename StateIO<TS>::Raw S[8];
 #pragma unroll
     for (int it = 0; it < 8; ++it) S[it] = StateIO<TS>::load(p.state_in, sbase + (size_t)(it * 8 + rg) * kN + c0);
 
@@ -137,145 +170,137 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
     if (p.prefetch_state) grid_dependency_wait();
     if (tid == 0) grid_launch_dependents();  // the output projection sets up and streams weights under this grid's tail
 
-    // ---- all operands of the recurrence, requested before the first is used: four columns per thread, and the value row
-    const bool interp = MODE == kRaw && p.v_first != nullptr && p.v_gate != nullptr;
-    const Raw4<T> q_r = ld_raw4<T>(p.r, vbase + c0), q_a = ld_raw4<T>(p.a, vbase + c0), q_k = ld_raw4<T>(p.k, vbase + c0);
-    const T* vrow = reinterpret_cast<const T*>(p.v) + vbase;
-    T q_v{}, q_gate{}, q_vf{}, q_gb{};
-    if (tid < kN) {
-        q_v = vrow[tid];
-        if (interp) {
-            q_gate = reinterpret_cast<const T*>(p.v_gate)[vbase + tid];
-            q_vf = reinterpret_cast<const T*>(p.v_first)[vsbase + tid];
-            if (p.v_gate_bias) q_gb = reinterpret_cast<const T*>(p.v_gate_bias)[hbase + tid];
-        }
-    }
-    float r[4], w[4], k[4], kk[4], a[4];
-    if constexpr (MODE == kRaw) {
-        const Raw4<T> q_w = ld_raw4<T>(p.w, vbase + c0), q_ks = ld_raw4<T>(p.k_k, hbase + c0), q_ka = ld_raw4<T>(p.k_a, hbase + c0);
-        const bool has_ab = p.a_is_raw && p.a_bias != nullptr;
-        const Raw4<T> q_wb = ld_raw4<T>(p.w_bias, hbase + c0, p.w_bias != nullptr), q_ab = ld_raw4<T>(p.a_bias, hbase + c0, has_ab);
-        float wr[4], kr[4], ks[4], ka[4];
-        cvt4(q_r, r);
-        cvt4(q_a, a);
-        cvt4(q_w, wr);
-        cvt4(q_k, kr);
-        cvt4(q_ks, ks);
-        cvt4(q_ka, ka);
-        if (p.w_bias) {
-            float wb[4];
-            cvt4(q_wb, wb);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) wr[c] = round_to<T>(wr[c] + wb[c]);
-        }
-        if (p.a_is_raw) {
-            float ab[4];
-            cvt4(q_ab, ab);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) a[c] = round_to<T>(sigmoidf_(round_to<T>(a[c] + ab[c])));
-        }
-        float n2 = 0.f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            kk[c] = kr[c] * ks[c];
-            n2 += kk[c] * kk[c];
-        }
-        n2 = group_sum<16>(n2);
-        const float inv = 1.0f / fmaxf(sqrtf(n2), 1e-12f);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            kk[c] *= inv;
-            k[c] = kr[c] * (1.0f + (a[c] - 1.0f) * ka[c]);
-            w[c] = decay_from_raw(wr[c]);
-        }
-        if constexpr (sizeof(TS) == 2) {
-            if (p.elapsed != nullptr) {  // (decay - 1 + rotator) rounded to fp16, as the reference's FP16-state kernel forms it
-                const int phase = p.elapsed[srow] + hbase + c0;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) w[c] = 1.0f + __half2float(__float2half_rn(w[c] - 1.0f + rotator1(phase + c)));
+    // ---- the vectors of the head, two channels a lane, one warp each; shared.  (Formed by every row group for itself they were
+    // two thirds of the kernel's instructions.)
+    const float2 r = cvt2(ld_raw2<T>(p.r, vbase + c2));
+    auto put = [&](float* s, float x, float y) { *reinterpret_cast<float2*>(s + c2) = make_float2(x, y); };
+    Raw2<T> q_gw{}, q_gb{}, q_g{};
+    if (warp == 0) {
+        float2 w;
+        if constexpr (MODE == kRaw) {
+            const Raw2<T> q_w = ld_raw2<T>(p.w, vbase + c2), q_wb = ld_raw2<T>(p.w_bias, hbase + c2, p.w_bias != nullptr);
+            w = cvt2(q_w);
+            if (p.w_bias) {
+                const float2 wb = cvt2(q_wb);
+                w = make_float2(round_to<T>(w.x + wb.x), round_to<T>(w.y + wb.y));
             }
+            w = make_float2(decay_from_raw(w.x), decay_from_raw(w.y));
+            if constexpr (sizeof(TS) == 2) {
+                if (p.elapsed != nullptr) {  // (decay - 1 + rotator) rounded to fp16, as the reference's FP16-state kernel forms it
+                    const int phase = p.elapsed[srow] + hbase + c2;
+                    w.x = 1.0f + __half2float(__float2half_rn(w.x - 1.0f + rotator1(phase)));
+                    w.y = 1.0f + __half2float(__float2half_rn(w.y - 1.0f + rotator1(phase + 1)));
+                }
+            }
+        } else {
+            w = cvt2(ld_raw2<TW>(p.w, vbase + c2));
         }
-    } else {
-        const Raw4<TW> q_w = ld_raw4<TW>(p.w, vbase + c0);
-        const Raw4<T> q_kk = ld_raw4<T>(p.kk, vbase + c0);
-        cvt4(q_r, r);
-        cvt4(q_a, a);
-        cvt4(q_w, w);
-        cvt4(q_k, k);
-        cvt4(q_kk, kk);
-    }
-    float kka[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) kka[c] = kk[c] * a[c];
-
-    // ---- row-indexed value vector (with the optional v_first interpolation)
-    if (tid < kN) {
-        float vv = to_f<T>(q_v);
+        put(s_w, w.x, w.y);
+        put(s_r, r.x, r.y);
+    } else if (warp == 1) {
+        const Raw2<T> q_a = ld_raw2<T>(p.a, vbase + c2), q_k = ld_raw2<T>(p.k, vbase + c2);
+        float2 k, kk, a;
+        if constexpr (MODE == kRaw) {
+            const bool has_ab = p.a_is_raw && p.a_bias != nullptr;
+            const Raw2<T> q_ks = ld_raw2<T>(p.k_k, hbase + c2), q_ka = ld_raw2<T>(p.k_a, hbase + c2), q_ab = ld_raw2<T>(p.a_bias, hbase + c2, has_ab);
+            a = cvt2(q_a);
+            k = cvt2(q_k);
+            if (p.a_is_raw) {
+                const float2 ab = cvt2(q_ab);
+                a.x = round_to<T>(sigmoidf_(round_to<T>(a.x + ab.x)));
+                a.y = round_to<T>(sigmoidf_(round_to<T>(a.y + ab.y)));
+            }
+            const float2 ks = cvt2(q_ks), ka = cvt2(q_ka);
+            kk = make_float2(k.x * ks.x, k.y * ks.y);
+            const float inv = 1.0f / fmaxf(sqrtf(group_sum<32>(kk.x * kk.x + kk.y * kk.y)), 1e-12f);
+            kk.x *= inv;
+            kk.y *= inv;
+            k.x *= 1.0f + (a.x - 1.0f) * ka.x;
+            k.y *= 1.0f + (a.y - 1.0f) * ka.y;
+        } else {
+            a = cvt2(q_a);
+            k = cvt2(q_k);
+            kk = cvt2(ld_raw2<T>(p.kk, vbase + c2));
+        }
+        put(s_k, k.x, k.y);
+        put(s_kk, kk.x, kk.y);
+        put(s_kka, kk.x * a.x, kk.y * a.y);
+        if constexpr (MODE != kUpdate) {
+            const float2 rk = cvt2(ld_raw2<T>(p.r_k, hbase + c2));
+            const float corr = group_sum<32>(r.x * k.x * rk.x + r.y * k.y * rk.y);
+            if (lane == 0) s_corr = corr;
+        }
+    } else if (warp == 2) {
+        // ---- row-indexed value vector (with the optional v_first interpolation); this warp also makes the output
+        const bool interp = MODE == kRaw && p.v_first != nullptr && p.v_gate != nullptr;
+        const Raw2<T> q_v = ld_raw2<T>(p.v, vbase + c2);
+        if constexpr (MODE != kUpdate) {
+            q_gw = ld_raw2<T>(p.gn_w, hbase + c2);
+            q_gb = ld_raw2<T>(p.gn_b, hbase + c2);
+            q_g = ld_raw2<T>(p.g, vbase + c2);
+        }
+        float2 v = cvt2(q_v);
         if constexpr (MODE == kRaw) {
             if (interp) {
-                float gate = to_f<T>(q_gate);
-                if (p.v_gate_is_raw) gate = round_to<T>(sigmoidf_(round_to<T>(gate + to_f<T>(q_gb))));
-                const float vf = to_f<T>(q_vf);
-                vv = round_to<T>(vv + (vf - vv) * gate);
+                const Raw2<T> q_gate = ld_raw2<T>(p.v_gate, vbase + c2), q_vf = ld_raw2<T>(p.v_first, vsbase + c2),
+                              q_vb = ld_raw2<T>(p.v_gate_bias, hbase + c2, p.v_gate_bias != nullptr);
+                float2 gate = cvt2(q_gate);
+                const float2 vf = cvt2(q_vf), vb = cvt2(q_vb);
+                if (p.v_gate_is_raw) {
+                    gate.x = round_to<T>(sigmoidf_(round_to<T>(gate.x + vb.x)));
+                    gate.y = round_to<T>(sigmoidf_(round_to<T>(gate.y + vb.y)));
+                }
+                v.x = round_to<T>(v.x + (vf.x - v.x) * gate.x);
+                v.y = round_to<T>(v.y + (vf.y - v.y) * gate.y);
             }
-            if (p.v_out) reinterpret_cast<T*>(p.v_out)[vsbase + tid] = from_f<T>(vv);
+            if (p.v_out) st2<T>(p.v_out, vsbase + c2, v.x, v.y);
         }
-        s_v[tid] = vv;
+        put(s_v, v.x, v.y);
     }
     __syncthreads();
 
-    // ---- the recurrence, row by row
+    // ---- the recurrence: eight rows a thread, sums over the columns of all of them together
+    {
+        auto four = [&](const float* s) { return *reinterpret_cast<const float4*>(s + c0); };
+        float sa[8], y[8];
+        const float4 kk = four(s_kk);
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-        const int i = it * 8 + rg;
-        float4 s = S[it];
-        float sa = s.x * kk[0] + s.y * kk[1] + s.z * kk[2] + s.w * kk[3];
-        sa = group_sum<16>(sa);
-        const float vi = s_v[i];
-        s.x = s.x * w[0] + vi * k[0] - sa * kka[0];
-        s.y = s.y * w[1] + vi * k[1] - sa * kka[1];
-        s.z = s.z * w[2] + vi * k[2] - sa * kka[2];
-        s.w = s.w * w[3] + vi * k[3] - sa * kka[3];
-        StateIO<TS>::store(p.state_out, sbase + (size_t)i * kN + c0, s);
-        if constexpr (sizeof(TS) == 2) {  // the output is formed from the state as stored
-            s.x = round_to<__half>(s.x); s.y = round_to<__half>(s.y); s.z = round_to<__half>(s.z); s.w = round_to<__half>(s.w);
+        for (int it = 0; it < 8; ++it) {
+            const float4 s = StateIO<TS>::value(S[it]);
+            sa[it] = s.x * kk.x + s.y * kk.y + s.z * kk.z + s.w * kk.w;
         }
-        float y = s.x * r[0] + s.y * r[1] + s.z * r[2] + s.w * r[3];
-        y = group_sum<16>(y);
-        if (l16 == 0) s_y[i] = y;
-    }
-
-    float corr = 0.f;
-    T q_gw{}, q_gnb{}, q_g{};
-    if constexpr (MODE != kUpdate) {
-        if (tid < kN) {
-            q_gw = reinterpret_cast<const T*>(p.gn_w)[hbase + tid];
-            q_gnb = reinterpret_cast<const T*>(p.gn_b)[hbase + tid];
-            q_g = reinterpret_cast<const T*>(p.g)[vbase + tid];
-        }
-        float rk[4];
-        load4(reinterpret_cast<const T*>(p.r_k) + hbase + c0, rk);
+        const float mine = sum_rows(sa, l16);
+        const float4 w = four(s_w), k = four(s_k), kka = four(s_kka), r4 = four(s_r);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) corr += r[c] * k[c] * rk[c];
-        corr = group_sum<16>(corr);
+        for (int it = 0; it < 8; ++it) {
+            const int i = it * 8 + rg;
+            float4 s = StateIO<TS>::value(S[it]);
+            const float vi = s_v[i], a = __shfl_sync(0xffffffffu, mine, it, 16);
+            s.x = s.x * w.x + vi * k.x - a * kka.x;
+            s.y = s.y * w.y + vi * k.y - a * kka.y;
+            s.z = s.z * w.z + vi * k.z - a * kka.z;
+            s.w = s.w * w.w + vi * k.w - a * kka.w;
+            StateIO<TS>::store(p.state_out, sbase + (size_t)i * kN + c0, s);
+            if constexpr (sizeof(TS) == 2) {  // the output is formed from the state as stored
+                s.x = round_to<__half>(s.x); s.y = round_to<__half>(s.y); s.z = round_to<__half>(s.z); s.w = round_to<__half>(s.w);
+            }
+            y[it] = s.x * r4.x + s.y * r4.y + s.z * r4.z + s.w * r4.w;
+        }
+        const float row = sum_rows(y, l16);
+        if (l16 < 8) s_y[l16 * 8 + rg] = row;
     }
     __syncthreads();
 
-    if (tid < kN) {
-        T* out = reinterpret_cast<T*>(p.out) + vbase;
-        const float y = s_y[tid];
+    if (warp == 2) {
+        const float2 y = *reinterpret_cast<const float2*>(s_y + c2);
         if constexpr (MODE == kUpdate) {
-            out[tid] = from_f<T>(y);
+            st2<T>(p.out, vbase + c2, y.x, y.y);
         } else {
-            // both warps 0 and 1 compute the head statistics redundantly from shared memory
-            const int lane = tid & 31;
-            const float y0 = s_y[lane], y1 = s_y[lane + 32];
-            const float mean = group_sum<32>(y0 + y1) * (1.0f / kN);
-            const float d0 = y0 - mean, d1 = y1 - mean;
-            const float var = group_sum<32>(d0 * d0 + d1 * d1) * (1.0f / kN);
-            const float normed = (y - mean) * rsqrtf(var + p.eps);
-            const float gw = to_f<T>(q_gw), gb = to_f<T>(q_gnb), gate = to_f<T>(q_g);
-            out[tid] = from_f<T>((normed * gw + gb + corr * s_v[tid]) * gate);
+            const float mean = group_sum<32>(y.x + y.y) * (1.0f / kN);
+            const float dx = y.x - mean, dy = y.y - mean;
+            const float rstd = rsqrtf(group_sum<32>(dx * dx + dy * dy) * (1.0f / kN) + p.eps), corr = s_corr;
+            const float2 gw = cvt2(q_gw), gb = cvt2(q_gb), gate = cvt2(q_g), v = *reinterpret_cast<const float2*>(s_v + c2);
+            st2<T>(p.out, vbase + c2, (dx * rstd * gw.x + gb.x + corr * v.x) * gate.x, (dy * rstd * gw.y + gb.y + corr * v.y) * gate.y);
         }
     }
 }
