@@ -42,6 +42,7 @@ struct StepArgs {
     int H;
     float eps;
     int prefetch_state;  // load the state tile before the grid-dependency wait (state_prefetch argument of the raw entry point)
+    int idle_slot;       // state pool: the row of padding rows, which are not computed (-1: none)
     const int* slots;    // state pool: row b of the batch lives in pool row slots[b] (state, v_first / v_out, elapsed); NULL = row b
     const int* elapsed;  // fp16 state, raw mode: per-sequence step counters [B] that phase the decay dither (NULL = no dither)
 };
@@ -146,6 +147,12 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
 
     // Launched programmatically: resident under the tail of the preceding kernel.  By default everything waits for it.
     if (!p.prefetch_state) grid_dependency_wait();
+    if (POOL && srow == p.idle_slot) {  // a padding row of a fixed-size batch: nobody's state, nobody reads the output
+        if (p.prefetch_state) grid_dependency_wait();
+        if (tid == 0) grid_launch_dependents();
+        if (tid < 32) st2<T>(p.out, vbase + c2, 0.f, 0.f);
+        return;
+    }
     // ---- state tile: issue all 8 row loads first (memory-level parallelism)
     const size_t sbase = sbh * kN * kN;
     typename StateIO<TS>::Raw S[8];
@@ -392,13 +399,14 @@ extern "C" int rwkv7_wkv7_output_prepare_raw(const void* r, const void* w_raw, c
 }
 
 // ---------------------------------------------------------------- state pool
-extern "C" int rwkv7_wkv7_output_prepare_raw_pool(const void* r, const void* w_raw, const void* k_raw, const void* v,
+extern "C" int rwkv7_wkv7_output_prepare_raw_pool_idle(const void* r, const void* w_raw, const void* k_raw, const void* v,
                                                   const void* a, float* state_pool, const int32_t* slot_ids, const void* g,
                                                   const void* k_k, const void* k_a, const void* r_k, const void* gn_w,
                                                   const void* gn_b, void* out, const void* w_bias, const void* a_bias,
                                                   int a_is_raw, const void* v_first_pool, const void* v_gate,
                                                   const void* v_gate_bias, int v_gate_is_raw, void* v_out_pool,
-                                                  int state_prefetch, int B, int H, int N, float eps, int dtype, void* stream) {
+                                                  int state_prefetch, int idle_slot, int B, int H, int N, float eps, int dtype,
+                                                  void* stream) {
     StepArgs p{};
     p.r = r; p.w = w_raw; p.k = k_raw; p.v = v; p.a = a;
     p.state_in = state_pool; p.state_out = state_pool; p.out = out; p.H = H;
@@ -409,6 +417,7 @@ extern "C" int rwkv7_wkv7_output_prepare_raw_pool(const void* r, const void* w_r
     p.v_out = v_out_pool;
     p.prefetch_state = state_prefetch != 0;
     p.slots = slot_ids;
+    p.idle_slot = idle_slot;
     RWKV7_REQUIRE(slot_ids && g && r_k && gn_w && gn_b && k_k && k_a, RWKV7_ERR_INVALID,
                   "wkv7_output_prepare_raw_pool: null tensor pointer");
     RWKV7_REQUIRE((v_first_pool == nullptr) == (v_gate == nullptr), RWKV7_ERR_INVALID,
@@ -417,6 +426,16 @@ extern "C" int rwkv7_wkv7_output_prepare_raw_pool(const void* r, const void* w_r
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, { return launch_step<T, T, kRaw, float, true>(p, B, st); });
     return RWKV7_OK;
+}
+
+extern "C" int rwkv7_wkv7_output_prepare_raw_pool(const void* r, const void* w_raw, const void* k_raw, const void* v, const void* a, float* state_pool,
+                                                  const int32_t* slot_ids, const void* g, const void* k_k, const void* k_a, const void* r_k,
+                                                  const void* gn_w, const void* gn_b, void* out, const void* w_bias, const void* a_bias, int a_is_raw,
+                                                  const void* v_first_pool, const void* v_gate, const void* v_gate_bias, int v_gate_is_raw,
+                                                  void* v_out_pool, int state_prefetch, int B, int H, int N, float eps, int dtype, void* stream) {
+    return rwkv7_wkv7_output_prepare_raw_pool_idle(r, w_raw, k_raw, v, a, state_pool, slot_ids, g, k_k, k_a, r_k, gn_w, gn_b, out, w_bias, a_bias, a_is_raw,
+                                                   v_first_pool, v_gate, v_gate_bias, v_gate_is_raw, v_out_pool, state_prefetch, -1, B, H, N, eps, dtype,
+                                                   stream);
 }
 
 // ---------------------------------------------------------------- fp16 recurrent state

@@ -228,10 +228,10 @@ class StepContext:
     GPU with one side stream per device."""
 
     def __init__(self, side_stream=None, all_reduce=None, tp_world: int = 1, tp_rank: int = 0, lane: int = 0,
-                 stream_base: int = 0, slot_ids=None, row_sum=None):
+                 stream_base: int = 0, slot_ids=None, row_sum=None, idle_slot: int = -1):
         # slot_ids (int32 [B] on the device): the recurrent buffers handed to the layer step are slot pools
-        # ([capacity, ...]) and batch row b lives in pool row slot_ids[b]
-        self.slot_ids = slot_ids
+        # ([capacity, ...]) and batch row b lives in pool row slot_ids[b]; rows in idle_slot only pad the batch
+        self.slot_ids, self.idle_slot = slot_ids, int(idle_slot)
         self._side_stream = side_stream
         self._all_reduce = all_reduce
         # row_sum(partial, lane) -> tp_comm.PeerRowSum or None: the communicator whose row kernels take the sum over
@@ -384,7 +384,7 @@ def block_ip_batched(x, state, xpa, xpf, v_first, p, sparse_ffn_out=None, fp16_e
     out, _ = _rec.fused_recurrent_output_prepare_raw(
         r, w_raw, k, v, a_pre, state, g, k_k, k_a, r_k, gn_w, gn_b, eps=float(eps), new_state=state, w_bias=w0, a_bias=a0,
         a_is_raw=True, state_prefetch=True, elapsed=elapsed,
-        advance_elapsed=bool(fp16_advance_elapsed) and elapsed is not None, slot_ids=slots, **extra)
+        advance_elapsed=bool(fp16_advance_elapsed) and elapsed is not None, slot_ids=slots, idle_slot=ctx.idle_slot, **extra)
     attn = apply_linear(Ow, out, static=True)
     if rows_comm is not None:
         x, mixed = rows_comm.ffn_add_norm_mix(x, attn, xpf, fn_w, fn_b, fx_k, slot_ids=slots)

@@ -122,7 +122,7 @@ def fused_recurrent_output_prepare_raw(r, w_raw, k_raw, v, a, state, g, k_k, k_a
                                        a_bias=None, a_is_raw: bool = False, v_first=None, v_gate=None,
                                        v_gate_bias=None, v_gate_is_raw: bool = False, v_out=None,
                                        state_prefetch: bool = False, elapsed=None, advance_elapsed: bool = False,
-                                       slot_ids=None):
+                                       slot_ids=None, idle_slot: int = -1):
     """Decode recurrence / output prep straight from raw w, k and sigmoid(a).
 
     The keyword arguments after ``force_fallback`` are extensions of this package (the reference
@@ -134,12 +134,13 @@ def fused_recurrent_output_prepare_raw(r, w_raw, k_raw, v, a, state, g, k_k, k_a
     (fp32 arithmetic, state rounded on the store); ``elapsed`` (int32 ``[B]``) adds the decay dither of the reference's
     native_wkv_fp16 extension and ``advance_elapsed`` increments it after the step.  ``slot_ids`` (int32 ``[B]``):
     ``state`` is a pool ``[capacity,H,N,N]`` (fp32) updated in place at rows ``slot_ids[b]``, and ``v_first`` / ``v_out``
-    are pools ``[capacity, H*N]`` indexed the same way; the returned state is the pool."""
+    are pools ``[capacity, H*N]`` indexed the same way; the returned state is the pool.  Rows that name ``idle_slot`` (padding of a
+    fixed-size batch) are not computed: zeros out, the pool row as it was."""
     no_fallback(force_fallback, "fused_recurrent_output_prepare_raw")
     if slot_ids is not None:
         return _output_prepare_raw_pool(r, w_raw, k_raw, v, a, state, g, k_k, k_a, r_k, group_norm_weight, group_norm_bias,
                                         float(eps), out, w_bias, a_bias, a_is_raw, v_first, v_gate, v_gate_bias,
-                                        v_gate_is_raw, v_out, state_prefetch, slot_ids)
+                                        v_gate_is_raw, v_out, state_prefetch, slot_ids, idle_slot)
     B, H, N = _state_shape(state, allow_f16=True)
     if elapsed is not None:
         if state.dtype != torch.float16:
@@ -182,7 +183,7 @@ def fused_recurrent_output_prepare_raw(r, w_raw, k_raw, v, a, state, g, k_k, k_a
 
 
 def _output_prepare_raw_pool(r, w_raw, k_raw, v, a, pool, g, k_k, k_a, r_k, gn_w, gn_b, eps, out, w_bias, a_bias, a_is_raw,
-                             v_first, v_gate, v_gate_bias, v_gate_is_raw, v_out, state_prefetch, slot_ids):
+                             v_first, v_gate, v_gate_bias, v_gate_is_raw, v_out, state_prefetch, slot_ids, idle_slot):
     _, H, N = _state_shape(pool, allow_f16=False)
     B = int(slot_ids.numel())
     if not (slot_ids.is_cuda and slot_ids.dtype == torch.int32 and slot_ids.is_contiguous()):
@@ -206,10 +207,10 @@ def _output_prepare_raw_pool(r, w_raw, k_raw, v, a, pool, g, k_k, k_a, r_k, gn_w
     same_dtype(r_, w_, k_, v_, a_, g_, *params, *opt, v_first, v_out, what="fused_recurrent_output_prepare_raw")
     if out is None:
         out = torch.empty_like(r_)
-    _lib.check(_lib.lib.rwkv7_wkv7_output_prepare_raw_pool(
+    _lib.check(_lib.lib.rwkv7_wkv7_output_prepare_raw_pool_idle(
         ptr(r_), ptr(w_), ptr(k_), ptr(v_), ptr(a_), ptr(pool), ptr(slot_ids), ptr(g_), ptr(params[0]), ptr(params[1]),
         ptr(params[2]), ptr(params[3]), ptr(params[4]), ptr(out), ptr(opt[0]), ptr(opt[1]), int(bool(a_is_raw)),
-        ptr(v_first), ptr(opt[2]), ptr(opt[3]), int(bool(v_gate_is_raw)), ptr(v_out), int(bool(state_prefetch)), B, H, N,
+        ptr(v_first), ptr(opt[2]), ptr(opt[3]), int(bool(v_gate_is_raw)), ptr(v_out), int(bool(state_prefetch)), int(idle_slot), B, H, N,
         eps, dt_code(r_), stream_ptr(r_)), "fused_recurrent_output_prepare_raw")
     return (out.reshape(B, hidden) if flat else out.reshape(B, H, N)), pool
 

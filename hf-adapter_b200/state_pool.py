@@ -316,7 +316,7 @@ class RWKV7StatePool:
     def _step(self, ids, slot_vec, greedy):
         m = self.model
         x = torch.nn.functional.embedding(ids, m.model.embeddings.weight)
-        ctx = _pk.StepContext(m._side_stream, None, 1, 0, 0, 0, slot_ids=slot_vec)
+        ctx = _pk.StepContext(m._side_stream, None, 1, 0, 0, 0, slot_ids=slot_vec, idle_slot=self.scratch_slot)
         packs, _, _, _ = _pk.extract_graph_packs(m, unused_as_zeros=False)
         for l, p in enumerate(packs):
             x = _pk.block_ip_batched(x, self.S_pool[l], self.xpa_pool[l], self.xpf_pool[l], self.vfirst_pool, p, context=ctx)

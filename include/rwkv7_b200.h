@@ -198,6 +198,16 @@ int rwkv7_wkv7_output_prepare_raw_pool(const void* r, const void* w_raw, const v
                                        const void* v_first_pool, const void* v_gate, const void* v_gate_bias,
                                        int v_gate_is_raw, void* v_out_pool, int state_prefetch,
                                        int B, int H, int N, float eps, int dtype, void* stream);
+/* The same with a pool row that belongs to nobody: rows of the batch that name it (those that pad a batch to a fixed size) are not computed,
+ * their output is zero.  -1: none. */
+int rwkv7_wkv7_output_prepare_raw_pool_idle(const void* r, const void* w_raw, const void* k_raw, const void* v, const void* a,
+                                       float* state_pool, const int32_t* slot_ids, const void* g,
+                                       const void* k_k, const void* k_a, const void* r_k,
+                                       const void* gn_w, const void* gn_b, void* out,
+                                       const void* w_bias, const void* a_bias, int a_is_raw,
+                                       const void* v_first_pool, const void* v_gate, const void* v_gate_bias,
+                                       int v_gate_is_raw, void* v_out_pool, int state_prefetch, int idle_slot,
+                                       int B, int H, int N, float eps, int dtype, void* stream);
 
 /* Plain LayerNorm (pre_norm of layer 0 and the final norm; rwkv7_hf/native.py:404,450). */
 int rwkv7_layer_norm(const void* x, const void* norm_w, const void* norm_b, void* out,
