@@ -27,7 +27,11 @@ constexpr int kWarps = 8, kThreads = kWarps * 32;
 constexpr int kSlots = 16;  // partial sums per CTA: warps x cluster size
 constexpr int TM = 2, kTile = TM * 16;  // channels of a warp: with one 16-channel tile the reads of x weigh double (4096 -> 16384
                                         // int4, 8 rows: 24.6 us against 17.5)
-constexpr int kW4Block = 8704, kW4Scales = 8192, kW4Zeros = 8448, kW8Block = 16384;  // tiled formats: per [128 ch x 128 k]
+// Tiled formats (w4g_umma.cu): blocks of [128 channels x 128 k], eight pieces of 16 channels each: [4 or 8 chunks of k][channel][16 bytes],
+// for int4 then eight bytes for channels c and c + 8: their scales, their zeros.  Read by warps of 16 channels such pieces run at 5.9 TB/s; from
+// blocks of [chunk][128 channels][16 bytes], where a warp's part of a block is 256 bytes here and there, at 3.6 (cp.async of nothing but
+// weights).  In this kernel, which also converts, 4096 -> 16384 took 15.2 us, 14.8 with pieces, 14.4 with the scales of two channels in one load.
+constexpr int kW4Block = 8704, kW8Block = 16384, kW4Piece = 1088, kW8Piece = 2048, kW4Scales = 1024, kChunk = 256;
 enum Fmt { kDense = 0, kInt4 = 1, kInt8 = 2 };
 
 struct Problem {
@@ -99,7 +103,7 @@ template <> struct Unit<kInt8> { static constexpr int K = 128, W16 = 2, X16 = 4;
 
 template <int FMT> struct Regs {
     uint4 w[TM][2][Unit<FMT>::W16];  // [16-channel tile][channel gid / gid + 8][piece]
-    uint32_t sc[FMT == kInt4 ? TM : 1][2], z[FMT == kInt4 ? TM : 1][2];
+    uint2 sz[FMT == kInt4 ? TM : 1];  // scales of the lane's two channels of a tile, their zeros
     uint4 x[Unit<FMT>::X16];
 };
 
@@ -131,7 +135,7 @@ __device__ __forceinline__ void unit_mma(float (&acc)[TM][2][4], const Regs<FMT>
                     a[hh][0] = v.x; a[hh][1] = v.y; a[hh][2] = v.z; a[hh][3] = v.w;
                 } else if constexpr (FMT == kInt4) {
                     const uint4 v = r.w[t][hh][0];
-                    int4_word(q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w, r.z[t][hh], r.sc[t][hh] * 0x00010001u, a[hh]);
+                    int4_word(q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w, (r.sz[t].y >> (hh * 8)) & 255u, __byte_perm(r.sz[t].x, 0, hh ? 0x3232 : 0x1010), a[hh]);
                 } else {
                     const uint4 v = r.w[t][hh][q >> 1];
                     int8_word(q & 1 ? v.z : v.x, a[hh][0], a[hh][1]);
@@ -155,8 +159,8 @@ __device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, co
     const size_t row8 = (size_t)K * 16;  // dense: bytes between channels n and n + 8
     if constexpr (FMT == kDense) wp = reinterpret_cast<const char*>(p.W) + ((size_t)(n0 + gid) * K + (size_t)u0 * 64 + tig * 8) * 2;
     else wp = reinterpret_cast<const char*>(p.W) + ((size_t)(n0 >> 7) * (K >> 7) + u0) * (FMT == kInt4 ? kW4Block : kW8Block) +
-              ((n0 & 127) + gid) * 16 + tig * 2048;
-    const int soff = kW4Scales - ((n0 & 127) + gid) * 14 - tig * 2048, zoff = kW4Zeros - ((n0 & 127) + gid) * 15 - tig * 2048;
+              ((n0 >> 4) & 7) * (FMT == kInt4 ? kW4Piece : kW8Piece) + gid * 16 + tig * kChunk;
+    const int soff = kW4Scales - gid * 8 - tig * kChunk;
     const int rows8 = (p.N - n0 - gid + 7) >> 3;  // dense: channels n0 + gid + 8 i that exist
     auto load_w = [&](Regs<FMT>& r, int u) {
 #pragma unroll
@@ -169,12 +173,10 @@ __device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, co
                     for (int q = 0; q < 2; ++q)
                         r.w[t][hh][q] = (i < rows8 && u * 64 + q * 32 + tig * 8 < K) ? ldg_stream(wp + i * row8 + q * 64) : make_uint4(0, 0, 0, 0);
                 } else {
-                    r.w[t][hh][0] = ldg_stream(wp + i * 128);
-                    if constexpr (FMT == kInt8) r.w[t][hh][1] = ldg_stream(wp + i * 128 + 4 * 2048);
-                    else {
-                        r.sc[t][hh] = *reinterpret_cast<const unsigned short*>(wp + soff + i * 16);
-                        r.z[t][hh] = *reinterpret_cast<const unsigned char*>(wp + zoff + i * 8);
-                    }
+                    const char* q = wp + t * (FMT == kInt4 ? kW4Piece : kW8Piece);
+                    r.w[t][hh][0] = ldg_stream(q + hh * 128);
+                    if constexpr (FMT == kInt8) r.w[t][hh][1] = ldg_stream(q + hh * 128 + 4 * kChunk);
+                    else if (hh == 0) r.sz[t] = *reinterpret_cast<const uint2*>(q + soff);
                 }
             }
         wp += FMT == kDense ? 128 : FMT == kInt4 ? kW4Block : kW8Block;

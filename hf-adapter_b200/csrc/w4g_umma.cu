@@ -7,8 +7,8 @@
 // HBM exactly once, so the contraction goes to tcgen05.mma:
 //
 //   * the weights are read from a TILED copy of the reference's [Nout, K/2] array (rwkv7_w4g_repack, built once at
-//     load): one 8.5 KiB block per [128 channels x 128 k] tile (nibbles, then the tile's scales and zero-points),
-//     blocks of a channel tile consecutive in memory, so every CTA streams one contiguous region, one bulk copy per
+//     load): one 8.5 KiB block per [128 channels x 128 k] tile (eight times the nibbles, scales and zero-points of 16
+//     channels), blocks of a channel tile consecutive in memory, so every CTA streams one contiguous region, one bulk copy per
 //     block -- row-strided 64-byte pieces of the row-major array reach under 1 TB/s on HBM3e, contiguous blocks run
 //     at copy speed;
 //   * dequant warps (thread = output channel) read their 64 packed bytes, expand them to 128 fp16 values in
@@ -68,11 +68,15 @@ namespace rwkv7 {
 namespace w4 {
 constexpr int TILE_N = 128;  // output channels per CTA = UMMA M
 constexpr int KB = 128;      // k elements per block
-constexpr int RAW_BYTES = TILE_N * KB / 2;  // 8192 packed nibbles
-constexpr int SC_OFF = RAW_BYTES;           // then 128 fp16 scales of the k-block
-constexpr int Z_OFF = SC_OFF + TILE_N * 2;  // then 128 u8 zero-points, then padding
-constexpr int W4_BLOCK_BYTES = 8704;        // one int4 tile block in memory = one bulk copy (68 x 128 B)
-constexpr int W8_BLOCK_BYTES = TILE_N * KB;  // int8 per-channel format: 16 KiB of offset-binary bytes (q + 128), scales apart
+// A block [128 channels x 128 k] is eight pieces of 16 channels: one bulk copy here, a KB or two in one place for a reader of 16
+// channels (row_gemv.cu).
+constexpr int SLICES = TILE_N / 16;
+constexpr int CHUNK = 16 * 16;              // a piece: 32 k (int4) or 16 k (int8) of its 16 channels, 16 bytes each, then the next k
+constexpr int SC_OFF = 16 * KB / 2;         // int4: then for channels c and c + 8 eight bytes: two fp16 scales, two u8 zero-points, padding
+__host__ __device__ constexpr int scale_off(int r) { return SC_OFF + (r & 7) * 8 + (r >> 3) * 2; }  // of channel r of the 16
+__host__ __device__ constexpr int zero_off(int r) { return SC_OFF + (r & 7) * 8 + 4 + (r >> 3); }
+constexpr int W4_PIECE = 1088, W8_PIECE = 16 * KB;  // int8: offset-binary bytes (q + 128), one scale per channel apart
+constexpr int W4_BLOCK_BYTES = SLICES * W4_PIECE, W8_BLOCK_BYTES = SLICES * W8_PIECE;
 constexpr int TMEM_COLS = 512;
 constexpr int HANDOFF_THREADS = 128 + 32;   // a dequant group arrives, its issuer warp syncs
 
@@ -114,8 +118,8 @@ struct Cfg {
 constexpr int kW4MaxGroup = 4;  // projections of equal shape served by one launch (r / k / v of a layer)
 
 struct W4UmmaArgs {
-    const uint8_t* tw[kW4MaxGroup];  // tiled weights: [tiles][K/128] blocks; int4: [4 chunks][128 channels][16 B] | scales | zeros,
-                                     // int8: [8 chunks][128 channels][16 B]
+    const uint8_t* tw[kW4MaxGroup];  // tiled weights: [tiles][K/128] blocks; int4: 8 x ([4 chunks][16 channels][16 B] | scales | zeros),
+                                     // int8: 8 x [8 chunks][16 channels][16 B]
     const __half* rscale[kW4MaxGroup];  // int8 format: one scale per output channel
     __half* out[kW4MaxGroup];
     const __half* residual;          // add epilogue (single projection only)
@@ -331,15 +335,15 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
             ok = __shfl_sync(0xffffffffu, ok, 0);
             uint32_t v[4][16];
             if (ok) {
-                // this channel's 64 packed bytes: chunk c (32 k) of all 128 channels is one 2 KiB slab, so the
-                // threads of a warp read consecutive 16-byte pieces (no bank conflicts, no swizzle)
-                const unsigned char* rrow = wblk + row * 16;
+                // this channel's 64 packed bytes: a chunk (32 k) of 16 channels is one 256-byte slab, so eight threads of a
+                // warp read consecutive 16-byte pieces (no bank conflicts, no swizzle)
+                const unsigned char *piece = wblk + (row >> 4) * (BLOCK_BYTES / SLICES), *rrow = piece + (row & 15) * 16;
                 if constexpr (FMT == 0) {
                     uint4 pk[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * 2048);
-                    const uint32_t s16 = reinterpret_cast<const unsigned short*>(wblk + SC_OFF)[row];
-                    const uint32_t z = (wblk + Z_OFF)[row];
+                    for (int c = 0; c < 4; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * CHUNK);
+                    const uint32_t s16 = *reinterpret_cast<const unsigned short*>(piece + scale_off(row & 15));
+                    const uint32_t z = piece[zero_off(row & 15)];
                     const uint32_t sc = s16 * 0x00010001u;               // (scale, scale)
                     const uint32_t zlo = z * 0x00010001u + 0x64006400u;  // 1024 + z as fp16: 0x6400 | z
                     const uint32_t zhi = z * 0x00100010u + 0xD400D400u;  // -(64 + z) as fp16: 0xD400 | (z << 4)
@@ -353,10 +357,10 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                         dequant_word(pk[c].w, zlo, zhi, sc, v[c] + 12);
                     }
                 } else {
-                    // 128 bytes per channel: chunk c (16 k) of all 128 channels is one 2 KiB slab
+                    // 128 bytes per channel, 16 k a chunk
                     uint4 pk[8];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * 2048);
+                    for (int c = 0; c < 8; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * CHUNK);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&wempty[aa]);
 #pragma unroll
@@ -550,16 +554,16 @@ __global__ void w4g_repack_kernel(const uint8_t* __restrict__ packed, const T* _
 #pragma unroll
         for (int i = 0; i < 8; ++i) out |= ((w >> (4 * order[i])) & 15u) << (4 * i);
     }
-    uint8_t* block = tiled + blk * w4::W4_BLOCK_BYTES;
-    reinterpret_cast<uint32_t*>(block)[widx & 2047] = out;
+    uint8_t* piece = tiled + blk * w4::W4_BLOCK_BYTES + (r >> 4) * w4::W4_PIECE;
+    reinterpret_cast<uint32_t*>(piece + c * w4::CHUNK + (r & 15) * 16)[j] = out;
     if (c == 0 && j == 0) {
         const long long gi = n * (K / group) + (b * 128) / group;
-        reinterpret_cast<T*>(block + w4::SC_OFF)[r] = (n < Nout) ? scales[gi] : from_f<T>(0.f);
-        (block + w4::Z_OFF)[r] = (n < Nout && zeros) ? zeros[gi] : (uint8_t)8;
+        *reinterpret_cast<T*>(piece + w4::scale_off(r & 15)) = (n < Nout) ? scales[gi] : from_f<T>(0.f);
+        piece[w4::zero_off(r & 15)] = (n < Nout && zeros) ? zeros[gi] : (uint8_t)8;
     }
 }
 
-// int8 per-channel weights q [Nout, K] -> [tiles][K/128] blocks of [8 chunks][128 channels][16 B], bytes stored as
+// int8 per-channel weights q [Nout, K] -> [tiles][K/128] blocks of 8 x [8 chunks][16 channels][16 B], bytes stored as
 // q + 128 (offset binary: the kernel's byte -> fp16 conversion needs no sign handling).  One thread per 16-byte piece.
 __global__ void w8_repack_kernel(const int8_t* __restrict__ q, uint8_t* __restrict__ tiled, int K, int Nout, long long total_pieces) {
     const long long pidx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -576,7 +580,7 @@ __global__ void w8_repack_kernel(const int8_t* __restrict__ q, uint8_t* __restri
         v = *reinterpret_cast<const uint4*>(q + n * K + b * 128 + c * 16);
         v.x ^= 0x80808080u; v.y ^= 0x80808080u; v.z ^= 0x80808080u; v.w ^= 0x80808080u;
     }
-    reinterpret_cast<uint4*>(tiled)[pidx] = v;
+    *reinterpret_cast<uint4*>(tiled + blk * w4::W8_BLOCK_BYTES + (r >> 4) * w4::W8_PIECE + c * w4::CHUNK + (r & 15) * 16) = v;
 }
 
 // Tiled buffers written by rwkv7_w4g_repack / rwkv7_w8_repack and not yet read by a projection.  The projection kernel streams the
