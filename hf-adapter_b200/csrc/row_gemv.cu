@@ -11,8 +11,8 @@
 // epilogue, so here the weights go HBM -> registers -> mma.sync m16n8k16 with M as the narrow n side:
 //   * every lane loads 16 bytes of one channel; the k order inside a unit is permuted so that those bytes ARE its
 //     fragments of the A operand (x is read in the same order), no shared memory and no shuffle in between;
-//   * a warp works on 32 channels, two units of K ahead; the warps of a CTA, and the CTAs of a cluster where one CTA
-//     per channel tile would leave SMs idle, split K, and their sums are added in fixed order;
+//   * a warp works on 32 channels, two units of K ahead; the warps of a CTA (eight, or four), and the CTAs of a cluster where
+//     one CTA per channel tile would leave SMs idle, split K, and their sums are added in fixed order;
 //   * the first units of weights are requested before the grid-dependency wait, under the preceding kernel's tail.
 #include "umma.cuh"
 
@@ -23,7 +23,7 @@ bool take_tiled_fresh(const void* tiled);  // w4g_umma.cu: the tiled copy was wr
 namespace rg {
 constexpr int kMaxProblems = 8;
 constexpr int kMaxRows = 8;
-constexpr int kWarps = 8, kThreads = kWarps * 32;
+constexpr int kWarps = 8, kThreads = kWarps * 32;  // of a CTA at most
 constexpr int kSlots = 16;  // partial sums per CTA: warps x cluster size
 constexpr int TM = 2, kTile = TM * 16;  // channels of a warp: with one 16-channel tile the reads of x weigh double (4096 -> 16384
                                         // int4, 8 rows: 24.6 us against 17.5)
@@ -215,7 +215,7 @@ __device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, co
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2) rows_gemv_kernel(const __grid_constant__ Args args) {
     __shared__ float slots[kSlots][kMaxRows * (kTile + 1)];  // partial sums [row][channel], padded
-    const int S = args.splits, wk = args.wk, groups = kWarps / wk;  // `groups` channel tiles per CTA, wk warps each
+    const int S = args.splits, wk = args.wk, threads = blockDim.x, groups = (threads >> 5) / wk;  // `groups` channel tiles per CTA, wk warps each
     const int rank = blockIdx.x % S, cta = blockIdx.x / S;
     int pi = 0;
     while (pi + 1 < args.n && cta >= args.p[pi + 1].cta0) ++pi;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kThreads, 2) rows_gemv_kernel(const __grid_con
         __syncthreads();
     }
     const int channels = groups * kTile, nbase = (cta - p.cta0) * channels;
-    for (int i = threadIdx.x; i < channels * args.M; i += kThreads) {
+    for (int i = threadIdx.x; i < channels * args.M; i += threads) {
         const int c = i % channels, m = i / channels, n = nbase + c;
         if (n >= p.N) continue;
         const int o = m * (kTile + 1) + c % kTile, s0 = c / kTile * parts;
@@ -308,11 +308,23 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
         max_units = units > max_units ? units : max_units;
     }
     a.wk = max_units >= 8 ? 8 : max_units >= 4 ? 4 : max_units >= 2 ? 2 : 1;
-    const int per = kWarps / a.wk * kTile;
-    int ctas = 0;
-    for (int i = 0; i < n_problems; ++i) {
-        a.p[i].cta0 = ctas;
-        ctas += (N[i] + per - 1) / per;
+    // Two CTAs of eight warps fit an SM, or four of four, which take twice as long over their tile: those where the eight-warp CTAs
+    // would start a second wave that is nearly empty.  us, 8 -> 4 warps, 1 / 8 rows: int4 2048 -> 9600 7.4 / 8.6 -> 6.9 / 8.3, 4096 -> 16384 14.7 / 17.2 ->
+    // 12.9 / 14.9, 4096 -> 18944 15.2 / 17.6 -> 13.3 / 15.2, 4096 -> 32768 26.5 / 30.2 -> 23.8 / 28.1; int8 2560 -> 10240 11.0 -> 9.1; dense 2560 -> 10240 14.1 /
+    // 15.0 -> 12.4 / 13.0, 2560 -> 14336 15.4 / 16.1 -> 13.7 / 14.5.  With as many waves either way but one: dense 4096 -> 20480 33.8 / 35.1 -> 38.5 / 39.9.
+    const auto deal = [&](int warps) {
+        const int per = warps / a.wk * kTile;
+        int ctas = 0;
+        for (int i = 0; i < n_problems; ++i) {
+            a.p[i].cta0 = ctas;
+            ctas += (N[i] + per - 1) / per;
+        }
+        return ctas;
+    };
+    int warps = kWarps, ctas = deal(warps);
+    if (a.wk == kWarps && ctas > 2 * 148 && 2 * ((ctas + 4 * 148 - 1) / (4 * 148)) <= (ctas + 2 * 148 - 1) / (2 * 148)) {
+        warps = a.wk = kWarps / 2;
+        ctas = deal(warps);
     }
     // Up to one CTA an SM and at least two units a warp: pairs of CTAs halve K.  1 row, fp16 / int4 / int8, one CTA against two:
     // 2560 x 2560 5.7 / 4.0 / 4.3 -> 4.6 / 3.9 / 4.2 us, 10240 -> 2560 19.9 / 13.1 / 13.4 -> 13.1 / 8.9 / 9.7, 16384 -> 4096
@@ -322,7 +334,7 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
     auto kern = dtype == RWKV7_F16 ? rows_gemv_kernel<__half> : rows_gemv_kernel<__nv_bfloat16>;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas * a.splits);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(warps * 32);
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -173,3 +173,23 @@ def test_prefill_lora_pairs(rows_, rank, dt, first):
             # the hidden value is rounded twice, the result once: each at most half an ulp of its size
             half_ulp = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -20}[dt]
             assert y.shape == want.shape and float((y.double() - want).norm()) <= 2 * half_ulp * float(want.norm())
+
+
+@pytest.mark.parametrize("N", [9472, 9504, 18944, 18976, 28448])
+@pytest.mark.parametrize("fmt", ["dense", "int8"])
+def test_either_side_of_the_wave_limits(N, fmt):
+    """CTAs of eight warps up to 296 tiles of 32 channels, of four up to 592 and from 889 on."""
+    K, M = 512, 3
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(M, K, generator=g, device="cuda").half()
+    lin = torch.nn.Linear(K, N, bias=False, device="cuda", dtype=torch.float16)
+    with torch.no_grad():
+        lin.weight.normal_(0.0, K ** -0.5, generator=g)
+    if fmt == "dense":
+        y, = rows.rows_gemv((x,), (lin.weight,), out_features=(N,), fmts=(0,))
+        p = x.double() @ lin.weight.double().t()
+    else:
+        m8 = hb.MM8Linear(lin, rowwise=True)
+        y, = rows.rows_gemv((x,), (m8.tiled_for(x),), out_features=(N,), fmts=(2,), scales=(m8.row_scale,))
+        p = x.double() @ (m8.q_row.double() * m8.row_scale.double()[:, None]).t()
+    _close(y, p.float(), torch.float16)
