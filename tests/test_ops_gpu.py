@@ -179,6 +179,27 @@ def test_scan_tile_choice_by_grid(B, T, Hh):
     assert sh.dtype == torch.float16 and rel_err(npf(sh), soh) < 1e-3
 
 
+@pytest.mark.parametrize("Hh", [2, 149])
+@pytest.mark.parametrize("T", [8, 40, 41, 47, 48, 81])
+def test_scan_in_pieces_is_the_scan(T, Hh):
+    """Blocks of 8 tokens in a ring of five: a token's place in it is no part of its arithmetic (the same bits), whether its block
+    is whole, the last one, or behind others.  Against the oracle as in the test above."""
+    r, w, k, v, kk, a = wkv_inputs(1, T, Hh, N, seed=T, dtype=np.float32)
+    rng = np.random.default_rng(T)
+    f = lambda *sh: rng.standard_normal(sh).astype(np.float32)
+    seq, s0 = [cu(x) for x in (r, w, k, v, kk, a)], 0.1 * f(1, Hh, N, N)
+    g, rk, gw, gb = cu(f(1, T, Hh, N)), cu(0.1 * f(Hh, N)), cu(1 + 0.1 * f(Hh * N)), cu(0.1 * f(Hh * N))
+    y, s = hb.fused_recurrent_scan_output_prepare(*seq, cu(s0), g, rk, gw, gb, eps=EPS)
+    _, so = O.recurrent_scan(r, w, k, v, kk, a, s0)
+    assert rel_err(npf(s), so) < 2e-6
+    for cut in (1, 3, 7):
+        state, ys = cu(s0), []
+        for t0, t1 in ((0, cut), (cut, T)):
+            yt, state = hb.fused_recurrent_scan_output_prepare(*(x[:, t0:t1].contiguous() for x in seq), state, g[:, t0:t1].contiguous(), rk, gw, gb, eps=EPS)
+            ys.append(yt)
+        assert torch.equal(torch.cat([x.reshape(-1) for x in ys]), y.reshape(-1)) and torch.equal(state, s)
+
+
 @pytest.mark.parametrize("dt", ["fp16", "bf16", "fp32"])
 @pytest.mark.parametrize("Hh", [3, 149, 297])
 def test_scan_parameters_of_any_alignment(dt, Hh):
