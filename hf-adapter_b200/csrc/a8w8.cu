@@ -15,27 +15,64 @@ namespace rwkv7 {
 // ONCE: each thread keeps its 8-element chunks in registers between the amax pass and the quantising pass (rows up to
 // 256 * 8 * CHUNKS elements; longer rows re-read the tail, which then comes from L2).
 //
-// Bound: HBM (3 bytes an fp16 element); the IEEE division per element was what it spent its time on, and registers for
-// eight chunks kept three CTAs on an SM.
+// Bound: HBM (3 bytes an fp16 element): 4096 rows of 16384 in fp16 38 us (5.3 TB/s; 62.5 with two conversions an element on the
+// slow unit), of 4096 13.2 (19.0); bf16 53 (93) and 16.9 (19.2), fp32 56 (81) and 16.6 (18.2).
 
 // bf16 rows hold few distinct quotients, which tie in some rows for many elements, and a warp with one tie forms 32
-// quotients after all: below this many rows (few CTAs an SM) bf16 divides without asking.  64 rows of 16384 / 10240 / 4096:
-// 8.72 / 6.32 / 3.60 us with the product, 6.28 / 4.64 / 2.93 without; 4096 rows of 4096: 16.9 us with it (34.7 without).
-constexpr int kA8RecipRows = 512;
+// quotients after all: below this many rows (few CTAs an SM) bf16 divides without asking.  64 rows of 16384: 11.0 us with the
+// product, 6.9 without; 256 of 10240: 9.0 either way; 511 of 16384: 13.6 with it, 17.2 without.
+constexpr int kA8RecipRows = 256;
 
-// The quotient only matters where it rounds: x * (1 / s) is within 1.5 * 2^-23 of x / s relative to it, less than 3e-5 for
-// |x / s| <= 127, so away from a rounding boundary by 1e-4 the product rounds like the IEEE quotient; nearer (and for
-// NaN) the quotient itself is formed.  RECIP false: always.
+__device__ __forceinline__ float quant_quotient(float v, float s) {
+    const float t = __fdiv_rn(v, s);
+    return fminf(fmaxf((t >= 0.f) ? floorf(t + 0.5f) : ceilf(t - 0.5f), -127.f), 127.f);
+}
+
+// Eight elements to eight bytes.  The quotient only matters where it rounds: x * (1 / s) is within 2^-23 of x / s relative to
+// it, and x / s and the half added to it are rounded once each: 2.5e-5 in all for |x / s| <= 127.  So away from a rounding boundary
+// by 4e-5 the integer nearest to the product is the one that the IEEE quotient rounds to; nearer (and for NaN) the quotient itself is
+// formed.  RECIP false: always.  The nearest integer is the low byte of the product + 1.5 * 2^23: three operations an element, none
+// of them on the slow unit that floorf and the conversion share.
 template <bool RECIP>
-__device__ __forceinline__ int8_t quant_one(float v, float s, float inv) {
-    const float u = fabsf(v * inv) + 0.5f, f = floorf(u), d = u - f;
-    float r = copysignf(f, v);
-    if (!RECIP || !(d >= 1e-4f && d <= 0.9999f)) {
-        const float t = __fdiv_rn(v, s);
-        r = (t >= 0.f) ? floorf(t + 0.5f) : ceilf(t - 0.5f);
+__device__ __forceinline__ uint2 quant8(const float (&v)[8], float s, float inv) {
+    constexpr float kMagic = 12582912.f, kSure = 0.5f - 4e-5f;
+    uint32_t b[8];
+    if (RECIP) {
+        float off[8], worst = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float u = v[e] * inv, m = __fadd_rn(u, kMagic);
+            off[e] = fabsf(u - __fadd_rn(m, -kMagic));
+            asm("max.NaN.f32 %0, %0, %1;" : "+f"(worst) : "f"(off[e]));
+            b[e] = __float_as_uint(m);
+        }
+        if (!(worst <= kSure)) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (!(off[e] <= kSure)) b[e] = (uint32_t)(int)quant_quotient(v[e], s);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = (uint32_t)(int)quant_quotient(v[e], s);
     }
-    r = fminf(fmaxf(r, -127.f), 127.f);
-    return (int8_t)(int)r;
+    auto four = [](uint32_t x, uint32_t y, uint32_t z, uint32_t w) { return __byte_perm(__byte_perm(x, y, 0x0040), __byte_perm(z, w, 0x0040), 0x5410); };
+    return make_uint2(four(b[0], b[1], b[2], b[3]), four(b[4], b[5], b[6], b[7]));
+}
+
+// |x| of a chunk's largest element; pairs of 16-bit elements at once.  NaN is passed over, as fmaxf does.
+template <typename T>
+__device__ __forceinline__ float chunk_amax(const Vec8<T>& x) {
+    if constexpr (sizeof(T) == 4) {
+        float m = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(x.v[e]));
+        return m;
+    } else {
+        using T2 = std::conditional_t<std::is_same<T, __half>::value, __half2, __nv_bfloat162>;
+        const T2* h = reinterpret_cast<const T2*>(x.v);
+        const T2 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+        return fmaxf(fmaxf(to_f<T>(m.x), to_f<T>(m.y)), 0.f);
+    }
 }
 
 template <typename T, int CHUNKS, bool RECIP>
@@ -46,10 +83,7 @@ __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, 
     const T* xr = x + row * K;
     Vec8<T> keep[CHUNKS];  // the row's chunks in their storage type: 4 registers per chunk for 16-bit inputs
     float amax = 0.f;
-    auto take = [&](int c) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(to_f<T>(keep[c].v[e])));
-    };
+    auto take = [&](int c) { amax = fmaxf(amax, chunk_amax<T>(keep[c])); };
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
         const int k = (c * 256 + threadIdx.x) * 8;
@@ -76,19 +110,16 @@ __global__ void __launch_bounds__(256) a8_quant_kernel(const T* __restrict__ x, 
     for (int c = 0; c < CHUNKS; ++c) {
         const int k = (c * 256 + threadIdx.x) * 8;
         if (k < K) {
-            alignas(8) int8_t o[8];
+            float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = quant_one<RECIP>(to_f<T>(keep[c].v[e]), s, inv);
-            *reinterpret_cast<uint2*>(q + row * K + k) = *reinterpret_cast<const uint2*>(o);
+            for (int e = 0; e < 8; ++e) v[e] = to_f<T>(keep[c].v[e]);
+            *reinterpret_cast<uint2*>(q + row * K + k) = quant8<RECIP>(v, s, inv);
         }
     }
     for (int k = (CHUNKS * 256 + threadIdx.x) * 8; k < K; k += 256 * 8) {
         float v[8];
         load8(xr + k, v);
-        alignas(8) int8_t o[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = quant_one<RECIP>(v[e], s, inv);
-        *reinterpret_cast<uint2*>(q + row * K + k) = *reinterpret_cast<const uint2*>(o);
+        *reinterpret_cast<uint2*>(q + row * K + k) = quant8<RECIP>(v, s, inv);
     }
 }
 

@@ -56,6 +56,28 @@ def test_a8_quantiser_at_rounding_boundaries(K, amax):
     np.testing.assert_array_equal(q.cpu().numpy(), qo)
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,K", [(7, 8), (7, 2056), (300, 4096), (300, 4104), (9, 16392)])
+def test_a8_quantiser_of_every_type(dt, rows, K):
+    """The bytes are those of the division: random rows, half-way points that the type can hold, zeros, infinities, NaN; rows that
+    end inside a thread's pieces and past them; bf16 on both sides of its rule on rows."""
+    gen = torch.Generator().manual_seed(K)
+    x = torch.randn(rows, K, generator=gen)
+    x[1] = (torch.arange(K) % 253 - 126) / 2  # ties, with the scale 1 that the next line makes
+    x[1, -1] = 127.0
+    x[2] = 0
+    x[3, K // 2] = float("nan")
+    x[4, 0] = float("inf")
+    x[5] *= 1e-6
+    x = x.to(dt)
+    f = x.float()
+    s = (f.nan_to_num(nan=0.0, posinf=float("inf")).abs().amax(1) / 127.0).clamp_min(1e-5)
+    t = f / s[:, None]
+    want = torch.where(t >= 0, (t + 0.5).floor(), (t - 0.5).ceil()).nan_to_num(nan=-127.0).clamp(-127, 127).to(torch.int8)
+    q, scale = hb.dynamic_a8_quant(x.cuda())
+    assert torch.equal(scale.cpu().reshape(-1), s) and torch.equal(q.cpu(), want)
+
+
 @pytest.mark.parametrize("M,K,Nn", [(1, 16, 8), (17, 64, 24), (64, 256, 96), (130, 4096, 136), (256, 512, 256), (384, 1024, 512)])
 def test_int8_gemm_bit_exact(M, K, Nn):
     rng = np.random.default_rng(M * 7 + Nn)
