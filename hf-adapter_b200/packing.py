@@ -304,7 +304,7 @@ def _wide_projections(ctx, x, ops, xs, downs, ups, down_x):
     if tiled is not None:
         # int4 / int8 r / k / v of equal shape: one launch streams all three weight sets (one pipeline fill, no split-K
         # exchange).  The LoRA chain is two launches long and leads, behind the kernel that made its inputs; they branch off
-        lora = lora_chain()
+        lora = lora_chain(lean=int(x.shape[0]) > 16)
         branched = rkv = branch(0, xs, lambda: _rkv_launch(ops, xs, tiled))
     elif _lora_leads(ops[0], int(x.shape[0]), int(xs[0].shape[-1])):
         # independent projections on separate branches: the tail of one overlaps the ramp-up of the next
