@@ -43,6 +43,14 @@ def same_dtype(first, *rest, what: str) -> None:
             raise ValueError(f"{what}: dtype mismatch ({t.dtype} vs {first.dtype})")
 
 
+def zero_lists(*lists) -> None:
+    """Zeros into every tensor of lists that are of one type each: a launch a list, not one a tensor (a prefill begins with the
+    buffers of all layers, and the GPU idles meanwhile: 32 layers 0.9 ms)."""
+    for ts in lists:
+        if ts:
+            torch._foreach_zero_(ts)
+
+
 def ptr(t):
     return 0 if t is None else t.data_ptr()
 

@@ -6,6 +6,8 @@ from __future__ import annotations
 
 import torch
 
+from ._util import zero_lists
+
 _METRIC_NAMES = ("clones", "detaches", "device_moves", "select_batch_calls", "batch_select_calls", "batch_select_indices_calls",
                  "batch_repeat_interleave_calls", "reorder_calls", "crops", "resets", "native_graph_bound_selects")
 
@@ -66,11 +68,13 @@ class NativeRWKV7Cache:
     def allocate(cls, num_layers, batch, hidden, heads, head_dim, device, dtype, state_dtype=torch.float32):
         """Zero state (rwkv7_hf/native.py:283-295).  ``state_dtype=torch.float16`` allocates the FP16-state lane's
         cache (half the recurrent-state bytes, plus the ``elapsed`` counters of its decay dither)."""
-        z = lambda *s, dt=dtype: torch.zeros(*s, device=device, dtype=dt)
-        return cls([z(batch, heads, head_dim, head_dim, dt=state_dtype) for _ in range(num_layers)],
-                   [z(batch, hidden) for _ in range(num_layers)], [z(batch, hidden) for _ in range(num_layers)],
-                   z(batch, heads * head_dim), 0,
-                   elapsed=z(batch, dt=torch.int32) if state_dtype == torch.float16 else None)
+        e = lambda *s, dt=dtype: torch.empty(*s, device=device, dtype=dt)
+        cache = cls([e(batch, heads, head_dim, head_dim, dt=state_dtype) for _ in range(num_layers)],
+                    [e(batch, hidden) for _ in range(num_layers)], [e(batch, hidden) for _ in range(num_layers)],
+                    e(batch, heads * head_dim), 0,
+                    elapsed=e(batch, dt=torch.int32) if state_dtype == torch.float16 else None)
+        zero_lists(cache._state, [*cache._xpa, *cache._xpf, cache._v_first], [] if cache._elapsed is None else [cache._elapsed])
+        return cache
 
     def _tensors(self):
         """Every tensor of the cache as one flat list (the order `_set_tensors` takes)."""

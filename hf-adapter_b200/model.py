@@ -425,11 +425,12 @@ class RWKV7ForCausalLM(nn.Module):
                 w, k, v, kk, a_sig = _prep.fused_prefill_state_prep(
                     w_raw, k_raw, v_raw, a_pre, at.k_k, at.k_a, v_first=vf, v_gate=vg, num_heads=H, head_dim=N,
                     a_is_raw=True, v_gate_is_raw=True, return_gate=True)
-                out, new_state = _rec.fused_recurrent_scan_output_prepare(
+                out, new_state = _rec.scan_output_prepare_inplace(
                     r, w, k, v, kk, a_sig, state[i], g, at.r_k, at.g_norm.weight, at.g_norm.bias, eps=N * 1e-5)
             if i == 0:
                 v_first = v
-            state[i].copy_(new_state)
+            if new_state is not state[i]:
+                state[i].copy_(new_state)
             if self.tp_world == 1:
                 x = _linear(at.o_proj, out, residual=x)  # the residual add rides in the projection's epilogue
             else:

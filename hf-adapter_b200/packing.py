@@ -27,6 +27,7 @@ from . import norm_mix as _nm
 from . import quant as _q
 from . import recurrent as _rec
 from . import rows as _rowsk
+from ._util import zero_lists
 
 PACK_SLOTS = 41
 _QUANT_TYPES = (_q.MM4Linear, _q.MM8Linear, _q.A8W8Linear)
@@ -111,9 +112,10 @@ def init_batched_from_packs(packs, batch_size: int, device, dtype, *, state_dtyp
     hid = int(packs[0][7].numel())
     if state_dtype is None:
         state_dtype = torch.float32
-    state = [torch.zeros(batch_size, H, N, N, device=device, dtype=state_dtype) for _ in range(n)]
-    xpa = [torch.zeros(batch_size, hid, device=device, dtype=dtype) for _ in range(n)]
-    xpf = [torch.zeros(batch_size, hid, device=device, dtype=dtype) for _ in range(n)]
+    state = [torch.empty(batch_size, H, N, N, device=device, dtype=state_dtype) for _ in range(n)]
+    xpa = [torch.empty(batch_size, hid, device=device, dtype=dtype) for _ in range(n)]
+    xpf = [torch.empty(batch_size, hid, device=device, dtype=dtype) for _ in range(n)]
+    zero_lists(state, [*xpa, *xpf])
     return state, xpa, xpf
 
 

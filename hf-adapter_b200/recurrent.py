@@ -284,6 +284,13 @@ def fused_recurrent_scan_output_prepare(r, w, k, v, kk, a, state, g, r_k, group_
                  prep=(g, r_k, group_norm_weight, group_norm_bias), eps=eps)
 
 
+def scan_output_prepare_inplace(r, w, k, v, kk, a, state, g, r_k, group_norm_weight, group_norm_bias, *, eps: float):
+    """``fused_recurrent_scan_output_prepare`` that leaves the final state in ``state`` (which it returns), where that is
+    contiguous: a CTA reads its head's state before the first token and writes it after the last."""
+    return _scan("scan_output_prepare_inplace", r, w, k, v, kk, a, state, 0, prep=(g, r_k, group_norm_weight, group_norm_bias),
+                 eps=eps, new_state=state if state.is_contiguous() else None)
+
+
 def fused_recurrent_scan_state_prep(r, w_raw, k_raw, v_raw, a, state, k_k, k_a, *, v_first=None, v_gate=None,
                                     block_n: int = 64, block_m=None, num_warps=None, force_fallback: bool = False):
     """State prep folded into the scan (rwkv7_hf/fused_recurrent_update.py:1541): raw w / k / v and sigmoided a / v-gate

@@ -132,6 +132,7 @@ int rwkv7_wkv7_output_prepare_raw_f16state(const void* r, const void* w_raw, con
  * (rwkv7_hf/dplr_prefill.py:505).  Inputs [B,T,H,64]; y [B,T,H,64]; state [B,H,64,64] fp32.
  *   w_mode: 0 = w is the decay in `dtype`, 1 = decay in fp32, 2 = raw w in `dtype` (decay computed in-kernel)
  *   g/r_k/gn_w/gn_b: all NULL = plain scan; all non-NULL = fused per-token GroupNorm/bonus/gate.
+ *   state_out may equal state_in (rwkv7_wkv7_scan and _f16state).
  */
 int rwkv7_wkv7_scan(const void* r, const void* w, const void* k, const void* v, const void* kk, const void* a,
                     const float* state_in, float* state_out, void* y,

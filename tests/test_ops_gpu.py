@@ -222,6 +222,26 @@ def test_scan_parameters_of_any_alignment(dt, Hh):
         assert all(torch.equal(x, y) for x, y in zip(got, want))
 
 
+@pytest.mark.parametrize("Hh,sd", [(3, torch.float32), (149, torch.float16), (300, torch.float32)])
+def test_scan_in_place_is_the_scan(Hh, sd):
+    """The final state over the first one: the same bits as in a buffer of its own; a strided state is left alone."""
+    from hf_adapter_b200.recurrent import scan_output_prepare_inplace
+    T = 19
+    rng = np.random.default_rng(Hh)
+    f = lambda *sh: cu(rng.standard_normal(sh).astype(np.float16))
+    seq = [cu(x) for x in wkv_inputs(1, T, Hh, N, seed=Hh)]
+    seq[1] = seq[1].to(torch.float16)
+    rest = f(1, T, Hh, N), 0.1 * f(Hh, N), f(Hh * N), f(Hh * N)
+    s0 = (0.1 * f(2, Hh, N, N).float()).to(sd)
+    want, final = hb.fused_recurrent_scan_output_prepare(*seq, s0[:1], *rest, eps=EPS)
+    state = s0[:1].clone()
+    got, same = scan_output_prepare_inplace(*seq, state, *rest, eps=EPS)
+    assert same is state and torch.equal(got, want) and torch.equal(state, final)
+    strided = s0[:1].transpose(2, 3).contiguous().transpose(2, 3)
+    got, other = scan_output_prepare_inplace(*seq, strided, *rest, eps=EPS)
+    assert other is not strided and torch.equal(got, want) and torch.equal(other, final) and torch.equal(strided, s0[:1])
+
+
 def test_scan_empty_sequence_passes_state_through():
     s0 = torch.randn(2, 2, N, N, device="cuda")
     e = torch.empty(2, 0, 2, N, device="cuda", dtype=torch.float16)
