@@ -435,15 +435,29 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
         cluster_wait();
     }
 
+    grid_dependency_wait();  // residual reads and output writes are ordered after the preceding kernel (returns at once here)
     // ---- split-K reduction (fixed rank order) + epilogue, from this CTA's own shared memory
+    // Each thread owns one channel pair (n, n + 1) and walks the rows of this rank's share.  Above 64 rows a pass EU at a time: their
+    // residuals are requested together, the first ones under the barrier, where one by one, with a store in between, each costs a
+    // round trip to L2.  Step of 256 rows, 7.2B int4: 7408 -> 7318 us, 100 rows 4136 -> 4126; of 64 rows (three turns of the loop) 2797 -> 2824.
+    constexpr int EU = NB > 64 ? 4 : 1, RSTEP = NTHREADS / 64;  // full 64-thread row teams (a trailing half team sits out)
+    const int en = (tid & 63) * 2, e_begin = split * rows_per_rank, e_end = (tid >> 6) < RSTEP ? min(m_rows, e_begin + rows_per_rank) : 0;
+    const bool e_ok = n0 + en < p.Nout, e_pair = n0 + en + 1 < p.Nout && (p.Nout & 1) == 0;
+    __half2 e_res[EU];
+    auto residuals = [&](int m) {
+#pragma unroll
+        for (int u = 0; u < EU; ++u)
+            if (p.epilogue == RWKV7_EPI_ADD && e_pair && m + u * RSTEP < e_end)
+                e_res[u] = *reinterpret_cast<const __half2*>(p.residual + (size_t)(m0 + m + u * RSTEP) * p.Nout + n0 + en);
+    };
     if (clustered) {
         cluster_arrive_release();
+        residuals(e_begin + (tid >> 6));
         cluster_wait();
     } else {
         __syncthreads();
     }
     const bool aborted = (*abort_flag != 0);
-    grid_dependency_wait();  // residual reads and output writes are ordered after the preceding kernel (returns at once here)
     if (!aborted && !clustered) {
         // 16-byte pieces of the staged rows: 16 threads cover the 256 bytes of a row
         for (int idx = tid; idx < m_rows * (TILE_N / 8); idx += NTHREADS) {
@@ -474,50 +488,50 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
         }
     }
     if (!aborted && clustered) {
-        // Each thread owns one channel pair (n, n+1) and walks the rows of this rank's share: float2 loads of the rank
-        // slots in fixed order, fp16 rounding, epilogue, one 4-byte store; 64 consecutive threads cover one 256-byte
-        // output row segment.
-        const int m_begin = split * rows_per_rank;
-        const int m_end = min(m_rows, m_begin + rows_per_rank);
-        const int n = (tid & 63) * 2;
-        const bool n_ok = n0 + n < p.Nout;
-        const bool pair = (n0 + n + 1 < p.Nout) && ((p.Nout & 1) == 0);
-        constexpr int RSTEP = NTHREADS / 64;  // full 64-thread row teams (a trailing half team sits out)
-        const float* Q0 = Q + n - (size_t)m_begin * TILE_N;  // slot r, global row m: Q0[(r * rows_per_rank + m) * TILE_N]
+        // float2 loads of the rank slots in fixed order, fp16 rounding, epilogue, one 4-byte store; 64 consecutive threads cover one
+        // 256-byte output row segment
+        const float* Q0 = Q + en - (size_t)e_begin * TILE_N;  // slot r, global row m: Q0[(r * rows_per_rank + m) * TILE_N]
         const int slot = rows_per_rank * TILE_N;
         float rs0 = 1.f, rs1 = 1.f;
-        if (FMT == 1 && n_ok) {
-            rs0 = __half2float(p.rscale[grp_idx][n0 + n]);
-            if (n0 + n + 1 < p.Nout) rs1 = __half2float(p.rscale[grp_idx][n0 + n + 1]);
+        if (FMT == 1 && e_ok) {
+            rs0 = __half2float(p.rscale[grp_idx][n0 + en]);
+            if (n0 + en + 1 < p.Nout) rs1 = __half2float(p.rscale[grp_idx][n0 + en + 1]);
         }
-        for (int m = m_begin + (tid >> 6); m < m_end && n_ok && (tid >> 6) < RSTEP; m += RSTEP) {
-            const float* qq = Q0 + m * TILE_N;
-            float2 acc = *reinterpret_cast<const float2*>(qq);
-            for (int r = 1; r < p.splits; ++r) {
-                const float2 t2 = *reinterpret_cast<const float2*>(qq + r * slot);
-                acc.x += t2.x;
-                acc.y += t2.y;
-            }
-            const size_t o = (size_t)(m0 + m) * p.Nout + n0 + n;
-            float y0 = __half2float(__float2half_rn(acc.x * rs0)), y1 = __half2float(__float2half_rn(acc.y * rs1));
-            if (p.epilogue == RWKV7_EPI_RELU2) {
-                y0 = fmaxf(y0, 0.f); y0 *= y0;
-                y1 = fmaxf(y1, 0.f); y1 *= y1;
-            } else if (p.epilogue == RWKV7_EPI_ADD) {
-                if (pair) {
-                    const float2 rr = __half22float2(*reinterpret_cast<const __half2*>(p.residual + o));
-                    y0 += rr.x;
-                    y1 += rr.y;
-                } else {
-                    y0 += __half2float(p.residual[o]);
-                    if (n0 + n + 1 < p.Nout) y1 += __half2float(p.residual[o + 1]);
+        const int first = e_begin + (tid >> 6);
+        for (int mb = first; mb < e_end && e_ok; mb += EU * RSTEP) {
+            if (mb > first) residuals(mb);
+#pragma unroll
+            for (int u = 0; u < EU; ++u) {
+                const int m = mb + u * RSTEP;
+                if (m >= e_end) break;
+                const float* qq = Q0 + m * TILE_N;
+                float2 acc = *reinterpret_cast<const float2*>(qq);
+                for (int r = 1; r < p.splits; ++r) {
+                    const float2 t2 = *reinterpret_cast<const float2*>(qq + r * slot);
+                    acc.x += t2.x;
+                    acc.y += t2.y;
                 }
-            }
-            if (pair) {
-                *reinterpret_cast<__half2*>(outp + o) = __floats2half2_rn(y0, y1);
-            } else {
-                outp[o] = __float2half_rn(y0);
-                if (n0 + n + 1 < p.Nout) outp[o + 1] = __float2half_rn(y1);
+                const size_t o = (size_t)(m0 + m) * p.Nout + n0 + en;
+                float y0 = __half2float(__float2half_rn(acc.x * rs0)), y1 = __half2float(__float2half_rn(acc.y * rs1));
+                if (p.epilogue == RWKV7_EPI_RELU2) {
+                    y0 = fmaxf(y0, 0.f); y0 *= y0;
+                    y1 = fmaxf(y1, 0.f); y1 *= y1;
+                } else if (p.epilogue == RWKV7_EPI_ADD) {
+                    if (e_pair) {
+                        const float2 rr = __half22float2(e_res[u]);
+                        y0 += rr.x;
+                        y1 += rr.y;
+                    } else {
+                        y0 += __half2float(p.residual[o]);
+                        if (n0 + en + 1 < p.Nout) y1 += __half2float(p.residual[o + 1]);
+                    }
+                }
+                if (e_pair) {
+                    *reinterpret_cast<__half2*>(outp + o) = __floats2half2_rn(y0, y1);
+                } else {
+                    outp[o] = __float2half_rn(y0);
+                    if (n0 + en + 1 < p.Nout) outp[o + 1] = __float2half_rn(y1);
+                }
             }
         }
     }
