@@ -281,37 +281,46 @@ __device__ __forceinline__ Raw8<T> ld_row8(const T* p) {
     }
 }
 
-// LayerNorm and token-shift mixes of a sequence in one pass: a CTA takes one token and normalises its row and the row before it
+// LayerNorm and token-shift mixes of a sequence in one pass: a CTA takes R tokens and normalises their rows and the row before them
 // (which L2 has, because the token before is read at about the same time), rounded to the storage type as stored ones would be, so
-// that the normalised sequence is neither written nor read.  The two rows' statistics share their barriers.  A thread has 8 NV
+// that the normalised sequence is neither written nor read.  The rows' statistics share their barriers.  A thread has 8 NV
 // elements of each (as many threads as the row needs, up to 512).
+//
+// Bound: with more CTAs than are resident, the parameters and the second reading of every row (a token's reads weigh five times its
+// own row with one mix, 64 registers let few CTAs overlap them): two tokens a CTA read three rows for two and the parameters once.
+// us, fp16, one token a CTA -> two, six mixes / one mix: 777 x 2560 8.5 / 6.2 -> 7.5 / 5.0, 2331 x 2560 20.8 / 14.3 -> 17.6 / 10.9, 8192 x 768 19.0 / 13.2 ->
+// 17.6 / 10.5, 32768 x 4096 one mix 293 -> 210 (5.1 TB/s).
 constexpr int kSeqThreads = 512;
-template <typename T, int NMIX, int NV>
+template <typename T, int NMIX, int NV, int R>
 __global__ void __launch_bounds__(kSeqThreads, NV == 1 ? 2 : 1) seq_norm_mix_kernel(const SeqNormMixArgs p) {
-    __shared__ float2 red[2][kSeqThreads / 32];
+    constexpr int ROWS = R + 1;  // row 0: the one before the CTA's tokens (before the first of a sequence: the initial state, normalised already)
+    __shared__ float red[2][ROWS][kSeqThreads / 32];
     const int D = p.D, nvec = D / 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const size_t row = blockIdx.x;
-    const int t = (int)(row % p.T);
-    const size_t b = row / p.T;
-    auto block_sums = [&](float u, float v, float2* r) {
-        u = group_sum<32>(u);
-        v = group_sum<32>(v);
-        if (lane == 0) r[warp] = make_float2(u, v);
+    const int per_seq = (p.T + R - 1) / R, t0 = (int)(blockIdx.x % per_seq) * R, nt = R == 1 ? 1 : min(R, p.T - t0);
+    const size_t b = blockIdx.x / per_seq, row0 = b * p.T + t0;
+    auto block_sums = [&](float (&v)[ROWS], float (*r)[kSeqThreads / 32]) {
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) v[i] = group_sum<32>(v[i]);
+        if (lane == 0)
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) r[i][warp] = v[i];
         __syncthreads();
-        const float2 q = lane < warps ? r[lane] : make_float2(0.f, 0.f);
-        return make_float2(group_sum<32>(q.x), group_sum<32>(q.y));
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) v[i] = group_sum<32>(lane < warps ? r[i][lane] : 0.f);
     };
-    float x[NV][8], pv[NV][8];  // this row and the one before it (t = 0: the initial state, which is normalised already)
-    float sx = 0.f, sp = 0.f;
+    float x[ROWS][NV][8];
+    float mean[ROWS] = {}, rstd[ROWS] = {};
+    Raw8<T> cw[NV], cb[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int vi = threadIdx.x + i * kSeqThreads;
         if (vi < nvec) {
-            load8(reinterpret_cast<const T*>(p.x) + row * D + vi * 8, x[i]);
-            load8(t > 0 ? reinterpret_cast<const T*>(p.x) + (row - 1) * D + vi * 8 : reinterpret_cast<const T*>(p.init_prev) + b * D + vi * 8, pv[i]);
+            load8(t0 > 0 ? reinterpret_cast<const T*>(p.x) + (row0 - 1) * D + vi * 8 : reinterpret_cast<const T*>(p.init_prev) + b * D + vi * 8, x[0][i]);
+#pragma unroll
+            for (int j = 1; j < ROWS; ++j)  // past the sequence's end: the last token again, for nobody
+                load8(reinterpret_cast<const T*>(p.x) + (row0 + (R == 1 ? 0 : min(j, nt) - 1)) * D + vi * 8, x[j][i]);
         }
     }
-    Raw8<T> cw[NV], cb[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int vi = threadIdx.x + i * kSeqThreads;
@@ -319,29 +328,29 @@ __global__ void __launch_bounds__(kSeqThreads, NV == 1 ? 2 : 1) seq_norm_mix_ker
             cw[i] = ld_row8(reinterpret_cast<const T*>(p.nw) + vi * 8);
             cb[i] = ld_row8(reinterpret_cast<const T*>(p.nb) + vi * 8);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                sx += x[i][e];
-                sp += pv[i][e];
-            }
+            for (int e = 0; e < 8; ++e)
+#pragma unroll
+                for (int j = 0; j < ROWS; ++j) mean[j] += x[j][i][e];
         }
     }
-    float2 mean = block_sums(sx, sp, red[0]);
-    mean.x /= (float)D;
-    mean.y /= (float)D;
-    float qx = 0.f, qp = 0.f;
+    block_sums(mean, red[0]);
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) mean[j] /= (float)D;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         if (threadIdx.x + i * kSeqThreads < nvec) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float dx = x[i][e] - mean.x, dp = pv[i][e] - mean.y;
-                qx += dx * dx;
-                qp += dp * dp;
-            }
+            for (int e = 0; e < 8; ++e)
+#pragma unroll
+                for (int j = 0; j < ROWS; ++j) {
+                    const float d = x[j][i][e] - mean[j];
+                    rstd[j] += d * d;
+                }
         }
     }
-    const float2 var = block_sums(qx, qp, red[1]);
-    const float rx = rsqrtf(var.x / (float)D + p.eps), rp = rsqrtf(var.y / (float)D + p.eps);
+    block_sums(rstd, red[1]);
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) rstd[j] = rsqrtf(rstd[j] / (float)D + p.eps);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int vi = threadIdx.x + i * kSeqThreads;
@@ -349,18 +358,27 @@ __global__ void __launch_bounds__(kSeqThreads, NV == 1 ? 2 : 1) seq_norm_mix_ker
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const float w = to_f<T>(cw[i].v[e]), bb = to_f<T>(cb[i].v[e]);
-            x[i][e] = round_to<T>((x[i][e] - mean.x) * rx * w + bb);
-            const float h = round_to<T>((pv[i][e] - mean.y) * rp * w + bb);
-            pv[i][e] = (t > 0 ? h : pv[i][e]) - x[i][e];
+#pragma unroll
+            for (int j = 0; j < ROWS; ++j) {
+                const float h = round_to<T>((x[j][i][e] - mean[j]) * rstd[j] * w + bb);
+                x[j][i][e] = j > 0 || t0 > 0 ? h : x[j][i][e];
+            }
         }
-        if (t == p.T - 1) store8(reinterpret_cast<T*>(p.next_state) + b * D + vi * 8, x[i]);
+#pragma unroll
+        for (int j = 1; j < ROWS; ++j)
+            if (t0 + j == p.T) store8(reinterpret_cast<T*>(p.next_state) + b * D + vi * 8, x[j][i]);
 #pragma unroll
         for (int m = 0; m < NMIX; ++m) {
-            float mx[8], o[8];
+            float mx[8];
             load8(reinterpret_cast<const T*>(p.mix[m]) + vi * 8, mx);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = x[i][e] + pv[i][e] * mx[e];
-            store8(reinterpret_cast<T*>(p.out[m]) + row * D + vi * 8, o);
+            for (int j = 1; j < ROWS; ++j) {
+                if (R > 1 && j > nt) break;
+                float o[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) o[e] = x[j][i][e] + (x[j - 1][i][e] - x[j][i][e]) * mx[e];
+                store8(reinterpret_cast<T*>(p.out[m]) + (row0 + j - 1) * D + vi * 8, o);
+            }
         }
     }
 }
@@ -511,9 +529,15 @@ extern "C" int rwkv7_seq_norm_mix(const void* x, const void* norm_w, const void*
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, TT, {
         const bool wide = D > 8 * kSeqThreads;
-        auto kern = wide ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 2> : seq_norm_mix_kernel<TT, 1, 2>)
-                         : (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 1> : seq_norm_mix_kernel<TT, 1, 1>);
-        kern<<<B * T, wide ? kSeqThreads : (D / 8 + 31) / 32 * 32, 0, st>>>(p);
+        const int threads = wide ? kSeqThreads : (D / 8 + 31) / 32 * 32, per_sm = 65536 / (64 * threads);
+        // Two tokens a CTA where one each would not all be resident.  Below that they only halve the CTAs (300 x 2560, six / one mix 4.9 / 3.8 ->
+        // 5.6 / 3.8); with six mixes the stores weigh more, in fp32 from two waves on (777 x 2560 16.6 -> 17.7, 2331 x 2560 40.3 -> 38.6), and at
+        // two CTAs an SM not at all (768 x 4096 12.5 -> 13.6, 2048 x 3072 22.5 -> 23.2).
+        const bool two = !wide && T > 1 && (n_mix == 1 || per_sm >= 3) && (long long)B * T > 148ll * per_sm * (n_mix == 6 && sizeof(TT) == 4 ? 2 : 1);
+        auto kern = wide  ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 2, 1> : seq_norm_mix_kernel<TT, 1, 2, 1>)
+                    : two ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 1, 2> : seq_norm_mix_kernel<TT, 1, 1, 2>)
+                          : (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 1, 1> : seq_norm_mix_kernel<TT, 1, 1, 1>);
+        kern<<<B * (two ? (T + 1) / 2 : T), threads, 0, st>>>(p);
         return check_launch("seq_norm_mix_kernel");
     });
     return RWKV7_OK;

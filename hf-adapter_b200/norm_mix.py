@@ -9,7 +9,7 @@ from ._util import dt_code, no_fallback, ptr, require_cuda, same_dtype, stream_p
 
 
 def _one_norm_mix(rows: int, width: int, dtype) -> bool:
-    """Whether the norm and the mixes of a sequence are one kernel, which normalises every row twice (once as the row before the next):
+    """Whether the norm and the mixes of a sequence are one kernel that takes a token a CTA and normalises every row twice (once as the row before the next):
     few CTAs do not notice, many do, and the fewer fit an SM the sooner (a CTA is width / 8 threads up to 4096, above that 512 with
     two vectors each)."""
     # us, two kernels -> one, six mixes / one mix.  fp16: 2331 x 2560 25.7 / 17.6 -> 24.9 / 16.5, 2048 x 3072 25.7 / 17.5 -> 24.7 / 16.1; 768 x 4096
@@ -18,6 +18,14 @@ def _one_norm_mix(rows: int, width: int, dtype) -> bool:
     # waits for memory: 2048 x 768 21.3 / 9.1 -> 13.9 / 6.3, 1600 x 3584 56.2 / 22.7 -> 44.2 / 21.7, 768 x 8192 65.2 / 29.3 -> 59.6 / 27.3.
     most = 6 if dtype == torch.float32 or width <= 3072 else 3 if width <= 4096 else 1
     return rows * width <= most << 20
+
+
+def _one_kernel(rows: int, tokens: int, width: int, dtype, mixes: int) -> bool:
+    """``_one_norm_mix``, or a form in which a CTA takes two tokens of a sequence and reads three rows for them: one kernel at any size."""
+    # us, two kernels -> that.  One mix, up to 4096 wide: fp16 2331 x 2560 14.0 -> 10.9, 768 x 4096 8.7 -> 7.3, 32768 x 4096 261 -> 210, bf16 289 -> 219, fp32
+    # 393 -> 285.  Six, up to 2560 wide: fp16 2331 x 2560 22.8 -> 17.6, 16384 x 2560 157 -> 108, bf16 169 -> 112, fp32 361 -> 210.  Wider, six mixes keep to one
+    # token a CTA (32768 x 4096 in fp16 would be 460 -> 416 so, 1554 x 4096 23.2 -> 25.2, bf16 8192 x 3072 98 -> 105).
+    return (tokens > 1 and width <= (4096 if mixes == 1 else 2560)) or _one_norm_mix(rows, width, dtype)
 
 
 def _rows(x, name):
@@ -174,7 +182,7 @@ def sequence_norm_mix(x, initial_prev, norm_weight, norm_bias, mixes, eps: float
     nw, nb = norm_weight.contiguous(), norm_bias.contiguous()
     mp, _k1 = _lib.ptr_array([m.data_ptr() for m in flat])
     op, _k2 = _lib.ptr_array([o.data_ptr() for o in outs])
-    if _one_norm_mix(B * T, D, x.dtype):
+    if _one_kernel(B * T, T, D, x.dtype, len(mixes)):
         _lib.check(_lib.lib.rwkv7_seq_norm_mix(ptr(src), ptr(nw), ptr(nb), ptr(initial), mp, op, ptr(nxt), B, T, D, len(mixes), float(eps),
                                                dt_code(src), stream_ptr(src)), "sequence_norm_mix")
     else:

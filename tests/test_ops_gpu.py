@@ -402,6 +402,32 @@ def test_sequence_norm_mix(dt, B, T, D):
 
 
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,T,D,piece", [(3, 148, 2560, 90), (3, 149, 2560, 91), (297, 3, 2560, 1), (1, 2963, 768, 100), (1, 297, 4096, 99), (2, 149, 3072, 61),
+                                         (1, 8193, 4096, 256)])
+def test_sequence_norm_mix_of_two_tokens_a_cta(dt, B, T, D, piece):
+    """Either side of the row counts at which a CTA takes two tokens, odd lengths and sequences of three among them, and of the sizes at
+    which one kernel becomes two: a long call gives the bits of short ones (one token a CTA) that carry the state."""
+    from hf_adapter_b200 import norm_mix as NM
+    g = torch.Generator(device="cuda").manual_seed(B * T + D)
+    n = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dt)
+    x, state, w, b = n(B, T, D), n(B, D), n(D), n(D)
+    mixes = [torch.rand(D, generator=g, device="cuda").to(dt) for _ in range(6)]
+    for k in (6, 1):
+        one = NM._one_kernel(B * T, T, D, dt, k)
+        outs, nxt = NM.sequence_norm_mix(x, state, w, b, mixes[:k])
+        carried, parts = state, []
+        for t in range(0, T, piece):
+            got, carried = NM.sequence_norm_mix(x[:, t:t + piece].contiguous(), carried, w, b, mixes[:k])
+            parts.append(got)
+        whole = [torch.cat(p, 1) for p in zip(*parts)]
+        if one:
+            assert torch.equal(carried, nxt) and all(torch.equal(p.reshape(-1), q.reshape(-1)) for p, q in zip(whole, outs))
+        else:  # two kernels: the row's statistics in another order, so a unit of the rounded rows, as in the test above
+            eps = max(torch.finfo(dt).eps, 2e-6)
+            assert all(((p.reshape(-1).float() - q.reshape(-1).float()).abs() <= 4 * eps * (8 + q.reshape(-1).float().abs())).all() for p, q in zip(whole, outs))
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,Hh", [(1, 1), (33, 1), (4095, 3), (12287, 1), (12288, 1), (4099, 3)])
 def test_state_prep_either_side_of_its_two_forms(dt, rows, Hh):
     """8- and 16-byte pieces a lane (they change at 12288 heads) against 64 bits.  Each result is rounded once from fp32 arithmetic of a
