@@ -113,16 +113,16 @@ def few_rows_quant(rows: int, in_features: int, out_features: int) -> bool:
     the tcgen05 one.  At 8 rows the activations weigh as much as the weights of a long row, and few channels with a long row
     leave SMs idle.  Time of the row kernel over the other's, int4 / int8, by rows:
 
-        4096 -> 4096    1 0.75 / 0.80   4 0.79 / 0.83   8 0.86 / 0.87
-        2560 -> 10240   1 0.89 / 1.00   5 0.87 / 1.00   8 0.90 / 1.06
-        4096 -> 16384   1 0.86 / 0.87   5 0.82 / 0.84   8 0.89 / 0.96
-        7168 -> 4096    1 0.89 / 0.90   5 0.99 / 0.94   8 0.86 / 0.80
-        8192 -> 8192    1 0.81 / 0.83   7 0.95 / 0.89   8 1.13 / 1.05
-        10240 -> 2560   1 0.84 / 0.83   5 0.98 / 0.88   6 1.05 / 0.96   8 1.09 / 1.00
-        12288 -> 8192   1 0.85 / 0.85   5 0.92 / 0.87   6 1.15 / 1.09   8 1.20 / 1.09
-        16384 -> 4096   1 0.73 / 0.77   3 0.87 / 0.85   4 1.04 / 1.04   8 1.15 / 1.07
-        8192 -> 1024    1 1.00 / 0.94   8 1.06 / 0.98
-        12288 -> 1024   1 1.19 / 1.14   8 1.20 / 1.16"""
+        4096 -> 4096    1 0.91 / 1.00   4 0.68 / 0.74   8 0.98 / 0.97
+        2560 -> 10240   1 0.73 / 0.72   5 0.77 / 0.81   8 0.87 / 0.80
+        4096 -> 16384   1 0.72 / 0.77   5 0.75 / 0.78   8 0.83 / 0.83
+        7168 -> 4096    1 1.01 / 0.75   5 1.01 / 0.99   8 0.96 / 1.04
+        8192 -> 8192    1 0.69 / 0.74   7 0.91 / 0.85   8 1.10 / 1.07
+        10240 -> 2560   1 0.97 / 0.97   5 1.06 / 1.03   6 0.99 / 0.92   8 1.16 / 1.07
+        12288 -> 8192   1 0.87 / 0.85   5 0.85 / 0.84   6 1.10 / 1.08   8 1.13 / 1.08
+        16384 -> 4096   1 0.80 / 0.78   3 1.00 / 0.96   4 1.05 / 1.07   8 1.13 / 1.11
+        8192 -> 1024    1 1.23 / 1.26   8 1.12 / 1.09
+        12288 -> 1024   1 1.34 / 1.35   8 1.26 / 1.25"""
     most = 8 if in_features <= 7168 else 7 if in_features <= 8192 else 5 if in_features <= 12288 else 3
     return 1 <= rows <= min(most, _rowsk.MAX_ROWS) and in_features < 8 * out_features
 

@@ -43,13 +43,12 @@ def prefers_dense(rows: int, K: int, N: int, fused: bool, early: bool) -> bool:
     it.  ``fused``: an epilogue rides in it; ``early``: its weights may be requested under the kernel before it.  Library
     against this kernel in us, fp16, 1 / 8 rows:
 
-    * a short K leaves the reads of x and the epilogue: 64 -> 2560 2.2 against 2.1 / 4.6, + residual 3.6 against 2.3 / 6.0; 256 ->
+    * a short K leaves the reads of x and the epilogue: 64 -> 2560 2.4 / 2.8 against 1.9 / 4.2, + residual 3.6 against 2.3 / 6.0; 256 ->
       2048 at 0.82 / 0.97 of the library's time, + residual 0.58 / 0.73;
-    * more channels than a wave of CTAs takes: 2560 -> 2560 8.5 against 5.6 / 6.0, but 2560 -> 10240 11.2 against 14.7 / 15.4 and
-      768 -> 32768 11.6 against 15.6 / 16.7; 1024 -> 8192 at 0.84 / 0.93 of the library, 4096 -> 5120 at 1.04 / 1.08, with the
-      residual 0.93 / 0.95;
-    * early, behind a norm kernel: 2560 -> 10240 + relu^2 17.0 against 16.1 / 17.1, 4096 -> 16384 32.8 against 27.8 / 28.5, 8192 ->
-      8192 28.7 against 27.3 / 28.2; but 5120 -> 20480 42.1 against 45.9 / 46.7 and 20480 -> 5120 + residual 48.2 against 51.3 / 53.1."""
+    * more channels than a wave of CTAs takes: 2560 -> 2560 8.1 / 7.7 against 4.5 / 4.8, but 2560 -> 10240 10.8 against 12.3 / 12.9; 768 ->
+      32768 10.7 against 10.1 / 11.4; 1024 -> 8192 5.6 against 4.2 / 4.4, 4096 -> 5120 10.5 against 10.1 / 10.5;
+    * early, behind a norm kernel and with relu^2: 2560 -> 10240 13.9 / 14.2 against 12.4 / 12.9, 4096 -> 16384 25.6 / 26.7 against 23.2 / 24.0, 8192 ->
+      8192 26.3 / 26.8 against 23.1 / 23.6; but 5120 -> 20480 37.4 against 41.3 / 42.4, and 20480 -> 5120 + residual 48.2 against 51.3 / 53.1."""
     if K < (32 if fused else 64) * rows or K * N > 1 << 26:
         return False
     if early:
