@@ -147,9 +147,9 @@ __device__ __forceinline__ void unit_mma(float (&acc)[TM][2][4], const Regs<FMT>
         }
 }
 
-// units [u0, u1) of the 32 channels from n0
-template <typename T, int FMT>
-__device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, const Args& args, int n0, int u0, int u1) {
+// units [u0, u1) of the 32 channels from n0.  HALVES: the sums of those before `mid` go to slot 2 x warp
+template <typename T, int FMT, bool HALVES>
+__device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, const Args& args, int n0, int u0, int mid, int u1, float (*slots)[kMaxRows * (kTile + 1)]) {
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
     const int K = p.K;
     const uint4* xrow = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.x) + (size_t)gid * K);
@@ -186,6 +186,16 @@ __device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, co
     for (int t = 0; t < TM; ++t)
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[t][e >> 2][e & 3] = 0.f;
+    auto leave_first = [&] {
+        float* first = slots[(threadIdx.x >> 5) * 2];  // (nothing but the lane's place is kept for this through the loop)
+#pragma unroll
+        for (int t = 0; t < TM; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                first[(tig * 2 + (e & 1)) * (kTile + 1) + t * 16 + (e >> 1) * 8 + gid] = acc[t][0][e] + acc[t][1][e];
+                acc[t][0][e] = acc[t][1][e] = 0.f;
+            }
+    };
     Regs<FMT> r[2];
     if (!args.early) grid_dependency_wait();
     if (u0 < u1) load_w(r[0], u0);
@@ -198,6 +208,7 @@ __device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, co
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             if (u + b < u1) {
+                if (HALVES && u + b == mid) leave_first();
                 unit_mma<T, FMT>(acc, r[b]);
                 if (u + b + 2 < u1) {
                     load_w(r[b], u + b + 2);
@@ -206,16 +217,18 @@ __device__ __forceinline__ void stream(float (&sum)[TM][4], const Problem& p, co
             }
         }
     }
+    if (HALVES && mid >= u1) leave_first();  // (a part of one unit or none)
 #pragma unroll
     for (int t = 0; t < TM; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) sum[t][e] = acc[t][0][e] + acc[t][1][e];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) rows_gemv_kernel(const __grid_constant__ Args args) {
+template <typename T, bool HALVES>
+__global__ void __launch_bounds__(HALVES ? kThreads / 2 : kThreads, HALVES ? 4 : 2) rows_gemv_kernel(const __grid_constant__ Args args) {
     __shared__ float slots[kSlots][kMaxRows * (kTile + 1)];  // partial sums [row][channel], padded
-    const int S = args.splits, wk = args.wk, threads = blockDim.x, groups = (threads >> 5) / wk;  // `groups` channel tiles per CTA, wk warps each
+    constexpr int threads = HALVES ? kThreads / 2 : kThreads;
+    const int S = HALVES ? 1 : args.splits, wk = HALVES ? kWarps / 2 : args.wk, groups = (threads >> 5) / wk;  // `groups` channel tiles per CTA, wk warps each
     const int rank = blockIdx.x % S, cta = blockIdx.x / S;
     int pi = 0;
     while (pi + 1 < args.n && cta >= args.p[pi + 1].cta0) ++pi;
@@ -226,13 +239,18 @@ __global__ void __launch_bounds__(kThreads, 2) rows_gemv_kernel(const __grid_con
     const int units = n0 >= p.N ? 0 : p.fmt == kDense ? (p.K + 63) >> 6 : p.K >> 7;
     const int part = rank * wk + warp % wk, parts = S * wk;
     const int u0 = (int)((long long)units * part / parts), u1 = (int)((long long)units * (part + 1) / parts);
-    if (p.fmt == kDense) stream<T, kDense>(sum, p, args, n0, u0, u1);
-    else if (p.fmt == kInt4) stream<__half, kInt4>(sum, p, args, n0, u0, u1);
-    else stream<__half, kInt8>(sum, p, args, n0, u0, u1);
+    // as many partial sums as eight warps would leave, and the same bits: with one chain of MMAs twice as long the sums were a little
+    // further from the exact ones (4096 -> 16384 int4, one row: 0.37 % of the results not the correctly rounded ones, 0.26 % so).  In a kernel
+    // of its own: the branch in the loop cost the others 2 %.
+    constexpr int H = HALVES ? 1 : 0;
+    const int mid = HALVES ? (int)((long long)units * (2 * part + 1) / (2 * parts)) : 0, nslots = parts << H;
+    if (p.fmt == kDense) stream<T, kDense, HALVES>(sum, p, args, n0, u0, mid, u1, slots);
+    else if (p.fmt == kInt4) stream<__half, kInt4, HALVES>(sum, p, args, n0, u0, mid, u1, slots);
+    else stream<__half, kInt8, HALVES>(sum, p, args, n0, u0, mid, u1, slots);
 
     // rank 0 of the cluster receives every partial sum and adds them in fixed order
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-    float* mine = slots[t * parts + part];
+    float* mine = slots[t * nslots + (part << H) + H];
     const uint32_t dst = S > 1 ? mapa_shared(smem_u32(mine), 0) : 0;
     if (S > 1) cluster_wait();
 #pragma unroll
@@ -254,9 +272,9 @@ __global__ void __launch_bounds__(kThreads, 2) rows_gemv_kernel(const __grid_con
     for (int i = threadIdx.x; i < channels * args.M; i += threads) {
         const int c = i % channels, m = i / channels, n = nbase + c;
         if (n >= p.N) continue;
-        const int o = m * (kTile + 1) + c % kTile, s0 = c / kTile * parts;
+        const int o = m * (kTile + 1) + c % kTile, s0 = c / kTile * nslots;
         float v = 0.f;
-        for (int r = 0; r < parts; ++r) v += slots[s0 + r][o];
+        for (int r = 0; r < nslots; ++r) v += slots[s0 + r][o];
         if (p.fmt == kInt8) v *= to_f<T>(reinterpret_cast<const T*>(p.scale)[n]);
         v = round_to<T>(v);
         const size_t oo = (size_t)m * p.N + n;
@@ -322,8 +340,10 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
         return ctas;
     };
     int warps = kWarps, ctas = deal(warps);
+    bool halves = false;  // a warp has the K of two of eight, and leaves the partial sums of either
     if (a.wk == kWarps && ctas > 2 * 148 && 2 * ((ctas + 4 * 148 - 1) / (4 * 148)) <= (ctas + 2 * 148 - 1) / (2 * 148)) {
         warps = a.wk = kWarps / 2;
+        halves = true;
         ctas = deal(warps);
     }
     // Up to one CTA an SM and at least two units a warp: pairs of CTAs halve K.  1 row, fp16 / int4 / int8, one CTA against two:
@@ -331,7 +351,8 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
     // 34.7 / 20.6 / 21.6 -> 25.0 / 14.2 / 16.0; beyond one CTA an SM pairs only add their exchange (4096 -> 16384 int4
     // 15.0 -> 19.9), and so do fours (16384 -> 4096 int4 18.5).
     a.splits = ctas <= 148 && max_units >= 16 ? 2 : 1;
-    auto kern = dtype == RWKV7_F16 ? rows_gemv_kernel<__half> : rows_gemv_kernel<__nv_bfloat16>;
+    auto kern = dtype == RWKV7_F16 ? (halves ? rows_gemv_kernel<__half, true> : rows_gemv_kernel<__half, false>)
+                                   : (halves ? rows_gemv_kernel<__nv_bfloat16, true> : rows_gemv_kernel<__nv_bfloat16, false>);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas * a.splits);
     cfg.blockDim = dim3(warps * 32);

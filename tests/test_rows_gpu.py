@@ -193,3 +193,17 @@ def test_either_side_of_the_wave_limits(N, fmt):
         y, = rows.rows_gemv((x,), (m8.tiled_for(x),), out_features=(N,), fmts=(2,), scales=(m8.row_scale,))
         p = x.double() @ (m8.q_row.double() * m8.row_scale.double()[:, None]).t()
     _close(y, p.float(), torch.float16)
+
+
+@pytest.mark.parametrize("M", [1, 8])
+def test_short_problems_beside_one_of_many_waves(M):
+    """CTAs of four warps leave two partial sums each: of parts of one unit of K, of none, and of an odd number."""
+    sizes = [(512, 9600), (64, 40), (72, 33), (136, 64), (704, 32)]
+    g = torch.Generator(device="cuda").manual_seed(M)
+    xs = [torch.randn(M, K, generator=g, device="cuda").half() for K, _ in sizes]
+    ws = [(torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).half() for K, N in sizes]
+    ys = rows.rows_gemv(xs, ws, out_features=[N for _, N in sizes], fmts=[0] * len(sizes))
+    for x, w, y in zip(xs, ws, ys):
+        _close(y, (x.double() @ w.double().t()).float(), torch.float16)
+        alone, = rows.rows_gemv((x,), (w,), out_features=(int(w.shape[0]),), fmts=(0,))
+        _close(alone, y.float(), torch.float16)
