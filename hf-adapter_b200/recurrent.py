@@ -286,9 +286,13 @@ def fused_recurrent_scan_output_prepare(r, w, k, v, kk, a, state, g, r_k, group_
 
 def scan_output_prepare_inplace(r, w, k, v, kk, a, state, g, r_k, group_norm_weight, group_norm_bias, *, eps: float):
     """``fused_recurrent_scan_output_prepare`` that leaves the final state in ``state`` (which it returns), where that is
-    contiguous: a CTA reads its head's state before the first token and writes it after the last."""
-    return _scan("scan_output_prepare_inplace", r, w, k, v, kk, a, state, 0, prep=(g, r_k, group_norm_weight, group_norm_bias),
-                 eps=eps, new_state=state if state.is_contiguous() else None)
+    contiguous: a CTA reads its head's state before the first token and writes it after the last.  Counted as a change of ``state``, as the
+    copy of a new state into it would be, so that a backward pass that saved it before says so."""
+    out, final = _scan("scan_output_prepare_inplace", r, w, k, v, kk, a, state, 0, prep=(g, r_k, group_norm_weight, group_norm_bias),
+                       eps=eps, new_state=state if state.is_contiguous() else None)
+    if final is state:
+        torch.autograd.graph.increment_version(state)
+    return out, final
 
 
 def fused_recurrent_scan_state_prep(r, w_raw, k_raw, v_raw, a, state, k_k, k_a, *, v_first=None, v_gate=None,

@@ -242,6 +242,20 @@ def test_scan_in_place_is_the_scan(Hh, sd):
     assert other is not strided and torch.equal(got, want) and torch.equal(other, final) and torch.equal(strided, s0[:1])
 
 
+def test_scan_in_place_is_a_change_of_the_state():
+    """A backward pass through something that saved the state before a prefill moved it on is refused, not silently wrong."""
+    from hf_adapter_b200.recurrent import scan_output_prepare_inplace
+    T = 5
+    f = lambda *sh: torch.randn(*sh, device="cuda", dtype=torch.float16)
+    state, weight = torch.randn(1, 3, N, N, device="cuda"), torch.ones((), device="cuda", requires_grad=True)
+    loss = (state * weight).sum()
+    with torch.no_grad():
+        _, same = scan_output_prepare_inplace(*(f(1, T, 3, N) for _ in range(6)), state, f(1, T, 3, N), f(3, N), f(3 * N), f(3 * N), eps=EPS)
+    assert same is state
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
+
+
 def test_scan_empty_sequence_passes_state_through():
     s0 = torch.randn(2, 2, N, N, device="cuda")
     e = torch.empty(2, 0, 2, N, device="cuda", dtype=torch.float16)
