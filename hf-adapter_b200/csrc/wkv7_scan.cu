@@ -179,7 +179,7 @@ __device__ __forceinline__ void scan_block(f2 (&S)[R][C / 2], Operands& op, int 
 
 // ---- grids that leave an SM with one or two CTAs: the serial chain of a token is all there is -----------------------------
 // Operands of one token in registers: the columns of a lane (4 cg .. + 3 and 32 + 4 cg .. + 3) and the values of its four rows.
-constexpr int kFewBlocks = 5;               // blocks of operands in shared memory: two ahead, two behind the one that runs
+constexpr int kFewBlocks = 3;               // blocks of operands in shared memory: one ahead, one behind the one that runs
 constexpr int kFewRows = 4, kFewLanes = 8;  // rows a thread has eight columns of, lanes that share them
 struct TokenRegs {
     f2 kk[4], w[4], k[4], nb[4], r[4];
@@ -206,14 +206,14 @@ template <typename T> struct alignas(2 * sizeof(T)) Pair { T x, y; };
 template <typename T> __device__ __forceinline__ float2 to_f2(const Pair<T>& q) { return make_float2(to_f<T>(q.x), to_f<T>(q.y)); }
 
 // A CTA owns one (sequence, head).  Warps 0..3 run the recurrence: 8 lanes share four rows, a lane has 8 columns of each.  Warps
-// 4, 5 read a block of tokens ahead (in registers while the block before it runs) and convert it, warps 6, 7 write out a block that
+// 4, 5 read a block of tokens ahead (in registers while the block before it runs) and convert it, warps 6, 7 write out the block that
 // is done.  In the token loop everything that does not wait for S.kk of this token sits in its shadow: the operands of the next
-// token, the decay and the v k^T term, the output sums of the token before.  Five blocks are in flight so that this also holds
-// for the first token of a block: its operands are there a barrier early, and the last output of the block before leaves with it.
+// token, the decay and the v k^T term, the output sums of the token before.  (Five blocks in flight, so that this also holds for the first
+// token of a block, cost two more barriers a call: against three, 16 tokens took 9..12 % longer, 64 3..6 %, 512 0..3 %, in fp32 1 % less.)
 // What bounds it: the instructions of four warps, one a scheduler (about 190 a token and warp at 2.2 cycles; two tokens a step, with
 // half the chain and as many instructions, took as long), and the shared-memory pipe, which hands a warp its 16-byte operand pieces
 // at four cycles each whoever shares them: two rows a thread on twice the warps are 30 % slower.  A partial sum is one chain of
-// four packed steps and one add (two chains and three adds: 5 % slower).  120 CTAs x 512 tokens 128.5 -> 120.3 us (235 ns a token).
+// four packed steps and one add (two chains and three adds: 5 % slower).  120 CTAs x 512 tokens 126.7 -> 115.7 us (226 ns a token).
 template <typename T, bool PREP, int CTAS>
 __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs p) {
     constexpr int R = kFewRows, G = kFewLanes, NT = kSN / R * G;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
                 S[i][2 * j] = pack2(x[0], x[1]);
                 S[i][2 * j + 1] = pack2(x[2], x[3]);
             }
-        float y[R] = {};
+        float y[R];
         auto dot = [&](float (&out)[R], const f2 (&x)[4]) {
 #pragma unroll
             for (int i = 0; i < R; ++i) {
@@ -284,26 +284,26 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
             y1 += y1q;
             y1q = xchg(y1, 1);
         };
-        auto token = [&](float* yprev, const TokenRegs& o) {  // `yprev`: where the output of the token before goes
+        auto token = [&](Operands& op, int t, bool prev, const TokenRegs& o) {
             float sa[R], q[R];
             dot(sa, o.kk);
 #pragma unroll
             for (int i = 0; i < R; ++i) q[i] = xchg(sa[i], 4);
-            y_step4();
+            if (prev) y_step4();
             decay_rows(0, o);
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 sa[i] += q[i];
                 q[i] = xchg(sa[i], 2);
             }
-            y_step2();
+            if (prev) y_step2();
             decay_rows(R / 2, o);
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 sa[i] += q[i];
                 q[i] = xchg(sa[i], 1);
             }
-            y_step1();
+            if (prev) y_step1();
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 sa[i] += q[i];
@@ -311,41 +311,38 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
 #pragma unroll
                 for (int j = 0; j < 4; ++j) S[i][j] = fma2(s2, o.nb[j], S[i][j]);
             }
-            if (ystore) yprev[yrow] = y1 + y1q;
+            if (prev && ystore) op.y[t - 1][yrow] = y1 + y1q;
             dot(y, o.r);
         };
-        TokenRegs o[CTAS == 1 ? 2 : 1];
-        for (int it = -2; it <= nblocks + 1; ++it) {
+        for (int it = -1; it <= nblocks; ++it) {
             if (it >= 0 && it < nblocks) {
                 Operands& op = ops[it % kFewBlocks];
-                const Operands& next = ops[(it + 1) % kFewBlocks];  // its operands are there since the last barrier; past the end: nobody's
-                float* y0 = it > 0 ? ops[(it - 1) % kFewBlocks].y[kTS - 1] : op.y[0];  // of the block before; first: overwritten by the next token
                 const int nt = min(kTS, T_ - it * kTS);
-                if (it == 0) load_token(o[0], op, 0, row0, cg);
                 if (nt == kTS) {
+                    TokenRegs o[CTAS == 1 ? 2 : 1];
+                    load_token(o[0], op, 0, row0, cg);
 #pragma unroll
                     for (int t = 0; t < kTS; ++t) {
-                        const Operands& from = t + 1 < kTS ? op : next;
                         if constexpr (CTAS == 1) {  // the next token's operands a token ahead
-                            load_token(o[(t + 1) & 1], from, (t + 1) % kTS, row0, cg);
-                            token(t > 0 ? op.y[t - 1] : y0, o[t & 1]);
+                            if (t + 1 < kTS) load_token(o[(t + 1) & 1], op, t + 1, row0, cg);
+                            token(op, t, t > 0, o[t & 1]);
                         } else {  // two CTAs an SM: no registers for that, and less need
-                            token(t > 0 ? op.y[t - 1] : y0, o[0]);
-                            load_token(o[0], from, (t + 1) % kTS, row0, cg);
+                            token(op, t, t > 0, o[0]);
+                            if (t + 1 < kTS) load_token(o[0], op, t + 1, row0, cg);
                         }
                     }
                 } else {
 #pragma unroll 1
                     for (int t = 0; t < nt; ++t) {
-                        load_token(o[0], op, t, row0, cg);
-                        token(t > 0 ? op.y[t - 1] : y0, o[0]);
+                        TokenRegs o;
+                        load_token(o, op, t, row0, cg);
+                        token(op, t, t > 0, o);
                     }
                 }
-            } else if (it == nblocks) {
                 y_step4();
                 y_step2();
                 y_step1();
-                if (ystore) ops[(it - 1) % kFewBlocks].y[T_ - 1 - (it - 1) * kTS][yrow] = y1 + y1q;
+                if (ystore) op.y[nt - 1][yrow] = y1 + y1q;
             }
             __syncthreads();
         }
@@ -396,8 +393,8 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
         fetch(0);
         announce(1);
         announce(2);
-        for (int it = -2; it <= nblocks + 1; ++it) {
-            const int s = it + 2;
+        for (int it = -1; it <= nblocks; ++it) {
+            const int s = it + 1;
             if (s < nblocks) {
                 Operands& op = ops[s % kFewBlocks];
 #pragma unroll
@@ -451,8 +448,8 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
             load_param(p.gn_w, gw);
             load_param(p.gn_b, gb);
         }
-        for (int it = -2; it <= nblocks + 1; ++it) {
-            const int s = it - 2;
+        for (int it = -1; it <= nblocks; ++it) {
+            const int s = it - 1;
             if (s >= 0) {
                 const Operands& op = ops[s % kFewBlocks];
                 const int t = s * kTS + tt;
@@ -478,8 +475,8 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
                 if (live) store8(reinterpret_cast<T*>(p.y) + base + (size_t)t * tok_stride + c, y);
             }
             if constexpr (PREP) {  // the gate of the block that is written next
-                const int t = (s + 1) * kTS + tt;
-                if (s >= -1 && t < T_) {
+                const int t = it * kTS + tt;
+                if (it >= 0 && t < T_) {
                     const T* q = reinterpret_cast<const T*>(p.g) + base + (size_t)t * tok_stride + c;
                     reinterpret_cast<uint4*>(&g)[0] = reinterpret_cast<const uint4*>(q)[0];
                     if constexpr (sizeof(T) == 4) reinterpret_cast<uint4*>(&g)[1] = reinterpret_cast<const uint4*>(q)[1];
@@ -662,8 +659,8 @@ template <typename T, bool PREP>
 static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     // Chosen by how many CTAs an SM gets.  Up to one, and up to two (with fewer registers a thread): the form with loads, output
     // and recurrence on warps of their own.  More: the CTAs of an SM hide each other's loads and the extra warps only take
-    // registers.  us for 512 tokens, fp16, output prepared, by CTAs, before -> now: 12 120 -> 115, 148 131 -> 121, 149 196 -> 189,
-    // 296 200 -> 192.  320: 405, where the form for fewer takes two waves (438).
+    // registers.  us for 512 tokens, fp16, output prepared, by CTAs, before -> now: 12 126 -> 115, 148 129 -> 116, 149 193 -> 186,
+    // 296 194 -> 186; for 16 tokens 7.4 -> 7.2, 7.7 -> 7.6, 9.4 -> 9.2, 10.0 -> 9.8.  320: 405, where the form for fewer takes two waves (438).
     const int ctas = B * p.H;
     const bool few = ctas <= 2 * kSMs;
     void (*kern)(const ScanArgs) = ctas <= kSMs ? wkv7_scan_few_kernel<T, PREP, 1> : few ? wkv7_scan_few_kernel<T, PREP, 2> : wkv7_scan_kernel<T, PREP, 2, 32>;
