@@ -19,9 +19,10 @@ namespace rwkv7 {
 // slow unit), of 4096 13.2 (19.0); bf16 53 (93) and 16.9 (19.2), fp32 56 (81) and 16.6 (18.2).
 
 // bf16 rows hold few distinct quotients, which tie in some rows for many elements, and a warp with one tie forms 32
-// quotients after all: below this many rows (few CTAs an SM) bf16 divides without asking.  64 rows of 16384: 11.0 us with the
-// product, 6.9 without; 256 of 10240: 9.0 either way; 511 of 16384: 13.6 with it, 17.2 without.
-constexpr int kA8RecipRows = 256;
+// quotients after all: up to this many rows (two CTAs an SM, and the slowest of them decides) bf16 divides without asking.  us, with
+// the product / without: 256 x 2560 3.5 / 3.1, 296 x 10240 6.9 / 6.1, 296 x 16384 9.5 / 8.5; 297 x 10240 7.0 / 7.6, 297 x 16384 9.6 / 11.2, 511 x 16384
+// 12.0 / 14.8; rows of 768 are level or 2..7 % the other way up to 511.
+constexpr int kA8DivideRows = 2 * 148;
 
 __device__ __forceinline__ float quant_quotient(float v, float s) {
     const float t = __fdiv_rn(v, s);
@@ -318,7 +319,7 @@ extern "C" int rwkv7_a8_quant(const void* x, int8_t* q, float* scale, int rows, 
         auto launch = [&](auto kern) { kern<<<rows, 256, 0, st>>>(reinterpret_cast<const T*>(x), q, scale, K); };
         const bool two = K <= 2 * 256 * 8;
         if constexpr (sizeof(T) == 2 && !std::is_same<T, __half>::value) {
-            if (rows < kA8RecipRows) {
+            if (rows <= kA8DivideRows) {
                 two ? launch(a8_quant_kernel<T, 2, false>) : launch(a8_quant_kernel<T, 8, false>);
                 return check_launch("a8_quant_kernel");
             }

@@ -78,6 +78,13 @@ def test_a8_quantiser_of_every_type(dt, rows, K):
     assert torch.equal(scale.cpu().reshape(-1), s) and torch.equal(q.cpu(), want)
 
 
+@pytest.mark.parametrize("rows", [296, 297])
+@pytest.mark.parametrize("K", [264, 4104])
+def test_a8_quantiser_either_side_of_its_rule_on_rows(rows, K):
+    """Up to two CTAs an SM bf16 divides, above it multiplies and divides where that could round the other way: the same bytes."""
+    test_a8_quantiser_of_every_type(torch.bfloat16, rows, K)
+
+
 @pytest.mark.parametrize("M,K,Nn", [(1, 16, 8), (17, 64, 24), (64, 256, 96), (130, 4096, 136), (256, 512, 256), (384, 1024, 512)])
 def test_int8_gemm_bit_exact(M, K, Nn):
     rng = np.random.default_rng(M * 7 + Nn)
