@@ -530,10 +530,15 @@ extern "C" int rwkv7_seq_norm_mix(const void* x, const void* norm_w, const void*
     RWKV7_DISPATCH_DTYPE(dtype, TT, {
         const bool wide = D > 8 * kSeqThreads;
         const int threads = wide ? kSeqThreads : (D / 8 + 31) / 32 * 32, per_sm = 65536 / (64 * threads);
-        // Two tokens a CTA where one each would not all be resident.  Below that they only halve the CTAs (300 x 2560, six / one mix 4.9 / 3.8 ->
-        // 5.6 / 3.8); with six mixes the stores weigh more, in fp32 from two waves on (777 x 2560 16.6 -> 17.7, 2331 x 2560 40.3 -> 38.6), and at
-        // two CTAs an SM not at all (768 x 4096 12.5 -> 13.6, 2048 x 3072 22.5 -> 23.2).
-        const bool two = !wide && T > 1 && (n_mix == 1 || per_sm >= 3) && (long long)B * T > 148ll * per_sm * (n_mix == 6 && sizeof(TT) == 4 ? 2 : 1);
+        // Two tokens a CTA where one each would not all be resident (below that they only halve the CTAs), by waves of CTAs that one token each
+        // would make.  One mix: from the first full wave on at 0.74..0.96 of the time.  Six, whose stores weigh more: where half the CTAs do
+        // not start a nearly empty wave of their own, at three CTAs an SM and more.  Time of two tokens over one, fp16 / bf16 / fp32, 512..2560 wide: 1.05
+        // waves 0.80..1.07 / 0.81..0.85 / 0.89..1.08, 1.4 to 2 0.79..0.92 / 0.80..0.90 / 0.96..1.13, 2.05 to 2.6 0.99..1.12 / 0.93..1.06 / 1.00..1.16, 3.05 to 3.6
+        // 0.90..0.99 / 0.87..0.94 / 0.94..1.06, 4.1 to 6 0.83..0.95 / 0.83..0.90 / 0.91..1.01, 16 0.79..0.86.  At two CTAs an SM 768 x 4096 12.5 -> 13.6 us.
+        // Sequences of 3 and 5, whose last CTA has one token: one mix, 400 x 3 x 4096 11.9 -> 12.7, 300 x 5 x 3072 11.6 -> 12.0.
+        const long long tokens = (long long)B * T, wave = 148ll * per_sm;
+        const bool even = sizeof(TT) == 4 ? tokens > 4 * wave : (4 * tokens > 5 * wave && tokens <= 2 * wave) || tokens > 3 * wave;
+        const bool two = !wide && T > 1 && T != 3 && T != 5 && (n_mix == 1 ? tokens > wave : per_sm >= 3 && even);
         auto kern = wide  ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 2, 1> : seq_norm_mix_kernel<TT, 1, 2, 1>)
                     : two ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 1, 2> : seq_norm_mix_kernel<TT, 1, 1, 2>)
                           : (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 1, 1> : seq_norm_mix_kernel<TT, 1, 1, 1>);

@@ -21,11 +21,11 @@ def _one_norm_mix(rows: int, width: int, dtype) -> bool:
 
 
 def _one_kernel(rows: int, tokens: int, width: int, dtype, mixes: int) -> bool:
-    """``_one_norm_mix``, or a form in which a CTA takes two tokens of a sequence and reads three rows for them: one kernel at any size."""
+    """``_one_norm_mix``, or a form in which a CTA takes two tokens of a sequence (not of 3 or 5) and reads three rows for them: one kernel at any size."""
     # us, two kernels -> that.  One mix, up to 4096 wide: fp16 2331 x 2560 14.0 -> 10.9, 768 x 4096 8.7 -> 7.3, 32768 x 4096 261 -> 210, bf16 289 -> 219, fp32
     # 393 -> 285.  Six, up to 2560 wide: fp16 2331 x 2560 22.8 -> 17.6, 16384 x 2560 157 -> 108, bf16 169 -> 112, fp32 361 -> 210.  Wider, six mixes keep to one
     # token a CTA (32768 x 4096 in fp16 would be 460 -> 416 so, 1554 x 4096 23.2 -> 25.2, bf16 8192 x 3072 98 -> 105).
-    return (tokens > 1 and width <= (4096 if mixes == 1 else 2560)) or _one_norm_mix(rows, width, dtype)
+    return (tokens not in (1, 3, 5) and width <= (4096 if mixes == 1 else 2560)) or _one_norm_mix(rows, width, dtype)
 
 
 def _rows(x, name):

@@ -442,6 +442,15 @@ def test_sequence_norm_mix_of_two_tokens_a_cta(dt, B, T, D, piece):
 
 
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,T,D,piece", [(1, 555, 2560, 222), (1, 556, 2560, 139), (1, 888, 2560, 222), (1, 889, 2560, 127), (1, 1333, 2560, 333), (1, 1777, 2560, 355),
+                                         (149, 3, 2560, 1), (112, 5, 2560, 3), (280, 3, 4096, 1)])
+def test_sequence_norm_mix_either_side_of_its_waves(dt, B, T, D, piece):
+    """Six mixes in two tokens a CTA from 1.25 waves to two and from three on (fp32: four); sequences of 3 and 5, one token a CTA or two
+    kernels: the bits of short calls that carry the state, as in the test above."""
+    test_sequence_norm_mix_of_two_tokens_a_cta(dt, B, T, D, piece)
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,Hh", [(1, 1), (33, 1), (4095, 3), (12287, 1), (12288, 1), (4099, 3)])
 def test_state_prep_either_side_of_its_two_forms(dt, rows, Hh):
     """8- and 16-byte pieces a lane (they change at 12288 heads) against 64 bits.  Each result is rounded once from fp32 arithmetic of a
