@@ -342,9 +342,9 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                     uint4 pk[4];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * CHUNK);
-                    const uint32_t s16 = *reinterpret_cast<const unsigned short*>(piece + scale_off(row & 15));
-                    const uint32_t z = piece[zero_off(row & 15)];
-                    const uint32_t sc = s16 * 0x00010001u;               // (scale, scale)
+                    const uint2 sz = *reinterpret_cast<const uint2*>(piece + SC_OFF + (row & 7) * 8);  // of channels c and c + 8
+                    const uint32_t z = (sz.y >> (row & 8)) & 255u;
+                    const uint32_t sc = __byte_perm(sz.x, 0, row & 8 ? 0x3232 : 0x1010);  // (scale, scale)
                     const uint32_t zlo = z * 0x00010001u + 0x64006400u;  // 1024 + z as fp16: 0x6400 | z
                     const uint32_t zhi = z * 0x00100010u + 0xD400D400u;  // -(64 + z) as fp16: 0xD400 | (z << 4)
                     __syncwarp();
