@@ -200,7 +200,7 @@ def _rows_operand(op, x):
     """``(fmt, weight, scale, out_features)`` when the projection ``op`` of the few rows ``x`` runs on the row kernel."""
     if isinstance(op, _q.MM4Linear) or (isinstance(op, _q.MM8Linear) and op.sm7x_rowwise):
         ok = (op.bias is None and x.is_contiguous() and int(x.shape[-1]) == op.in_features
-              and _q.few_rows_quant(int(x.shape[0]), op.in_features, op.out_features))
+              and _q.few_rows_quant(int(x.shape[0]), op.in_features, op.out_features, 4 if isinstance(op, _q.MM4Linear) else 8))
         tiled = op.tiled_for(x) if ok else None
         if tiled is None:
             return None

@@ -108,22 +108,29 @@ def w4_repack_tiled(q, scales, in_features, group_size=128, zeros=None):
     return tiled
 
 
-def few_rows_quant(rows: int, in_features: int, out_features: int) -> bool:
+def few_rows_quant(rows: int, in_features: int, out_features: int, bits: int = 4) -> bool:
     """Whether a tiled int4 / int8 projection of ``rows`` activation rows runs on the row kernel (csrc/row_gemv.cu) and not on
     the tcgen05 one.  At 8 rows the activations weigh as much as the weights of a long row, and few channels with a long row
-    leave SMs idle.  Time of the row kernel over the other's, int4 / int8, by rows:
+    leave SMs idle.
 
-        4096 -> 4096    1 0.91 / 1.00   4 0.68 / 0.74   8 0.98 / 0.97
-        2560 -> 10240   1 0.73 / 0.72   5 0.77 / 0.81   8 0.87 / 0.80
-        4096 -> 16384   1 0.72 / 0.77   5 0.75 / 0.78   8 0.83 / 0.83
-        7168 -> 4096    1 1.01 / 0.75   5 1.01 / 0.99   8 0.96 / 1.04
-        8192 -> 8192    1 0.69 / 0.74   7 0.91 / 0.85   8 1.10 / 1.07
-        10240 -> 2560   1 0.97 / 0.97   5 1.06 / 1.03   6 0.99 / 0.92   8 1.16 / 1.07
-        12288 -> 8192   1 0.87 / 0.85   5 0.85 / 0.84   6 1.10 / 1.08   8 1.13 / 1.08
-        16384 -> 4096   1 0.80 / 0.78   3 1.00 / 0.96   4 1.05 / 1.07   8 1.13 / 1.11
-        8192 -> 1024    1 1.23 / 1.26   8 1.12 / 1.09
-        12288 -> 1024   1 1.34 / 1.35   8 1.26 / 1.25"""
+    us of a launch, row kernel minus the other, int4 / int8 by rows, in captured decode steps that differ in that projection alone and are
+    replayed in turn (spread 0.1; the same kernels behind one another, without a step around them, differ by up to 2 us from row to
+    row, and a product of a weight that was just tiled waits for it, so it is no measure):
+
+        2560 -> 2560    1 -1.0 / -0.6   2 -1.6 / -0.8   3 -1.3 / -1.0   4 -1.1 / -0.9   6 -1.2 / -1.5   8 -1.2 / -1.7
+        2560 -> 10240   1 -3.8 / -3.2   2 -3.0 / -2.7   3 -3.0 / -2.8   4 -2.8 / -2.6   6 -2.1 / -1.9   8 -1.6 / -1.6
+        10240 -> 2560   1 -0.8 / -1.3   2 -0.1 / -1.1   3 -0.1 / -0.7   4 +0.3 / +0.5   5 +0.7 / -0.5   6 +0.9 / -0.1   8 +1.3 / +1.1
+        4096 -> 4096    1 -1.1 / -1.3   2 -1.4 / -1.2   3 -3.3 / -1.0   4 -1.7 / -1.1   6 -1.0 / -0.5   8 -0.6 / -0.6
+        4096 -> 16384   1 -5.1 / -5.5   2 -5.1 / -5.4   3 -4.3 / -4.9   4 -3.8 / -4.1   6 -3.8 / -3.9   8 -3.1 / -3.4
+        16384 -> 4096   1 -3.1 / -4.4   2 -3.2 / -1.4   3 -0.7 / -2.0   4 +0.8 / +0.5   6 +1.7 / +0.5   8 +2.5 / +0.8
+
+    Other shapes, time over the other's behind a norm kernel: 7168 -> 4096 0.81..1.02 / 0.79..1.00 up to 7 rows, 1.11 / 1.05 at 8 (0.99 on
+    another run); 8192 -> 8192 0.7..0.9 up to 7, 1.12 / 1.10 at 8; 8192 -> 4096 0.8..1.07 / 0.8..1.0 up to 7; 12288 -> 8192 0.75..0.90 / 0.79..0.84 up to 5,
+    1.10 / 1.08 at 6; 12288 -> 4096 0.92..1.06 / 0.84..1.03 up to 5; 12288 -> 2048, where the other runs clusters of eight, 0.6; 8192 -> 1024 1.02..1.07 /
+    1.07..1.12; 12288 -> 1024 1.13..1.20 / 1.19..1.23."""
     most = 8 if in_features <= 7168 else 7 if in_features <= 8192 else 5 if in_features <= 12288 else 3
+    if bits == 4 and in_features > 8192 and in_features >= 4 * out_features > 8192:
+        most = 3
     return 1 <= rows <= min(most, _rowsk.MAX_ROWS) and in_features < 8 * out_features
 
 
@@ -199,7 +206,7 @@ def w8_tiled_linear_group(xs, tileds, scales, out_features, in_features, *, relu
     if (res is not None or out is not None) and G != 1:
         raise ValueError("residual / out apply to a single projection")
     ys = [torch.empty((M, Nout), device=x2[0].device, dtype=x2[0].dtype) if out is None else out.reshape(M, Nout) for _ in range(G)]
-    if few_rows_quant(M, K, Nout) and x2[0].dtype == torch.float16 and all(t.is_contiguous() for t in x2):
+    if few_rows_quant(M, K, Nout, 8) and x2[0].dtype == torch.float16 and all(t.is_contiguous() for t in x2):
         _rowsk.rows_gemv(x2, tileds, out_features=[Nout] * G, fmts=[_rowsk.INT8] * G, scales=sc, residuals=[res] * G, outs=ys,
                          epilogues=[epi] * G, static_weights=True)
         return [y.reshape(*x.shape[:-1], Nout) for y, x in zip(ys, xs)]

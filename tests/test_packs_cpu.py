@@ -32,3 +32,10 @@ def test_quantised_products_on_the_row_kernel():
     for K, N, most in [(128, 24, 8), (128, 16, 0), (7168, 4096, 8), (7296, 4096, 7), (8192, 1032, 7), (8320, 8192, 5), (12288, 8192, 5), (12416, 8192, 3),
                        (16384, 4096, 3), (12288, 1024, 0)]:
         assert [m for m in range(10) if few_rows_quant(m, K, N)] == list(range(1, most + 1))
+
+
+def test_quantised_products_of_few_channels_on_the_row_kernel():
+    from hf_adapter_b200.quant import few_rows_quant
+    for K, N, bits, most in [(10240, 2560, 4, 3), (10240, 2560, 8, 5), (10240, 2568, 4, 5), (8192, 2056, 4, 7), (8200, 2056, 4, 5), (8320, 2064, 4, 3),
+                             (8320, 2048, 4, 5), (12288, 2048, 4, 5), (16384, 4096, 8, 3)]:
+        assert [m for m in range(10) if few_rows_quant(m, K, N, bits)] == list(range(1, most + 1)), (K, N, bits)
