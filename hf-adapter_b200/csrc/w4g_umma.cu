@@ -333,6 +333,14 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
             // one lane per warp polls; the others wait at the shuffle
             if (lane == 0 && ok) ok = mbar_wait(&wfull[aa], (i / NA) & 1, actx, kErrWaitFull);
             ok = __shfl_sync(0xffffffffu, ok, 0);
+            __syncwarp();  // what lane 0 saw land, the others see (a shuffle does not order memory)
+            // The warp gives the stage back once its loads have RETURNED, in every lane: loads that are still on their way when it arrives
+            // can meet the next copy into the stage, which the async proxy does not order behind them (seen: a step of 128 rows in 700 had a
+            // few channels of one k-block from the block that took its stage).  `seen` has a bit of every load, the vote needs it of every
+            // lane, and its result is the lane that arrives.  (A proxy fence by every lane would do, for 5..14 % of a launch of up to 64 rows.)
+            const auto release = [&](uint32_t seen) {
+                if (lane == (int)(__ballot_sync(0xffffffffu, seen & 1u) & 31u)) mbar_arrive(&wempty[aa]);
+            };
             uint32_t v[4][16];
             if (ok) {
                 // this channel's 64 packed bytes: a chunk (32 k) of 16 channels is one 256-byte slab, so eight threads of a
@@ -347,8 +355,7 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                     const uint32_t sc = __byte_perm(sz.x, 0, row & 8 ? 0x3232 : 0x1010);  // (scale, scale)
                     const uint32_t zlo = z * 0x00010001u + 0x64006400u;  // 1024 + z as fp16: 0x6400 | z
                     const uint32_t zhi = z * 0x00100010u + 0xD400D400u;  // -(64 + z) as fp16: 0xD400 | (z << 4)
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&wempty[aa]);
+                    release(pk[0].x ^ pk[1].x ^ pk[2].x ^ pk[3].x ^ sz.x);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         dequant_word(pk[c].x, zlo, zhi, sc, v[c] + 0);
@@ -361,8 +368,7 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                     uint4 pk[8];
 #pragma unroll
                     for (int c = 0; c < 8; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * CHUNK);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&wempty[aa]);
+                    release(pk[0].x ^ pk[1].x ^ pk[2].x ^ pk[3].x ^ pk[4].x ^ pk[5].x ^ pk[6].x ^ pk[7].x);
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         uint32_t* o = v[c >> 1] + (c & 1) * 8;
