@@ -179,10 +179,27 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
 
     // ---- the vectors of the head, two channels a lane, one warp each; shared.  (Formed by every row group for itself they were
     // two thirds of the kernel's instructions.)
-    const float2 r = cvt2(ld_raw2<T>(p.r, vbase + c2));
+    float2 r{};
+    if constexpr (MODE != kUpdate) r = cvt2(ld_raw2<T>(p.r, vbase + c2));
     auto put = [&](float* s, float x, float y) { *reinterpret_cast<float2*>(s + c2) = make_float2(x, y); };
     Raw2<T> q_gw{}, q_gb{}, q_g{};
-    if (warp == 0) {
+    // The plain update has nothing to make of them: every lane takes its four columns from the operands.  (Through shared memory a
+    // grid of more than eight CTAs an SM took longer than before: 22 rows of 64 heads 8.7 -> 9.5 us, so 8.3; 48 rows into a new state 13.6 -> 15.1, so 12.8.)
+    float4 w4, k4, kk4, kka4, r4;
+    if constexpr (MODE == kUpdate) {
+        auto vec4 = [&](auto tag, const void* base) {
+            float x[4];
+            load4(reinterpret_cast<const decltype(tag)*>(base) + vbase + c0, x);
+            return make_float4(x[0], x[1], x[2], x[3]);
+        };
+        if (tid < kN) s_v[tid] = to_f<T>(reinterpret_cast<const T*>(p.v)[vbase + tid]);
+        kk4 = vec4(T{}, p.kk);
+        w4 = vec4(TW{}, p.w);
+        k4 = vec4(T{}, p.k);
+        const float4 a4 = vec4(T{}, p.a);
+        r4 = vec4(T{}, p.r);
+        kka4 = make_float4(kk4.x * a4.x, kk4.y * a4.y, kk4.z * a4.z, kk4.w * a4.w);
+    } else if (warp == 0) {
         float2 w;
         if constexpr (MODE == kRaw) {
             const Raw2<T> q_w = ld_raw2<T>(p.w, vbase + c2), q_wb = ld_raw2<T>(p.w_bias, hbase + c2, p.w_bias != nullptr);
@@ -232,20 +249,16 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
         put(s_k, k.x, k.y);
         put(s_kk, kk.x, kk.y);
         put(s_kka, kk.x * a.x, kk.y * a.y);
-        if constexpr (MODE != kUpdate) {
-            const float2 rk = cvt2(ld_raw2<T>(p.r_k, hbase + c2));
-            const float corr = group_sum<32>(r.x * k.x * rk.x + r.y * k.y * rk.y);
-            if (lane == 0) s_corr = corr;
-        }
+        const float2 rk = cvt2(ld_raw2<T>(p.r_k, hbase + c2));
+        const float corr = group_sum<32>(r.x * k.x * rk.x + r.y * k.y * rk.y);
+        if (lane == 0) s_corr = corr;
     } else if (warp == 2) {
         // ---- row-indexed value vector (with the optional v_first interpolation); this warp also makes the output
         const bool interp = MODE == kRaw && p.v_first != nullptr && p.v_gate != nullptr;
         const Raw2<T> q_v = ld_raw2<T>(p.v, vbase + c2);
-        if constexpr (MODE != kUpdate) {
-            q_gw = ld_raw2<T>(p.gn_w, hbase + c2);
-            q_gb = ld_raw2<T>(p.gn_b, hbase + c2);
-            q_g = ld_raw2<T>(p.g, vbase + c2);
-        }
+        q_gw = ld_raw2<T>(p.gn_w, hbase + c2);
+        q_gb = ld_raw2<T>(p.gn_b, hbase + c2);
+        q_g = ld_raw2<T>(p.g, vbase + c2);
         float2 v = cvt2(q_v);
         if constexpr (MODE == kRaw) {
             if (interp) {
@@ -270,14 +283,20 @@ __global__ void __launch_bounds__(kStepThreads, 8) wkv7_step_kernel(const StepAr
     {
         auto four = [&](const float* s) { return *reinterpret_cast<const float4*>(s + c0); };
         float sa[8], y[8];
-        const float4 kk = four(s_kk);
+        const float4 kk = MODE == kUpdate ? kk4 : four(s_kk);
 #pragma unroll
         for (int it = 0; it < 8; ++it) {
             const float4 s = StateIO<TS>::value(S[it]);
             sa[it] = s.x * kk.x + s.y * kk.y + s.z * kk.z + s.w * kk.w;
         }
         const float mine = sum_rows(sa, l16);
-        const float4 w = four(s_w), k = four(s_k), kka = four(s_kka), r4 = four(s_r);
+        float4 w = w4, k = k4, kka = kka4;
+        if constexpr (MODE != kUpdate) {
+            w = four(s_w);
+            k = four(s_k);
+            kka = four(s_kka);
+            r4 = four(s_r);
+        }
 #pragma unroll
         for (int it = 0; it < 8; ++it) {
             const int i = it * 8 + rg;
