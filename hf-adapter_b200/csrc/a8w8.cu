@@ -22,7 +22,7 @@ namespace rwkv7 {
 // quotients after all: up to this many rows (two CTAs an SM, and the slowest of them decides) bf16 divides without asking.  us, with
 // the product / without: 256 x 2560 3.5 / 3.1, 296 x 10240 6.9 / 6.1, 296 x 16384 9.5 / 8.5; 297 x 10240 7.0 / 7.6, 297 x 16384 9.6 / 11.2, 511 x 16384
 // 12.0 / 14.8; rows of 768 are level or 2..7 % the other way up to 511.
-constexpr int kA8DivideRows = 2 * 148;
+constexpr int kA8DivideRows = 2 * kSMs;
 
 __device__ __forceinline__ float quant_quotient(float v, float s) {
     const float t = __fdiv_rn(v, s);
@@ -347,7 +347,7 @@ static int a8w8_dequant_impl(const int32_t* acc, const float* sa, const float* s
     RWKV7_REQUIRE(acc && sa && sw && out, RWKV7_ERR_INVALID, "a8w8_dequant: null pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long total = (long long)M * Nout;
-    const int grid = (int)((total + 255) / 256 < 148LL * 16 ? (total + 255) / 256 : 148LL * 16);
+    const int grid = (int)((total + 255) / 256 < (long long)kSMs * 16 ? (total + 255) / 256 : (long long)kSMs * 16);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
         a8w8_dequant_kernel<T><<<grid, 256, 0, st>>>(acc, sa, sw, reinterpret_cast<const T*>(bias),
                                                     reinterpret_cast<const T*>(residual), reinterpret_cast<T*>(out), M, Nout, relu2);

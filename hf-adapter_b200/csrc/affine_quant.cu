@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) affine_dequant_kernel(const uint8_t* __re
 
 static int affine_splits(int K, int Nout) {
     const int tiles = (Nout + kAffTileN - 1) / kAffTileN;
-    int S = (148 * 2 + tiles - 1) / tiles;
+    int S = (kSMs * 2 + tiles - 1) / tiles;
     if (S > 32) S = 32;
     while (S > 1 && K / S < 64) --S;
     return S < 1 ? 1 : S;
@@ -195,7 +195,7 @@ extern "C" int rwkv7_affine_dequant(const uint8_t* q, const void* mx, const void
     RWKV7_REQUIRE(q && mx && rx && my && ry && W, RWKV7_ERR_INVALID, "affine_dequant: null pointer");
     const int row_bytes = bits == 8 ? Nout : (Nout + 1) / 2;
     const long long total = (long long)K * ((Nout + 7) / 8);
-    const int grid = (int)((total + 255) / 256 < 148LL * 32 ? (total + 255) / 256 : 148LL * 32);
+    const int grid = (int)((total + 255) / 256 < (long long)kSMs * 32 ? (total + 255) / 256 : (long long)kSMs * 32);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
         if (bits == 8)

@@ -17,6 +17,8 @@
 
 namespace rwkv7 {
 
+constexpr int kSMs = 148;  // B200
+
 // ---- error plumbing -------------------------------------------------------
 void set_error(const char* fmt, ...);  // defined in capi.cu (thread-local buffer)
 constexpr int kMaxDevices = 64;        // device indices the per-device address caches cover

@@ -273,7 +273,7 @@ static int small_gemm_group(int n_problems, const void* const* x, const void* co
     // four downs of a layer (ranks 64, 64, 128, 32; fp16): 2560 wide 2331 rows 33.9 / 35.1 / 35.6, 4096 rows 36.1 / 44.1 / 51.0, 6000 54.8 / 45.8 / 54.6,
     // 12000 85.4 / 74.8 / 92.0; 4096 wide 4096 rows 50.6 / 63.6 / 75.0, 6000 79.3 / 65.8 / 81.8, 12000 125.4 / 102.2 / 134.6; 768 wide 6000 24.3 / 20.7 / 21.7,
     // 12000 38.1 / 33.4 / 33.0
-    const bool one_wave = tiles * row_blocks * splits <= 3 * 148;
+    const bool one_wave = tiles * row_blocks * splits <= 3 * kSMs;
     if (dtype == RWKV7_F16) e = !deep ? launch_group<__half, 2>(cfg, a) : one_wave ? launch_group<__half, 4>(cfg, a) : launch_group<__half, 3>(cfg, a);
     else e = !deep ? launch_group<__nv_bfloat16, 2>(cfg, a) : one_wave ? launch_group<__nv_bfloat16, 4>(cfg, a) : launch_group<__nv_bfloat16, 3>(cfg, a);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "small_gemm_group launch: %s", cudaGetErrorString(e));

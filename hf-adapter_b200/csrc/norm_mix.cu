@@ -536,7 +536,7 @@ extern "C" int rwkv7_seq_norm_mix(const void* x, const void* norm_w, const void*
         // waves 0.80..1.07 / 0.81..0.85 / 0.89..1.08, 1.4 to 2 0.79..0.92 / 0.80..0.90 / 0.96..1.13, 2.05 to 2.6 0.99..1.12 / 0.93..1.06 / 1.00..1.16, 3.05 to 3.6
         // 0.90..0.99 / 0.87..0.94 / 0.94..1.06, 4.1 to 6 0.83..0.95 / 0.83..0.90 / 0.91..1.01, 16 0.79..0.86.  At two CTAs an SM 768 x 4096 12.5 -> 13.6 us.
         // Sequences of 3 and 5, whose last CTA has one token: one mix, 400 x 3 x 4096 11.9 -> 12.7, 300 x 5 x 3072 11.6 -> 12.0.
-        const long long tokens = (long long)B * T, wave = 148ll * per_sm;
+        const long long tokens = (long long)B * T, wave = (long long)kSMs * per_sm;
         const bool even = sizeof(TT) == 4 ? tokens > 4 * wave : (4 * tokens > 5 * wave && tokens <= 2 * wave) || tokens > 3 * wave;
         const bool two = !wide && T > 1 && T != 3 && T != 5 && (n_mix == 1 ? tokens > wave : per_sm >= 3 && even);
         auto kern = wide  ? (n_mix == 6 ? seq_norm_mix_kernel<TT, 6, 2, 1> : seq_norm_mix_kernel<TT, 1, 2, 1>)
@@ -567,7 +567,7 @@ extern "C" int rwkv7_seq_shift_mix(const void* x, const void* initial_prev, cons
                   "seq_shift_mix: unaligned pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long blocks = (p.total_vec + 255) / 256;
-    const int grid = (int)(blocks < 148LL * 16 ? blocks : 148LL * 16);
+    const int grid = (int)(blocks < (long long)kSMs * 16 ? blocks : (long long)kSMs * 16);
     RWKV7_DISPATCH_DTYPE(dtype, TT, {
         seq_shift_mix_kernel<TT><<<grid, 256, 0, st>>>(p);
         return check_launch("seq_shift_mix_kernel");

@@ -268,7 +268,7 @@ extern "C" int rwkv7_relu2(const void* x, void* y, long long n, int dtype, void*
     RWKV7_REQUIRE(x && y, RWKV7_ERR_INVALID, "relu2: null pointer");
     RWKV7_REQUIRE(aligned(x, 16) && aligned(y, 16), RWKV7_ERR_ALIGN, "relu2: unaligned pointer");
     const long long nvec = n / 8;
-    const int grid = (int)((nvec + 255) / 256 < 148LL * 32 ? (nvec + 255) / 256 : 148LL * 32);
+    const int grid = (int)((nvec + 255) / 256 < (long long)kSMs * 32 ? (nvec + 255) / 256 : (long long)kSMs * 32);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RWKV7_DISPATCH_DTYPE(dtype, T, {
         relu2_kernel<T><<<grid, 256, 0, st>>>(reinterpret_cast<const T*>(x), reinterpret_cast<T*>(y), nvec);

@@ -341,7 +341,7 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
     };
     int warps = kWarps, ctas = deal(warps);
     bool halves = false;  // a warp has the K of two of eight, and leaves the partial sums of either
-    if (a.wk == kWarps && ctas > 2 * 148 && 2 * ((ctas + 4 * 148 - 1) / (4 * 148)) <= (ctas + 2 * 148 - 1) / (2 * 148)) {
+    if (a.wk == kWarps && ctas > 2 * kSMs && 2 * ((ctas + 4 * kSMs - 1) / (4 * kSMs)) <= (ctas + 2 * kSMs - 1) / (2 * kSMs)) {
         warps = a.wk = kWarps / 2;
         halves = true;
         ctas = deal(warps);
@@ -350,7 +350,7 @@ extern "C" int rwkv7_rows_gemv(int n_problems, const void* const* x, const void*
     // 2560 x 2560 5.7 / 4.0 / 4.3 -> 4.6 / 3.9 / 4.2 us, 10240 -> 2560 19.9 / 13.1 / 13.4 -> 13.1 / 8.9 / 9.7, 16384 -> 4096
     // 34.7 / 20.6 / 21.6 -> 25.0 / 14.2 / 16.0; beyond one CTA an SM pairs only add their exchange (4096 -> 16384 int4
     // 15.0 -> 19.9), and so do fours (16384 -> 4096 int4 18.5).
-    a.splits = ctas <= 148 && max_units >= 16 ? 2 : 1;
+    a.splits = ctas <= kSMs && max_units >= 16 ? 2 : 1;
     auto kern = dtype == RWKV7_F16 ? (halves ? rows_gemv_kernel<__half, true> : rows_gemv_kernel<__half, false>)
                                    : (halves ? rows_gemv_kernel<__nv_bfloat16, true> : rows_gemv_kernel<__nv_bfloat16, false>);
     cudaLaunchConfig_t cfg{};

@@ -651,7 +651,7 @@ static int rows_per_pass(int M, int tiles, int G, int total_kb, int splits128, i
     const auto cost = [&](int nb, int splits) {
         const long long ctas = (long long)tiles * ((M + nb - 1) / nb) * G * splits;
         const long long exchange = splits == 1 ? 450 : nb == 128 ? 1400 : 2200;
-        return (ctas + 147) / 148 * ((long long)(total_kb / splits) * (nb == 128 ? 105 : 164) + exchange);
+        return (ctas + kSMs - 1) / kSMs * ((long long)(total_kb / splits) * (nb == 128 ? 105 : 164) + exchange);
     };
     return cost(256, splits256) < cost(128, splits128) ? 256 : 128;
 }
@@ -667,7 +667,7 @@ int launch_w4g_umma_tiled(const void* const* xs, const uint8_t* const* tws, cons
     const int total_kb = K / KB;
     const auto splits_for = [&](int nb) {
         for (int s = 8; s >= 2; s >>= 1)
-            if ((long long)tiles * ((M + nb - 1) / nb) * G * s <= 148 && total_kb % s == 0 && total_kb / s >= 4) return s;
+            if ((long long)tiles * ((M + nb - 1) / nb) * G * s <= kSMs && total_kb % s == 0 && total_kb / s >= 4) return s;
         return 1;
     };
     const int NB = rows_per_pass(M, tiles, G, total_kb, splits_for(128), splits_for(256));

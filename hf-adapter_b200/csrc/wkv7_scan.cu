@@ -14,7 +14,6 @@ namespace rwkv7 {
 
 constexpr int kSN = 64;
 constexpr int kTS = 8;     // tokens per shared-memory block
-constexpr int kSMs = 148;  // B200
 
 struct ScanArgs {
     const void *r, *w, *k, *v, *kk, *a;

@@ -293,7 +293,8 @@ class RWKV7StatePool:
     def decode(self, token_ids, slot_ids, generations=None, *, use_graph: bool = True, greedy: bool = False):
         """One token for every scheduled request, state updated in place inside the pools.  Returns logits
         ``[len(slot_ids), V]`` (or the greedy tokens).  With ``use_graph`` the step replays a CUDA graph captured for the
-        next bucket size (1, 2, 4, ...); padding rows read and write the scratch slot only."""
+        next bucket size (1, 2, 4, ...); padding rows name the scratch slot: its shift states are
+        read and written, its recurrent state is left alone."""
         slots = self._check(slot_ids, generations)
         n = len(slots)
         ids = torch.as_tensor(token_ids, device=self.S_pool.device).reshape(-1)

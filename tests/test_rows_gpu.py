@@ -178,7 +178,7 @@ def test_prefill_lora_pairs(rows_, rank, dt, first):
 @pytest.mark.parametrize("N", [9472, 9504, 18944, 18976, 28448])
 @pytest.mark.parametrize("fmt", ["dense", "int8"])
 def test_either_side_of_the_wave_limits(N, fmt):
-    """CTAs of eight warps up to 296 tiles of 32 channels, of four up to 592 and from 889 on."""
+    """CTAs of eight warps up to 296 tiles of 32 channels, of four up to 592, of eight up to 888, of four up to 1184."""
     K, M = 512, 3
     g = torch.Generator(device="cuda").manual_seed(N)
     x = torch.randn(M, K, generator=g, device="cuda").half()
@@ -207,3 +207,30 @@ def test_short_problems_beside_one_of_many_waves(M):
         _close(y, (x.double() @ w.double().t()).float(), torch.float16)
         alone, = rows.rows_gemv((x,), (w,), out_features=(int(w.shape[0]),), fmts=(0,))
         _close(alone, y.float(), torch.float16)
+
+
+@pytest.mark.parametrize("M,epi", [(1, 0), (3, 1), (8, 2)])
+@pytest.mark.parametrize("N,fewer", [(9504, 9472), (37920, 37888), (47392, 47360)])
+@pytest.mark.parametrize("fmt", ["fp16", "bf16", "int4", "int8"])
+def test_ctas_of_four_warps_give_the_bits_of_eight(M, epi, N, fewer, fmt):
+    """Channels of a weight of N rows and of its first rows alone, either side of the limits at 296, 1184 and 1480 tiles: the same partial
+    sums in the same order, whatever the warps of a CTA.  11 quantised units of K and 22 dense ones, so that halves are odd."""
+    K = 1408
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    dt = torch.bfloat16 if fmt == "bf16" else torch.float16
+    x = torch.randn(M, K, generator=g, device="cuda").to(dt)
+    res = torch.randn(M, N, generator=g, device="cuda").to(dt) if epi == 2 else None
+    if fmt == "int4":
+        q = torch.randint(0, 256, (N, K // 2), generator=g, device="cuda", dtype=torch.uint8)
+        sc = (torch.rand(N, K // 128, generator=g, device="cuda") * 0.01).half()
+        weight, scale = (lambda n: hb.w4_repack_tiled(q[:n].contiguous(), sc[:n].contiguous(), K, 128)), None
+    elif fmt == "int8":
+        q = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+        weight, scale = (lambda n: hb.w8_repack_tiled(q[:n].contiguous())), (torch.rand(N, generator=g, device="cuda") * 0.01).half()
+    else:
+        w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(dt)
+        weight, scale = (lambda n: w[:n].contiguous()), None
+    outs = [rows.rows_gemv((x,), (weight(n),), out_features=(n,), fmts=({"int4": 1, "int8": 2}.get(fmt, 0),), epilogues=(epi,),
+                           scales=(None if scale is None else scale[:n].contiguous(),),
+                           residuals=(None if res is None else res[:, :n].contiguous(),))[0] for n in (N, fewer)]
+    assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0][:, :fewer], outs[1])
