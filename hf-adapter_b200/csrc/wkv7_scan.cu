@@ -208,11 +208,12 @@ template <typename T> __device__ __forceinline__ float2 to_f2(const Pair<T>& q) 
 // 4, 5 read a block of tokens ahead (in registers while the block before it runs) and convert it, warps 6, 7 write out the block that
 // is done.  In the token loop everything that does not wait for S.kk of this token sits in its shadow: the operands of the next
 // token, the decay and the v k^T term, the output sums of the token before.  (Five blocks in flight, so that this also holds for the first
-// token of a block, cost two more barriers a call: against three, 16 tokens took 9..12 % longer, 64 3..6 %, 512 0..3 %, in fp32 1 % less.)
+// token of a block, cost two more barriers a call.  Time of three over five: up to 8 tokens 0.89..0.98, 9 to 64 0.87..0.98, 72 to 192 0.96..1.01,
+// from 256 on 1.01..1.03 with the output prepared and one CTA an SM, 0.98..1.00 else.)
 // What bounds it: the instructions of four warps, one a scheduler (about 190 a token and warp at 2.2 cycles; two tokens a step, with
 // half the chain and as many instructions, took as long), and the shared-memory pipe, which hands a warp its 16-byte operand pieces
 // at four cycles each whoever shares them: two rows a thread on twice the warps are 30 % slower.  A partial sum is one chain of
-// four packed steps and one add (two chains and three adds: 5 % slower).  120 CTAs x 512 tokens 126.7 -> 115.7 us (226 ns a token).
+// four packed steps and one add (two chains and three adds: 5 % slower).  120 CTAs x 512 tokens 127.3 -> 116.0 us (227 ns a token).
 template <typename T, bool PREP, int CTAS>
 __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs p) {
     constexpr int R = kFewRows, G = kFewLanes, NT = kSN / R * G;
@@ -658,8 +659,8 @@ template <typename T, bool PREP>
 static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     // Chosen by how many CTAs an SM gets.  Up to one, and up to two (with fewer registers a thread): the form with loads, output
     // and recurrence on warps of their own.  More: the CTAs of an SM hide each other's loads and the extra warps only take
-    // registers.  us for 512 tokens, fp16, output prepared, by CTAs, before -> now: 12 126 -> 115, 148 129 -> 116, 149 193 -> 186,
-    // 296 194 -> 186; for 16 tokens 7.4 -> 7.2, 7.7 -> 7.6, 9.4 -> 9.2, 10.0 -> 9.8.  320: 405, where the form for fewer takes two waves (438).
+    // registers.  us for 512 tokens, fp16, output prepared, by CTAs, before -> now: 12 126 -> 115, 148 129 -> 117, 149 193 -> 185,
+    // 296 194 -> 185; for 16 tokens 7.2 -> 7.0, 7.7 -> 7.5, 9.4 -> 9.2, 9.8 -> 9.6.  320: 405, where the form for fewer takes two waves (438).
     const int ctas = B * p.H;
     const bool few = ctas <= 2 * kSMs;
     void (*kern)(const ScanArgs) = ctas <= kSMs ? wkv7_scan_few_kernel<T, PREP, 1> : few ? wkv7_scan_few_kernel<T, PREP, 2> : wkv7_scan_kernel<T, PREP, 2, 32>;
