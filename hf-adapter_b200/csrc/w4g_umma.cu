@@ -44,8 +44,8 @@
 //
 // Warps: 0 weight-stream producer, 1 activation producer + tensor-memory owner, 2..1+NISS issuers, then G dequant groups of
 // four warps (group g takes k-blocks g, g + G, ...).  NA = 2 G A buffers: a group waits for the MMAs of its block before
-// last, never for the previous one.  Weight ring: NA stages of one block (two per group, released as soon as the block is
-// in registers).  Weight stage, A buffer and "done" barrier of block i have index i mod NA and always belong to group
+// last, never for the previous one.  Weight ring: NA stages of one block (two per group, released once the block is in
+// tensor memory).  Weight stage, A buffer and "done" barrier of block i have index i mod NA and always belong to group
 // i mod G and issuer i mod NISS (NA is a multiple of both); its activation stage has index i mod XST, released by a barrier of its
 // own, or with XST = NA by the "done" barrier.  So every waiter sees every phase of the barriers it waits on (a waiter
 // that skips phases passes a parity wait one phase early).  G, NA, NISS, XST by rows a pass: Cfg below.  Above 64 rows the split-K
@@ -207,7 +207,7 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
     uint64_t* xfree = bars + XST;        // [XST] the MMAs that read the tile completed (unused when SHARED_DONE)
     uint64_t* done = xfree + XST;        // [NA]  the MMAs of the block completed: its A buffer is free
     uint64_t* wfull = done + NA;         // [NA]  weight block landed
-    uint64_t* wempty = wfull + NA;       // [NA]  the group's four warps hold the block in registers
+    uint64_t* wempty = wfull + NA;       // [NA]  the group's four warps have the block in tensor memory
     uint64_t* d_full = wempty + NA;      // [1]   every issuer's last MMA completed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_full + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -334,13 +334,6 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
             if (lane == 0 && ok) ok = mbar_wait(&wfull[aa], (i / NA) & 1, actx, kErrWaitFull);
             ok = __shfl_sync(0xffffffffu, ok, 0);
             __syncwarp();  // what lane 0 saw land, the others see (a shuffle does not order memory)
-            // The warp gives the stage back once its loads have RETURNED, in every lane: loads that are still on their way when it arrives
-            // can meet the next copy into the stage, which the async proxy does not order behind them (seen: a step of 128 rows in 700 had a
-            // few channels of one k-block from the block that took its stage).  `seen` has a bit of every load, the vote needs it of every
-            // lane, and its result is the lane that arrives.  (A proxy fence by every lane would do, for 5..14 % of a launch of up to 64 rows.)
-            const auto release = [&](uint32_t seen) {
-                if (lane == (int)(__ballot_sync(0xffffffffu, seen & 1u) & 31u)) mbar_arrive(&wempty[aa]);
-            };
             uint32_t v[4][16];
             if (ok) {
                 // this channel's 64 packed bytes: a chunk (32 k) of 16 channels is one 256-byte slab, so eight threads of a
@@ -355,7 +348,6 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                     const uint32_t sc = __byte_perm(sz.x, 0, row & 8 ? 0x3232 : 0x1010);  // (scale, scale)
                     const uint32_t zlo = z * 0x00010001u + 0x64006400u;  // 1024 + z as fp16: 0x6400 | z
                     const uint32_t zhi = z * 0x00100010u + 0xD400D400u;  // -(64 + z) as fp16: 0xD400 | (z << 4)
-                    release(pk[0].x ^ pk[1].x ^ pk[2].x ^ pk[3].x ^ sz.x);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         dequant_word(pk[c].x, zlo, zhi, sc, v[c] + 0);
@@ -368,7 +360,6 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                     uint4 pk[8];
 #pragma unroll
                     for (int c = 0; c < 8; ++c) pk[c] = *reinterpret_cast<const uint4*>(rrow + c * CHUNK);
-                    release(pk[0].x ^ pk[1].x ^ pk[2].x ^ pk[3].x ^ pk[4].x ^ pk[5].x ^ pk[6].x ^ pk[7].x);
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         uint32_t* o = v[c >> 1] + (c & 1) * 8;
@@ -390,6 +381,12 @@ w4g_umma_kernel(const __grid_constant__ W4Maps maps, const W4UmmaArgs p) {
                 for (int c = 0; c < 4; ++c) tmem_st16(a_addr + c * 16, v[c]);
                 tc_wait_st();
                 tc_fence_before();
+                // The stage goes back only now that every word of it, in every lane, has gone into an instruction above: loads that are still on
+                // their way when the warp arrives can meet the next copy into the stage, which the async proxy does not order behind them
+                // (given back right behind the loads, a step of 128 rows in 700 had a few channels of one k-block from the block that took
+                // its stage).  A proxy fence by every lane behind the loads costs 5..14 % of a launch of up to 64 rows, a vote over the
+                // loaded words up to 5 %, this nothing.
+                if (lane == 0) mbar_arrive(&wempty[aa]);
             }
             named_arrive(1 + aa, HANDOFF_THREADS);  // never skipped
         }
