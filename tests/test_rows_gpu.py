@@ -178,7 +178,7 @@ def test_prefill_lora_pairs(rows_, rank, dt, first):
 @pytest.mark.parametrize("N", [9472, 9504, 18944, 18976, 28448])
 @pytest.mark.parametrize("fmt", ["dense", "int8"])
 def test_either_side_of_the_wave_limits(N, fmt):
-    """CTAs of eight warps up to 296 tiles of 32 channels, of four up to 592, of eight up to 888, of four up to 1184."""
+    """CTAs of eight warps up to 296 tiles of 32 channels, of four up to 592 and from 889 on."""
     K, M = 512, 3
     g = torch.Generator(device="cuda").manual_seed(N)
     x = torch.randn(M, K, generator=g, device="cuda").half()
@@ -213,8 +213,9 @@ def test_short_problems_beside_one_of_many_waves(M):
 @pytest.mark.parametrize("N,fewer", [(9504, 9472), (37920, 37888), (47392, 47360)])
 @pytest.mark.parametrize("fmt", ["fp16", "bf16", "int4", "int8"])
 def test_ctas_of_four_warps_give_the_bits_of_eight(M, epi, N, fewer, fmt):
-    """Channels of a weight of N rows and of its first rows alone, either side of the limits at 296, 1184 and 1480 tiles: the same partial
-    sums in the same order, whatever the warps of a CTA.  11 quantised units of K and 22 dense ones, so that halves are odd."""
+    """Channels of a weight of N rows and of its first rows alone, either side of the limits at 296, 1184 and 1480 tiles of 32 channels (CTAs
+    of eight warps up to 296, of four up to 592, of eight up to 888, of four up to 1184, of eight up to 1480, then of four): the same
+    partial sums in the same order, whatever the warps of a CTA.  11 quantised units of K and 22 dense ones, so that halves are odd."""
     K = 1408
     g = torch.Generator(device="cuda").manual_seed(N + M)
     dt = torch.bfloat16 if fmt == "bf16" else torch.float16
