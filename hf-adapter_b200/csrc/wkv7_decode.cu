@@ -19,7 +19,8 @@
 // What it costs beside the state is instructions, of which a head has few warps to hide them: the vectors of the head are
 // made once, by one warp each (when all eight row groups made them for themselves that was two thirds of the kernel), and the
 // sums over the columns of a thread's eight rows run together (sum_rows).  us a launch, before -> now: 64 rows of 64 heads, fp32
-// state 27.7 -> 22.9 (5.9 TB/s), 256 rows 100 -> 82 (6.5); 64 rows of 40 heads, fp16 state 18.3 -> 13; one row of 12 heads 5.9 -> 4.0.
+// state 27.7 -> 22.9 (6.0 TB/s of the bytes above), 256 rows 100 -> 82 (6.7: above the rate of a copy, because up to an L2 of written state
+// drains under the kernels behind; at 64 rows DRAM sees 80 of the 138 MB within the kernel); 64 rows of 40 heads, fp16 state 18.3 -> 13; one row of 12 heads 5.9 -> 4.0.
 #include "common.cuh"
 
 namespace rwkv7 {
