@@ -178,7 +178,6 @@ __device__ __forceinline__ void scan_block(f2 (&S)[R][C / 2], Operands& op, int 
 
 // ---- grids that leave an SM with one or two CTAs: the serial chain of a token is all there is -----------------------------
 // Operands of one token in registers: the columns of a lane (4 cg .. + 3 and 32 + 4 cg .. + 3) and the values of its four rows.
-constexpr int kFewBlocks = 3;               // blocks of operands in shared memory: one ahead, one behind the one that runs
 constexpr int kFewRows = 4, kFewLanes = 8;  // rows a thread has eight columns of, lanes that share them
 struct TokenRegs {
     f2 kk[4], w[4], k[4], nb[4], r[4];
@@ -207,18 +206,20 @@ template <typename T> __device__ __forceinline__ float2 to_f2(const Pair<T>& q) 
 // A CTA owns one (sequence, head).  Warps 0..3 run the recurrence: 8 lanes share four rows, a lane has 8 columns of each.  Warps
 // 4, 5 read a block of tokens ahead (in registers while the block before it runs) and convert it, warps 6, 7 write out the block that
 // is done.  In the token loop everything that does not wait for S.kk of this token sits in its shadow: the operands of the next
-// token, the decay and the v k^T term, the output sums of the token before.  (Five blocks in flight, so that this also holds for the first
-// token of a block, cost two more barriers a call.  Time of three over five: up to 8 tokens 0.89..0.98, 9 to 64 0.87..0.98, 72 to 192 0.96..1.01,
-// from 256 on 1.01..1.03 with the output prepared and one CTA an SM, 0.98..1.00 else.)
+// token, the decay and the v k^T term, the output sums of the token before.  With three BLOCKS of operands in shared memory (one ahead,
+// one behind the one that runs) a block's first token has no such shadow; with five (two and two) it has, at two more barriers a call.
 // What bounds it: the instructions of four warps, one a scheduler (about 190 a token and warp at 2.2 cycles; two tokens a step, with
 // half the chain and as many instructions, took as long), and the shared-memory pipe, which hands a warp its 16-byte operand pieces
 // at four cycles each whoever shares them: two rows a thread on twice the warps are 30 % slower.  A partial sum is one chain of
-// four packed steps and one add (two chains and three adds: 5 % slower).  120 CTAs x 512 tokens 127.3 -> 116.0 us (227 ns a token).
-template <typename T, bool PREP, int CTAS>
+// four packed steps and one add (two chains and three adds: 5 % slower).  120 CTAs x 512 tokens 127.3 -> 116.0 us with three blocks (227 ns a
+// token), with five 2 us less.
+template <typename T, bool PREP, int CTAS, int BLOCKS>
 __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs p) {
-    constexpr int R = kFewRows, G = kFewLanes, NT = kSN / R * G;
+    constexpr int R = kFewRows, G = kFewLanes, NT = kSN / R * G, LAG = BLOCKS / 2;
+    constexpr bool ACROSS = BLOCKS == 5;  // a token's shadow reaches across the blocks
+    static_assert(BLOCKS == 3 || (BLOCKS == 5 && CTAS == 1), "LAG blocks on either side; five with one CTA an SM");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Operands* ops = reinterpret_cast<Operands*>(smem_raw);  // [kFewBlocks]
+    Operands* ops = reinterpret_cast<Operands*>(smem_raw);  // [BLOCKS]
     const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
     const int tid = threadIdx.x;
     const int T_ = p.T;
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
                 S[i][2 * j] = pack2(x[0], x[1]);
                 S[i][2 * j + 1] = pack2(x[2], x[3]);
             }
-        float y[R];
+        float y[R] = {};
         auto dot = [&](float (&out)[R], const f2 (&x)[4]) {
 #pragma unroll
             for (int i = 0; i < R; ++i) {
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
             y1 += y1q;
             y1q = xchg(y1, 1);
         };
-        auto token = [&](Operands& op, int t, bool prev, const TokenRegs& o) {
+        auto token = [&](bool prev, float* yprev, const TokenRegs& o) {  // `yprev`: where the output of the token before goes
             float sa[R], q[R];
             dot(sa, o.kk);
 #pragma unroll
@@ -311,38 +312,48 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
 #pragma unroll
                 for (int j = 0; j < 4; ++j) S[i][j] = fma2(s2, o.nb[j], S[i][j]);
             }
-            if (prev && ystore) op.y[t - 1][yrow] = y1 + y1q;
+            if (prev && ystore) yprev[yrow] = y1 + y1q;
             dot(y, o.r);
         };
-        for (int it = -1; it <= nblocks; ++it) {
+        auto last_output = [&](float* ylast) {
+            y_step4();
+            y_step2();
+            y_step1();
+            if (ystore) ylast[yrow] = y1 + y1q;
+        };
+        TokenRegs o[CTAS == 1 ? 2 : 1];
+        for (int it = -LAG; it < nblocks + LAG; ++it) {
             if (it >= 0 && it < nblocks) {
-                Operands& op = ops[it % kFewBlocks];
+                Operands& op = ops[it % BLOCKS];
+                const Operands& next = ops[(it + 1) % BLOCKS];  // ACROSS: there since the last barrier; past the end: nobody's
+                // before a block's first token comes the last one of the block before; before the first of all: overwritten by the next token
+                float* y0 = ACROSS && it > 0 ? ops[(it - 1) % BLOCKS].y[kTS - 1] : op.y[0];
                 const int nt = min(kTS, T_ - it * kTS);
+                if (ACROSS && it == 0) load_token(o[0], op, 0, row0, cg);
                 if (nt == kTS) {
-                    TokenRegs o[CTAS == 1 ? 2 : 1];
-                    load_token(o[0], op, 0, row0, cg);
+                    if (!ACROSS) load_token(o[0], op, 0, row0, cg);
 #pragma unroll
                     for (int t = 0; t < kTS; ++t) {
+                        float* yprev = t > 0 ? op.y[t - 1] : y0;
                         if constexpr (CTAS == 1) {  // the next token's operands a token ahead
-                            if (t + 1 < kTS) load_token(o[(t + 1) & 1], op, t + 1, row0, cg);
-                            token(op, t, t > 0, o[t & 1]);
+                            const Operands& from = t + 1 < kTS ? op : next;
+                            if (ACROSS || t + 1 < kTS) load_token(o[(t + 1) & 1], from, (t + 1) % kTS, row0, cg);
+                            token(ACROSS || t > 0, yprev, o[t & 1]);
                         } else {  // two CTAs an SM: no registers for that, and less need
-                            token(op, t, t > 0, o[0]);
+                            token(t > 0, yprev, o[0]);
                             if (t + 1 < kTS) load_token(o[0], op, t + 1, row0, cg);
                         }
                     }
                 } else {
 #pragma unroll 1
                     for (int t = 0; t < nt; ++t) {
-                        TokenRegs o;
-                        load_token(o, op, t, row0, cg);
-                        token(op, t, t > 0, o);
+                        load_token(o[0], op, t, row0, cg);
+                        token(ACROSS || t > 0, t > 0 ? op.y[t - 1] : y0, o[0]);
                     }
                 }
-                y_step4();
-                y_step2();
-                y_step1();
-                if (ystore) op.y[nt - 1][yrow] = y1 + y1q;
+                if (!ACROSS) last_output(op.y[nt - 1]);
+            } else if (ACROSS && it == nblocks) {
+                last_output(ops[(it - 1) % BLOCKS].y[T_ - 1 - (it - 1) * kTS]);
             }
             __syncthreads();
         }
@@ -393,10 +404,10 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
         fetch(0);
         announce(1);
         announce(2);
-        for (int it = -1; it <= nblocks; ++it) {
-            const int s = it + 1;
+        for (int it = -LAG; it < nblocks + LAG; ++it) {
+            const int s = it + LAG;
             if (s < nblocks) {
-                Operands& op = ops[s % kFewBlocks];
+                Operands& op = ops[s % BLOCKS];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int tt = tt0 + u;
@@ -448,10 +459,10 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
             load_param(p.gn_w, gw);
             load_param(p.gn_b, gb);
         }
-        for (int it = -1; it <= nblocks; ++it) {
-            const int s = it - 1;
+        for (int it = -LAG; it < nblocks + LAG; ++it) {
+            const int s = it - LAG;
             if (s >= 0) {
-                const Operands& op = ops[s % kFewBlocks];
+                const Operands& op = ops[s % BLOCKS];
                 const int t = s * kTS + tt;
                 const bool live = t < T_;  // the shuffles below run in all lanes
                 float y[8];
@@ -475,8 +486,8 @@ __global__ void __launch_bounds__(256, CTAS) wkv7_scan_few_kernel(const ScanArgs
                 if (live) store8(reinterpret_cast<T*>(p.y) + base + (size_t)t * tok_stride + c, y);
             }
             if constexpr (PREP) {  // the gate of the block that is written next
-                const int t = it * kTS + tt;
-                if (it >= 0 && t < T_) {
+                const int t = (s + 1) * kTS + tt;
+                if (s >= -1 && t < T_) {
                     const T* q = reinterpret_cast<const T*>(p.g) + base + (size_t)t * tok_stride + c;
                     reinterpret_cast<uint4*>(&g)[0] = reinterpret_cast<const uint4*>(q)[0];
                     if constexpr (sizeof(T) == 4) reinterpret_cast<uint4*>(&g)[1] = reinterpret_cast<const uint4*>(q)[1];
@@ -663,9 +674,17 @@ static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     // 296 194 -> 185; for 16 tokens 7.2 -> 7.0, 7.7 -> 7.5, 9.4 -> 9.2, 9.8 -> 9.6.  320: 405, where the form for fewer takes two waves (438).
     const int ctas = B * p.H;
     const bool few = ctas <= 2 * kSMs;
-    void (*kern)(const ScanArgs) = ctas <= kSMs ? wkv7_scan_few_kernel<T, PREP, 1> : few ? wkv7_scan_few_kernel<T, PREP, 2> : wkv7_scan_kernel<T, PREP, 2, 32>;
+    // Five blocks instead of three with the output prepared and one CTA an SM, from where their two barriers are paid for.  us, three -> five, 12 / 120 CTAs,
+    // fp16: 16 tokens 6.6 / 7.3 -> 7.3 / 7.9, 128 31.4 / 32.1 -> 31.7 / 32.7, 192 45.1 / 46.0 -> 45.0 / 46.2, 224 52.0 / 53.0 -> 51.7 / 52.9, 256 59.0 / 60.1 -> 58.4 / 59.8, 512 114.0 /
+    // 116.0 -> 111.7 / 114.7, 777 171.6 / 176.5 -> 167.4 / 173.3; fp32: 192 46.1 / 47.0 -> 45.8 / 46.7, 777 176.9 / 180.7 -> 172.8 / 176.4.  Without it, or at two CTAs an SM,
+    // five take 0..2 % longer at every length.
+    const bool across = PREP && ctas <= kSMs && p.T > 192;
+    void (*kern)(const ScanArgs) = !few           ? wkv7_scan_kernel<T, PREP, 2, 32>
+                                   : ctas > kSMs  ? wkv7_scan_few_kernel<T, PREP, 2, 3>
+                                   : across       ? wkv7_scan_few_kernel<T, PREP, 1, PREP ? 5 : 3>
+                                                  : wkv7_scan_few_kernel<T, PREP, 1, 3>;
     const int threads = few ? 256 : 64;
-    const size_t smem = few ? kFewBlocks * sizeof(Operands) : 2 * sizeof(RawStage<T>) + sizeof(Operands);
+    const size_t smem = few ? (across ? 5 : 3) * sizeof(Operands) : 2 * sizeof(RawStage<T>) + sizeof(Operands);
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     RWKV7_REQUIRE(e == cudaSuccess, RWKV7_ERR_CUDA, "wkv7_scan: %s", cudaGetErrorString(e));
     kern<<<ctas, threads, smem, st>>>(p);

@@ -200,6 +200,26 @@ def test_scan_in_pieces_is_the_scan(T, Hh):
         assert torch.equal(torch.cat([x.reshape(-1) for x in ys]), y.reshape(-1)) and torch.equal(state, s)
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T", [193, 200, 201, 208, 264])
+@pytest.mark.parametrize("Hh", [1, 148])
+def test_scan_of_many_tokens_is_the_scan_of_few(dt, T, Hh):
+    """Five blocks of operands in flight from 193 tokens on, three up to there: the bits of the same tokens in shorter calls, which the tests
+    above compare with the oracle."""
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    f = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    r, k, v, a, g = (f(1, T, Hh, N).to(dt) for _ in range(5))
+    seq = (r, torch.sigmoid(f(1, T, Hh, N)), k, v, torch.nn.functional.normalize(k.float(), dim=-1).to(dt), torch.sigmoid(a.float()).to(dt))
+    s0, par = 0.1 * f(1, Hh, N, N), [f(Hh, N).to(dt), f(Hh * N).to(dt), f(Hh * N).to(dt)]
+    y, s = hb.fused_recurrent_scan_output_prepare(*seq, s0, g, *par, eps=EPS)
+    assert bool(torch.isfinite(y).all()) and bool(torch.isfinite(s).all())
+    state, ys = s0, []
+    for t0, t1 in ((0, 1), (1, 100), (100, T)) if T > 193 else ((0, 1), (1, T)):
+        yt, state = hb.fused_recurrent_scan_output_prepare(*(x[:, t0:t1].contiguous() for x in seq), state, g[:, t0:t1].contiguous(), *par, eps=EPS)
+        ys.append(yt)
+    assert torch.equal(torch.cat([x.reshape(-1) for x in ys]), y.reshape(-1)) and torch.equal(state, s)
+
+
 @pytest.mark.parametrize("dt", ["fp16", "bf16", "fp32"])
 @pytest.mark.parametrize("Hh", [3, 149, 297])
 def test_scan_parameters_of_any_alignment(dt, Hh):
