@@ -25,7 +25,7 @@
 // each in turn, into a ring of six slots: decay products, scaled operands, the four 16 x 16 products, the inverse.  mma.sync
 // and not tcgen05: these products are 16 rows high, and through tensor memory every link of the chain costs a store, a
 // fence, an issue, a commit and a load, about 700 cycles (a tile of 64 tokens with five such links took 16.9 k cycles with one CTA
-// an SM).  8 sequences x 4096 tokens x 32 heads, in a row: 1154 -> 412 us (0.40 of the HBM floor of 165 us), raw decays 1209 -> 454.
+// an SM).  8 sequences x 4096 tokens x 32 heads, in a row: 1150 -> 434 us (0.38 of the HBM floor of 165 us; 420..436 by box), raw decays 1209 -> 454.
 //
 // Products that contain decay-scaled factors (range e^9.7 over 16 tokens with the model's decays) run on operands rounded to tf32;
 // products of bounded quantities (A_* against V and U, the keys decayed to the chunk's end) run in fp16; T is inverted in fp32.

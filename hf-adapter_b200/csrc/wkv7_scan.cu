@@ -670,7 +670,7 @@ template <typename T, bool PREP>
 static int dispatch_scan(const ScanArgs& p, int B, cudaStream_t st) {
     // Chosen by how many CTAs an SM gets.  Up to one, and up to two (with fewer registers a thread): the form with loads, output
     // and recurrence on warps of their own.  More: the CTAs of an SM hide each other's loads and the extra warps only take
-    // registers.  us for 512 tokens, fp16, output prepared, by CTAs, before -> now: 12 126 -> 115, 148 129 -> 117, 149 193 -> 185,
+    // registers.  us for 512 tokens, fp16, output prepared, by CTAs, before -> three blocks: 12 126 -> 115, 148 129 -> 117, 149 193 -> 185,
     // 296 194 -> 185; for 16 tokens 7.2 -> 7.0, 7.7 -> 7.5, 9.4 -> 9.2, 9.8 -> 9.6.  320: 405, where the form for fewer takes two waves (438).
     const int ctas = B * p.H;
     const bool few = ctas <= 2 * kSMs;
