@@ -52,7 +52,7 @@ def zero_lists(*lists) -> None:
     for ts in lists:
         if not ts:
             continue
-        if ts[0].element_size() == 4 and min(t.numel() for t in ts) > 10 << 20:
+        if ts[0].element_size() == 4 and ts[0].numel() > 10 << 20 and min(t.numel() for t in ts) > 10 << 20:
             for t in ts:
                 t.zero_()
         else:
